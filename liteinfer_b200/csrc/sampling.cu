@@ -1,4 +1,4 @@
-// Sampling: one block per row of logits.
+// Sampling: a row of logits is an arg-max, or a draw from what temperature, top-k and top-p leave of it.
 //
 // Order of operations as liteinfer/sampling/sampler.py:50-63: logits / temperature
 // -> top-k (exactly k survive; ties at the boundary do not widen it, :76-83)
@@ -11,7 +11,11 @@
 // arithmetic is 32-bit; the selections use exact integer sums (counts, and
 // probabilities in 2^-32 fixed point), so a given row always gives the same
 // token.  Among equal values the lower index comes first.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace li {
 
@@ -46,32 +50,31 @@ __device__ ArgMax block_argmax(ArgMax mine, ArgMax* scratch /* 32 */) {
   return r;
 }
 
-// Exclusive prefix of `v` over the block's threads in thread order, and the total.
-__device__ unsigned long long block_exclusive_scan(unsigned long long v, unsigned long long* scratch /* 33 */,
-                                                   unsigned long long* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  unsigned long long incl = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long n = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += n;
-  }
-  __syncthreads();
-  if (lane == 31) scratch[warp] = incl;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned long long run = 0;
-    for (int w = 0; w < nwarps; ++w) {
-      const unsigned long long t = scratch[w];
-      scratch[w] = run;
-      run += t;
-    }
-    scratch[32] = run;
-  }
-  __syncthreads();
-  *total = scratch[32];
-  return scratch[warp] + incl - v;
-}
+// ---- the sampling kernel --------------------------------------------------------------------------
+// A row belongs to a cluster of blocks (one per 2,048 columns, at most eight), each with its share of the columns in its
+// shared memory, so the logits are read once.  Every later pass runs over shared memory; what the blocks of a row must agree on (the maximum, a
+// histogram, a running weight) they read from one another's shared memory behind a cluster barrier, and each works
+// the answer out for itself.
+//
+// Top-k and top-p are the same selection: in descending order, keep the elements whose preceding weight (1 each, or
+// the probability) is within a limit.  The first histogram bins by the distance below the row's maximum, in steps of
+// 1/46 up to where probabilities in 2^-32 vanish: the interesting values spread over hundreds of bins, so the atomics
+// rarely meet.  Elements above the boundary bin are in, those below are out; the others are told apart by histograms over
+// ever narrower ranges of their keys (two more, as a rule).  What can still be chosen is listed after the first histogram,
+// in the order of the columns, so the passes behind it walk a few hundred columns instead of the vocabulary.
+//
+// Bound by the instructions of the passes over the whole row (load and maximum, histogram, listing) and by the
+// barriers between the others (a pass over 16,000 columns with a division and an exponential each takes a block some 10 us
+// when three share an SM).  Measured on B200, 48 rows of 128,256 bfloat16 logits, all kinds of parameters: 83 us, against
+// 2,075 for a block of 1,024 threads a row that read the row from L2 a dozen times, with 64-bit atomics into 256 bins of
+// the key's bits, most of them into the same bin, and one thread that walked the bins; one row with top-k and top-p: 50 us.
+constexpr int kSampleThreads = 512, kSampleWarps = kSampleThreads / 32;
+constexpr int kMostRanks = 8;      // blocks of a row's cluster
+constexpr int kRankColumns = 2048; // a row of no more columns is one block's: fewer barriers between blocks
+constexpr int kBins = 1024;
+constexpr int kListed = 512;       // columns that a warp can list; where one has more its block goes on walking its whole share
+constexpr int kSampleMostSmem = 200 << 10;
+constexpr float kBinsPerUnit = 46.f;   // (kBins - 1) / 46 = 22.24 > 32 ln 2: a value in the last bin has no probability left
 
 struct Keep {        // the surviving set: key > beta, or key == beta and index <= tie_cut
   uint32_t beta;
@@ -79,182 +82,447 @@ struct Keep {        // the surviving set: key > beta, or key == beta and index 
   __device__ __forceinline__ bool has(uint32_t key, int i) const { return key > beta || (key == beta && i <= tie_cut); }
 };
 
-struct SelectSmem {
-  unsigned long long mass[256];
-  unsigned int count[256];
-  unsigned long long scan[33];
-  unsigned long long above;
-  uint32_t prefix;
-  int found;
-  int tie_cut;
-  unsigned long long n_tie;
+struct SampleSmem {
+  // Two histograms in turn: kBins counts, or the sums of the weights' lower 16 bits and, behind them, of the bits above;
+  // for a share of 2^16 columns or more, where those could overflow, kBins 64-bit sums.
+  alignas(16) uint32_t bins[2][2 * kBins];
+  unsigned long long exchange[8];           // what other blocks of the cluster read, one slot per exchange
+  unsigned long long warp[kSampleWarps];
+  ArgMax warp_best[32];
+  ArgMax best;
+  unsigned long long before, mass;          // of the boundary bin
+  int chosen;
+  uint16_t list[kSampleWarps][kListed];
 };
 
-// Among the elements of `within`, in descending order of value (equal values by
-// ascending index), keeps each element whose preceding weight sum is <= limit.
-// `unit` weights count elements (top-k with limit k-1); otherwise the weight is
-// exp(x - row_max) in 2^-32 fixed point (top-p with limit p * total).
-template <typename T, bool unit>
-__device__ Keep select_prefix(const T* __restrict__ row, int n, float temp, float row_max, Keep within,
-                              unsigned long long limit, SelectSmem& sm) {
-  if (threadIdx.x == 0) {
-    sm.prefix = 0;
-    sm.above = 0;
+// One block's share of a row: columns [base, base + n) of it, whose element i lies at data[i] (in shared memory, or the row
+// itself where a share does not fit).  The walks over a share go warp by warp: each warp has a run of columns, and once
+// `listed` is set a list of those of its columns that still count, so a walk is in the order of the columns.
+template <typename S>
+struct Share {
+  const S* data;
+  const uint16_t* list;      // this warp's list
+  int n, base;
+  int from, to;              // this warp's columns, or the length of its list (from 0)
+  bool listed, divided;      // divided: data holds value / temperature
+  bool wide;                 // the row's shares have 2^16 columns or more
+  float temp, row_max;
+  float bin_max, bin_scale;  // the maximum as it is stored in `data`, and bins per unit of what is stored there
+  uint32_t max_key;
+  __device__ __forceinline__ int column(int j) const { return listed ? list[j] : j; }
+  __device__ __forceinline__ float value(int i) const { return divided ? to_float(data[i]) : to_float(data[i]) / temp; }
+  __device__ __forceinline__ unsigned long long weight(float x) const {
+    return (unsigned long long)(expf(x - row_max) * 4294967296.0f);
   }
-  for (int pass = 0; pass < 4; ++pass) {
-    const int shift = 24 - 8 * pass;
-    for (int b = threadIdx.x; b < 256; b += blockDim.x) {
-      sm.mass[b] = 0;
-      sm.count[b] = 0;
-    }
-    __syncthreads();
-    const uint32_t prefix = sm.prefix;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const float x = to_float(row[i]) / temp;
-      const uint32_t key = ordered_key(x);
-      if (!within.has(key, i)) continue;
-      if (pass > 0 && (key >> (shift + 8)) != prefix) continue;
-      const int bin = (key >> shift) & 255;
-      const unsigned long long w = unit ? 1ull : (unsigned long long)(expf(x - row_max) * 4294967296.0f);
-      atomicAdd(&sm.mass[bin], w);
-      atomicAdd(&sm.count[bin], 1u);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      // The boundary lies in the lowest non-empty bin whose preceding mass is still <= limit.
-      unsigned long long above = sm.above, chosen_above = sm.above;
-      int chosen = -1;
-      for (int b = 255; b >= 0; --b) {
-        if (above > limit) break;
-        if (sm.count[b]) {
-          chosen = b;
-          chosen_above = above;
-        }
-        above += sm.mass[b];
-      }
-      if (chosen < 0) {  // even the largest element's predecessors exceed the limit: keep the top bin
-        for (int b = 255; b >= 0; --b)
-          if (sm.count[b]) { chosen = b; break; }
-        if (chosen < 0) chosen = 0;
-      }
-      sm.prefix = (prefix << 8) | (uint32_t)chosen;
-      sm.above = chosen_above;
-      if (pass == 3) {
-        const unsigned long long w_each = sm.count[chosen] ? sm.mass[chosen] / sm.count[chosen] : 0;
-        unsigned long long keep = sm.count[chosen];
-        if (limit >= chosen_above && w_each > 0) {
-          const unsigned long long fit = (limit - chosen_above) / w_each + 1;
-          if (fit < keep) keep = fit;
-        } else if (limit < chosen_above) {
-          keep = 1;
-        }
-        if (keep < 1) keep = 1;
-        sm.n_tie = keep;
-        sm.tie_cut = n;
-        sm.found = (int)sm.count[chosen];
-      }
-    }
-    __syncthreads();
+  // Never rises with the value, and equal values divided by the temperature are in one bin.  A difference that is no
+  // number (infinities, NaN) goes by the key.
+  __device__ __forceinline__ int bin(int i) const {
+    const float stored = to_float(data[i]), d = bin_max - stored;
+    if (!(d >= 0.f)) return ordered_key(divided ? stored : stored / temp) >= max_key ? 0 : kBins - 1;
+    return (int)fminf(d * bin_scale, (float)(kBins - 1));
   }
-  Keep out{sm.prefix, n};
-  const unsigned long long n_tie = sm.n_tie;
-  if (n_tie < (unsigned long long)sm.found) {
-    // Not every element equal to beta survives: find the index of the n_tie-th one.
-    const int seg = (n + blockDim.x - 1) / blockDim.x;
-    const int lo = min(n, (int)threadIdx.x * seg), hi = min(n, lo + seg);
-    unsigned long long mine = 0;
-    for (int i = lo; i < hi; ++i) {
-      const uint32_t key = ordered_key(to_float(row[i]) / temp);
-      mine += (key == out.beta && within.has(key, i)) ? 1 : 0;
+};
+
+__device__ __forceinline__ unsigned long long warp_inclusive(unsigned long long v, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long n = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += n;
+  }
+  return v;
+}
+
+// Sums the blocks' histograms `buf` and finds the last non-empty bin whose preceding weight is within the limit
+// (`whole`: the limit is the share `top_p` of the whole sum, and is left in `limit`).  Every thread returns with the bin,
+// the weight before it and its own weight.
+template <bool unit>
+__device__ void find_boundary(SampleSmem& sm, int buf, bool wide, unsigned long long above, bool whole, float top_p,
+                              unsigned long long& limit, int& chosen, unsigned long long& before, unsigned long long& mass) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  if (t == 0) sm.chosen = -1;
+  cluster.sync();
+  static_assert(kBins == 2 * kSampleThreads, "two bins a thread");
+  unsigned long long a = 0, b = 0;
+  const int ranks = (int)cluster.num_blocks();
+#pragma unroll
+  for (int r = 0; r < kMostRanks; ++r) {
+    if (r >= ranks) break;
+    if (!unit && wide) {
+      const ulonglong2 both = *reinterpret_cast<const ulonglong2*>(cluster.map_shared_rank(&sm.bins[buf][4 * t], r));
+      a += both.x;
+      b += both.y;
+      continue;
     }
-    unsigned long long total;
-    const unsigned long long before = block_exclusive_scan(mine, sm.scan, &total);
-    if (before < n_tie && before + mine >= n_tie) {
-      unsigned long long c = before;
-      for (int i = lo; i < hi; ++i) {
-        const uint32_t key = ordered_key(to_float(row[i]) / temp);
-        if (key == out.beta && within.has(key, i) && ++c == n_tie) {
-          sm.tie_cut = i;
-          break;
-        }
-      }
+    const uint2 lo = *reinterpret_cast<const uint2*>(cluster.map_shared_rank(&sm.bins[buf][2 * t], r));
+    a += lo.x;
+    b += lo.y;
+    if (!unit) {
+      const uint2 hi = *reinterpret_cast<const uint2*>(cluster.map_shared_rank(&sm.bins[buf][kBins + 2 * t], r));
+      a += (unsigned long long)hi.x << 16;
+      b += (unsigned long long)hi.y << 16;
     }
-    __syncthreads();
-    out.tie_cut = sm.tie_cut;
+  }
+  const unsigned long long incl = warp_inclusive(a + b, lane);
+  if (lane == 31) sm.warp[w] = incl;
+  __syncthreads();
+  unsigned long long start = above, total = 0;
+#pragma unroll
+  for (int i = 0; i < kSampleWarps; ++i) {
+    const unsigned long long v = sm.warp[i];
+    if (i < w) start += v;
+    total += v;
+  }
+  if (whole) limit = (unsigned long long)((double)top_p * (double)total);
+  const unsigned long long first = start + incl - (a + b), second = first + a;
+  int mine = -1;
+  if (a && first <= limit) mine = 2 * t;
+  if (b && second <= limit) mine = 2 * t + 1;
+  if (mine >= 0) atomicMax(&sm.chosen, mine);
+  __syncthreads();
+  if (mine >= 0 && mine == sm.chosen) {
+    sm.before = (mine & 1) ? second : first;
+    sm.mass = (mine & 1) ? b : a;
   }
   __syncthreads();
+  chosen = sm.chosen;       // -1: nothing has any weight (a row whose maximum is infinite)
+  before = sm.before;
+  mass = sm.mass;
+}
+
+// Among the elements of `within`, in descending order of value (equal values by ascending index), keeps each element
+// whose preceding weight sum is within the limit.  `unit` weights count elements (top-k with limit k - 1); otherwise the
+// weight is exp(x - row_max) in 2^-32 fixed point (top-p with limit p * total).  `turn`: the histogram to use next;
+// `slot`: the next free exchange.  Lists what survives the first histogram.
+template <typename S, bool unit>
+__device__ Keep select_prefix(Share<S>& share, bool all_in, Keep within, unsigned long long limit, float top_p, int vocab,
+                              int& turn, int& slot, SampleSmem& sm) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const bool wide = share.wide;
+  int first_bin = -1;
+  uint32_t low_key = 0, high_key = 0xffffffffu;
+  unsigned long long above = 0, mass = 0;
+  for (int level = 0;; ++level) {
+    const uint32_t range = high_key - low_key;
+    const int shift = level == 0 ? 32 : max(0, 32 - __clz(range) - 10);
+    uint32_t* bins = sm.bins[turn];
+    for (int i = threadIdx.x; i < 2 * kBins; i += kSampleThreads) bins[i] = 0;
+    __syncthreads();
+#pragma unroll 4
+    for (int j = share.from + lane; j < share.to; j += 32) {
+      const int i = share.column(j);
+      int bin = share.bin(i);
+      float x = 0.f;
+      if (!all_in || level > 0) {
+        x = share.value(i);
+        const uint32_t key = ordered_key(x);
+        if (!all_in && !within.has(key, share.base + i)) continue;
+        if (level > 0) {
+          if (bin != first_bin || key < low_key || key > high_key) continue;
+          bin = (int)((high_key - key) >> shift);
+        }
+      }
+      if (unit) {
+        atomicAdd(bins + bin, 1u);
+      } else if (bin < kBins - 1 || level > 0) {   // what weighs nothing lies behind every limit
+        const unsigned long long weight = share.weight(all_in && level == 0 ? share.value(i) : x);
+        if (!wide) {
+          atomicAdd(bins + bin, (uint32_t)weight & 0xffffu);
+          atomicAdd(bins + kBins + bin, (uint32_t)(weight >> 16));
+        } else {
+          atomicAdd(reinterpret_cast<unsigned long long*>(bins) + bin, weight);
+        }
+      }
+    }
+    int chosen;
+    find_boundary<unit>(sm, turn, wide, above, !unit && level == 0, top_p, limit, chosen, above, mass);
+    turn ^= 1;
+    if (chosen < 0) return within;
+    if (level == 0) {
+      first_bin = chosen;
+      const float far = (float)(chosen + 1) * (1.0001f / kBinsPerUnit), near = (float)chosen * (0.9999f / kBinsPerUnit);
+      const float slack = 1e-5f * (fabsf(share.row_max) + 1.f);
+      if (chosen > 0) high_key = ordered_key(share.row_max - near + slack);
+      if (chosen < kBins - 1) low_key = ordered_key(share.row_max - far - slack);
+      if (!(fabsf(share.row_max) < 3.0e38f)) low_key = 0, high_key = 0xffffffffu;
+      if (!share.listed && !wide) {   // list what the boundary bin and those above it hold
+        int listed = 0;
+        bool fits = true;
+        for (int j = share.from; j < share.to; j += 32) {
+          const int i = j + lane;
+          bool in = i < share.to && share.bin(i) <= first_bin;
+          if (in && !all_in) in = within.has(ordered_key(share.value(i)), share.base + i);
+          const unsigned votes = __ballot_sync(0xffffffffu, in);
+          const int many = __popc(votes);
+          if (listed + many > kListed) {
+            fits = false;
+            break;
+          }
+          if (in) sm.list[w][listed + __popc(votes & ((1u << lane) - 1))] = (uint16_t)i;
+          listed += many;
+        }
+        if (__syncthreads_and(fits)) {
+          share.listed = true;
+          share.list = sm.list[w];
+          share.from = 0;
+          share.to = listed;
+        }
+      }
+      continue;
+    }
+    high_key -= (uint32_t)chosen << shift;
+    if (shift == 0) break;
+    const uint32_t width = (1u << shift) - 1;
+    if (high_key - low_key > width) low_key = high_key - width;
+  }
+  cg::cluster_group cluster = cg::this_cluster();
+  const uint32_t beta = high_key;
+  const float beta_value = __uint_as_float((beta & 0x80000000u) ? beta & 0x7fffffffu : ~beta);
+  const unsigned long long each = unit ? 1ull : share.weight(beta_value);
+  const unsigned long long count = each ? mass / each : 1ull;
+  const unsigned long long ties = each ? min(count, (limit - above) / each + 1) : 1ull;   // above <= limit
+  Keep out{beta, vocab};
+  if (ties < count) {
+    // Not every element equal to beta survives: the index of the `ties`-th one, over the blocks in order.
+    const int from = share.from, to = share.to;
+    int mine = 0;
+    for (int j = from; j < to; j += 32) {
+      bool in = false;
+      if (j + lane < to) {
+        const int i = share.column(j + lane);
+        const uint32_t key = ordered_key(share.value(i));
+        in = key == beta && within.has(key, share.base + i);
+      }
+      mine += __popc(__ballot_sync(0xffffffffu, in));
+    }
+    if (lane == 0) sm.warp[w] = mine;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned long long all = 0;
+      for (int k = 0; k < kSampleWarps; ++k) all += sm.warp[k];
+      sm.exchange[slot] = all;
+      sm.exchange[slot + 1] = (unsigned long long)vocab;
+    }
+    cluster.sync();
+    unsigned long long before = 0;
+    for (unsigned r = 0; r < cluster.block_rank(); ++r) before += *cluster.map_shared_rank(&sm.exchange[slot], r);
+    for (int k = 0; k < w; ++k) before += sm.warp[k];
+    if (before < ties && ties <= before + mine) {
+      int left = (int)(ties - before);
+      for (int j = from; j < to; j += 32) {
+        int i = 0;
+        bool in = false;
+        if (j + lane < to) {
+          i = share.column(j + lane);
+          const uint32_t key = ordered_key(share.value(i));
+          in = key == beta && within.has(key, share.base + i);
+        }
+        const unsigned votes = __ballot_sync(0xffffffffu, in);
+        const int here = __popc(votes);
+        if (left <= here) {
+          if (in && __popc(votes & ((2u << lane) - 1)) == left) sm.exchange[slot + 1] = (unsigned long long)(share.base + i);
+          break;
+        }
+        left -= here;
+      }
+    }
+    cluster.sync();
+    int cut = vocab;
+    for (unsigned r = 0; r < cluster.num_blocks(); ++r) cut = min(cut, (int)*cluster.map_shared_rank(&sm.exchange[slot + 1], r));
+    out.tie_cut = cut;
+  }
+  slot += 2;
   return out;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
-sample_kernel(const T* __restrict__ logits, int vocab, const float* __restrict__ temperature,
+// Grid: rows x (cluster size) blocks, a row's in one cluster.  `staged`: a block's share lies in its shared memory behind
+// `sm`, as S: the logits as they are, or as float, divided by the temperature.
+template <typename T, typename S>
+__global__ void __launch_bounds__(kSampleThreads, sizeof(S) == 2 ? 3 : 2)
+sample_kernel(const T* __restrict__ logits, int vocab, int share_size, bool staged, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ uniform,
               int* __restrict__ out) {
-  __shared__ ArgMax am_scratch[32];
-  __shared__ SelectSmem sm;
-  __shared__ int result;
-  const int r = blockIdx.x;
+  extern __shared__ __align__(16) char sample_smem[];
+  SampleSmem& sm = *reinterpret_cast<SampleSmem*>(sample_smem);
+  S* stage = reinterpret_cast<S*>(sample_smem + (sizeof(SampleSmem) + 15) / 16 * 16);
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks(), r = blockIdx.x / ranks;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const T* row = logits + (size_t)r * vocab;
+  const float temp = temperature ? temperature[r] : 0.f;
+  const bool greedy = !(temp > 0.f) || (top_k && top_k[r] == 1);
+  Share<S> share;
+  share.base = min(vocab, rank * share_size);
+  share.n = min(vocab, share.base + share_size) - share.base;
+  const T* mine_row = row + share.base;
+  share.divided = staged && sizeof(S) == 4 && !greedy;
 
   ArgMax mine{-INFINITY, 0x7fffffff};
-  for (int i = threadIdx.x; i < vocab; i += blockDim.x) mine = better(mine, ArgMax{to_float(row[i]), i});
-  const ArgMax top = block_argmax(mine, am_scratch);
-  const float temp = temperature ? temperature[r] : 0.f;
-  const int k = top_k ? top_k[r] : -1;
-  if (!(temp > 0.f) || k == 1) {
-    if (threadIdx.x == 0) out[r] = top.i;
+  constexpr int N = Vec16<T>::N;
+  int done = 0;
+  if (aligned16(mine_row)) {
+    done = share.n / N * N;
+#pragma unroll 2
+    for (int i = threadIdx.x * N; i < done; i += kSampleThreads * N) {
+      const Vec16<T> v = load16(mine_row + i);
+      float f[N];
+      unpack16(v, f);
+      float most = f[0];
+#pragma unroll
+      for (int k = 1; k < N; ++k) most = fmaxf(most, f[k]);
+      if (most > mine.v || mine.i == 0x7fffffff) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) mine = better(mine, ArgMax{f[k], share.base + i + k});
+      }
+      if (staged && !greedy) {
+        if constexpr (sizeof(S) == sizeof(T) && sizeof(T) == 2) {
+          store16(reinterpret_cast<T*>(stage) + i, v);
+        } else {
+#pragma unroll
+          for (int k = 0; k < N; k += 4) {
+            Vec16<float> d;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) d.set(e, f[k + e] / temp);
+            store16(reinterpret_cast<float*>(stage) + i + k, d);
+          }
+        }
+      }
+    }
+  }
+  for (int i = done + threadIdx.x; i < share.n; i += kSampleThreads) {
+    const T v = mine_row[i];
+    if (staged && !greedy) stage[i] = from_float<S>(sizeof(S) == 4 ? to_float(v) / temp : to_float(v));
+    mine = better(mine, ArgMax{to_float(v), share.base + i});
+  }
+  const ArgMax block_top = block_argmax(mine, sm.warp_best);
+  if (threadIdx.x == 0) sm.best = block_top;
+  cluster.sync();
+  ArgMax top = *cluster.map_shared_rank(&sm.best, 0);
+  for (int k = 1; k < ranks; ++k) top = better(top, *cluster.map_shared_rank(&sm.best, k));
+
+  if (greedy) {
+    if (rank == 0 && threadIdx.x == 0) out[r] = top.i;
+    cluster.sync();          // the others may still read this block's maximum
     return;
   }
-  const float row_max = top.v / temp;
+  const int part_size = (share.n + kSampleWarps - 1) / kSampleWarps;
+  share.from = min(share.n, w * part_size);
+  share.to = min(share.n, share.from + part_size);
+  share.listed = false;
+  share.wide = share_size >= 1 << 16;
+  share.list = nullptr;
+  share.temp = temp;
+  share.row_max = top.v / temp;
+  share.bin_max = share.divided ? share.row_max : top.v;
+  share.bin_scale = share.divided ? kBinsPerUnit : kBinsPerUnit / temp;
+  share.max_key = ordered_key(share.row_max);
 
-  Keep keep{0u, vocab};  // every finite value has a key > 0
-  if (k > 0 && k < vocab)
-    keep = select_prefix<T, true>(row, vocab, temp, row_max, keep, (unsigned long long)(k - 1), sm);
-
-  const float p = top_p ? top_p[r] : 1.f;
-  const int seg = (vocab + blockDim.x - 1) / blockDim.x;
-  const int lo = min(vocab, (int)threadIdx.x * seg), hi = min(vocab, lo + seg);
-  if (p > 0.f && p < 1.f) {
-    unsigned long long part = 0;
-    for (int i = lo; i < hi; ++i) {
-      const float x = to_float(row[i]) / temp;
-      if (keep.has(ordered_key(x), i)) part += (unsigned long long)(expf(x - row_max) * 4294967296.0f);
-    }
-    unsigned long long total;
-    block_exclusive_scan(part, sm.scan, &total);
-    const unsigned long long limit = (unsigned long long)((double)p * (double)total);
-    keep = select_prefix<T, false>(row, vocab, temp, row_max, keep, limit, sm);
+  if constexpr (sizeof(S) == sizeof(T)) {
+    if (!staged) reinterpret_cast<const T*&>(share.data) = mine_row;
+    else share.data = stage;
+  } else {
+    share.data = stage;
   }
+  const int k = top_k ? top_k[r] : -1;
+  const float p = top_p ? top_p[r] : 1.f;
+  const bool by_count = k > 0 && k < vocab;
+  int turn = 0, slot = 0;
+  Keep keep{0u, vocab};  // every finite value has a key > 0
+  if (by_count) keep = select_prefix<S, true>(share, true, keep, (unsigned long long)(k - 1), 0.f, vocab, turn, slot, sm);
+  if (p > 0.f && p < 1.f) keep = select_prefix<S, false>(share, !by_count, keep, 0, p, vocab, turn, slot, sm);
 
   // Draw: the first index (ascending) at which the running weight passes uniform * total.
+  const int from = share.from, to = share.to;
   unsigned long long part = 0;
-  for (int i = lo; i < hi; ++i) {
-    const float x = to_float(row[i]) / temp;
-    if (keep.has(ordered_key(x), i)) part += (unsigned long long)(expf(x - row_max) * 4294967296.0f);
+  for (int j = from + lane; j < to; j += 32) {
+    const int i = share.column(j);
+    const float x = share.value(i);
+    if (keep.has(ordered_key(x), share.base + i)) part += share.weight(x);
   }
-  unsigned long long total;
-  const unsigned long long before = block_exclusive_scan(part, sm.scan, &total);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+  __syncthreads();
+  if (lane == 0) sm.warp[w] = part;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long all = 0;
+    for (int i = 0; i < kSampleWarps; ++i) all += sm.warp[i];
+    sm.exchange[slot] = all;
+  }
+  cluster.sync();
+  unsigned long long before = 0, total = 0;
+  for (int i = 0; i < ranks; ++i) {
+    const unsigned long long v = *cluster.map_shared_rank(&sm.exchange[slot], i);
+    if (i < rank) before += v;
+    total += v;
+  }
+  for (int i = 0; i < w; ++i) before += sm.warp[i];
   double u = uniform ? (double)uniform[r] : 0.5;
   u = u < 0.0 ? 0.0 : (u >= 1.0 ? 0.99999994 : u);
   unsigned long long target = (unsigned long long)(u * (double)total);
   if (target >= total) target = total ? total - 1 : 0;
-  if (threadIdx.x == 0) result = top.i;  // total == 0 cannot happen (the maximum weighs 2^32); stay safe
-  __syncthreads();
-  if (part > 0 && before <= target && target < before + part) {
-    unsigned long long c = before;
-    for (int i = lo; i < hi; ++i) {
-      const float x = to_float(row[i]) / temp;
-      if (!keep.has(ordered_key(x), i)) continue;
-      c += (unsigned long long)(expf(x - row_max) * 4294967296.0f);
-      if (c > target) {
-        result = i;
+  if (total == 0) {                      // the maximum weighs 2^32: only a row without finite values comes here
+    if (rank == 0 && threadIdx.x == 0) out[r] = top.i;
+  } else if (part > 0 && before <= target && target < before + part) {
+    for (int j = from; j < to; j += 32) {
+      int i = 0;
+      unsigned long long weight = 0;
+      if (j + lane < to) {
+        i = share.column(j + lane);
+        const float x = share.value(i);
+        if (keep.has(ordered_key(x), share.base + i)) weight = share.weight(x);
+      }
+      const unsigned long long upto = before + warp_inclusive(weight, lane);
+      const unsigned passed = __ballot_sync(0xffffffffu, upto > target);
+      if (passed) {
+        if (lane == __ffs(passed) - 1) out[r] = share.base + i;
         break;
       }
+      before = __shfl_sync(0xffffffffu, upto, 31);
     }
   }
-  __syncthreads();
-  if (threadIdx.x == 0) out[r] = result;
+  cluster.sync();            // nobody leaves while another block reads
+}
+
+template <typename T, typename S>
+int launch_sample(const T* logits, int rows, int vocab, int ranks, int share, bool staged, const float* temperature,
+                  const int* top_k, const float* top_p, const float* uniform, int* out, cudaStream_t stream) {
+  const size_t smem = (sizeof(SampleSmem) + 15) / 16 * 16 + (staged ? (size_t)share * sizeof(S) : 0);
+  const cudaError_t status =
+      cudaFuncSetAttribute(sample_kernel<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleMostSmem);
+  if (status != cudaSuccess) return (int)status;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(rows * ranks);
+  config.blockDim = dim3(kSampleThreads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute[1];
+  attribute[0].id = cudaLaunchAttributeClusterDimension;
+  attribute[0].val.clusterDim.x = ranks;
+  attribute[0].val.clusterDim.y = 1;
+  attribute[0].val.clusterDim.z = 1;
+  config.attrs = attribute;
+  config.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&config, sample_kernel<T, S>, logits, vocab, share, staged, temperature, top_k, top_p,
+                                 uniform, out);
+}
+
+// Shares in shared memory where they fit.  bfloat16 is staged as divided floats while all of the launch's blocks are resident
+// at once that way, two an SM (64 KB of floats beside 33 KB): the passes then divide nothing.  A wider launch stages the
+// logits as they are, three blocks an SM, and divides again in the passes that need the quotient, so that 48 rows of
+// 128,256 (384 blocks) still are one wave; two waves would cost each row's chain of barriers twice.
+template <typename T>
+int sample_rows(const T* logits, int rows, int vocab, const float* temperature, const int* top_k, const float* top_p,
+                const float* uniform, int* out, cudaStream_t stream) {
+  int ranks = 1;
+  while (ranks < kMostRanks && ranks * kRankColumns < vocab) ranks *= 2;
+  const int share = ((vocab + ranks - 1) / ranks + 7) / 8 * 8;
+  if ((long long)rows * ranks > 0x7fffffffll) return LI_ERR_UNSUPPORTED;
+  const size_t room = kSampleMostSmem - (sizeof(SampleSmem) + 15) / 16 * 16;
+  const bool raw = (size_t)share * sizeof(T) <= room;
+  if (sizeof(T) == 4 || ((size_t)share * 4 <= room / 2 && rows * ranks <= 2 * 148))
+    return launch_sample<T, float>(logits, rows, vocab, ranks, share, raw, temperature, top_k, top_p, uniform, out, stream);
+  return launch_sample<T, T>(logits, rows, vocab, ranks, share, raw, temperature, top_k, top_p, uniform, out, stream);
 }
 
 template <typename T>
@@ -347,11 +615,6 @@ LI_EXPORT int li_argmax(int dtype, const void* logits, int rows, int vocab, int*
 LI_EXPORT int li_sample(int dtype, const void* logits, int rows, int vocab, const float* temperature,
                         const int* top_k, const float* top_p, const float* uniform, int* out, cudaStream_t stream) {
   if (rows == 0) return 0;
-  if (dtype == kFloat32)
-    sample_kernel<float><<<rows, kThreads, 0, stream>>>((const float*)logits, vocab, temperature, top_k, top_p,
-                                                        uniform, out);
-  else
-    sample_kernel<bf16><<<rows, kThreads, 0, stream>>>((const bf16*)logits, vocab, temperature, top_k, top_p, uniform,
-                                                       out);
-  LI_LAUNCH_CHECK();
+  if (dtype == kFloat32) return sample_rows((const float*)logits, rows, vocab, temperature, top_k, top_p, uniform, out, stream);
+  return sample_rows((const bf16*)logits, rows, vocab, temperature, top_k, top_p, uniform, out, stream);
 }

@@ -17,6 +17,7 @@ from __future__ import annotations
 
 import random
 
+import numpy as np
 import torch
 
 from liteinfer_b200 import ops
@@ -62,13 +63,14 @@ class Sampler:
         if all(p.greedy for p in params):
             return ops.argmax(logits, out)
         keys = keys or [None] * rows
+        # One list to one pinned buffer to one copy: temperature, top_p, uniform (float32) and top_k (the bits of int32).
+        greedy = [p.greedy for p in params]
+        values = [0.0 if g else p.temperature for g, p in zip(greedy, params)]
+        values += [p.top_p for p in params]
+        values += [0.0 if g else self._stream(p, k).random() for g, p, k in zip(greedy, params, keys)]
         host = torch.empty((4, rows), dtype=torch.float32, pin_memory=logits.is_cuda)
-        for i, p in enumerate(params):
-            host[0, i] = 0.0 if p.greedy else p.temperature
-            host[1, i] = p.top_p
-            host[2, i] = 0.0 if p.greedy else self._stream(p, keys[i]).random()
-            host[3, i] = 0.0
-        top_k = torch.tensor([p.top_k if p.top_k > 0 else 0 for p in params], dtype=torch.int32,
-                             pin_memory=logits.is_cuda)
+        staged = host.numpy()
+        staged[:3].reshape(-1)[:] = values
+        staged[3].view(np.int32)[:] = [p.top_k if p.top_k > 0 else 0 for p in params]
         dev = host.to(logits.device, non_blocking=True)
-        return ops.sample(logits, dev[0], top_k.to(logits.device, non_blocking=True), dev[1], dev[2], out)
+        return ops.sample(logits, dev[0], dev[3].view(torch.int32), dev[1], dev[2], out)

@@ -259,6 +259,59 @@ def test_sample_matches_the_rule(dtype, vocab):
                 assert int(got[r]) in (lo, hi), f"row {r}: got {int(got[r])}, rule gives {want}"
 
 
+def _sample_rule(x, k, p, u):
+    """The sampling rule for one row x (already divided by its temperature), sums in 64 bits, by a stable sort: the column
+    drawn, and the columns that could be."""
+    n = x.numel()
+    order = torch.sort(x, descending=True, stable=True).indices
+    w = torch.exp(x - x.max()).double()
+    keep = order[:k] if 0 < k < n else order
+    if 0.0 < p < 1.0:
+        before = torch.cumsum(w[keep], 0) - w[keep]
+        keep = keep[before <= p * float(w[keep].sum())]
+    keep = keep.sort().values
+    run = torch.cumsum(w[keep], 0)
+    return int(keep[min(int((run <= u * float(run[-1])).sum()), len(keep) - 1)]), keep
+
+
+# One block a row, two, four, eight; rows that start anywhere; rows too long for the blocks' shared memory, and for 16-bit
+# column numbers; as many rows as make bfloat16 be staged undivided.
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("vocab,rows", [(1, 12), (31, 12), (2048, 12), (2049, 12), (8190, 84), (50257, 12), (128256, 48),
+                                        (400003, 12), (600001, 12)])
+def test_sample_splits_a_row_over_blocks(dtype, vocab, rows):
+    from liteinfer_b200 import ops
+
+    g = torch.Generator().manual_seed(vocab)
+    logits = (torch.randn(rows, vocab, generator=g) * 2.5).to(dtype)
+    logits[1] = 3.25                                        # all equal: only the index decides
+    logits[2] = logits[2].float().round().to(dtype)         # a few values, thousands of ties
+    logits[3, :-1] = -torch.inf                             # one column left
+    logits[4, : vocab // 2] = torch.finfo(dtype).min        # masked with the type's lowest value
+    logits[5] = logits[5] * 40                              # most probabilities vanish
+    temps = torch.tensor([0.7, 1.0, 1.3, 1.0, 0.0, 1.0] * (rows // 6))
+    top_k = torch.tensor([50, 1000, 0, 7, 3, 200, 0, 0, 4097, 0, vocab // 2, 1] * (rows // 12), dtype=torch.int32)
+    top_p = torch.tensor([1.0, 0.5, 0.9, 0.95, 0.9, 0.99, 0.9, 0.3, 0.999, 1.0, 0.05, 0.5] * (rows // 12))
+    for trial in range(2):
+        u = torch.rand(rows, generator=g)
+        got = ops.sample(logits.cuda(), temps.cuda(), top_k.cuda(), top_p.cuda(), u.cuda(),
+                         torch.empty(rows, dtype=torch.int32, device="cuda")).cpu()
+        for r in range(rows):
+            if float(temps[r]) == 0.0 or int(top_k[r]) == 1:
+                assert int(got[r]) == int(torch.argmax(logits[r].float())), r
+                continue
+            x = logits[r].float() / temps[r]
+            # The kernel's weights are 32-bit exponentials (2^-22 of their own) cut to multiples of 2^-32 of the largest, so
+            # its running sums are within `off` of the whole, and the draw and the cut of top-p move by no more.
+            off = 2.0 ** -22 + vocab * 2.0 ** -32
+            k, p, v = int(top_k[r]), float(top_p[r]), float(u[r])
+            rules = [_sample_rule(x, k, p + dp, min(max(v + du, 0.0), 0.9999999)) for du in (-2 * off, 0.0, 2 * off)
+                     for dp in ((-2 * off, 0.0, 2 * off) if p < 1 else (0.0,))]
+            low, high = min(at for at, _ in rules), max(at for at, _ in rules)
+            assert low <= int(got[r]) <= high, f"row {r}: got {int(got[r])}, the rule gives {low} to {high}"
+            assert any(bool((keep == int(got[r])).any()) for _, keep in rules), f"row {r}: {int(got[r])} is not in what is kept"
+
+
 def test_sample_distribution():
     """Many draws of one row follow softmax(logits / T) restricted to the top-k."""
     from liteinfer_b200 import ops
