@@ -3,70 +3,302 @@
 // full-precision 32-bit mode), also instantiated for bfloat16 storage as the path
 // for shapes the tensor-core kernels refuse.
 //
-// Every output element adds its K products in the same order (k ascending,
-// one accumulator), whatever M and N are, so a row's result does not depend on
-// which other rows are in the batch.
+// Every output element adds its K products in the same order whatever M and N are, so a row's result does not depend on
+// which other rows are in the batch: chunks of 128 k, each one chain of fused multiply-adds in ascending order from zero,
+// and the chunks' sums in ascending order.  Both kernels keep that order; the chunks are what lets the narrow one give
+// each to a warp of its own (and the sum of short chains is nearer to the exact one than a single long chain was).
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace li {
 
-constexpr int BM = 64, BN = 64, BK = 16;
+constexpr int kChunk = 128;
 
-template <typename T>
-__global__ void __launch_bounds__(256)
-gemm_simt_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias, T* __restrict__ out,
-                 int M, int N, int K, int ldx, int ldo, long x_batch, long w_batch, long out_batch) {
-  __shared__ float xs[BK][BM + 1];
-  __shared__ float ws[BK][BN + 1];
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  x += blockIdx.z * x_batch;        // one product per blockIdx.z (a plain product is a batch of one)
-  w += blockIdx.z * w_batch;
-  out += blockIdx.z * out_batch;
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // 16 x 16 threads, 4 x 4 outputs each
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+struct SimtProduct {
+  const void *x, *w, *bias;
+  void* out;
+  int M, N, K, ldx, ldo;
+  long x_batch, w_batch, out_batch;     // one product per blockIdx.z (a plain product is a batch of one)
+};
 
-  const int lr = threadIdx.x / 4;         // 0..63: tile row this thread loads
-  const int lk = (threadIdx.x % 4) * 4;   // 0,4,8,12: first of its four k
-  for (int k0 = 0; k0 < K; k0 += BK) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int k = k0 + lk + i;
-      const int m = m0 + lr, n = n0 + lr;
-      xs[lk + i][lr] = (m < M && k < K) ? to_float(x[(size_t)m * ldx + k]) : 0.f;
-      ws[lk + i][lr] = (n < N && k < K) ? to_float(w[(size_t)n * K + k]) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = xs[k][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = ws[k][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
+// ---- many rows of x: 128 x 64 tiles, 8 x 4 outputs a thread ------------------------------------------------------
+// Bound by the FFMA pipe: four k are 128 multiply-adds a thread on 12 vector loads from shared memory, rows along k in
+// both operands (threads have rows 16 apart, which with rows of 36 words keeps the reads off one another's banks).  Three
+// steps of 32 k are on their way (cp.async) while a fourth is multiplied, so a grid of few tiles does not wait for every
+// step's loads.
+// Measured on B200, 1,250 rows: 3072 x 2048 488 us (32 TFLOP/s), 16384 x 2048 2,170 us (39), 1280 x 768 98 us; the tiles of
+// 64 x 64 before them (4 x 4 a thread, scalar loads between two barriers of every 16 k) took 833, 4,073 and 141 us.
+constexpr int BN = 64, BK = 32, kTileThreads = 256, kTileStages = 4;
+constexpr int kTileRow = BK + 4;
+template <int BM> constexpr size_t kTileSmem = (size_t)kTileStages * (BM + BN) * kTileRow * sizeof(float);
+
+__device__ __forceinline__ void copy16_async(float* dst, const float* src, int bytes = 16) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(bytes));
+}
+
+// Four neighbours along k, `left` of which exist: to shared memory, asynchronously where `vec` (the row lies on 16 bytes).
+__device__ __forceinline__ void stage_four(float* dst, const float* src, int left, bool vec) {
+  if (vec) {
+    copy16_async(dst, left > 0 ? src : src - (4 - left) / 4 * 4, left > 0 ? 16 : 0);   // K is a multiple of four
+    return;
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
-    if (m >= M) continue;
+  for (int i = 0; i < 4; ++i) dst[i] = i < left ? src[i] : 0.f;
+}
+__device__ __forceinline__ void stage_four(float* dst, const bf16* src, int left, bool vec) {
+  if (vec && left > 0) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(src);
+    *reinterpret_cast<float4*>(dst) = make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u),
+                                                  __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u));
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) dst[i] = i < left ? widen(src[i]) : 0.f;
+}
+
+template <typename T, int BM>
+__global__ void __launch_bounds__(kTileThreads, 2) gemm_simt_tile_kernel(SimtProduct p, bool vec) {
+  extern __shared__ __align__(16) float tile_smem[];      // [stage][x rows, then w rows][kTileRow]
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN, K = p.K;
+  const T* x = static_cast<const T*>(p.x) + blockIdx.z * p.x_batch;
+  const T* w = static_cast<const T*>(p.w) + blockIdx.z * p.w_batch;
+  T* out = static_cast<T*>(p.out) + blockIdx.z * p.out_batch;
+  const T* bias = static_cast<const T*>(p.bias);
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+  const int steps = (K + BK - 1) / BK;
+  const int lr = threadIdx.x / 8, lk = threadIdx.x % 8 * 4;   // the first row and the k of this thread's loads
+
+  // Rows beyond a matrix repeat its last one: their outputs are not stored.
+  const auto fill = [&](int step) {
+    if (step < steps) {
+      float* dst = tile_smem + (step % kTileStages) * ((BM + BN) * kTileRow) + lr * kTileRow + lk;
+      const int k = step * BK + lk, left = K - k;
+#pragma unroll
+      for (int r = 0; r < BM; r += kTileThreads / 8)
+        stage_four(dst + r * kTileRow, x + (size_t)min(m0 + lr + r, p.M - 1) * p.ldx + k, left, vec);
+#pragma unroll
+      for (int r = 0; r < BN; r += kTileThreads / 8)
+        stage_four(dst + (BM + r) * kTileRow, w + (size_t)min(n0 + lr + r, p.N - 1) * K + k, left, vec);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  float acc[BM / 16][4], total[BM / 16][4];
+#pragma unroll
+  for (int i = 0; i < BM / 16; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = total[i][j] = 0.f;
+
+  for (int step = 0; step < kTileStages - 1; ++step) fill(step);
+  for (int step = 0; step < steps; ++step) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kTileStages - 2) : "memory");
+    __syncthreads();                   // this step's operands are in place, and everyone is done with the step before
+    fill(step + kTileStages - 1);      // into the stage of the step before
+    const float* stage = tile_smem + (step % kTileStages) * ((BM + BN) * kTileRow);
+    const float* xr = stage + ty * kTileRow;
+    const float* wr = stage + (BM + tx) * kTileRow;
+#pragma unroll 2
+    for (int k = 0; k < BK; k += 4) {
+      float4 b[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(wr + j * 16 * kTileRow + k);
+#pragma unroll
+      for (int i = 0; i < BM / 16; ++i) {
+        const float4 a = *reinterpret_cast<const float4*>(xr + i * 16 * kTileRow + k);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          acc[i][j] = fmaf(a.w, b[j].w, fmaf(a.z, b[j].z, fmaf(a.y, b[j].y, fmaf(a.x, b[j].x, acc[i][j]))));
+      }
+    }
+    if ((step + 1) * BK % kChunk == 0 || step + 1 == steps) {
+#pragma unroll
+      for (int i = 0; i < BM / 16; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          total[i][j] += acc[i][j];
+          acc[i][j] = 0.f;
+        }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < BM / 16; ++i) {
+    const int m = m0 + ty + 16 * i;
+    if (m >= p.M) continue;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n >= N) continue;
-      float v = acc[i][j];
+      const int n = n0 + tx + 16 * j;
+      if (n >= p.N) continue;
+      float v = total[i][j];
       if (bias) v += to_float(bias[n]);
-      out[(size_t)m * ldo + n] = from_float<T>(v);
+      out[(size_t)m * p.ldo + n] = from_float<T>(v);
     }
   }
+}
+
+// ---- few rows of x (float32): 64 rows of w and one chunk of k a warp -----------------------------------------------
+// Bound by reading w (a decode step) and by how much of it is on its way at once: a block copies all of its w, 64 rows of
+// one to four chunks, to shared memory before it multiplies anything (and before it waits for the kernel ahead, which only x
+// depends on), and the chunks of a row lie in different warps and blocks.  A lane has two rows of w; x is read as
+// broadcasts, R rows a warp, G warps on the same chunk of w.  The chunks' sums meet in the shared memory of the blocks of a
+// cluster (along k) and are added in order.
+// Measured on B200, 12 rows: 1280 x 768 6.6 us, 768 x 2048 6.9, 16000 x 768 26 (1.9 TB/s); one row of 16384 x 2048 41 us
+// (3.3 TB/s).  On the 64 x 64 tiles, a dozen blocks that waited for every 16 k, these took 55, 140, 99 and 252 us.
+constexpr int kRowStride = kChunk + 4;     // 16-byte reads of 32 rows at the same k: off the banks' period
+constexpr int kRowsN = 64;
+constexpr int kMostCluster = 8, kMostChunks = 4, kMostRounds = 4;
+
+// Grid: (64 rows of w) x cluster, R * G rows of x, batch.  Block: `chunks` chunks of G warps, `rounds` times.
+template <int R, int G>
+__global__ void __launch_bounds__(32 * kMostChunks * G) gemm_simt_rows_kernel(SimtProduct p, int chunks, int rounds,
+                                                                                          int all_chunks) {
+  extern __shared__ __align__(16) float rows_smem[];
+  grid_launch_dependents();
+  cg::cluster_group cluster = cg::this_cluster();
+  const int ranks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, mine = warp / G, part = warp % G;
+  const int n0 = blockIdx.x / ranks * kRowsN, m0 = blockIdx.y * (R * G);
+  const float* x = static_cast<const float*>(p.x) + blockIdx.z * p.x_batch;
+  const float* w = static_cast<const float*>(p.w) + blockIdx.z * p.w_batch;
+  float* out = static_cast<float*>(p.out) + blockIdx.z * p.out_batch;
+  const float* bias = static_cast<const float*>(p.bias);
+  float* wt = rows_smem + mine * (kRowsN * kRowStride);
+  float* xt = rows_smem + chunks * (kRowsN * kRowStride) + mine * (R * G * kChunk);
+  float* sums = rows_smem + chunks * (kRowsN * kRowStride + R * G * kChunk);      // [rounds * chunks][R * G][kRowsN]
+  const int rows_w = min(kRowsN, p.N - n0), rows_x = min(R * G, p.M - m0);
+  static_assert(kChunk == 128, "a row of a chunk is one 16-byte piece a lane");
+  for (int round = 0; round < rounds; ++round) {
+    const int place = round * chunks + mine, k0 = (rank * rounds * chunks + place) * kChunk;
+    const int fours = max(0, min(kChunk, p.K - k0)) / 4;
+    if (round > 0) __syncthreads();        // the warps of a chunk are done with its operands
+    // The G warps of a chunk copy its operands between them, a row at a time.
+    if (lane < fours) {
+#pragma unroll 8
+      for (int r = part; r < rows_w; r += G)
+        copy16_async(wt + r * kRowStride + 4 * lane, w + (size_t)(n0 + r) * p.K + k0 + 4 * lane);
+    }
+    if (round == 0) grid_dependency_wait();
+    if (lane < fours) {
+#pragma unroll 4
+      for (int r = part; r < rows_x; r += G)
+        copy16_async(xt + r * kChunk + 4 * lane, x + (size_t)(m0 + r) * p.ldx + k0 + 4 * lane);
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    float acc[R][2];
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r][0] = acc[r][1] = 0.f;
+    const float4* w0 = reinterpret_cast<const float4*>(wt + lane * kRowStride);
+    const float4* w1 = reinterpret_cast<const float4*>(wt + (lane + 32) * kRowStride);
+    const float4* xr = reinterpret_cast<const float4*>(xt + part * R * kChunk);
+#pragma unroll 2
+    for (int f = 0; f < fours; ++f) {
+      const float4 b0 = w0[f], b1 = w1[f];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {        // rows beyond x or w hold what the memory held: their sums are not stored
+        const float4 a = xr[r * (kChunk / 4) + f];
+        acc[r][0] = fmaf(a.w, b0.w, fmaf(a.z, b0.z, fmaf(a.y, b0.y, fmaf(a.x, b0.x, acc[r][0]))));
+        acc[r][1] = fmaf(a.w, b1.w, fmaf(a.z, b1.z, fmaf(a.y, b1.y, fmaf(a.x, b1.x, acc[r][1]))));
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      float* mine_sums = sums + (place * (R * G) + part * R + r) * kRowsN + lane;
+      mine_sums[0] = acc[r][0];
+      mine_sums[32] = acc[r][1];
+    }
+  }
+  cluster.sync();
+  for (int i = rank * blockDim.x + threadIdx.x; i < rows_x * kRowsN; i += ranks * blockDim.x) {
+    const int m = i / kRowsN, n = i % kRowsN;
+    if (n >= rows_w) continue;
+    const int share = rounds * chunks;
+    float total = 0.f;
+#pragma unroll 4
+    for (int c = 0; c < all_chunks; ++c)
+      total += *cluster.map_shared_rank(sums + (c % share * (R * G) + m) * kRowsN + n, c / share);
+    if (bias) total += bias[n0 + n];
+    out[(size_t)(m0 + m) * p.ldo + n0 + n] = total;
+  }
+  cluster.sync();        // nobody leaves while another block reads its sums
+}
+
+template <int R, int G>
+int launch_rows(const SimtProduct& p, int batch, cudaStream_t stream) {
+  const int all_chunks = (p.K + kChunk - 1) / kChunk;
+  const int each = (all_chunks + kMostCluster - 1) / kMostCluster;          // chunks of a block
+  const int rounds = (each + kMostChunks - 1) / kMostChunks, chunks = (each + rounds - 1) / rounds;
+  const int ranks = (all_chunks + rounds * chunks - 1) / (rounds * chunks);
+  const size_t smem = (size_t)chunks * (kRowsN * kRowStride + R * G * (kChunk + rounds * kRowsN)) * sizeof(float);
+  const long blocks = (long)((p.N + kRowsN - 1) / kRowsN) * ranks, groups = (p.M + R * G - 1) / (R * G);
+  if (blocks > 0x7fffffffL || groups > 65535 || batch > 65535) return LI_ERR_UNSUPPORTED;
+  const cudaError_t status =
+      cudaFuncSetAttribute(gemm_simt_rows_kernel<R, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  if (status != cudaSuccess) return (int)status;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3((unsigned)blocks, (unsigned)groups, batch);
+  config.blockDim = dim3(32 * G * chunks);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attributes[2];
+  attributes[0].id = cudaLaunchAttributeClusterDimension;
+  attributes[0].val.clusterDim.x = ranks;
+  attributes[0].val.clusterDim.y = 1;
+  attributes[0].val.clusterDim.z = 1;
+  attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[1].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attributes;
+  config.numAttrs = pdl_enabled(p.M) ? 2 : 1;
+  return (int)cudaLaunchKernelEx(&config, gemm_simt_rows_kernel<R, G>, p, chunks, rounds, all_chunks);
+}
+
+template <typename T, int BM>
+int launch_tiles(const SimtProduct& p, bool vec, int batch, cudaStream_t stream) {
+  const dim3 grid((p.N + BN - 1) / BN, (p.M + BM - 1) / BM, batch);
+  if (grid.y > 65535 || batch > 65535) return LI_ERR_UNSUPPORTED;
+  const cudaError_t status =
+      cudaFuncSetAttribute(gemm_simt_tile_kernel<T, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem<BM>);
+  if (status != cudaSuccess) return (int)status;
+  gemm_simt_tile_kernel<T, BM><<<grid, kTileThreads, kTileSmem<BM>, stream>>>(p, vec);
+  LI_LAUNCH_CHECK();
+}
+
+// Which kernel, by what each was measured to take (B200, microseconds, float32).  The narrow one: 4 and 2.2 for every million
+// weights of a group of 16 rows (16384 x 2048: 73 for 12 rows; 1280 x 768: 10.2 for 64).  Tiles of 32 rows: 26 per 768 k
+// while each SM has one or none, then 0.15 a tile (1280 x 768: 26 for 192 rows, 120 for 1,250); tiles of 128 rows: 54 per 768 k
+// up to one an SM, 98 up to two, then 0.37 a tile (1280 x 768: 54 for 256 rows, 98 for 1,250; 4096 x 768: 239 for 1,250).
+constexpr int kMostRows = 256;
+inline float rows_cost(const SimtProduct& p, int batch) {
+  return 4.f + 2.2e-6f * (float)p.N * p.K * ((p.M + 15) / 16) * batch;
+}
+inline float tiles_cost(const SimtProduct& p, int batch, int rows) {
+  const float tiles = (float)((p.N + BN - 1) / BN) * ((p.M + rows - 1) / rows) * batch, depth = p.K / 768.f;
+  if (rows == 32) return depth * fmaxf(26.f, 0.15f * tiles);
+  return depth * (tiles <= 148.f ? 54.f : fmaxf(98.f, 0.37f * tiles));
+}
+
+int launch_product(int dtype, const SimtProduct& p, int batch, cudaStream_t stream) {
+  const size_t element = dtype == kFloat32 ? 4 : 2, four = 4 * element;
+  // Loads of four k at once: every row of x and w starts on their size.
+  const bool vec = p.K % 4 == 0 && p.ldx % 4 == 0 && p.x_batch % 4 == 0 && p.w_batch % 4 == 0 &&
+                   reinterpret_cast<uintptr_t>(p.x) % four == 0 && reinterpret_cast<uintptr_t>(p.w) % four == 0;
+  const float small = tiles_cost(p, batch, 32), large = tiles_cost(p, batch, 128);
+  if (dtype == kFloat32 && vec && p.K > 0 && p.M <= kMostRows && p.K <= kMostRounds * kMostChunks * kMostCluster * kChunk &&
+      batch <= 65535 && rows_cost(p, batch) < fminf(small, large)) {
+    if (p.M == 1) return launch_rows<1, 1>(p, batch, stream);
+    if (p.M <= 4) return launch_rows<4, 1>(p, batch, stream);
+    if (p.M <= 8) return launch_rows<4, 2>(p, batch, stream);
+    if (p.M <= 12) return launch_rows<6, 2>(p, batch, stream);
+    return launch_rows<8, 2>(p, batch, stream);
+  }
+  const bool narrow = small < large && (p.M + 31) / 32 <= 65535;
+  if (dtype == kFloat32)
+    return narrow ? launch_tiles<float, 32>(p, vec, batch, stream) : launch_tiles<float, 128>(p, vec, batch, stream);
+  return narrow ? launch_tiles<bf16, 32>(p, vec, batch, stream) : launch_tiles<bf16, 128>(p, vec, batch, stream);
 }
 
 }  // namespace li
@@ -76,15 +308,7 @@ using namespace li;
 LI_EXPORT int li_gemm_simt(int dtype, const void* x, const void* w, const void* bias, void* out, int M, int N, int K,
                            cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;
-  const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  if (grid.y > 65535) return LI_ERR_UNSUPPORTED;
-  if (dtype == kFloat32)
-    gemm_simt_kernel<float><<<grid, 256, 0, stream>>>((const float*)x, (const float*)w, (const float*)bias,
-                                                      (float*)out, M, N, K, K, N, 0, 0, 0);
-  else
-    gemm_simt_kernel<bf16><<<grid, 256, 0, stream>>>((const bf16*)x, (const bf16*)w, (const bf16*)bias, (bf16*)out, M,
-                                                     N, K, K, N, 0, 0, 0);
-  LI_LAUNCH_CHECK();
+  return launch_product(dtype, SimtProduct{x, w, bias, out, M, N, K, K, N, 0, 0, 0}, 1, stream);
 }
 
 // A batch of products: out[b][m][n] = sum_k x[b][m][k] * w[b][n][k], b < batch.  x[b] starts at x + b * x_batch
@@ -93,13 +317,6 @@ LI_EXPORT int li_gemm_simt(int dtype, const void* x, const void* w, const void* 
 LI_EXPORT int li_gemm_simt_batched(int dtype, const void* x, const void* w, void* out, int M, int N, int K, int batch,
                                    int ldx, int ldo, long x_batch, long w_batch, long out_batch, cudaStream_t stream) {
   if (M == 0 || N == 0 || batch == 0) return 0;
-  const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
-  if (grid.y > 65535 || batch > 65535) return LI_ERR_UNSUPPORTED;
-  if (dtype == kFloat32)
-    gemm_simt_kernel<float><<<grid, 256, 0, stream>>>((const float*)x, (const float*)w, nullptr, (float*)out, M, N, K,
-                                                      ldx, ldo, x_batch, w_batch, out_batch);
-  else
-    gemm_simt_kernel<bf16><<<grid, 256, 0, stream>>>((const bf16*)x, (const bf16*)w, nullptr, (bf16*)out, M, N, K, ldx,
-                                                     ldo, x_batch, w_batch, out_batch);
-  LI_LAUNCH_CHECK();
+  return launch_product(dtype, SimtProduct{x, w, nullptr, out, M, N, K, ldx, ldo, x_batch, w_batch, out_batch}, batch,
+                        stream);
 }

@@ -96,6 +96,29 @@ def test_gemm_simt_rows_do_not_depend_on_the_batch():
     assert torch.equal(full[33:34], one)
 
 
+# One chunk of k and part of one; several in a cluster of odd size; several a block; the narrow kernel's last size and the
+# first beyond it; a k that is not a multiple of four.
+@pytest.mark.parametrize("N,K", [(33, 40), (100, 128), (1000, 772), (64, 1024), (96, 2052), (65, 4096), (40, 4100), (65, 8196), (70, 301)])
+def test_gemm_simt_widths_agree_bit_for_bit(N, K):
+    from liteinfer_b200 import ops
+
+    x, w = _randn(200, K, dtype=torch.float32), _randn(N, K, dtype=torch.float32, seed=1)
+    b = _randn(N, dtype=torch.float32, seed=2)
+    full = ops.gemm_simt(x, w, torch.empty(200, N, device="cuda"), b)
+    # Chains of at most 128 products and then at most 34 sums, each rounding by 2^-24 of what it has.
+    bound = (x.double().abs() @ w.double().abs().t() + b.double().abs()) * (128 + 34) * 2.0 ** -24
+    assert bool(((full.double() - (x.double() @ w.double().t() + b.double())).abs() <= bound).all())
+    for M in (1, 2, 4, 5, 8, 9, 16, 17, 63, 64, 65, 129):
+        part = ops.gemm_simt(x[3:3 + M].contiguous(), w, torch.empty(M, N, device="cuda"), b)
+        assert torch.equal(part, full[3:3 + M]), M
+    if K % 4 == 0:
+        wide = torch.randn(2, 17, K + 8, device="cuda")
+        batched = ops.batched_linear(wide[:, :, 4:K + 4], torch.stack([w, 2 * w]), torch.empty(2, 17, N, device="cuda"))
+        for i in range(2):
+            one = ops.gemm_simt(wide[i, :, 4:K + 4].contiguous(), (i + 1) * w, torch.empty(17, N, device="cuda"))
+            assert torch.equal(batched[i], one)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 3072, 2048), (8, 2048, 8192), (64, 1000, 96), (300, 512, 64), (2048, 256, 2048)])
 def test_linear_bfloat16(M, N, K):
     from liteinfer_b200 import ops
@@ -171,6 +194,50 @@ def test_rope_write_then_attention(dtype, heads, kv_heads, head_dim, page_size, 
         assert torch.equal(torch.isnan(got.float()), ~written)      # nothing written outside the requests' slots
         torch.testing.assert_close(got.float()[written], want.float()[written], **_tol(dtype))
     assert torch.isfinite(outs[0][3].float()).all()
+
+
+# Rows walked by one warp and by teams, one unit of keys and several rounds of them, every width of values.
+@pytest.mark.parametrize("heads,kv_heads,head_dim,page_size", [(3, 1, 64, 16), (9, 1, 20, 16), (2, 2, 128, 16), (6, 3, 256, 8),
+                                                               (2, 1, 320, 16), (34, 2, 33, 5)])
+@pytest.mark.parametrize("window,keep_first,softcap,sink", [(0, 0, 0.0, False), (70, 0, 0.0, True), (100, 68, 20.0, False),
+                                                            (-96, 0, 0.0, False)])
+def test_generic_attention_cuts_agree_bit_for_bit(heads, kv_heads, head_dim, page_size, window, keep_first, softcap, sink):
+    from liteinfer_b200 import ops
+
+    ctx = 1100
+    case = _paged_case(torch.float32, heads, kv_heads, head_dim, page_size, [ctx], [ctx])
+    sinks = _randn(heads, dtype=torch.float32, seed=9) if sink else None
+    ops.rope_kv_write(case["qkv"], case["positions"], case["seq_of"], case["table"], case["k_pool"], case["v_pool"], None,
+                      heads, kv_heads, head_dim, 0)
+
+    def attend(start, count):
+        qkv = case["qkv"][start:start + count]
+        out = torch.empty(count, heads * head_dim, device="cuda")
+        ops.paged_attention_generic(qkv, qkv.stride(0), out, case["k_pool"], case["v_pool"], case["table"],
+                                    torch.tensor([0, count], dtype=torch.int32, device="cuda"),
+                                    torch.tensor([start + count], dtype=torch.int32, device="cuda"), 1, count, heads, kv_heads,
+                                    head_dim, head_dim ** -0.5, window, keep_first, softcap, sinks)
+        return out
+
+    whole = attend(0, ctx)
+    q, k, v = (t.double().unflatten(1, (-1, head_dim)) for t in case["qkv"].split(
+        [heads * head_dim, kv_heads * head_dim, kv_heads * head_dim], dim=1))
+    k, v = (t.repeat_interleave(heads // kv_heads, dim=1) for t in (k, v))
+    score = torch.einsum("thd,shd->hts", q, k) * head_dim ** -0.5
+    score = softcap * torch.tanh(score / softcap) if softcap else score
+    i, j = torch.arange(ctx, device="cuda")[:, None], torch.arange(ctx, device="cuda")[None]
+    seen = j <= i
+    if window > 0:
+        seen &= (i - j < window) | (j < keep_first)
+    elif window < 0:
+        seen &= i // -window == j // -window
+    score = score.masked_fill(~seen, -torch.inf)
+    if sink:
+        score = torch.cat([score, sinks.double()[:, None, None].expand(-1, ctx, 1)], -1)
+    want = torch.einsum("hts,shd->thd", torch.softmax(score, -1)[..., :ctx], v).flatten(1)
+    torch.testing.assert_close(whole.double(), want, rtol=1e-5, atol=1e-5)
+    for start, count in ((0, 1), (62, 2), (64, 1), (127, 3), (130, 1), (500, 9), (1099, 1)):
+        assert torch.equal(attend(start, count), whole[start:start + count]), (start, count)
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
