@@ -24,6 +24,7 @@ from dataclasses import dataclass, field
 
 import torch
 
+from liteinfer_b200 import ops
 from liteinfer_b200.cache.pages import CacheExhaustedError, OutOfPagesError, PageAllocator, SlotAllocator
 from liteinfer_b200.parts.context import KVCacheView, KVNeed, LayerCache, StateNeed
 from liteinfer_b200.parts.spec import ScheduleEntry
@@ -98,6 +99,7 @@ class CacheManager:
         self._slot_of: dict[str, int] = {}
         self._length: dict[str, int] = {}
         self._state_tensors: list[torch.Tensor] = []
+        self._slot_states: ops.SlotStates | None = None     # of those, on a GPU, once a slot has been zeroed
         self._table_version: dict[str, int] = {}            # changes whenever a block table of the request does
         self._versions = 0
 
@@ -233,18 +235,19 @@ class CacheManager:
                     f"cache group {g} needs {wanted[g]} more pages, {group.allocator.num_free} of "
                     f"{group.allocator.num_pages} are free")
         newcomers = [r for r in request_ids if r not in self._length]
+        taken = []
         if len(newcomers) > self.slots.num_free:
             raise CacheExhaustedError(
                 f"{len(newcomers)} new requests but {self.slots.num_free} of {self.max_requests} state slots are free")
         for request_id in newcomers:
             slot = self.slots.allocate_one()
+            taken.append(slot)
             self._slot_of[request_id] = slot
             self._length[request_id] = 0
-            for state in self._state_tensors:
-                state[slot].zero_()
             for group in self.groups:
                 group.tables[request_id] = []
             self._touch(request_id)
+        self._zero_states(taken)
         for request_id, total in zip(request_ids, new_totals, strict=True):
             old = self._length[request_id]
             for group in self.groups:
@@ -258,6 +261,19 @@ class CacheManager:
                     while len(table) <= block:
                         table.append(-1)
                     table[block] = page
+
+    def _zero_states(self, slots: list[int]) -> None:
+        """The states of slots that have just been handed out: zero, on a GPU by one launch for all of them."""
+        if not slots or not self._state_tensors:
+            return
+        if self.device.type == "cuda":
+            if self._slot_states is None:
+                self._slot_states = ops.SlotStates(self._state_tensors)
+            self._slot_states.zero(slots)
+            return
+        for slot in slots:
+            for state in self._state_tensors:
+                state[slot].zero_()
 
     def commit(self, request_id: str, new_total: int) -> None:
         """The step that wrote up to `new_total` succeeded: count it, and give back what no later token reads."""

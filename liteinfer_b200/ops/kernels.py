@@ -12,7 +12,7 @@ from __future__ import annotations
 
 import ctypes
 import os
-from ctypes import c_float, c_int, c_long, c_size_t, c_void_p
+from ctypes import c_float, c_int, c_long, c_longlong, c_size_t, c_void_p
 
 from dataclasses import dataclass
 
@@ -40,6 +40,7 @@ _functions: dict[str, ctypes._CFuncPtr] = {}
 _SIGNATURES = {
     "li_embedding": ("elementwise", [c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]),
     "li_scatter_tokens": ("elementwise", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
+    "li_zero_slots": ("elementwise", [c_void_p, c_void_p, c_int, c_longlong, c_void_p, c_int, c_void_p]),
     "li_stage_batch": ("elementwise", [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
     "li_rmsnorm": ("elementwise", [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float,
                                    c_int, c_void_p]),
@@ -306,6 +307,12 @@ class beside:
     Tensors: what the second stream reads must stay alive until the join, and what it makes is used behind the join."""
 
     _streams: dict[torch.device, "torch.cuda.Stream"] = {}
+    _open: set[torch.device] = set()        # devices whose second stream holds work that nobody has joined yet
+
+    @staticmethod
+    def is_free(device: torch.device) -> bool:
+        """Whether the second stream holds nothing that is still to be joined: work that is put there would wait for it."""
+        return _lane == 0 and normalise_device(device) not in beside._open
 
     def __init__(self, device: torch.device) -> None:
         self.device = normalise_device(device)
@@ -322,6 +329,7 @@ class beside:
         for context in self.entered:
             context.__enter__()
         _lane = 1
+        beside._open.add(self.device)
         return self
 
     def __exit__(self, *exc):
@@ -333,6 +341,7 @@ class beside:
 
     def join(self) -> None:
         torch.cuda.current_stream(self.device).wait_stream(self.stream)
+        beside._open.discard(self.device)
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:
@@ -371,7 +380,7 @@ def scatter_tokens(tokens: torch.Tensor, dst: torch.Tensor, src: torch.Tensor, s
 
 
 # Batches up to this many 32-bit words are brought to the device by a kernel that reads the pinned buffer in place
-# (one block; a copy engine's latency is longer than that for a few kilobytes, shorter for many).
+# (a copy engine's latency is longer than that for a few kilobytes, shorter for many).
 STAGE_KERNEL_MAX_WORDS = 16384
 
 
@@ -392,6 +401,25 @@ def stage_batch(device: torch.Tensor, host: torch.Tensor, tokens: torch.Tensor, 
         return False
     _check(code, "stage_batch")
     return True
+
+
+class SlotStates:
+    """The state tensors [slots, ...] of a cache on a GPU, for `zero`: their addresses and sizes, on the device.  Keeps the
+    tensors, so the addresses stay theirs."""
+
+    def __init__(self, tensors: list[torch.Tensor]) -> None:
+        _on_gpu(*tensors)
+        self.tensors = tensors
+        sizes = [t[0].numel() * t.element_size() for t in tensors]
+        self.most = max(sizes, default=0)
+        self.table = torch.tensor([[t.data_ptr() for t in tensors], sizes], dtype=torch.int64, device=tensors[0].device)
+
+    def zero(self, slots: list[int]) -> None:
+        """tensor[slot] = 0 in every tensor, for every slot: one launch (per 64 slots)."""
+        array = (c_int * len(slots))(*slots)
+        assert all(0 <= slot < t.shape[0] for t in self.tensors[:1] for slot in slots)
+        _check(_fn("li_zero_slots")(self.table[0].data_ptr(), self.table[1].data_ptr(), len(self.tensors), self.most, array,
+                                    len(slots), _stream()), "zero_slots")
 
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor,
@@ -1079,6 +1107,13 @@ def tensor_core_sizes(key_dim: int, value_dim: int, heads: int, kv_heads: int) -
 MASKED_ON_MMA = os.environ.get("LITEINFER_TCGEN05_ATTN", "1") == "0"
 
 
+# In a step that has both, the attention of the single tokens runs on a second stream beside that of the portions, which
+# up to this many queries leaves blocks of the device idle.  Measured on B200 (1B sizes, 23 decoding at
+# up to 700 keys): a step with 509 tokens of a prompt behind 1,024 takes 2,160 us beside one another and 2,242 in turn, with 1,400
+# 3,419 and 3,529; 48 decoding beside 40 tokens at the 3B sizes 2,953 and 3,483, beside 1,900 tokens 11,784 and 12,122.
+MIXED_BESIDE_TOKENS = 2048
+
+
 def paged_attention(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_pool: torch.Tensor,
                     v_pool: torch.Tensor, block_table: torch.Tensor, query_start_loc: torch.Tensor,
                     context_lens: torch.Tensor, num_seqs: int, max_q_len: int, heads: int, kv_heads: int,
@@ -1128,6 +1163,18 @@ def paged_attention(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_poo
     if plan is None:
         return paged_attention_mma(*common, None, num_seqs, max_q_len, heads, kv_heads, head_dim, scale, window,
                                    **options)
+    def single_tokens():
+        bound = min(plan.max_decode_context_len, reach) if reach else plan.max_decode_context_len
+        streaming = not (keep_first > 0 and window > 0) and stream_attention_supports(q.dtype, heads, kv_heads, head_dim, page_size)
+        splits = decode_splits or decode_splits_for(plan.num_decode, kv_heads * parts, bound, head_dim, streaming)
+        paged_attention_mma(*common, plan.decode_seqs, plan.num_decode, 1, heads, kv_heads, head_dim, scale,
+                            window, splits, newest, streaming, **options)
+
+    lane = None
+    if plan.num_prefill and plan.num_decode and plan.max_prefill_query_len <= MIXED_BESIDE_TOKENS and beside.is_free(out.device):
+        lane = beside(out.device)
+        with lane:
+            single_tokens()
     if plan.num_prefill:
         if tcgen05_attention_supports(q.dtype, heads, kv_heads, head_dim, page_size) and not MASKED_ON_MMA:
             paged_attention_tcgen05(*common, plan.prefill_seqs, plan.num_prefill, plan.max_prefill_query_len, heads,
@@ -1135,12 +1182,10 @@ def paged_attention(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_poo
         else:
             paged_attention_mma(*common, plan.prefill_seqs, plan.num_prefill, plan.max_prefill_query_len, heads,
                                 kv_heads, head_dim, scale, window, **options)
-    if plan.num_decode:
-        bound = min(plan.max_decode_context_len, reach) if reach else plan.max_decode_context_len
-        streaming = not (keep_first > 0 and window > 0) and stream_attention_supports(q.dtype, heads, kv_heads, head_dim, page_size)
-        splits = decode_splits or decode_splits_for(plan.num_decode, kv_heads * parts, bound, head_dim, streaming)
-        paged_attention_mma(*common, plan.decode_seqs, plan.num_decode, 1, heads, kv_heads, head_dim, scale,
-                            window, splits, newest, streaming, **options)
+    if lane is not None:
+        lane.join()
+    elif plan.num_decode:
+        single_tokens()
     return out
 
 

@@ -573,17 +573,18 @@ def test_stage_batch_equals_copy_and_scatter(words, n_late):
     from liteinfer_b200 import ops
 
     g = torch.Generator().manual_seed(words)
-    tok_len, n = 16, max(n_late, 1)                      # layout: tokens [0, 16), dst [20, 20 + n), src after it
+    tok_len, n = (16 if words < 16384 else 3000), max(n_late, 1)    # layout: tokens first, dst 4 words behind, src after it
     host = torch.randint(0, 1000, (words,), generator=g, dtype=torch.int32)
     dst = torch.full((n,), -1, dtype=torch.int32)
     places = torch.randperm(tok_len, generator=g).to(torch.int32)
     for i in range(0, min(n_late, 2 * tok_len), 2):      # every second entry names a place, each place once
         dst[i] = places[i // 2]
-    host[20:20 + n] = dst
-    host[20 + n:20 + 2 * n] = torch.randint(0, 32, (n,), generator=g, dtype=torch.int32)
+    at = tok_len + 4
+    host[at:at + n] = dst
+    host[at + n:at + 2 * n] = torch.randint(0, 32, (n,), generator=g, dtype=torch.int32)
     host = host.pin_memory()
     source = torch.randint(0, 50000, (32,), generator=g, dtype=torch.int32).cuda()
-    views = lambda t: (t[:tok_len], t[20:20 + n], t[20 + n:20 + 2 * n])
+    views = lambda t: (t[:tok_len], t[at:at + n], t[at + n:at + 2 * n])
     want = host.cuda()
     if n_late:
         ops.scatter_tokens(*views(want), source)
@@ -593,6 +594,22 @@ def test_stage_batch_equals_copy_and_scatter(words, n_late):
     if done:
         torch.cuda.synchronize()
         assert torch.equal(device, want)
+
+
+@pytest.mark.parametrize("shapes", [[(3, 5)], [(16, 128, 128), (7,), (4, 1000)], [(1,)] * 40])
+def test_zeroed_slots(shapes):
+    """The slots named, and no others, are zero in every state tensor, whatever a slot's size and alignment."""
+    from liteinfer_b200 import ops
+
+    slots = 70
+    tensors = [torch.full((slots, *shape), 3.0, dtype=DTYPES[i % 2], device="cuda") for i, shape in enumerate(shapes)]
+    states = ops.SlotStates(tensors)
+    states.zero([4])
+    assert all(bool((t[4] == 0).all()) and int((t == 0).sum()) == t[4].numel() for t in tensors)
+    named = [0, *range(5, slots)]
+    states.zero(named)
+    for t in tensors:
+        assert bool((t[0] == 0).all() and (t[4:] == 0).all() and (t[1:4] == 3).all())
 
 
 def test_split_policy():
