@@ -196,6 +196,28 @@ def test_rope_write_then_attention(dtype, heads, kv_heads, head_dim, page_size, 
     assert torch.isfinite(outs[0][3].float()).all()
 
 
+# Launches of few blocks, whose keys two blocks share from eight tiles of 64 on (one tile short of it, just there, an odd
+# number of tiles, keys hidden by a window, a sequence too short to share beside one that is not).
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 2, 64), (3, 1, 128), (8, 8, 128), (32, 1, 64)])
+@pytest.mark.parametrize("q_lens,ctx_lens,window", [([40], [448], 0), ([40], [449], 0), ([130, 2], [1111, 70], 0), ([70, 33], [700, 1000], 600),
+                                                    ([3], [2000], 513)])
+def test_prompt_attention_with_shared_keys(heads, kv_heads, head_dim, q_lens, ctx_lens, window):
+    from liteinfer_b200 import ops
+
+    case = _paged_case(torch.bfloat16, heads, kv_heads, head_dim, 16, q_lens, ctx_lens)
+    qkv, k_pool, v_pool = case["qkv"], case["k_pool"], case["v_pool"]
+    ops.rope_kv_write(qkv, case["positions"], case["seq_of"], case["table"], k_pool, v_pool, None, heads, kv_heads, head_dim, 0)
+    common = (case["table"], case["qsl"], case["ctx"])
+    out = torch.empty(case["T"], heads * head_dim, dtype=torch.bfloat16, device="cuda")
+    ops.paged_attention_tcgen05(qkv, qkv.stride(0), out, k_pool, v_pool, *common, torch.arange(len(q_lens), dtype=torch.int32, device="cuda"),
+                                len(q_lens), max(q_lens), heads, kv_heads, head_dim, head_dim ** -0.5, window)
+    want = torch.empty_like(out)
+    ref.paged_attention(qkv, qkv.shape[1], want, k_pool, v_pool, *common, len(q_lens), max(q_lens), heads, kv_heads, head_dim,
+                        head_dim ** -0.5, window)
+    torch.testing.assert_close(out.float(), want.float(), **_tol(torch.bfloat16))
+    assert ops.gemm_error_flag("cuda:0") == 0
+
+
 # Rows walked by one warp and by teams, one unit of keys and several rounds of them, every width of values.
 @pytest.mark.parametrize("heads,kv_heads,head_dim,page_size", [(3, 1, 64, 16), (9, 1, 20, 16), (2, 2, 128, 16), (6, 3, 256, 8),
                                                                (2, 1, 320, 16), (34, 2, 33, 5)])
