@@ -71,8 +71,6 @@ __device__ ArgMax block_argmax(ArgMax mine, ArgMax* scratch /* 32 */) {
 constexpr int kSampleThreads = 512, kSampleWarps = kSampleThreads / 32;
 constexpr int kMostRanks = 8;      // blocks of a row's cluster
 constexpr int kRankColumns = 2048; // a row of no more columns is one block's: fewer barriers between blocks
-constexpr int kBins = 1024;
-constexpr int kListed = 512;       // columns that a warp can list; where one has more its block goes on walking its whole share
 constexpr int kSampleMostSmem = 200 << 10;
 constexpr float kBinsPerUnit = 46.f;   // (kBins - 1) / 46 = 22.24 > 32 ln 2: a value in the last bin has no probability left
 
@@ -281,7 +279,8 @@ __device__ Keep select_prefix(Share<S>& share, bool all_in, Keep within, unsigne
   const unsigned long long each = unit ? 1ull : share.weight(beta_value);
   const unsigned long long count = each ? mass / each : 1ull;
   const unsigned long long ties = each ? min(count, (limit - above) / each + 1) : 1ull;   // above <= limit
-  Keep out{beta, vocab};
+  // (Where the cut falls on the value that `within` was cut at, that cut stays.)
+  Keep out{beta, beta == within.beta ? within.tie_cut : vocab};
   if (ties < count) {
     // Not every element equal to beta survives: the index of the `ties`-th one, over the blocks in order.
     const int from = share.from, to = share.to;

@@ -366,7 +366,7 @@ def _sample_rule(x, k, p, u):
 # One block a row, two, four, eight; rows that start anywhere; rows too long for the blocks' shared memory, and for 16-bit
 # column numbers; as many rows as make bfloat16 be staged undivided.
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("vocab,rows", [(1, 12), (31, 12), (2048, 12), (2049, 12), (8190, 84), (50257, 12), (128256, 48),
+@pytest.mark.parametrize("vocab,rows", [(1, 12), (31, 12), (8192, 12), (8193, 12), (20011, 12), (32766, 84), (50257, 12), (128256, 48),
                                         (400003, 12), (600001, 12)])
 def test_sample_splits_a_row_over_blocks(dtype, vocab, rows):
     from liteinfer_b200 import ops
