@@ -51,7 +51,7 @@ __device__ ArgMax block_argmax(ArgMax mine, ArgMax* scratch /* 32 */) {
 }
 
 // ---- the sampling kernel --------------------------------------------------------------------------
-// A row belongs to a cluster of blocks (one per 2,048 columns, at most eight), each with its share of the columns in its
+// A row belongs to a cluster of blocks (one per 8,192 columns, at most eight), each with its share of the columns in its
 // shared memory, so the logits are read once.  Every later pass runs over shared memory; what the blocks of a row must agree on (the maximum, a
 // histogram, a running weight) they read from one another's shared memory behind a cluster barrier, and each works
 // the answer out for itself.
@@ -70,7 +70,12 @@ __device__ ArgMax block_argmax(ArgMax mine, ArgMax* scratch /* 32 */) {
 // the key's bits, most of them into the same bin, and one thread that walked the bins; one row with top-k and top-p: 50 us.
 constexpr int kSampleThreads = 512, kSampleWarps = kSampleThreads / 32;
 constexpr int kMostRanks = 8;      // blocks of a row's cluster
-constexpr int kRankColumns = 2048; // a row of no more columns is one block's: fewer barriers between blocks
+// A row of no more columns is one block's, and so on.  The passes over a share get longer, but there are fewer blocks to meet at
+// every barrier, and more rows at once: 12 rows of 16,000 columns take 27.7 us in two blocks each and 35.8 in eight, 64 rows of
+// 32,000 42 in four and 74 in eight; with twice as many columns a block 34.7 and 40.
+constexpr int kRankColumns = 8192;
+constexpr int kBins = 1024;
+constexpr int kListed = 512;       // columns that a warp can list; where one has more its block goes on walking its whole share
 constexpr int kSampleMostSmem = 200 << 10;
 constexpr float kBinsPerUnit = 46.f;   // (kBins - 1) / 46 = 22.24 > 32 ln 2: a value in the last bin has no probability left
 
