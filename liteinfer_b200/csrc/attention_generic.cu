@@ -15,9 +15,8 @@
 // `softcap` > 0 turns a scaled score s into softcap * tanh(s / softcap) before the softmax; `sink` [heads]
 // (float, optional): exp(sink[h]) is one more term of head h's denominator, with no key and no value.
 //
-// Work split: block = (query tile, KV head, sequence).  A row (query, head-in-group) walks its keys in units of 64 that
-// start at multiples of 64, 32 keys at a time with the online softmax from nothing in each unit; the units' results are
-// merged in ascending order.  So the order of every sum depends on the row's position only, never on how the batch was cut
+// Work split: block = (query tile, KV head, sequence).  A row (query, head-in-group) walks its keys in units of 32 that
+// start at multiples of 32, each with a softmax of its own; the units' results are merged in ascending order.  So the order of every sum depends on the row's position only, never on how the batch was cut
 // or on who walks a unit: where a block has more rows than warps each warp takes rows in turn and walks all of a row's
 // units; where it has fewer (decode) a row belongs to a team of warps, which walk a unit each and meet for the merge.
 // Masked keys are not read at all: a page that was never written, or holds another request's tokens, cannot leak
@@ -25,7 +24,7 @@
 //
 // Bound by the latency of a unit's loads: a lane asks for 64 numbers of its key at once in 16-byte pieces, and for 32 of the
 // values' numbers, without a branch between the loads.  Measured on B200 (float32, 12 heads
-// on 4, head size 64, generating 24 tokens for 12 sequences of 19 to 190): 24 us a launch on average, prompts included (13 for
+// on 4, head size 64, generating 24 tokens for 12 sequences of 19 to 190): 24 us a launch on average, prompts included (9 for
 // a decode step), against 238 when a warp walked all of a row's keys one load after another.
 #include "common.cuh"
 
@@ -33,7 +32,7 @@ namespace li {
 
 constexpr int kMaxKeyDim = 1024;
 constexpr int kQueriesPerBlock = 8;
-constexpr int kUnit = 64;
+constexpr int kUnit = 32;
 constexpr int kMostWarps = 16;
 
 template <typename T>
@@ -47,6 +46,7 @@ struct GenericParams {
   int window, keep_first;
   float scale, softcap;
   bool vec;      // keys lie on 16 bytes and are a multiple of them long
+  bool row_blocks;   // single tokens: a block has one row (blockIdx.x is the head in its group)
 };
 
 // What a walk over keys has so far: the maximum, the sum and the weighted values (lane + 32 i of them in acc[i]).
@@ -167,14 +167,16 @@ template <typename T, int kDimsPerLane>
 __global__ void __launch_bounds__(kDimsPerLane <= 8 ? 32 * kMostWarps : 256, 1)
 paged_attention_generic_kernel(const GenericParams<T> p) {
   extern __shared__ __align__(16) float q_smem[];
+  grid_launch_dependents();       // (what follows may be a product that asks for its weights first)
+  grid_dependency_wait();
   const int seq = blockIdx.z, kvh = blockIdx.y;
   const int q_begin = p.query_start_loc[seq], q_len = p.query_start_loc[seq + 1] - q_begin;
-  const int tile_start = blockIdx.x * kQueriesPerBlock;
+  const int tile_start = p.row_blocks ? 0 : blockIdx.x * kQueriesPerBlock;
   if (tile_start >= q_len) return;
   const int ctx = p.context_lens[seq];
   const int groups = p.heads / p.kv_heads;
   const int tile_q = min(kQueriesPerBlock, q_len - tile_start);
-  const int rows = tile_q * groups;
+  const int first_row = p.row_blocks ? blockIdx.x : 0, rows = p.row_blocks ? 1 : tile_q * groups;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const int q_stride = (p.head_dim + 3) / 4 * 4;
   float* qs = q_smem + warp * q_stride;
@@ -190,8 +192,8 @@ paged_attention_generic_kernel(const GenericParams<T> p) {
   // A team has one row, and every warp of the block takes part in its barriers.
   for (int row = warp / team; team > 1 ? row == warp / team : row < rows; row += teams) {
     const bool real = row < rows && warp < teams * team;
-    const int qi = tile_start + (real ? row / groups : 0);          // query index within the sequence's queries
-    const int head = kvh * groups + (real ? row % groups : 0);
+    const int qi = tile_start + (real ? (first_row + row) / groups : 0);          // query index within the sequence's queries
+    const int head = kvh * groups + (real ? (first_row + row) % groups : 0);
     const int qpos = ctx - q_len + qi;                 // absolute position of this query
     __syncwarp();
     if (real) {
@@ -262,8 +264,7 @@ int launch_generic(dim3 grid, int threads, const GenericParams<T>& p, cudaStream
                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (status != cudaSuccess) return (int)status;
   }
-  paged_attention_generic_kernel<T, kDimsPerLane><<<grid, threads, smem, stream>>>(p);
-  LI_LAUNCH_CHECK();
+  return (int)launch_pdl(0, paged_attention_generic_kernel<T, kDimsPerLane>, grid, dim3(threads), smem, stream, p);
 }
 
 template <typename T>
@@ -299,16 +300,20 @@ LI_EXPORT int li_paged_attention_generic(int dtype, const void* q, int q_row_str
   if (head_dim < 1 || head_dim > kMaxKeyDim || kv_heads < 1 || heads % kv_heads) return LI_ERR_UNSUPPORTED;
   if (v_dim < 1 || v_dim > 32 * 32) return LI_ERR_UNSUPPORTED;
   if (kv_heads > 65535 || num_seqs > 65535) return LI_ERR_UNSUPPORTED;
-  // Few rows a block (decode): more warps share a row's units.
-  const int rows = (max_q_len < kQueriesPerBlock ? max_q_len : kQueriesPerBlock) * (heads / kv_heads);
+  // Few rows a block (decode): more warps share a row's units.  Single tokens of few sequences: a block for every row, whose
+  // warps then walk sixteen units at once (12 sequences of 19 to 190 keys, 12 heads on 4: 9.2 us a launch, 12.9 with the three
+  // rows of a KV head in a block; 64 sequences of 500, whose keys every row's block would fetch again: 72 and 52).
+  const int groups = heads / kv_heads;
+  const bool row_blocks = max_q_len == 1 && groups > 1 && (long)num_seqs * heads <= 2 * 148;
+  const int rows = row_blocks ? 1 : (max_q_len < kQueriesPerBlock ? max_q_len : kQueriesPerBlock) * groups;
   const int threads = rows >= 8 || v_dim > 256 ? 256 : 32 * kMostWarps;
-  const dim3 grid((max_q_len + kQueriesPerBlock - 1) / kQueriesPerBlock, kv_heads, num_seqs);
+  const dim3 grid(row_blocks ? groups : (max_q_len + kQueriesPerBlock - 1) / kQueriesPerBlock, kv_heads, num_seqs);
   const auto run = [&](auto p) {
     p.block_table = block_table, p.query_start_loc = query_start_loc, p.context_lens = context_lens, p.sink = sink;
     p.q_row_stride = q_row_stride, p.out_row_stride = out_row_stride, p.table_stride = table_stride;
     p.heads = heads, p.kv_heads = kv_heads, p.head_dim = head_dim, p.v_dim = v_dim;
     p.page_size = page_size, p.num_pages = num_pages, p.window = window, p.keep_first = keep_first;
-    p.scale = scale, p.softcap = softcap;
+    p.scale = scale, p.softcap = softcap, p.row_blocks = row_blocks;
     p.vec = aligned16(k_pool) && (size_t)head_dim * sizeof(*p.k_pool) % 16 == 0;
     return launch_generic(grid, threads, p, stream);
   };
