@@ -363,6 +363,15 @@ static int plan_and_launch(const CUtensorMap& map, const StreamParams& p, cudaSt
       // (with at most three chunks of k a warp and one tile of rows, a warp keeps its share of x in registers)
       if (NT == 1 && (p.K + kChunkK - 1) / kChunkK <= 18 && !getenv("LITEINFER_STREAM_NO_X_CACHE"))
         return launch_stream_gemm<1, 6, 3, false, 3>(map, p, min(tiles, 2 * sms), stream);
+      // Longer rows, whose x does not fit those registers: one block of eight warps per SM with deep rings, at most three or
+      // four chunks of k a warp, so that x stays in registers all the same.  Without, every warp reads its share of x again
+      // for every tile.  Measured on B200 at 3 rows: 28672 x 4096 with its activation 34.4 us (39.8), 6144 x 4096 8.5 (11.8),
+      // at 8 rows 16384 x 3072 16.1 (18.5); a decode step of three sequences at the 8B sizes 3,243 us (3,439).  A weight of
+      // very many tiles gains more from two blocks' rings than from x at hand: 128256 x 4096 152 us with them, 158 without.
+      if (NT == 1 && tiles <= 24 * sms) {
+        if ((p.K + kChunkK - 1) / kChunkK <= 24) return launch_stream_gemm<1, 8, 5, false, 3>(map, p, min(tiles, sms), stream);
+        if ((p.K + kChunkK - 1) / kChunkK <= 32) return launch_stream_gemm<1, 8, 5, false, 4>(map, p, min(tiles, sms), stream);
+      }
       return launch_stream_gemm<NT, 6, 3, false>(map, p, min(tiles, 2 * sms), stream);
     default: return launch_stream_gemm<NT, 8, 3, false>(map, p, tiles <= 2 * sms ? tiles : sms, stream);
   }

@@ -870,6 +870,25 @@ def test_fused_decode_layer_chain_matches_the_unfused_one(monkeypatch):
     torch.testing.assert_close(s2.sumsq.sum(0), b.float().pow(2).sum(-1), rtol=1e-5, atol=1e-5)
 
 
+# More tiles than two for every SM with rows of 19 to 24 chunks of 128 k, of 25 to 32 and of more; and very many tiles.
+@pytest.mark.parametrize("M", [1, 8, 9])
+@pytest.mark.parametrize("N,K", [(4752, 2312), (6144, 3072), (5001, 3080), (9000, 4096), (4752, 4104), (57000, 2440)])
+def test_gemm_stream_of_long_rows(M, N, K):
+    from liteinfer_b200 import ops
+
+    x, w = _randn(M, K, dtype=torch.bfloat16), _randn(N, K, dtype=torch.bfloat16, seed=1, scale=0.05)
+    b = _randn(N, dtype=torch.bfloat16, seed=2)
+    got = ops.gemm_stream(x, w, torch.empty(M, N, dtype=torch.bfloat16, device="cuda"), b)
+    torch.testing.assert_close(got.double(), x.double() @ w.double().t() + b.double(), rtol=2 ** -7, atol=2 ** -7)
+    if N % 16 == 0:
+        pairs = (x.double() @ w.double().t()).view(M, -1, 2, 8).bfloat16().double()
+        want = (pairs[:, :, 0] * torch.sigmoid(pairs[:, :, 0])).bfloat16().double() * pairs[:, :, 1]
+        got = ops.gemm_stream(x, w, torch.empty(M, N // 2, dtype=torch.bfloat16, device="cuda"), None, "silu")
+        # Both factors are rounded to 2^-8 of themselves, the gate's through an activation of slope up to 1.1, and their product.
+        torch.testing.assert_close(got.double(), want.flatten(1), rtol=2 ** -5, atol=2 ** -6)
+    assert ops.gemm_error_flag("cuda:0") == 0
+
+
 @pytest.mark.parametrize("M", [1, 2, 7, 8, 9, 16])
 @pytest.mark.parametrize("N,K", [(3072, 2048), (2048, 8192), (1000, 96), (17, 40), (128256 // 8, 2048), (48, 16384),
                                  (16384, 2048), (5000, 200)])
