@@ -172,13 +172,27 @@ __global__ void delta_gates_kernel(const T* __restrict__ qkv, size_t row_width, 
   }
 }
 
-// R values of T starting at p (R a multiple of 4; p aligned to 16 bytes when kVector) as floats.
+// Which entries of a column of 8 R a lane keeps, where everything is vectors: pieces of four, the eight lanes' pieces side by
+// side, so that the lanes of a column read 128 neighbouring bytes at once.
+__device__ __forceinline__ int piece_at(int c, int part) { return (c * 8 + part) * 4; }
+
+__device__ __forceinline__ float4 load_piece(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load_piece(const bf16* p) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  return make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16),
+                     __uint_as_float(raw.y & 0xffff0000u));
+}
+
+// A lane's R values of a row as floats: its pieces of the row at p (16-byte aligned) when kVector, else the `live` first of
+// the R that start at p.
 template <typename T, int R, bool kVector>
-__device__ __forceinline__ void load_slice(float (&dst)[R], const T* __restrict__ p, int live) {
+__device__ __forceinline__ void load_slice(float (&dst)[R], const T* __restrict__ p, int live, int part) {
   if (kVector) {
-    constexpr int N = Vec16<T>::N;
 #pragma unroll
-    for (int c = 0; c < R / N; ++c) unpack16(load16(p + c * N), dst + c * N);
+    for (int c = 0; c < R / 4; ++c) {
+      const float4 v = load_piece(p + piece_at(c, part));
+      dst[c * 4] = v.x; dst[c * 4 + 1] = v.y; dst[c * 4 + 2] = v.z; dst[c * 4 + 3] = v.w;
+    }
   } else {
 #pragma unroll
     for (int r = 0; r < R; ++r) dst[r] = r < live ? to_float(p[r]) : 0.f;
@@ -190,8 +204,8 @@ struct DeltaToken {   // what a lane needs of one token: its slices of q and k, 
   float q[R], k[R], v, q_inv, k_inv, beta, g;
 };
 
-// The state is kept column by column: state[slot][head][column][dim], so that a lane's slice of a column (R
-// entries) is contiguous and a warp's four columns are 4 * dim * 4 bytes in a row.
+// The state is kept column by column: state[slot][head][column][dim], so that the lanes of a column read 128 bytes in a row
+// and a warp's four columns are 4 * dim * 4 bytes.
 // R: entries of a column that one lane keeps (dim <= 8 R).  kAhead: tokens whose inputs are in flight while one is
 // computed (1 for steps of single tokens).  kVector: dim == 8 R and every row is 16-byte aligned.
 template <typename T, int R, int kAhead, bool kVector>
@@ -209,7 +223,7 @@ gated_delta_rule_kernel(const T* __restrict__ qkv, const float* __restrict__ sca
   const int part = lane >> 2;                                   // which eighth of the column
   const int column = blockIdx.x * 32 + warp * 4 + (lane & 3);
   const bool live = column < vdim;
-  const int first = part * R;
+  const int first = kVector ? 0 : part * R;                     // (a vector's pieces: see piece_at)
   const int mine_dims = min(R, max(0, dim - first));            // entries of this lane's slice that exist
   const int qk_width = kv_heads * dim;
   const size_t row_width = 2 * (size_t)qk_width + (size_t)heads * vdim;
@@ -222,7 +236,7 @@ gated_delta_rule_kernel(const T* __restrict__ qkv, const float* __restrict__ sca
   if (kVector) {
 #pragma unroll
     for (int c = 0; c < R / 4; ++c) {
-      const float4 v = live ? *reinterpret_cast<const float4*>(mine + c * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 v = live ? *reinterpret_cast<const float4*>(mine + piece_at(c, part)) : make_float4(0.f, 0.f, 0.f, 0.f);
       S[c * 4] = v.x; S[c * 4 + 1] = v.y; S[c * 4 + 2] = v.z; S[c * 4 + 3] = v.w;
     }
   } else {
@@ -237,14 +251,14 @@ gated_delta_rule_kernel(const T* __restrict__ qkv, const float* __restrict__ sca
     if (kAhead > 1) {
       // From the kernel in front: q and k as unit vectors in float, and the gates.
       const float* unit = scales + ((size_t)t * kv_heads + kv_head) * 2 * (size_t)dim + first;
-      load_slice<float, R, kVector>(tok.q, unit, mine_dims);
-      load_slice<float, R, kVector>(tok.k, unit + dim, mine_dims);
+      load_slice<float, R, kVector>(tok.q, unit, mine_dims, part);
+      load_slice<float, R, kVector>(tok.k, unit + dim, mine_dims, part);
       const float2 ga = *reinterpret_cast<const float2*>(gates + ((size_t)t * heads + head) * 2);
       tok.q_inv = 1.f; tok.k_inv = 1.f; tok.beta = ga.x; tok.g = ga.y;
       return;
     }
-    load_slice<T, R, kVector>(tok.q, row + q_at, mine_dims);
-    load_slice<T, R, kVector>(tok.k, row + k_at, mine_dims);
+    load_slice<T, R, kVector>(tok.q, row + q_at, mine_dims, part);
+    load_slice<T, R, kVector>(tok.k, row + k_at, mine_dims, part);
     if (kAhead == 1) {
       // Steps of single tokens: no kernel in front; the block works out the token's scales and gates itself.
       float qq = 0.f, kk = 0.f;
@@ -338,7 +352,7 @@ gated_delta_rule_kernel(const T* __restrict__ qkv, const float* __restrict__ sca
   if (kVector) {
 #pragma unroll
     for (int c = 0; c < R / 4; ++c)
-      *reinterpret_cast<float4*>(mine + c * 4) = make_float4(S[c * 4], S[c * 4 + 1], S[c * 4 + 2], S[c * 4 + 3]);
+      *reinterpret_cast<float4*>(mine + piece_at(c, part)) = make_float4(S[c * 4], S[c * 4 + 1], S[c * 4 + 2], S[c * 4 + 3]);
   } else {
 #pragma unroll
     for (int r = 0; r < R; ++r)
@@ -346,12 +360,41 @@ gated_delta_rule_kernel(const T* __restrict__ qkv, const float* __restrict__ sca
   }
 }
 
+// Two 32-bit numbers in one register pair: a fused multiply-add of both is one instruction, rounded like two.
+typedef unsigned long long pair32;
+__device__ __forceinline__ pair32 both(float v) {
+  pair32 r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ pair32 mul_pair(pair32 a, pair32 b) {
+  pair32 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ pair32 fma_pair(pair32 a, pair32 b, pair32 c) {
+  pair32 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ float sum_pair(pair32 a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+  return x + y;
+}
+
 // The same recurrence for prompts and portions, with the tokens' inputs staged in shared memory: the loads of a
 // register ring several tokens deep share a warp's few scoreboards, so a wait for one token's inputs also waits
 // for the ones just asked for, and a token cost a whole trip to the second-level cache (0.5 us, whatever the head
-// size).  Here a block copies eight tokens at a time (unit q and k in float, gates, the block's 16 values of v)
+// size).  Here a block copies eight tokens at a time (unit q and k in float, gates, the block's values of v)
 // with cp.async, whose groups are waited for in order, two chunks in flight, and reads them with shared-memory
 // loads.  For dim == 8 R, vdim a multiple of 16 and 16-byte aligned rows.
+//
+// Bound by instructions: a token is about 90 a warp of four columns, one after the other in a launch of a few hundred warps
+// (a prompt or two: each waits for the one before, some 3.5 cycles), and one of several warps' on every scheduler in a wide
+// one.  So a multiply-add works on two numbers, a chunk's tokens lie at places known to the compiler, and what a thread copies
+// comes from pointers that move on by a constant.  Measured on B200, 16 heads of 128 x 128: one prompt of 512 tokens 98 us
+// (148 before these three), eight 304 (404).  Two columns a lane, which share the reads of q and k: 119 and 309.
 constexpr int kStageTokens = 8;
 
 template <typename T, int R>
@@ -360,62 +403,105 @@ gated_delta_rule_staged_kernel(const T* __restrict__ qkv, const float* __restric
                                float* __restrict__ state, const int* __restrict__ query_start_loc,
                                const int* __restrict__ state_slots, float* __restrict__ out, int heads, int kv_heads,
                                int vdim) {
-  // Four warps and 16 columns a block: a prompt alone is a few hundred chains (heads x vdim columns / 4 a warp),
-  // fewer than the device has schedulers, so each warp gets a scheduler of its own and as little of a column's
-  // arithmetic as the lanes of a column can share.
   extern __shared__ __align__(16) unsigned char staged[];
-  constexpr int dim = 8 * R, kColumns = 16;
+  constexpr int dim = 8 * R, kColumns = 16, kPieces = R / 4;
   constexpr int kUnitBytes = 8 * dim, kValueBytes = kColumns * (int)sizeof(T);
   constexpr int kTokenBytes = kUnitBytes + 16 + (kValueBytes + 15) / 16 * 16;   // units | gates (8 bytes, padded) | v
-  constexpr int kCopies = kUnitBytes / 16 + 1 + kValueBytes / 16;               // per token: 16-byte copies, one of 8 for the gates
   grid_dependency_wait();
   const int seq = blockIdx.z, head = blockIdx.y;
   const int begin = query_start_loc[seq], end = query_start_loc[seq + 1];
   if (end <= begin) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int part = lane >> 2;
+  const int part = lane >> 2;                                   // which eighth of the column
   const int local_column = warp * 4 + (lane & 3), column = blockIdx.x * kColumns + local_column;
-  const int first = part * R;
   const int qk_width = kv_heads * dim;
   const size_t row_width = 2 * (size_t)qk_width + (size_t)heads * vdim;
   const int kv_head = head / (heads / kv_heads);
   const size_t v_at = 2 * (size_t)qk_width + (size_t)head * vdim + (size_t)blockIdx.x * kColumns;
-  float* mine = state + (((size_t)state_slots[seq] * heads + head) * vdim + column) * dim + first;
+  float* mine = state + (((size_t)state_slots[seq] * heads + head) * vdim + column) * dim;
 
-  float S[R];
+  pair32 S[kPieces][2];
 #pragma unroll
-  for (int c = 0; c < R / 4; ++c) {
-    const float4 v = *reinterpret_cast<const float4*>(mine + c * 4);
-    S[c * 4] = v.x; S[c * 4 + 1] = v.y; S[c * 4 + 2] = v.z; S[c * 4 + 3] = v.w;
+  for (int c = 0; c < kPieces; ++c) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(mine + piece_at(c, part));
+    S[c][0] = v.x;
+    S[c][1] = v.y;
   }
 
+  // A thread's copies of a chunk: one piece of the unit vectors of every kRound-th token, and for some threads a piece of v
+  // or a token's gates.  Where they come from moves on by the same distance every chunk.
+  constexpr int kUnitPieces = kUnitBytes / 16, kRound = 128 / kUnitPieces > 0 ? 128 / kUnitPieces : 1;
+  constexpr int kValuePieces = kValueBytes / 16 > 0 ? kValueBytes / 16 : 1;
+  static_assert(kValueBytes % 16 == 0 && 128 % kUnitPieces == 0 && kStageTokens * kValuePieces <= 128, "a chunk's copies");
+  const size_t unit_row = (size_t)kv_heads * 2 * dim;             // of floats, a token
+  const int unit_token = threadIdx.x / kUnitPieces, unit_piece = threadIdx.x % kUnitPieces;
+  const float* unit_src = units + ((size_t)(begin + unit_token) * kv_heads + kv_head) * 2 * dim + unit_piece * 4;
+  const int value_token = threadIdx.x / kValuePieces, value_piece = threadIdx.x % kValuePieces;
+  const T* value_src = qkv + (size_t)(begin + value_token) * row_width + v_at + value_piece * (16 / (int)sizeof(T));
+  const float* gate_src = gates + ((size_t)(begin + threadIdx.x) * heads + head) * 2;
+  const unsigned stage = (unsigned)__cvta_generic_to_shared(staged);
   auto copy_chunk = [&](int chunk) {
-    unsigned char* buffer = staged + (size_t)(chunk & 1) * kStageTokens * kTokenBytes;
-    const int t0 = begin + chunk * kStageTokens;
-    for (int i = threadIdx.x; i < kStageTokens * kCopies; i += 128) {
-      const int j = i / kCopies, c = i - j * kCopies, t = t0 + j;
-      if (t >= end) continue;
-      unsigned char* dst = buffer + (size_t)j * kTokenBytes;
-      if (c < kUnitBytes / 16) {
-        const char* src = reinterpret_cast<const char*>(units + ((size_t)t * kv_heads + kv_head) * 2 * dim) + c * 16;
-        const unsigned d = (unsigned)__cvta_generic_to_shared(dst + c * 16);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src));
-      } else if (c == kUnitBytes / 16) {
-        const char* src = reinterpret_cast<const char*>(gates + ((size_t)t * heads + head) * 2);
-        const unsigned d = (unsigned)__cvta_generic_to_shared(dst + kUnitBytes);
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src));
-      } else {
-        const int k = c - kUnitBytes / 16 - 1;
-        const char* src = reinterpret_cast<const char*>(qkv + (size_t)t * row_width + v_at) + k * 16;
-        const unsigned d = (unsigned)__cvta_generic_to_shared(dst + kUnitBytes + 16 + k * 16);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src));
-      }
-    }
+    const unsigned buffer = stage + (unsigned)(chunk & 1) * (kStageTokens * kTokenBytes);
+    const int left = end - begin - chunk * kStageTokens;          // tokens from the chunk's first on
+#pragma unroll
+    for (int j = 0; j < kStageTokens; j += kRound)
+      if (unit_token + j < left && unit_token + j < kStageTokens)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(buffer + (unit_token + j) * kTokenBytes + unit_piece * 16),
+                     "l"(unit_src + j * unit_row));
+    if (value_token < kStageTokens && value_token < left)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(buffer + value_token * kTokenBytes + kUnitBytes + 16 + value_piece * 16),
+                   "l"(value_src));
+    if (threadIdx.x < kStageTokens && (int)threadIdx.x < left)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(buffer + threadIdx.x * kTokenBytes + kUnitBytes), "l"(gate_src));
     asm volatile("cp.async.commit_group;" ::);
+    unit_src += kStageTokens * unit_row;
+    value_src += kStageTokens * row_width;
+    gate_src += (size_t)kStageTokens * heads * 2;
   };
 
+  // Where the column's read-out of the token before goes.
+  const size_t out_row = (size_t)heads * vdim;
+  float* out_at = out + (size_t)begin * out_row + (size_t)head * vdim + column - out_row;
   float o_parts = 0.f;
-  int o_token = -1;
+  const int lane_at = part * 16, column_at = kUnitBytes + 16 + local_column * (int)sizeof(T);
+  bool stores = false;          // not yet: the first token has none before it
+  // One token, whose inputs lie at `tok` (a lane's pieces of a row: see piece_at).
+  auto step = [&](const unsigned char* tok) {
+    const unsigned char *q = tok + lane_at, *k = q + dim * 4;
+    const float2 ga = *reinterpret_cast<const float2*>(tok + kUnitBytes);
+    const float v = widen(*reinterpret_cast<const T*>(tok + column_at));
+    pair32 kk[kPieces][2], d0, d1, o0, o1;
+#pragma unroll
+    for (int c = 0; c < kPieces; ++c) {
+      const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(k + c * 128);
+      kk[c][0] = k4.x;
+      kk[c][1] = k4.y;
+      d0 = c == 0 ? mul_pair(S[c][0], k4.x) : fma_pair(S[c][0], k4.x, d0);
+      d1 = c == 0 ? mul_pair(S[c][1], k4.y) : fma_pair(S[c][1], k4.y, d1);
+    }
+    // The read-out of the token before is added up over the lanes together with this token's S^T k.
+    float dsum = sum_pair(d0) + sum_pair(d1), osum = o_parts;
+#pragma unroll
+    for (int offset = 4; offset <= 16; offset <<= 1) {
+      const float a = __shfl_xor_sync(0xffffffffu, dsum, offset), b = __shfl_xor_sync(0xffffffffu, osum, offset);
+      dsum += a;
+      osum += b;
+    }
+    if (stores) *out_at = osum;
+    stores = part == 0;
+    out_at += out_row;
+    const pair32 g2 = both(ga.y), c2 = both(ga.x * (v - dsum * ga.y));
+#pragma unroll
+    for (int c = 0; c < kPieces; ++c) {
+      const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(q + c * 128);
+      S[c][0] = fma_pair(S[c][0], g2, mul_pair(kk[c][0], c2));
+      S[c][1] = fma_pair(S[c][1], g2, mul_pair(kk[c][1], c2));
+      o0 = c == 0 ? mul_pair(S[c][0], q4.x) : fma_pair(S[c][0], q4.x, o0);
+      o1 = c == 0 ? mul_pair(S[c][1], q4.y) : fma_pair(S[c][1], q4.y, o1);
+    }
+    o_parts = sum_pair(o0) + sum_pair(o1);
+  };
+
   const int chunks = (end - begin + kStageTokens - 1) / kStageTokens;
   copy_chunk(0);
   for (int chunk = 0; chunk < chunks; ++chunk) {
@@ -426,55 +512,22 @@ gated_delta_rule_staged_kernel(const T* __restrict__ qkv, const float* __restric
       asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
     __syncthreads();
-    const unsigned char* buffer = staged + (size_t)(chunk & 1) * kStageTokens * kTokenBytes;
-    const int t0 = begin + chunk * kStageTokens, count = min(kStageTokens, end - t0);
-#pragma unroll 2
-    for (int j = 0; j < count; ++j) {
-      const unsigned char* tok = buffer + (size_t)j * kTokenBytes;
-      const float* q = reinterpret_cast<const float*>(tok) + first;
-      const float* k = q + dim;
-      const float2 ga = *reinterpret_cast<const float2*>(tok + kUnitBytes);
-      const float v = widen(reinterpret_cast<const T*>(tok + kUnitBytes + 16)[local_column]);
-      float kk[R];
-      float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
-#pragma unroll
-      for (int r = 0; r < R; r += 4) {
-        const float4 k4 = *reinterpret_cast<const float4*>(k + r);
-        kk[r] = k4.x; kk[r + 1] = k4.y; kk[r + 2] = k4.z; kk[r + 3] = k4.w;
-        d0 = fmaf(S[r], k4.x, d0); d1 = fmaf(S[r + 1], k4.y, d1);
-        d2 = fmaf(S[r + 2], k4.z, d2); d3 = fmaf(S[r + 3], k4.w, d3);
-      }
-      // The read-out of the token before is added up over the lanes together with this token's S^T k.
-      float dsum = (d0 + d1) + (d2 + d3), osum = o_parts;
-#pragma unroll
-      for (int offset = 4; offset <= 16; offset <<= 1) {
-        const float a = __shfl_xor_sync(0xffffffffu, dsum, offset), b = __shfl_xor_sync(0xffffffffu, osum, offset);
-        dsum += a;
-        osum += b;
-      }
-      if (o_token >= 0 && part == 0) out[(size_t)o_token * heads * vdim + (size_t)head * vdim + column] = osum;
-      const float c = ga.x * (v - dsum * ga.y);
-      float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
-#pragma unroll
-      for (int r = 0; r < R; r += 4) {
-        const float4 q4 = *reinterpret_cast<const float4*>(q + r);
-        S[r] = fmaf(S[r], ga.y, kk[r] * c); S[r + 1] = fmaf(S[r + 1], ga.y, kk[r + 1] * c);
-        S[r + 2] = fmaf(S[r + 2], ga.y, kk[r + 2] * c); S[r + 3] = fmaf(S[r + 3], ga.y, kk[r + 3] * c);
-        o0 = fmaf(S[r], q4.x, o0); o1 = fmaf(S[r + 1], q4.y, o1);
-        o2 = fmaf(S[r + 2], q4.z, o2); o3 = fmaf(S[r + 3], q4.w, o3);
-      }
-      o_parts = (o0 + o1) + (o2 + o3);
-      o_token = t0 + j;
+    const unsigned char* tok = staged + (size_t)(chunk & 1) * kStageTokens * kTokenBytes;
+    const int count = min(kStageTokens, end - begin - chunk * kStageTokens);
+    if (count == kStageTokens) {           // at places known when this is compiled
+#pragma unroll 4
+      for (int j = 0; j < kStageTokens; ++j) step(tok + j * kTokenBytes);
+    } else {
+#pragma unroll 1
+      for (int j = 0; j < count; ++j) step(tok + j * kTokenBytes);
     }
     __syncthreads();     // the buffer is written again two chunks on
   }
-  {
-    const float o = sum_over_column_lanes(o_parts);
-    if (part == 0) out[(size_t)o_token * heads * vdim + (size_t)head * vdim + column] = o;
-  }
+  const float total = sum_over_column_lanes(o_parts);
+  if (part == 0) *out_at = total;
 #pragma unroll
-  for (int c = 0; c < R / 4; ++c)
-    *reinterpret_cast<float4*>(mine + c * 4) = make_float4(S[c * 4], S[c * 4 + 1], S[c * 4 + 2], S[c * 4 + 3]);
+  for (int c = 0; c < kPieces; ++c)
+    *reinterpret_cast<ulonglong2*>(mine + piece_at(c, part)) = make_ulonglong2(S[c][0], S[c][1]);
 }
 
 template <typename T, int R>

@@ -634,6 +634,49 @@ def test_zeroed_slots(shapes):
         assert bool((t[0] == 0).all() and (t[4:] == 0).all() and (t[1:4] == 3).all())
 
 
+# Sequences of less than a chunk of eight tokens, whole chunks, and a rest, together and each alone, at every head size the
+# staged kernel has; the plain recurrence checks the first.
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,dim,vdim", [(16, 128, 128), (4, 128, 32), (20, 64, 64), (40, 32, 96), (3, 256, 16)])
+def test_delta_rule_chunks(dtype, heads, dim, vdim):
+    from liteinfer_b200 import ops
+
+    lengths = [21, 1, 8, 9, 40, 2]
+    n, count = sum(lengths), len(lengths)
+    qkv = _randn(n, 2 * heads * dim + heads * vdim, dtype=dtype)
+    ab = _randn(n, 2 * heads, dtype=dtype, seed=1)
+    a_log, dt_bias = _randn(heads, dtype=torch.float32, seed=2), _randn(heads, dtype=torch.float32, seed=3)
+    before = _randn(count, heads, vdim, dim, dtype=torch.float32, seed=4)
+
+    def run(first, last):
+        rows = slice(sum(lengths[:first]), sum(lengths[:last]))
+        state, out = before[first:last].clone(), torch.empty(rows.stop - rows.start, heads * vdim, device="cuda")
+        starts = torch.tensor([0] + torch.tensor(lengths[first:last]).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+        slots = torch.arange(last - first, dtype=torch.int32, device="cuda")
+        ops.gated_delta_rule(qkv[rows], ab[rows], a_log, dt_bias, state, starts, slots, last - first, heads, heads, dim, vdim, out,
+                             max(2, max(lengths[first:last])))
+        return out, state
+
+    out, state = run(0, count)
+    at = 0
+    for i, length in enumerate(lengths[:5]):
+        alone, kept = run(i, i + 1)
+        assert torch.equal(alone, out[at:at + length]) and torch.equal(kept[0], state[i]), i
+        at += length
+    q, k, v = (t.double().unflatten(1, (heads, -1)) for t in qkv[:21].split([heads * dim, heads * dim, heads * vdim], dim=1))
+    q, k = (t / torch.sqrt(t.pow(2).sum(-1, keepdim=True) + 1e-6) for t in (q, k))
+    beta, raw = torch.sigmoid(ab[:21, :heads].double()), ab[:21, heads:].double() + dt_bias.double()
+    decay = torch.exp(-a_log.double().exp() * torch.nn.functional.softplus(raw))
+    S = before[0].double()                                  # [heads, vdim, dim]
+    for t in range(21):
+        S = decay[t][:, None, None] * S
+        u = beta[t][:, None] * (v[t] - torch.einsum("hvd,hd->hv", S, k[t]))
+        S = S + u[:, :, None] * k[t][:, None, :]
+        want = torch.einsum("hvd,hd->hv", S, q[t]) * dim ** -0.5
+        torch.testing.assert_close(out[t].double(), want.flatten(), rtol=1e-4, atol=1e-4)
+    torch.testing.assert_close(state[0].double(), S, rtol=1e-4, atol=1e-4)
+
+
 def test_split_policy():
     from liteinfer_b200.ops import decode_splits_for
 
