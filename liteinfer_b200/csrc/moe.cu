@@ -221,7 +221,7 @@ moe_router_kernel(const T* __restrict__ x, size_t x_stride, const float* __restr
 #pragma unroll
     for (int t = 0; t < TOK; ++t) xr[t] = x + (size_t)min(t0 + t, tokens - 1) * x_stride;
     if (wide) {
-#pragma unroll(TOK == 1 ? 8 : 1)
+#pragma unroll(TOK == 1 ? 8 : 2)
       for (int k = lane * 4; k < K; k += 128) {
         float4 wv[EXP];
 #pragma unroll
@@ -288,31 +288,46 @@ moe_sort_kernel(const int* __restrict__ ids, int pairs, int experts, int tile_ro
   int* cursor = sort_smem + experts;
   for (int e = threadIdx.x; e < experts; e += blockDim.x) counts[e] = 0;
   grid_dependency_wait();
+  // One block, so what takes its time is one thing waiting for another: a thread's first ids are asked for at once and kept
+  // for the second walk, and every expert's thread works out for itself where its run and its tiles begin.  8,192 pairs of 32
+  // experts: 8.1 us, 12.3 with loads one after the other, twice, and one thread that wrote the tiles.
+  constexpr int kHeld = 8;
+  int held[kHeld];
+#pragma unroll
+  for (int h = 0; h < kHeld; ++h) {
+    const int i = threadIdx.x + h * blockDim.x;
+    held[h] = i < pairs ? ids[i] : -1;
+  }
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
+#pragma unroll
+  for (int h = 0; h < kHeld; ++h)
+    if (held[h] >= 0 && held[h] < experts) atomicAdd(&counts[held[h]], 1);
+  for (int i = threadIdx.x + kHeld * blockDim.x; i < pairs; i += blockDim.x) {
     const int e = ids[i];
     if (e >= 0 && e < experts) atomicAdd(&counts[e], 1);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  for (int e = threadIdx.x; e <= experts; e += blockDim.x) {
     int run = 0, tile = 0;
-    for (int e = 0; e < experts; ++e) {
-      offsets[e] = run;
+    for (int j = 0; j < e; ++j) {
+      run += counts[j];
+      tile += (counts[j] + tile_rows - 1) / tile_rows;
+    }
+    offsets[e] = run;
+    if (e < experts) {
       cursor[e] = run;
       const int n = counts[e];
       for (int r = 0; r < n && tile < max_tiles; r += tile_rows, ++tile) {
         tile_expert[tile] = e;
         tile_row0[tile] = run + r;
       }
-      run += n;
+    } else {
+      for (; tile < max_tiles; ++tile) tile_expert[tile] = -1;
     }
-    offsets[experts] = run;
-    for (; tile < max_tiles; ++tile) tile_expert[tile] = -1;
   }
   __syncthreads();
   // The order of an expert's rows among themselves does not matter: every row of the products is computed alone.
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-    const int e = ids[i];
+  const auto put = [&](int i, int e) {
     if (e >= 0 && e < experts) {
       const int at = atomicAdd(&cursor[e], 1);
       order[at] = i;
@@ -320,7 +335,13 @@ moe_sort_kernel(const int* __restrict__ ids, int pairs, int experts, int tile_ro
     } else if (place != nullptr) {
       place[i] = -1;
     }
+  };
+#pragma unroll
+  for (int h = 0; h < kHeld; ++h) {
+    const int i = threadIdx.x + h * blockDim.x;
+    if (i < pairs) put(i, held[h]);
   }
+  for (int i = threadIdx.x + kHeld * blockDim.x; i < pairs; i += blockDim.x) put(i, ids[i]);
 }
 
 // out[m] = x[order[m] / top]: every pair's token row, in the order of the experts' runs.

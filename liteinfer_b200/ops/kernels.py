@@ -2026,6 +2026,11 @@ MOE_TCGEN05 = os.environ.get("LITEINFER_MOE_TCGEN05", "1") != "0"
 MOE_TCGEN05_MIN_PAIRS = int(os.environ.get("LITEINFER_MOE_TCGEN05_MIN_PAIRS", "1"))
 
 
+# Rows of an expert's tile in the products on the tcgen05 kernel (a pair of CTAs multiplies as many of them, in sixteens, as
+# the tile has).
+EXPERT_TILE_ROWS = 256
+
+
 def moe_tile_rows(dtype: torch.dtype, hidden: int, ff: int, pairs: int | None = None) -> int:
     """Rows of a tile of an expert's products: 128 where the tcgen05 kernel takes them (bfloat16, sizes in eights, a
     step of many pairs), 64 where both run on mma.sync tiles, else 32 (FFMA tiles)."""
@@ -2073,12 +2078,12 @@ def moe_grouped_tcgen05(mode: str, a: torch.Tensor, weight: torch.Tensor, out: t
                         activation: str = "swiglu", limit: float = 0.0, alpha: float = 1.0,
                         pair_weights: torch.Tensor | None = None) -> torch.Tensor:
     """`moe_grouped` on the tcgen05 kernel (bfloat16): `a` [pairs, K] and `out` hold their rows in the order of the
-    experts' runs (`plan.order`), the plan's tiles are 128 rows, and in mode "gate_up" an expert's gate and up rows lie
+    experts' runs (`plan.order`), the plan's tiles are `EXPERT_TILE_ROWS` rows, and in mode "gate_up" an expert's gate and up rows lie
     interleaved in eights.  mode "down" multiplies row m by pair_weights[plan.order[m]]; mode "up": experts without a gate."""
     _on_gpu(a, weight, out, pair_weights)
     experts, rows, K = weight.shape
     pairs = plan.order.numel()
-    assert plan.tile_rows == 128 and mode in ("gate_up", "down", "up") and a.dtype == weight.dtype == out.dtype == torch.bfloat16
+    assert plan.tile_rows == EXPERT_TILE_ROWS and mode in ("gate_up", "down", "up") and a.dtype == weight.dtype == out.dtype == torch.bfloat16
     assert a.shape == (pairs, K) and out.shape == (pairs, rows // 2 if mode == "gate_up" else rows)
     act = {"down": -1, "up": -2}.get(mode)
     if act is None:
@@ -2142,7 +2147,8 @@ def moe_expert_rows(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor, 
     gated = activation not in UNGATED_EXPERT_ACTIVATIONS
     first = "gate_up" if gated else "up"
     tile = moe_tile_rows(x.dtype, hidden, ff, pairs if eights or not gated else None)
-    plan = moe_sort(ids, experts, tile, with_place=tile == 128 or partial, in_pairs=tile != 128)
+    plan = moe_sort(ids, experts, EXPERT_TILE_ROWS if tile == 128 else tile, with_place=tile == 128 or partial,
+                    in_pairs=tile != 128)
     act = torch.empty((pairs, ff), dtype=x.dtype, device=x.device)
     each = torch.empty((pairs, hidden), dtype=x.dtype, device=x.device)
     scale = weights.view(-1)

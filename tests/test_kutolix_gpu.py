@@ -390,6 +390,37 @@ def test_expert_products_on_the_tcgen05_kernel(tokens, hidden, ff, experts, top,
     assert ops.gemm_error_flag(DEV) == 0
 
 
+# Experts with several tiles of 256 rows, with none, with one row; weights of part of a tile and of more than one.
+@pytest.mark.parametrize("hidden,ff", [(264, 72), (512, 256), (136, 520)])
+@pytest.mark.parametrize("counts", [[600, 0, 256, 1, 40], [17, 16, 255, 257, 33], [1, 0, 0, 0, 0]])
+@pytest.mark.parametrize("mode", ["capped_swiglu", "relu_squared"])
+def test_expert_tiles_of_every_height(hidden, ff, counts, mode):
+    from liteinfer_b200 import ops
+
+    dtype, tokens, experts = torch.bfloat16, sum(counts), len(counts)
+    x = _randn(tokens, hidden, seed=1, dtype=dtype)
+    up = _randn(experts, ff, hidden, seed=5, scale=hidden ** -0.5, dtype=dtype)
+    gate = _randn(experts, ff, hidden, seed=2, scale=hidden ** -0.5, dtype=dtype)
+    down = _randn(experts, hidden, ff, seed=3, scale=ff ** -0.5, dtype=dtype)
+    first = up if mode == "relu_squared" else torch.stack([gate.unflatten(1, (-1, 8)), up.unflatten(1, (-1, 8))], 2).flatten(1, 3)
+    ids = torch.repeat_interleave(torch.arange(experts), torch.tensor(counts))[torch.randperm(tokens, generator=torch.Generator().manual_seed(6))]
+    ids = ids.to(torch.int32).to(DEV)[:, None].contiguous()
+    weights = _randn(tokens, 1, seed=7).abs()
+    got = ops.moe_experts(x, first.contiguous(), down, ids, weights, mode, 1.2, 1.702, mode != "relu_squared",
+                          torch.empty(tokens, hidden, dtype=dtype, device=DEV))
+    e = ids[:, 0].long()
+    each = lambda a, w: torch.cat([(a[i:i + 64].double()[:, None] @ w[e[i:i + 64]].double().mT)[:, 0] for i in range(0, tokens, 64)])
+    u, g = each(x, up), each(x, gate)
+    if mode == "relu_squared":
+        h = torch.relu(u).square()
+    else:
+        g, u = g.clamp(max=1.2), u.clamp(-1.2, 1.2)
+        h = g * torch.sigmoid(1.702 * g) * (u + 1)
+    want = each(h.bfloat16(), down) * weights.double()
+    torch.testing.assert_close(got.double(), want, **_tol(dtype))
+    assert ops.gemm_error_flag(DEV) == 0
+
+
 def test_router_gives_every_row_an_expert_whatever_it_holds():
     """A row of padding may hold anything (what an attention that found no work left in its output): NaN and
     infinities still choose experts inside the table, so that nothing behind the router reads out of bounds."""
