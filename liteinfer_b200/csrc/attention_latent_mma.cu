@@ -20,8 +20,9 @@
 // once), either as two blocks of eight warps per SM (rounds of 32 keys, two stages) or as one block of sixteen
 // warps (rounds of 64 keys from five stages of 32), their keys split over `num_splits`
 // blocks whose partial results (normalised, with the logarithm of their denominators) a second kernel merges,
-// sink included.  Sequences that bring more run with MT = 4, KT = 32 and three stages: four consecutive queries
-// share every tile of keys.
+// sink included.  Sequences that bring more run on the kernel of attention_latent_tcgen05.cuh where it takes
+// their sizes, else with MT = 4, KT = 32 and three stages: four consecutive queries share every tile of keys.
+#include "attention_latent_tcgen05.cuh"
 #include "attention_mma.cuh"
 #include "tcgen05.cuh"
 
@@ -616,7 +617,25 @@ LI_EXPORT int li_latent_attention_mma(const void* q_lat, long q_lat_head_stride,
   if (!aligned16(q_lat) || !aligned16(pool) || (q_lat_token_stride % 8) || (q_lat_head_stride % 8) || (out_token_stride % 2) ||
       (out_head_stride % 2))
     return LI_ERR_ALIGNMENT;
-  if (max_q_len != 1) num_splits = 1;
+  if (max_q_len != 1) {
+    latent_tc::Params t;
+    t.q_lat = (const bf16*)q_lat; t.q_lat_head_stride = q_lat_head_stride; t.q_lat_token_stride = q_lat_token_stride;
+    t.q_raw = (const bf16*)q_raw; t.q_raw_token_stride = q_raw_token_stride; t.q_raw_head_stride = q_raw_head_stride;
+    t.q_rot_off = q_rot_off; t.out = (bf16*)out; t.out_head_stride = out_head_stride; t.out_token_stride = out_token_stride;
+    t.block_table = block_table; t.table_stride = table_stride; t.query_start_loc = query_start_loc;
+    t.context_lens = context_lens; t.seq_index = seq_index; t.inv_freq = inv_freq; t.sink = sink; t.heads = heads;
+    t.rot_dims = rot_dims; t.page_size = page_size; t.page_shift = 0; t.num_pages = num_pages;
+    while ((1 << t.page_shift) < page_size) ++t.page_shift;
+    t.scale_log2 = scale * kLog2e; t.window = window; t.cs_scale = cos_sin_scale; t.error_flag = error_flag;
+    CUtensorMap map;
+    if (latent_tc::takes(t, pool, num_seqs, max_q_len, kv_rank, rot_dim) &&
+        latent_tc::make_entry_map(&map, pool, (long)num_pages * page_size, page_size < 32 ? page_size : 32, kv_rank + rot_dim)) {
+      if (kv_rank == 128) return latent_tc::launch<128>(t, map, num_seqs, max_q_len, stream);
+      if (kv_rank == 256) return latent_tc::launch<256>(t, map, num_seqs, max_q_len, stream);
+      return latent_tc::launch<512>(t, map, num_seqs, max_q_len, stream);
+    }
+    num_splits = 1;
+  }
   if (num_splits > kMaxSplits) num_splits = kMaxSplits;
   if (num_splits > 1 && (!partial_out || !partial_lse)) return LI_ERR_UNSUPPORTED;
   LatentParams p;

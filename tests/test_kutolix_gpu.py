@@ -227,6 +227,37 @@ def test_latent_window_on_tensor_cores(heads, c, r, page, window):
     assert ops.gemm_error_flag(DEV) == 0
 
 
+@pytest.mark.parametrize("heads,c,dims,page,window", [(16, 512, 64, 16, 0), (16, 512, 64, 64, 70), (8, 512, 40, 32, 33), (128, 512, 64, 16, 0),
+                                                      (24, 256, 64, 16, 31), (12, 256, 0, 64, 0), (33, 128, 64, 32, 100), (7, 512, 64, 16, 0)])
+def test_latent_prompts_by_rows_of_128(heads, c, dims, page, window):
+    """Prompts in tiles of 128 rows (128 // heads queries): one query less and more than a tile, contexts that end on both
+    sides of a tile of 32 keys, unwritten slots and pages behind the window that hold NaN, parts that do not turn; seven
+    heads stay on the tiles of four queries.  Probabilities are bfloat16: 2^-8 of a sum of values of size one."""
+    from liteinfer_b200 import ops
+
+    dtype, d, r, q = torch.bfloat16, 8, 64, 128 // heads
+    query_lens = [2, q + 1, max(2, q - 1), 3 * q + 2, 2, 70]
+    context_lens = [2, q + 32, max(2, q - 1) + 31, 3 * q + 2, 129, 70 + 3 * page]
+    pages = sum(-(-n // page) for n in context_lens) + 3
+    table, qsl, ctxl, pool, q_lat, q_raw = _attention_inputs(dtype, heads, c, r, d, query_lens, context_lens, page, pages, 7)
+    for s, (n, total) in enumerate(zip(query_lens, context_lens)):
+        if total % page:
+            pool[int(table[s, total // page]), 0, total % page:] = float("nan")
+        gone = max(0, total - n - window + 1) // page if window else 0
+        if gone:
+            pool[table[s, :gone].long()] = float("nan")
+            table[s, :gone] = -1
+    inv_freq = (1000.0 ** (-torch.arange(dims // 2, dtype=torch.float64) * 2 / max(dims, 1))).float().to(DEV)
+    sinks = _randn(heads, seed=9)
+    common = (q_lat, q_raw, d + r, d)
+    rest = (pool, table, qsl, ctxl, inv_freq, sinks, len(query_lens), 70, heads, c, r, dims, 0.09)
+    want = ref.latent_attention(*common, torch.empty_like(q_lat), *rest, window=window, cos_sin_scale=0.9)
+    for plan in (None, _plan(query_lens, context_lens)):
+        got = ops.latent_attention(*common, torch.full_like(q_lat, 7.0), *rest, plan=plan, window=window, cos_sin_scale=0.9)
+        torch.testing.assert_close(got.float(), want.float(), **_tol(dtype))
+    assert ops.gemm_error_flag(DEV) == 0
+
+
 @pytest.mark.parametrize("dtype,c,r", [(torch.float32, 48, 8), (torch.bfloat16, 48, 8), (torch.bfloat16, 64, 32)])
 @pytest.mark.parametrize("decode", [False, True])
 def test_latent_key_just_inside_and_just_outside_the_window(dtype, c, r, decode):
