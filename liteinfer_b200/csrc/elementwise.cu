@@ -218,8 +218,10 @@ __global__ void act_mul_kernel(const T* __restrict__ gate_up, T* __restrict__ ou
 template <typename T>
 __global__ void act_mul_vec_kernel(const T* __restrict__ gate_up, T* __restrict__ out, size_t rows, int width, int act,
                                    float limit, float alpha) {
-  grid_launch_dependents();
-  grid_dependency_wait();
+  if (sizeof(T) == 4) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+  }
   constexpr int N = Vec16<T>::N;
   const int vec_per_row = width / N;
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -257,8 +259,6 @@ __global__ void act_mul_interleaved_kernel(const T* __restrict__ gate_up, T* __r
 // up values behind them.
 __global__ void act_mul_interleaved_vec_kernel(const bf16* __restrict__ gate_up, bf16* __restrict__ out, size_t rows,
                                                int width, int act, float limit, float alpha) {
-  grid_launch_dependents();
-  grid_dependency_wait();
   const int groups = width / 8;
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t n = rows * (size_t)groups, stride = (size_t)gridDim.x * blockDim.x;
@@ -315,8 +315,12 @@ int launch_act_mul(const void* gate_up, void* out, size_t rows, int width, int a
   constexpr int N = Vec16<T>::N;
   if (width % N == 0 && aligned16(gate_up) && aligned16(out)) {
     const size_t n = rows * (size_t)(width / N);
-    return (int)launch_pdl((long)rows, act_mul_vec_kernel<T>, dim3(grid_for(n, 256)), dim3(256), 0, s, (const T*)gate_up, (T*)out,
-                           rows, width, act, limit, alpha);
+    // Early in the 32-bit path only, where it was shown to help; a bfloat16 decode step of twelve at the 1B sizes, whose
+    // activations also started early, took 869 us where it had taken 859 (B200).
+    if (sizeof(T) == 4)
+      return (int)launch_pdl((long)rows, act_mul_vec_kernel<T>, dim3(grid_for(n, 256)), dim3(256), 0, s, (const T*)gate_up, (T*)out,
+                             rows, width, act, limit, alpha);
+    act_mul_vec_kernel<T><<<grid_for(n, 256), 256, 0, s>>>((const T*)gate_up, (T*)out, rows, width, act, limit, alpha);
   } else {
     act_mul_kernel<T><<<grid_for(rows * (size_t)width, 256), 256, 0, s>>>((const T*)gate_up, (T*)out, rows, width, act, limit,
                                                                           alpha);
@@ -471,8 +475,8 @@ LI_EXPORT int li_act_mul_interleaved(int dtype, const void* gate_up, void* out, 
     act_mul_interleaved_kernel<float><<<grid_for(n, 256), 256, 0, stream>>>((const float*)gate_up, (float*)out, rows,
                                                                             width, act, limit, alpha);
   else if (aligned16(gate_up) && aligned16(out))
-    return (int)launch_pdl((long)rows, act_mul_interleaved_vec_kernel, dim3(grid_for(n / 8, 256)), dim3(256), 0, stream,
-                           (const bf16*)gate_up, (bf16*)out, rows, width, act, limit, alpha);
+    act_mul_interleaved_vec_kernel<<<grid_for(n / 8, 256), 256, 0, stream>>>((const bf16*)gate_up, (bf16*)out, rows,
+                                                                             width, act, limit, alpha);
   else
     act_mul_interleaved_kernel<bf16><<<grid_for(n, 256), 256, 0, stream>>>((const bf16*)gate_up, (bf16*)out, rows,
                                                                           width, act, limit, alpha);
