@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) gemm_simt_tile_kernel(SimtPro
 // (3.3 TB/s).  On the 64 x 64 tiles, a dozen blocks that waited for every 16 k, these took 55, 140, 99 and 252 us.
 constexpr int kRowStride = kChunk + 4;     // 16-byte reads of 32 rows at the same k: off the banks' period
 constexpr int kRowsN = 64;
-constexpr int kMostCluster = 8, kMostChunks = 4, kMostRounds = 4;
+constexpr int kMostCluster = 8, kMostChunks = 4, kMostEach = 16;     // blocks along k, chunks of a block at a time, chunks of a block
 
 // Grid: (64 rows of w) x cluster, R * G rows of x, batch.  Block: `chunks` chunks of G warps, `rounds` times.
 template <int R, int G>
@@ -227,17 +227,40 @@ __global__ void __launch_bounds__(32 * kMostChunks * G) gemm_simt_rows_kernel(Si
   cluster.sync();        // nobody leaves while another block reads its sums
 }
 
+// How a block walks its share of `each` chunks: as many at a time as its shared memory holds beside the sums of all of them.
+struct RowsPlan {
+  int chunks, rounds;
+  size_t smem;
+};
+constexpr size_t kMostSmem = 227 * 1024;
+constexpr RowsPlan rows_plan(int each, int rows) {
+  RowsPlan plan = {};
+  for (int most = kMostChunks; most > 0; --most) {
+    plan.rounds = (each + most - 1) / most;
+    plan.chunks = (each + plan.rounds - 1) / plan.rounds;
+    plan.smem = sizeof(float) * plan.chunks * (size_t)(kRowsN * kRowStride + rows * (kChunk + plan.rounds * kRowsN));
+    if (plan.smem <= kMostSmem) break;
+  }
+  return plan;
+}
+constexpr bool every_plan_fits(int rows) {
+  for (int each = 1; each <= kMostEach; ++each)
+    if (rows_plan(each, rows).smem > kMostSmem) return false;
+  return true;
+}
+
 template <int R, int G>
 int launch_rows(const SimtProduct& p, int batch, cudaStream_t stream) {
+  static_assert(every_plan_fits(R * G), "a k that the narrow kernel is chosen for and that its shared memory does not hold");
   const int all_chunks = (p.K + kChunk - 1) / kChunk;
-  const int each = (all_chunks + kMostCluster - 1) / kMostCluster;          // chunks of a block
-  const int rounds = (each + kMostChunks - 1) / kMostChunks, chunks = (each + rounds - 1) / rounds;
+  const RowsPlan plan = rows_plan((all_chunks + kMostCluster - 1) / kMostCluster, R * G);
+  const int rounds = plan.rounds, chunks = plan.chunks;
   const int ranks = (all_chunks + rounds * chunks - 1) / (rounds * chunks);
-  const size_t smem = (size_t)chunks * (kRowsN * kRowStride + R * G * (kChunk + rounds * kRowsN)) * sizeof(float);
+  const size_t smem = plan.smem;
   const long blocks = (long)((p.N + kRowsN - 1) / kRowsN) * ranks, groups = (p.M + R * G - 1) / (R * G);
   if (blocks > 0x7fffffffL || groups > 65535 || batch > 65535) return LI_ERR_UNSUPPORTED;
   const cudaError_t status =
-      cudaFuncSetAttribute(gemm_simt_rows_kernel<R, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      cudaFuncSetAttribute(gemm_simt_rows_kernel<R, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostSmem);
   if (status != cudaSuccess) return (int)status;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3((unsigned)blocks, (unsigned)groups, batch);
@@ -287,7 +310,7 @@ int launch_product(int dtype, const SimtProduct& p, int batch, cudaStream_t stre
   const bool vec = p.K % 4 == 0 && p.ldx % 4 == 0 && p.x_batch % 4 == 0 && p.w_batch % 4 == 0 &&
                    reinterpret_cast<uintptr_t>(p.x) % four == 0 && reinterpret_cast<uintptr_t>(p.w) % four == 0;
   const float small = tiles_cost(p, batch, 32), large = tiles_cost(p, batch, 128);
-  if (dtype == kFloat32 && vec && p.K > 0 && p.M <= kMostRows && p.K <= kMostRounds * kMostChunks * kMostCluster * kChunk &&
+  if (dtype == kFloat32 && vec && p.K > 0 && p.M <= kMostRows && p.K <= kMostEach * kMostCluster * kChunk &&
       batch <= 65535 && rows_cost(p, batch) < fminf(small, large)) {
     if (p.M == 1) return launch_rows<1, 1>(p, batch, stream);
     if (p.M <= 4) return launch_rows<4, 1>(p, batch, stream);

@@ -96,8 +96,8 @@ def test_gemm_simt_rows_do_not_depend_on_the_batch():
     assert torch.equal(full[33:34], one)
 
 
-# One chunk of k and part of one; several in a cluster of odd size; several a block; the narrow kernel's last size and the
-# first beyond it; a k that is not a multiple of four.
+# One chunk of k and part of one; several in a cluster of odd size; four a block and the first k beyond that; eight; a k that is
+# not a multiple of four.
 @pytest.mark.parametrize("N,K", [(33, 40), (100, 128), (1000, 772), (64, 1024), (96, 2052), (65, 4096), (40, 4100), (65, 8196), (70, 301)])
 def test_gemm_simt_widths_agree_bit_for_bit(N, K):
     from liteinfer_b200 import ops
@@ -117,6 +117,23 @@ def test_gemm_simt_widths_agree_bit_for_bit(N, K):
         for i in range(2):
             one = ops.gemm_simt(wide[i, :, 4:K + 4].contiguous(), (i + 1) * w, torch.empty(17, N, device="cuda"))
             assert torch.equal(batched[i], one)
+
+
+# As many rows as the narrow kernel takes at once and one more, at a k that is the last of twelve chunks a block, the first of
+# thirteen, between, the narrow kernel's last and the first beyond it.
+@pytest.mark.parametrize("K", [12288, 12292, 14336, 16384, 16388])
+def test_gemm_simt_of_a_deep_k(K):
+    from liteinfer_b200 import ops
+
+    N = 130
+    x, w = _randn(256, K, dtype=torch.float32), _randn(N, K, dtype=torch.float32, seed=1)
+    full = ops.gemm_simt(x, w, torch.empty(256, N, device="cuda"))
+    # Chains of at most 128 products and then the chunks' sums, each rounding by 2^-24 of what it has.
+    bound = (x.double().abs() @ w.double().abs().t()) * (128 + -(-K // 128)) * 2.0 ** -24
+    assert bool(((full.double() - x.double() @ w.double().t()).abs() <= bound).all())
+    for M in (1, 4, 8, 12, 13, 16, 17, 48, 255):
+        part = ops.gemm_simt(x[1:1 + M].contiguous(), w, torch.empty(M, N, device="cuda"))
+        assert torch.equal(part, full[1:1 + M]), M
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 3072, 2048), (8, 2048, 8192), (64, 1000, 96), (300, 512, 64), (2048, 256, 2048)])
