@@ -154,9 +154,9 @@ _SIGNATURES = {
     "li_gemm_stream_supports": ("gemm_stream", [c_int, c_int, c_int]),
     "li_gemm_tcgen05": ("gemm_tcgen05", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float,
                                          c_void_p, c_void_p]),
-    "li_gemm_simt": ("gemm_simt", [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
+    "li_gemm_simt": ("gemm_simt", [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
     "li_gemm_simt_batched": ("gemm_simt", [c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
-                                           c_int, c_long, c_long, c_long, c_void_p]),
+                                           c_int, c_long, c_long, c_long, c_int, c_void_p]),
     "li_activation": ("elementwise", [c_int, c_void_p, c_void_p, c_size_t, c_int, c_void_p]),
     "li_embedding_streams": ("stream_mix", [c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int,
                                             c_void_p, c_void_p]),
@@ -346,6 +346,17 @@ class beside:
 
 def _ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
+
+
+def at_rest(t: torch.Tensor) -> torch.Tensor:
+    """Says of `t` that no kernel writes it from here on (a model's parameter): a float32 product may then read it, as its
+    weight, before the kernel ahead in the stream is done.  Of the tensor object alone: its views are as any other tensor."""
+    t.at_rest = True
+    return t
+
+
+def _at_rest(t: torch.Tensor) -> int:
+    return int(getattr(t, "at_rest", False))
 
 
 def _int32(t: torch.Tensor | None, what: str) -> None:
@@ -543,7 +554,9 @@ def linear(x: "torch.Tensor | PendingNorm", weight: torch.Tensor, out: torch.Ten
     float32 runs the FFMA kernel (a true 32-bit product: tensor cores have no such
     mode).  bfloat16 hands the product to the library GEMM, as the reference's
     `nn.Linear` does (liteinfer/models/llama.py:108-110,137-140), with 32-bit
-    accumulation, except for a handful of rows, which the weight-streaming kernel takes.
+    accumulation, except for a handful of rows, which the weight-streaming kernel takes.  That kernel asks for its
+    weight before the kernel ahead in the stream is done, whatever the weight is; the float32 one only where the weight
+    is `at_rest`.
 
     `x` may be a `PendingNorm`: the weight-streaming kernel then normalises on its way in; any other path runs
     the norm first.  With `residual` [M, N] the weight-streaming kernel adds its result into it
@@ -574,7 +587,7 @@ def linear(x: "torch.Tensor | PendingNorm", weight: torch.Tensor, out: torch.Ten
     assert out is None or (out.shape == (M, N) and out.dtype == x.dtype)
     if x.dtype == torch.float32:
         _check(_fn("li_gemm_simt")(0, x.data_ptr(), weight.data_ptr(), _ptr(bias), out.data_ptr(), M, N, K,
-                                   _stream()), "gemm_simt")
+                                   _at_rest(weight), _stream()), "gemm_simt")
         return out if activation is None else _unary(out, out, activation)
     if fused:
         return _skinny(x, weight, out, bias, -1 if activation is None else UNARY_ACT_BASE + UNARY_ACTIVATIONS[activation],
@@ -720,7 +733,7 @@ def gemm_simt(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, bias: to
     N = weight.shape[0]
     assert weight.shape[1] == K and out.shape == (M, N) and x.dtype == weight.dtype == out.dtype
     _check(_fn("li_gemm_simt")(_code(x), x.data_ptr(), weight.data_ptr(), _ptr(bias), out.data_ptr(), M, N, K,
-                               _stream()), "gemm_simt")
+                               _at_rest(weight), _stream()), "gemm_simt")
     return out
 
 
@@ -1821,7 +1834,7 @@ def batched_linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> 
         return out
     if x.dtype == torch.float32:
         _check(_fn("li_gemm_simt_batched")(0, x.data_ptr(), weight.data_ptr(), out.data_ptr(), M, N, K, B, x.stride(1),
-                                           N, x.stride(0), N * K, M * N, _stream()), "gemm_simt_batched")
+                                           N, x.stride(0), N * K, M * N, _at_rest(weight), _stream()), "gemm_simt_batched")
         return out
     torch.bmm(x, weight.transpose(1, 2), out=out)
     return out

@@ -32,6 +32,17 @@ from liteinfer_b200.parts.context import LayerCache, StepContext
 from liteinfer_b200.parts.registry import BLOCKS, build_part
 from liteinfer_b200.parts.spec import ModelSpec, TensorSpec
 
+
+def _held_by(part):
+    """The tensors that a part keeps, and those of parts inside it."""
+    for value in vars(part).values():
+        for one in value if isinstance(value, (list, tuple)) else (value,):
+            if isinstance(one, torch.Tensor):
+                yield one
+            elif hasattr(one, "tensor_specs"):
+                yield from _held_by(one)
+
+
 def _settled(hidden: torch.Tensor, delta, copies: int | None = None) -> torch.Tensor:
     """A copy of the residual stream with the pending delta added (for `StepContext.layer_trace`); of a residual
     kept as several streams, their sum."""
@@ -114,6 +125,8 @@ class Model:
         """Hand every part its tensors (by checkpoint name, already on the device)."""
         for prefix, part, renames in self._named_parts():
             part.bind({local: tensors[prefix + renames.get(local, local)] for local in part.tensor_specs()})
+            for value in _held_by(part):
+                ops.at_rest(value)
 
     @property
     def graph_safe(self) -> bool:

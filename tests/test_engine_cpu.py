@@ -290,3 +290,31 @@ def test_steps_launched_ahead_give_the_same_outputs(cpu_kernels, model_dirs):
     assert runs[1][0][0] == free[0][:1] and runs[1][0][1] == "stop"
     assert runs[1][3][1] == "length" and len(prompts[3]) + len(runs[1][3][0]) == 48
     assert all(-1 not in tokens for tokens, _, _ in runs[1])
+
+
+@pytest.mark.parametrize("family,name", [("tiny", "tiny_a"), ("gifudra", "gif_a"), ("karupel", "kar_a"), ("kegizen", "keg_a"),
+                                         ("kutolix", "kut_a"), ("lulisun", "lul_a"), ("sogazen", "sog_a")])
+def test_every_weight_of_a_product_is_at_rest(cpu_kernels, monkeypatch, tmp_path, family, name):
+    """What a bound model multiplies by may be read before the kernel ahead is done; a computed operand, or a view, may not."""
+    import importlib
+
+    from liteinfer_b200 import LLM, SamplingParams, ops
+    from liteinfer_b200.weights.random_init import write_random_model
+
+    config, seed, page = importlib.import_module(f"{family}_configs").ALL[name]
+    seen = []
+
+    def watched(product):
+        def run(x, weight, *args, **kwargs):
+            seen.append(weight)
+            return product(x, weight, *args, **kwargs)
+        return run
+
+    monkeypatch.setattr(ops, "linear", watched(ops.linear))
+    monkeypatch.setattr(ops, "batched_linear", watched(ops.batched_linear))
+    with LLM(str(write_random_model(config, tmp_path / name, seed)), dtype="float32", device="cpu", block_size=page,
+             max_num_seqs=2, max_model_len=64) as llm:
+        llm.generate(_prompts(config["vocab_size"] if family == "tiny" else 40, (9, 2)),
+                     SamplingParams(temperature=0.0, max_tokens=2, ignore_eos=True))
+    assert seen and all(ops.kernels._at_rest(w) for w in seen)
+    assert not ops.kernels._at_rest(torch.zeros(2, 2)) and not ops.kernels._at_rest(seen[0][:1])

@@ -136,6 +136,28 @@ def test_gemm_simt_of_a_deep_k(K):
         assert torch.equal(part, full[1:1 + M]), M
 
 
+@pytest.mark.parametrize("N,K", [(512, 256), (4096, 1024), (1000, 4096)])
+def test_a_second_operand_that_the_kernel_just_ahead_writes(N, K):
+    """The activation ahead lets the next kernel start while it still runs; what it writes is read behind it all the same."""
+    from liteinfer_b200 import ops
+
+    x, pairs = _randn(12, K, dtype=torch.float32), [_randn(N, 2 * K, dtype=torch.float32, seed=1 + i) for i in range(2)]
+    want = []
+    for pair in pairs:
+        y = ops.act_mul(pair, torch.empty(N, K, device="cuda"), "silu")
+        torch.cuda.synchronize()
+        want.append(ops.gemm_simt(x, y, torch.empty(12, N, device="cuda")))
+    torch.cuda.synchronize()
+    products = (ops.gemm_simt, ops.linear,
+                lambda a, b, out: ops.batched_linear(a[None], b[None], out[None])[0])
+    y, got = torch.empty(N, K, device="cuda"), []
+    for i in range(12):                 # y holds the other weights until the kernel ahead has written it
+        ops.act_mul(pairs[i % 2], y, "silu")
+        got.append(products[i % 3](x, y, torch.empty(12, N, device="cuda")))
+    for i, out in enumerate(got):
+        assert torch.equal(out, want[i % 2]), i
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 3072, 2048), (8, 2048, 8192), (64, 1000, 96), (300, 512, 64), (2048, 256, 2048)])
 def test_linear_bfloat16(M, N, K):
     from liteinfer_b200 import ops
