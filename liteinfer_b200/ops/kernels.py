@@ -304,7 +304,9 @@ class beside:
     """Within this context the kernels of this module (and library products) go to a second stream, with scratch of their
     own, behind what the current stream holds so far; the next `join` on the current stream waits for them.  Two runs of
     kernels that do not depend on one another share the device that way, in eager steps and inside a captured graph alike.
-    Tensors: what the second stream reads must stay alive until the join, and what it makes is used behind the join."""
+    Tensors: what the second stream reads must stay alive until the join, and what it makes is used behind the join.  An
+    exception within the context joins on its way out; whoever runs code between the context and the join joins in a
+    `finally`, so that nothing of a step that failed is still under way unnoticed."""
 
     _streams: dict[torch.device, "torch.cuda.Stream"] = {}
     _open: set[torch.device] = set()        # devices whose second stream holds work that nobody has joined yet
@@ -337,11 +339,15 @@ class beside:
         _lane = 0
         for context in reversed(self.entered):
             context.__exit__(*exc)
+        if exc and exc[0] is not None:
+            self.join()
         return False
 
     def join(self) -> None:
-        torch.cuda.current_stream(self.device).wait_stream(self.stream)
-        beside._open.discard(self.device)
+        try:
+            torch.cuda.current_stream(self.device).wait_stream(self.stream)
+        finally:
+            beside._open.discard(self.device)
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:
@@ -1176,6 +1182,7 @@ def paged_attention(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_poo
     if plan is None:
         return paged_attention_mma(*common, None, num_seqs, max_q_len, heads, kv_heads, head_dim, scale, window,
                                    **options)
+
     def single_tokens():
         bound = min(plan.max_decode_context_len, reach) if reach else plan.max_decode_context_len
         streaming = not (keep_first > 0 and window > 0) and stream_attention_supports(q.dtype, heads, kv_heads, head_dim, page_size)
@@ -1183,21 +1190,26 @@ def paged_attention(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_poo
         paged_attention_mma(*common, plan.decode_seqs, plan.num_decode, 1, heads, kv_heads, head_dim, scale,
                             window, splits, newest, streaming, **options)
 
-    lane = None
-    if plan.num_prefill and plan.num_decode and plan.max_prefill_query_len <= MIXED_BESIDE_TOKENS and beside.is_free(out.device):
-        lane = beside(out.device)
-        with lane:
-            single_tokens()
-    if plan.num_prefill:
+    def portions():
         if tcgen05_attention_supports(q.dtype, heads, kv_heads, head_dim, page_size) and not MASKED_ON_MMA:
             paged_attention_tcgen05(*common, plan.prefill_seqs, plan.num_prefill, plan.max_prefill_query_len, heads,
                                     kv_heads, head_dim, scale, window, **options)
         else:
             paged_attention_mma(*common, plan.prefill_seqs, plan.num_prefill, plan.max_prefill_query_len, heads,
                                 kv_heads, head_dim, scale, window, **options)
-    if lane is not None:
-        lane.join()
-    elif plan.num_decode:
+
+    if plan.num_prefill and plan.num_decode and plan.max_prefill_query_len <= MIXED_BESIDE_TOKENS and beside.is_free(out.device):
+        lane = beside(out.device)
+        with lane:
+            single_tokens()
+        try:
+            portions()
+        finally:
+            lane.join()
+        return out
+    if plan.num_prefill:
+        portions()
+    if plan.num_decode:
         single_tokens()
     return out
 

@@ -109,8 +109,10 @@ class ParallelNormsBlock:
             lane = ops.beside(hidden.device)
             with lane:
                 fed = self._sum(self.feed_forward, self.feed_forward.forward(also, ctx))
-            mixed = self._sum(self.mixer, self.mixer.forward(normed, ctx, cache))
-            lane.join()
+            try:
+                mixed = self._sum(self.mixer, self.mixer.forward(normed, ctx, cache))
+            finally:
+                lane.join()
             return hidden, mixed + fed
         mixed = self._sum(self.mixer, self.mixer.forward(normed, ctx, cache))
         return hidden, mixed + self._sum(self.feed_forward, self.feed_forward.forward(also, ctx))

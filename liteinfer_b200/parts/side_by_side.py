@@ -130,8 +130,10 @@ class SideBySide:
             lane = ops.beside(proj.device)
             with lane:
                 second = term(1)
-            first = term(0)
-            lane.join()
+            try:
+                first = term(0)
+            finally:
+                lane.join()
             return ops.SumDelta((first, second))
         return ops.SumDelta(tuple(term(i) for i in range(len(self.members))))
 
