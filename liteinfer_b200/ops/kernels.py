@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from ctypes import c_float, c_int, c_long, c_longlong, c_size_t, c_void_p
 
 from dataclasses import dataclass
@@ -207,11 +208,20 @@ def _check(code: int, name: str) -> None:
     raise KernelLibraryError(f"{name}: CUDA error {code} at launch")
 
 
-_pinned_stream: int | None = None
+class _Here(threading.local):
+    """Where a thread's launches go.  Of each thread its own: a step that another thread runs meanwhile, on a stream of its
+    own or the common one, neither follows this one's to the second stream nor takes that one's scratch."""
+
+    stream: int | None = None       # None: the current one, asked for at every launch
+    lane = 0                        # whose scratch the launches use: 0, or 1 within `beside`
+
+
+_here = _Here()
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream if _pinned_stream is None else _pinned_stream
+    pinned = _here.stream
+    return torch.cuda.current_stream().cuda_stream if pinned is None else pinned
 
 
 class on_current_stream:
@@ -220,14 +230,12 @@ class on_current_stream:
     was a noticeable part of a step's host time).  Contexts nest; leave the stream alone inside."""
 
     def __enter__(self):
-        global _pinned_stream
-        self.before = _pinned_stream
-        _pinned_stream = torch.cuda.current_stream().cuda_stream if torch.cuda.is_available() else None
+        self.before = _here.stream
+        _here.stream = torch.cuda.current_stream().cuda_stream if torch.cuda.is_available() else None
         return self
 
     def __exit__(self, *exc):
-        global _pinned_stream
-        _pinned_stream = self.before
+        _here.stream = self.before
         return False
 
 
@@ -276,7 +284,7 @@ class _Scratch:
 
 
 _scratch: dict[tuple[torch.device, int], _Scratch] = {}
-_lane = 0           # whose scratch the launches use: 0, or 1 within `beside`
+_lock = threading.Lock()        # of what the threads share: the scratch and the second streams
 
 
 def normalise_device(device: torch.device | str) -> torch.device:
@@ -289,14 +297,15 @@ def normalise_device(device: torch.device | str) -> torch.device:
 
 
 def scratch_for(device: torch.device | str) -> _Scratch:
-    device = normalise_device(device)
-    found = _scratch.get((device, _lane))
-    if found is None:       # (the error flags are one set for all)
-        errors = _scratch[device, 0].errors if (device, 0) in _scratch else None
-        found = _scratch[device, _lane] = _Scratch(device, errors)
-        for lane in (0, 1):
-            if lane != _lane and (device, lane) not in _scratch:
-                _scratch[device, lane] = _Scratch(device, found.errors)
+    device, lane = normalise_device(device), _here.lane
+    found = _scratch.get((device, lane))
+    if found is None:
+        with _lock:             # (the error flags are one set for all)
+            if (device, 0) not in _scratch:
+                first = _Scratch(device)
+                _scratch[device, 1] = _Scratch(device, first.errors)
+                _scratch[device, 0] = first
+            found = _scratch[device, lane]
     return found
 
 
@@ -306,7 +315,8 @@ class beside:
     kernels that do not depend on one another share the device that way, in eager steps and inside a captured graph alike.
     Tensors: what the second stream reads must stay alive until the join, and what it makes is used behind the join.  An
     exception within the context joins on its way out; whoever runs code between the context and the join joins in a
-    `finally`, so that nothing of a step that failed is still under way unnoticed."""
+    `finally`, so that nothing of a step that failed is still under way unnoticed.  A device has one second stream, whoever
+    uses it: its scratch is that stream's."""
 
     _streams: dict[torch.device, "torch.cuda.Stream"] = {}
     _open: set[torch.device] = set()        # devices whose second stream holds work that nobody has joined yet
@@ -314,29 +324,45 @@ class beside:
     @staticmethod
     def is_free(device: torch.device) -> bool:
         """Whether the second stream holds nothing that is still to be joined: work that is put there would wait for it."""
-        return _lane == 0 and normalise_device(device) not in beside._open
+        return _here.lane == 0 and normalise_device(device) not in beside._open
+
+    @classmethod
+    def claim(cls, device: torch.device) -> "beside | None":
+        """The second stream for one run, if it is free; None if another run, of this thread or of another, holds it."""
+        device = normalise_device(device)
+        with _lock:
+            if not cls.is_free(device):
+                return None
+            cls._open.add(device)
+        try:
+            return cls(device)
+        except BaseException:
+            cls._open.discard(device)
+            raise
 
     def __init__(self, device: torch.device) -> None:
         self.device = normalise_device(device)
-        stream = beside._streams.get(self.device)
-        if stream is None:
-            scratch_for(self.device)        # both lanes' buffers exist before a graph is captured
-            stream = beside._streams[self.device] = torch.cuda.Stream(device=self.device)
-        self.stream = stream
+        scratch_for(self.device)            # both lanes' buffers exist before a graph is captured
+        with _lock:
+            if self.device not in beside._streams:
+                beside._streams[self.device] = torch.cuda.Stream(device=self.device)
+            self.stream = beside._streams[self.device]
 
     def __enter__(self):
-        global _lane
-        self.stream.wait_stream(torch.cuda.current_stream(self.device))
-        self.entered = (torch.cuda.stream(self.stream), on_current_stream())
-        for context in self.entered:
-            context.__enter__()
-        _lane = 1
         beside._open.add(self.device)
+        try:
+            self.stream.wait_stream(torch.cuda.current_stream(self.device))
+            self.entered = (torch.cuda.stream(self.stream), on_current_stream())
+            for context in self.entered:
+                context.__enter__()
+        except BaseException:
+            beside._open.discard(self.device)
+            raise
+        _here.lane = 1
         return self
 
     def __exit__(self, *exc):
-        global _lane
-        _lane = 0
+        _here.lane = 0
         for context in reversed(self.entered):
             context.__exit__(*exc)
         if exc and exc[0] is not None:
@@ -1198,8 +1224,10 @@ def paged_attention(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_poo
             paged_attention_mma(*common, plan.prefill_seqs, plan.num_prefill, plan.max_prefill_query_len, heads,
                                 kv_heads, head_dim, scale, window, **options)
 
-    if plan.num_prefill and plan.num_decode and plan.max_prefill_query_len <= MIXED_BESIDE_TOKENS and beside.is_free(out.device):
-        lane = beside(out.device)
+    lane = None
+    if plan.num_prefill and plan.num_decode and plan.max_prefill_query_len <= MIXED_BESIDE_TOKENS:
+        lane = beside.claim(out.device)
+    if lane is not None:
         with lane:
             single_tokens()
         try:

@@ -3,6 +3,7 @@
 from __future__ import annotations
 
 import contextlib
+import threading
 from types import SimpleNamespace
 
 import pytest
@@ -71,7 +72,7 @@ def test_a_mixed_step_that_fails_joins_its_lane(streams, monkeypatch, failing):
     monkeypatch.setattr(kernels, "tcgen05_attention_supports", lambda *sizes: True)
     monkeypatch.setattr(kernels, "stream_attention_supports", lambda *sizes: True)
     for name in ("paged_attention_mma", "paged_attention_tcgen05"):
-        monkeypatch.setattr(kernels, name, lambda *a, _name=name, **k: (ran.append((_name, kernels._lane)), _name == failing and _fails()))
+        monkeypatch.setattr(kernels, name, lambda *a, _name=name, **k: (ran.append((_name, kernels._here.lane)), _name == failing and _fails()))
     ints = lambda *v: torch.tensor(v, dtype=torch.int32)
     q = torch.zeros(5, 64, dtype=torch.bfloat16)
     out = SimpleNamespace(dtype=q.dtype, device=DEVICE)
@@ -120,3 +121,53 @@ def test_mixers_side_by_side_that_fail_join_their_lane(streams, monkeypatch, fai
     with pytest.raises(RuntimeError, match="planted"):
         mixers._normed(Projection(), None, None)
     assert second in main.waited and ops.beside.is_free(DEVICE)
+
+
+def test_a_thread_does_not_follow_another_to_the_second_stream(streams, monkeypatch):
+    """While one thread's launches go to the second stream, another's stay where they were, with the first lane's scratch,
+    and the second stream is not to be had."""
+    main, second = streams
+    second.cuda_stream = 7
+    current = threading.local()
+    monkeypatch.setattr(torch.cuda, "is_available", lambda: True)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: getattr(current, "stream", main))
+
+    @contextlib.contextmanager
+    def on(stream):
+        current.stream = stream
+        yield
+        current.stream = main
+
+    monkeypatch.setattr(torch.cuda, "stream", on)
+    seen = []
+
+    def other():
+        with kernels.on_current_stream():
+            seen.append((kernels._stream(), kernels._here.lane, ops.beside.claim(DEVICE)))
+
+    lane = ops.beside.claim(DEVICE)
+    assert ops.beside.claim(DEVICE) is None
+    with lane:
+        assert (kernels._stream(), kernels._here.lane) == (7, 1)
+        thread = threading.Thread(target=other)
+        thread.start()
+        thread.join()
+        assert (kernels._stream(), kernels._here.lane) == (7, 1)
+    assert seen == [(0, 0, None)] and (kernels._stream(), kernels._here.lane) == (0, 0)
+    lane.join()
+    assert ops.beside.claim(DEVICE) is not None
+
+
+def test_claims_of_many_threads_are_one(streams):
+    gate, got = threading.Barrier(8), []
+
+    def run():
+        gate.wait()
+        got.append(ops.beside.claim(DEVICE))
+
+    threads = [threading.Thread(target=run) for _ in range(8)]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    assert sum(lane is not None for lane in got) == 1
