@@ -141,8 +141,9 @@ template <int X> constexpr int attn_threads() { return 32 + 32 * X + 128 * X; } 
 // kSplit: two blocks, a cluster, share a block's keys: each walks half of the tiles, the second hands its unnormalised rows to
 // the first through distributed shared memory.  A tile of keys is a chain (product, softmax, product) of some 0.7 us
 // however idle the device is, so a launch of few blocks over long contexts takes as long as its longest block.
-// Measured on B200 (32 heads on 8, head size 64): 509 queries over 1,533 keys 23.6 us against 30.4, 128 over 2,560 22.9 against
-// 34.8; 128 over 128, which are not shared, 7.4 against 7.0.
+// A row's result then depends, in its last bits, on how many blocks the launch has.
+// Measured on B200 (32 heads on 8, head size 64): 509 queries over 1,533 keys 23.5 us against 31.4, 128 over 1,152 15.1 against
+// 19.2, 2 over 1,026 16.8 against 23.4; 24 heads on 8 of size 128: 600 over 1,624 37.6 against 46.7.
 template <int D, int X, bool kOptions, bool kSpans, bool kSplit>
 __global__ void __launch_bounds__(attn_threads<X>(), (D == 64 && X == 1) ? 2 : 1)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -172,7 +173,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
   // Values wider than keys: the blocks of a KV head's parts lie side by side, each with all scores and D of a value's
   // dimensions.
   const int parts = kSpans ? (int)gridDim.x / p.kv_heads : 1;
-  const int kvh = kSpans ? (int)blockIdx.x / parts : kSplit ? (int)blockIdx.x >> 1 : (int)blockIdx.x, part = kSpans ? (int)blockIdx.x - kvh * parts : 0;
+  const int kvh = kSpans ? (int)blockIdx.x / parts : kSplit ? (int)blockIdx.x >> 1 : (int)blockIdx.x;
+  const int part = kSpans ? (int)blockIdx.x - kvh * parts : 0;
   const int q_begin = p.query_start_loc[seq], q_len = p.query_start_loc[seq + 1] - q_begin;
   const int groups = p.heads / p.kv_heads;
   const int tq = kRows / groups;
@@ -201,12 +203,23 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
   const int kept_end = (kOptions && p.window > 0 && p.keep_first > 0) ? min(p.keep_first, lo) : 0;
   const int kept_tiles = min((kept_end + kKeys - 1) / kKeys, tile_lo);
   const int all_tiles = kept_tiles + tile_hi - tile_lo;
-  // A split block's tiles: the first half or the second (few tiles are not split; the second block then has nothing to do).
-  const bool split = kSplit && all_tiles >= kSplitTiles;
-  const int rank = kSplit ? (int)cluster_cta_rank() : 0, first_half = (all_tiles + 1) / 2;
-  if (kSplit && !split && rank > 0) return;
-  const int tile0 = split && rank > 0 ? first_half : 0, ntiles = split ? (rank > 0 ? all_tiles - first_half : first_half) : all_tiles;
-  auto tile_at = [&](int t) { return tile0 + t < kept_tiles ? tile0 + t : tile_lo + tile0 + t - kept_tiles; };
+  // A split block's tiles: the first half or the second (the second of a block that is not split has nothing to do).
+  int tile0 = 0, ntiles = all_tiles;
+  bool split = false;
+  const int rank = kSplit ? (int)cluster_cta_rank() : 0;
+  if constexpr (kSplit) {
+    split = all_tiles >= kSplitTiles;
+    if (!split && rank > 0) return;
+    const int first_half = (all_tiles + 1) / 2;
+    if (split) {
+      tile0 = rank > 0 ? first_half : 0;
+      ntiles = rank > 0 ? all_tiles - first_half : first_half;
+    }
+  }
+  auto tile_at = [&](int t) {
+    if constexpr (kSplit) t += tile0;
+    return t < kept_tiles ? t : tile_lo + t - kept_tiles;
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kKvStages; ++s) {
@@ -310,8 +323,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
   const unsigned tmem_s[2] = {tmem_base + x * 128u, tmem_base + x * 128u + 64u};
   const unsigned tmem_o = tmem_base + X * 128u + x * D;
 
-  float row_m = -INFINITY, row_l = 0.f;      // of a softmax thread's row, at the end of its tiles
-  bool finished = false;
+  [[maybe_unused]] float row_m = -INFINITY, row_l = 0.f;      // kSplit: of a softmax thread's row, at the end of its tiles
+  [[maybe_unused]] bool finished = false;
   if (warp == 0) {
     // ------------------------------------------------------------------ loader
     for (int t = tiles_ahead; t < ntiles; ++t)
@@ -470,89 +483,120 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, const __grid
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full(buf));
     }
-    // The last P V done, the row's sums are complete.
-    finished = ok && ntiles > 0 &&
-               mbar_wait(pv_done((ntiles - 1) & 1), (unsigned)((ntiles - 1) >> 1) & 1, p.error_flag, 19);
-    tcgen05_fence_after();
-    row_m = m;
-    row_l = l;
+    if constexpr (kSplit) {
+      // The last P V done, the row's sums are complete.
+      finished = ok && ntiles > 0 &&
+                 mbar_wait(pv_done((ntiles - 1) & 1), (unsigned)((ntiles - 1) >> 1) & 1, p.error_flag, 19);
+      tcgen05_fence_after();
+      row_m = m;
+      row_l = l;
+    } else {
+      // Output: wait for the last P V, read the row, divide by the row's sum, store.
+      if (ok && ntiles > 0 && mbar_wait(pv_done((ntiles - 1) & 1), (unsigned)((ntiles - 1) >> 1) & 1, p.error_flag, 19)) {
+        tcgen05_fence_after();
+        const int qi = q0 + row / groups, head = kvh * groups + row % groups;
+        // The exponentials were taken against m (unscaled), so the sink's term is too.
+        // (Compiled into the kernel's form with options only, so that the plain form is what it was.)
+        if (kOptions && p.sink != nullptr && row < rows_used) l += exp2f(p.sink[head] * kLog2eF - m * p.scale_log2);
+        const float inv = l > 0.f ? 1.f / l : 0.f;
+        bf16* dst = p.out + (size_t)(q_begin + qi) * p.out_row_stride + (kSpans ? (size_t)head * parts + part : (size_t)head) * D;
+#pragma unroll
+        for (int half = 0; half < D / 32; ++half) {
+          unsigned o[32];
+          __syncwarp();
+          tmem_load32(tmem_o + lane_field + half * 32, o);
+          tmem_load_wait();
+          if (row < rows_used) {
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              unsigned w[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(o[v * 8 + 2 * e]) * inv,
+                                                         __uint_as_float(o[v * 8 + 2 * e + 1]) * inv);
+                w[e] = *reinterpret_cast<unsigned*>(&h);
+              }
+              *reinterpret_cast<uint4*>(dst + half * 32 + v * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+          }
+        }
+      }
+    }
   }
 
   // The second block's rows to the first: [D][128] unnormalised values, the maxima, the sums, over the first block's ring of
   // keys and values, which nobody reads or writes any more once both blocks have arrived.
-  const int quarter = warp & 3, row = quarter * 32 + lane;
-  const unsigned lane_field = (unsigned)(quarter * 32) << 16;
-  constexpr unsigned kPeerBytes = (D + 2) * kRows * 4;
-  static_assert(!kSplit || X * kPeerBytes <= 2 * kKvStages * kTileBytes, "a peer's rows fit the ring");
-  const unsigned peer_rows = k_smem + x * kPeerBytes + (unsigned)row * 4u;
-  if (split) {
-    tcgen05_fence_before();
-    __syncwarp();
-    cluster_sync_all();
-    tcgen05_fence_after();
-    if (rank > 0 && warp > X) {
-      unsigned remote;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(peer_rows), "r"(0));
-      const auto put = [&](int i, float v) {
-        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote + (unsigned)i * (kRows * 4)), "f"(v) : "memory");
-      };
+  if constexpr (kSplit) {
+    const int quarter = warp & 3, row = quarter * 32 + lane;
+    const unsigned lane_field = (unsigned)(quarter * 32) << 16;
+    constexpr unsigned kPeerBytes = (D + 2) * kRows * 4;
+    static_assert(X * kPeerBytes <= 2 * kKvStages * kTileBytes, "a peer's rows fit the ring");
+    const unsigned peer_rows = k_smem + x * kPeerBytes + (unsigned)row * 4u;
+    if (split) {
+      tcgen05_fence_before();
+      __syncwarp();
+      cluster_sync_all();
+      tcgen05_fence_after();
+      if (rank > 0 && warp > X) {
+        unsigned remote;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(peer_rows), "r"(0));
+        const auto put = [&](int i, float v) {
+          asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote + (unsigned)i * (kRows * 4)), "f"(v) : "memory");
+        };
+#pragma unroll
+        for (int half = 0; half < D / 32; ++half) {
+          unsigned o[32];
+          __syncwarp();
+          tmem_load32(tmem_o + lane_field + half * 32, o);
+          tmem_load_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) put(half * 32 + j, finished ? __uint_as_float(o[j]) : 0.f);
+        }
+        put(D, finished ? row_m : -INFINITY);
+        put(D + 1, finished ? row_l : 0.f);
+      }
+      __syncwarp();
+      cluster_sync_all();
+    }
+    // Output: read the row, divide by the row's sum, store.
+    if (warp > X && finished && rank == 0) {
+      const int qi = q0 + row / groups, head = kvh * groups + row % groups;
+      float l = row_l, own = 1.f, other = 0.f;
+      const float* peer = reinterpret_cast<const float*>(generic_base + (peer_rows - base));
+      if (split) {
+        const float peer_m = peer[D * kRows], m = fmaxf(row_m, peer_m);
+        own = row_m == -INFINITY ? 0.f : ex2((row_m - m) * p.scale_log2);
+        other = peer_m == -INFINITY ? 0.f : ex2((peer_m - m) * p.scale_log2);
+        l = row_l * own + peer[(D + 1) * kRows] * other;
+      }
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      own *= inv;
+      other *= inv;
+      bf16* dst = p.out + (size_t)(q_begin + qi) * p.out_row_stride + (size_t)head * D;
 #pragma unroll
       for (int half = 0; half < D / 32; ++half) {
         unsigned o[32];
         __syncwarp();
         tmem_load32(tmem_o + lane_field + half * 32, o);
         tmem_load_wait();
+        if (split) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) put(half * 32 + j, finished ? __uint_as_float(o[j]) : 0.f);
-      }
-      put(D, finished ? row_m : -INFINITY);
-      put(D + 1, finished ? row_l : 0.f);
-    }
-    __syncwarp();
-    cluster_sync_all();
-  }
-  // Output: read the row, divide by the row's sum, store.
-  if (warp > X && finished && rank == 0) {
-    const int qi = q0 + row / groups, head = kvh * groups + row % groups;
-    float m = row_m, l = row_l, own = 1.f, other = 0.f;
-    const float* peer = reinterpret_cast<const float*>(generic_base + (peer_rows - base));
-    if (split) {
-      const float peer_m = peer[D * kRows];
-      m = fmaxf(row_m, peer_m);
-      own = row_m == -INFINITY ? 0.f : ex2((row_m - m) * p.scale_log2);
-      other = peer_m == -INFINITY ? 0.f : ex2((peer_m - m) * p.scale_log2);
-      l = row_l * own + peer[(D + 1) * kRows] * other;
-    }
-    // The exponentials were taken against m (unscaled), so the sink's term is too.
-    // (Compiled into the kernel's form with options only, so that the plain form is what it was.)
-    if (kOptions && p.sink != nullptr && row < rows_used) l += exp2f(p.sink[head] * kLog2eF - m * p.scale_log2);
-    const float inv = l > 0.f ? 1.f / l : 0.f;
-    own *= inv;
-    other *= inv;
-    bf16* dst = p.out + (size_t)(q_begin + qi) * p.out_row_stride + (kSpans ? (size_t)head * parts + part : (size_t)head) * D;
+          for (int j = 0; j < 32; ++j)
+            o[j] = __float_as_uint(__uint_as_float(o[j]) * own + peer[(half * 32 + j) * kRows] * other);
+        }
+        const float times = split ? 1.f : inv;
+        if (row < rows_used) {
 #pragma unroll
-    for (int half = 0; half < D / 32; ++half) {
-      unsigned o[32];
-      __syncwarp();
-      tmem_load32(tmem_o + lane_field + half * 32, o);
-      tmem_load_wait();
-      if (split) {
+          for (int v = 0; v < 4; ++v) {
+            unsigned w[4];
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
-          o[j] = __float_as_uint(__uint_as_float(o[j]) * own + peer[(half * 32 + j) * kRows] * other);
-      }
-      const float times = split ? 1.f : inv;
-      if (row < rows_used) {
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          unsigned w[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(o[v * 8 + 2 * e]) * times,
-                                                     __uint_as_float(o[v * 8 + 2 * e + 1]) * times);
-            w[e] = *reinterpret_cast<unsigned*>(&h);
+            for (int e = 0; e < 4; ++e) {
+              __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(o[v * 8 + 2 * e]) * times,
+                                                       __uint_as_float(o[v * 8 + 2 * e + 1]) * times);
+              w[e] = *reinterpret_cast<unsigned*>(&h);
+            }
+            *reinterpret_cast<uint4*>(dst + half * 32 + v * 8) = make_uint4(w[0], w[1], w[2], w[3]);
           }
-          *reinterpret_cast<uint4*>(dst + half * 32 + v * 8) = make_uint4(w[0], w[1], w[2], w[3]);
         }
       }
     }
@@ -597,16 +641,27 @@ template <int D, int X, bool kOptions, bool kSpans, bool kSplit = false>
 static int launch_tc_attention_as(const CUtensorMap& mk, const CUtensorMap& mv, const TcAttnParams& p, dim3 grid,
                                   cudaStream_t stream);
 
-// Blocks of a launch up to which two share a block's keys: as many as leave room for their seconds, at two an SM at head size
-// 64 (the padded grid of a portion of 640 tokens has 160 for eight KV heads) and one at 128.
-template <int D> constexpr long kSplitBlocks = D == 64 ? 160 : 74;
+// Whether a launch goes out in pairs of blocks that share their keys: while its blocks are so few that all of their seconds find a
+// place (two places an SM at head size 64, one at 128; a portion of 640 tokens, whose 160 blocks' seconds do not, takes 32 us
+// behind 1,024 in pairs and 27 without).  `max_context` (0: not known): no sequence of the launch holds more tokens; contexts
+// that hardly fill the tiles from which a block is split are better off alone, the more so where a second's place is on an SM
+// that has another block: 128 blocks of 512 queries over themselves take 13.1 us in pairs and 12.3 without.
+constexpr long kSms = 148;
+template <int D, int X>
+static bool in_pairs(long blocks, int max_context, int window, int tq) {
+  const long places = (D == 64 ? 2 : 1) * kSms;
+  if (2 * blocks > places) return false;
+  long keys = max_context > 0 ? max_context : 0x7fffffffL;
+  if (window > 0 && keys > window + X * tq) keys = window + X * tq;      // what a block reads at most, but for a tile
+  return keys > (2 * blocks > kSms ? kSplitTiles + 1 : kSplitTiles - 1) * (long)kKeys;
+}
 
 template <int D, int X>
 static int launch_tc_attention(const CUtensorMap& mk, const CUtensorMap& mv, const TcAttnParams& p, dim3 grid,
-                               cudaStream_t stream) {
+                               int max_context, int tq, cudaStream_t stream) {
   const bool options = p.keep_first > 0 || p.cap_out > 0.f || p.sink != nullptr;
   const bool spans = p.window < 0 || (int)grid.x != p.kv_heads;
-  if (!spans && !options && (long)grid.x * grid.y * grid.z <= kSplitBlocks<D>)
+  if (!spans && !options && in_pairs<D, X>((long)grid.x * grid.y * grid.z, max_context, p.window, tq))
     return launch_tc_attention_as<D, X, false, false, true>(mk, mv, p, grid, stream);
   if (spans)
     return options ? launch_tc_attention_as<D, X, true, true>(mk, mv, p, grid, stream)
@@ -662,14 +717,14 @@ LI_EXPORT int li_paged_attention_tcgen05_supports(int heads, int kv_heads, int h
 
 // bfloat16; head_dim 64 or 128; page_size 16, 32 or 64; groups of at most 128 heads.  Sequences may bring any number of queries
 // (the kernel is meant for those that bring many).  window: see first_visible (common.cuh).  v_dim: the size of a value, a
-// multiple of head_dim.  error_flag (device int, zero): set if a wait inside gave up.
+// multiple of head_dim.  error_flag (device int, zero): set if a wait inside gave up.  max_context: see in_pairs.
 LI_EXPORT int li_paged_attention_tcgen05(const void* q, int q_row_stride, void* out, int out_row_stride,
                                          const void* k_pool, const void* v_pool, const int* block_table,
                                          int table_stride, const int* query_start_loc, const int* context_lens,
                                          const int* seq_index, int num_seqs, int max_q_len, int heads, int kv_heads,
                                          int head_dim, int page_size, int num_pages, float scale, int window,
                                          int* error_flag, int keep_first, float softcap, const float* sink,
-                                         int v_dim, cudaStream_t stream) {
+                                         int v_dim, int max_context, cudaStream_t stream) {
   if (num_seqs == 0 || max_q_len == 0) return 0;
   if (softcap > 0.f && scale == 0.f) return LI_ERR_UNSUPPORTED;
   if (!li_paged_attention_tcgen05_supports(heads, kv_heads, head_dim, page_size)) return LI_ERR_UNSUPPORTED;
@@ -695,8 +750,9 @@ LI_EXPORT int li_paged_attention_tcgen05(const void* q, int q_row_stride, void* 
   // (LITEINFER_TCGEN05_ATTN_TILES=1 keeps one).
   static const bool one_tile = [] { const char* e = getenv("LITEINFER_TCGEN05_ATTN_TILES"); return e && atoi(e) == 1; }();
   if (head_dim == 128 && max_q_len > tq && !one_tile)
-    return launch_tc_attention<128, 2>(mk, mv, p, dim3(kv_heads * v_parts, num_seqs, (max_q_len + 2 * tq - 1) / (2 * tq)), stream);
+    return launch_tc_attention<128, 2>(mk, mv, p, dim3(kv_heads * v_parts, num_seqs, (max_q_len + 2 * tq - 1) / (2 * tq)),
+                                       max_context, tq, stream);
   const dim3 grid(kv_heads * v_parts, num_seqs, (max_q_len + tq - 1) / tq);
-  return head_dim == 64 ? launch_tc_attention<64, 1>(mk, mv, p, grid, stream)
-                        : launch_tc_attention<128, 1>(mk, mv, p, grid, stream);
+  return head_dim == 64 ? launch_tc_attention<64, 1>(mk, mv, p, grid, max_context, tq, stream)
+                        : launch_tc_attention<128, 1>(mk, mv, p, grid, max_context, tq, stream);
 }

@@ -150,7 +150,8 @@ def _context(batch: _Batch, dev: torch.Tensor, device, counts, totals, decode_sp
     prefill_lens = [c for c in counts if c > 1]
     plan = AttentionPlan(
         num_decode=batch.n_decode, decode_seqs=dseq, decode_tokens=dtok, num_prefill=batch.n_prefill,
-        prefill_seqs=pseq, max_prefill_query_len=max(prefill_lens, default=0), max_decode_context_len=decode_bound)
+        prefill_seqs=pseq, max_prefill_query_len=max(prefill_lens, default=0), max_decode_context_len=decode_bound,
+        max_prefill_context_len=max((t for t, c in zip(totals, counts) if c > 1), default=0))
     return StepContext(
         num_tokens=batch.T, num_seqs=B, token_ids=tok, positions=pos, seq_of_token=seq, query_start_loc=qsl,
         context_lens=ctxl, block_tables=tables, state_slots=slots, logit_rows=rows, num_logit_rows=batch.R,
@@ -267,10 +268,11 @@ def _token_bucket(n: int) -> int:
 
 class _PaddedGraph:
     """One captured forward for any step that fits a padded shape: up to `tokens` tokens in up to `seqs` sequences,
-    of which up to `prefill` bring more than one token, with up to `rows` wanted rows."""
+    of which up to `prefill` bring more than one token, up to `portion` of them, and then hold up to `prefill_context`, with
+    up to `rows` wanted rows."""
 
-    def __init__(self, runner: ModelRunner, tokens: int, seqs: int, decode: bool, prefill: int, rows: int,
-                 max_model_len: int) -> None:
+    def __init__(self, runner: ModelRunner, tokens: int, seqs: int, decode: bool, prefill: int, portion: int,
+                 prefill_context: int, rows: int, max_model_len: int) -> None:
         cache = runner.cache
         pages = -(-max_model_len // cache.page_size)
         n_decode = seqs if decode else 0
@@ -280,8 +282,8 @@ class _PaddedGraph:
         tables = [t.view(seqs, w) for t, w in zip(tables, batch.widths)]
         # The kernels' launch bounds are those of the padded shape; what a step really holds is in the buffers.
         plan = AttentionPlan(num_decode=n_decode, decode_seqs=dseq, decode_tokens=dtok, num_prefill=prefill,
-                             prefill_seqs=pseq, max_prefill_query_len=tokens if prefill else 0,
-                             max_decode_context_len=max_model_len)
+                             prefill_seqs=pseq, max_prefill_query_len=portion if prefill else 0,
+                             max_decode_context_len=max_model_len, max_prefill_context_len=prefill_context)
         self.ctx = StepContext(
             num_tokens=tokens, num_seqs=seqs, token_ids=tok, positions=pos, seq_of_token=seq, query_start_loc=qsl,
             context_lens=ctxl, block_tables=tables, state_slots=slots, logit_rows=wanted, num_logit_rows=rows,
@@ -443,7 +445,12 @@ class ModelRunner:
         prefill = min(_pow2(len(entries) - n_decode), seqs) if n_decode < len(entries) else 0
         wanted = sum(len(e.want) for e in entries)
         rows = seqs if wanted <= seqs else _token_bucket(wanted)
-        key = (_token_bucket(tokens), seqs, n_decode > 0, prefill, rows)
+        # A single portion has the bucket of its own length (beside single tokens that of the step's may be the next one, and a
+        # launch sized for it a quarter too large); several share the step's.
+        brought = [(len(e.tokens), total) for e, total in zip(entries, totals) if len(e.tokens) > 1]
+        portion = _token_bucket(brought[0][0] if len(brought) == 1 else tokens)
+        context = kernels.context_class(max((total for _, total in brought), default=max_len), max_len)
+        key = (_token_bucket(tokens), seqs, n_decode > 0, prefill, portion, context, rows)
         graph = self._padded_graphs.get(key)
         if graph is None:
             if len(self._padded_graphs) >= _MAX_GRAPHS:      # the decode graphs have a table of their own

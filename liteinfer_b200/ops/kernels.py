@@ -142,7 +142,7 @@ _SIGNATURES = {
     "li_paged_attention_tcgen05": ("attention_tcgen05", [
         c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
         c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_float, c_void_p, c_int,
-        c_void_p]),
+        c_int, c_void_p]),
     "li_paged_attention_tcgen05_supports": ("attention_tcgen05", [c_int, c_int, c_int, c_int]),
     "li_gemm_skinny": ("gemm_skinny", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float,
                                        c_void_p, c_size_t, c_void_p, c_int, c_void_p]),
@@ -1102,10 +1102,11 @@ def fused_decode_supports(dtype: torch.dtype, heads: int, kv_heads: int, head_di
 
 def paged_attention_tcgen05(q, q_row_stride, out, k_pool, v_pool, block_table, query_start_loc, context_lens,
                             seq_index, num_seqs, max_q_len, heads, kv_heads, head_dim, scale, window=0, keep_first=0,
-                            softcap=0.0, sink=None) -> torch.Tensor:
+                            softcap=0.0, sink=None, max_context_len=0) -> torch.Tensor:
     """The tcgen05 / TMA / tensor-memory attention kernel for prompts and portions (bfloat16, head size 64 or 128,
     pages of 16, 32 or 64 tokens, groups of at most 128 heads; `keep_first` and `softcap` as in `paged_attention`;
-    `window` < 0: chunks of -window positions; values may be a multiple of the head size wide).
+    `window` < 0: chunks of -window positions; values may be a multiple of the head size wide).  `max_context_len`
+    (0: not known): the most tokens that a sequence holds; whether two blocks share a block's keys goes by it.
     `gemm_error_flag(device)` tells afterwards whether a wait inside the kernel ever gave up."""
     _rows2d(q, "q"); _rows2d(out, "out")
     _on_gpu(k_pool, v_pool, block_table, query_start_loc, context_lens, seq_index, sink)
@@ -1115,7 +1116,7 @@ def paged_attention_tcgen05(q, q_row_stride, out, k_pool, v_pool, block_table, q
         block_table.data_ptr(), block_table.stride(0), query_start_loc.data_ptr(), context_lens.data_ptr(),
         _ptr(seq_index), num_seqs, max_q_len, heads, kv_heads, head_dim, page_size, pages, float(scale),
         int(window), scratch_for(q.device).gemm_error.data_ptr(), int(keep_first), float(softcap), _ptr(sink),
-        v_pool.shape[3], _stream()),
+        v_pool.shape[3], int(max_context_len), _stream()),
         "paged_attention_tcgen05")
     return out
 
@@ -1150,6 +1151,16 @@ def tensor_core_sizes(key_dim: int, value_dim: int, heads: int, kv_heads: int) -
 
 # LITEINFER_TCGEN05_ATTN=0: prompts and portions run on the mma.sync kernel (a switch for measurements).
 MASKED_ON_MMA = os.environ.get("LITEINFER_TCGEN05_ATTN", "1") == "0"
+
+
+# Up to these contexts kernels for prompts are chosen differently (the shortest that two blocks of the tcgen05 attention share,
+# with few blocks and with more), so a step that is replayed from a graph keeps the class that its prompts' contexts lie in.
+CONTEXT_CLASSES = (448, 576)
+
+
+def context_class(longest: int, most: int) -> int:
+    """The bound of the class that a context of `longest` tokens lies in, where none is longer than `most`."""
+    return next((bound for bound in CONTEXT_CLASSES if longest <= bound < most), most)
 
 
 # In a step that has both, the attention of the single tokens runs on a second stream beside that of the portions, which
@@ -1219,7 +1230,8 @@ def paged_attention(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_poo
     def portions():
         if tcgen05_attention_supports(q.dtype, heads, kv_heads, head_dim, page_size) and not MASKED_ON_MMA:
             paged_attention_tcgen05(*common, plan.prefill_seqs, plan.num_prefill, plan.max_prefill_query_len, heads,
-                                    kv_heads, head_dim, scale, window, **options)
+                                    kv_heads, head_dim, scale, window, **options,
+                                    max_context_len=plan.max_prefill_context_len)
         else:
             paged_attention_mma(*common, plan.prefill_seqs, plan.num_prefill, plan.max_prefill_query_len, heads,
                                 kv_heads, head_dim, scale, window, **options)

@@ -107,6 +107,7 @@ class AttentionPlan:
     prefill_seqs: torch.Tensor | None = None    # [num_prefill] int32 batch rows with several queries
     max_prefill_query_len: int = 0
     max_decode_context_len: int = 0             # host bound on the decode rows' context (sizes the splits)
+    max_prefill_context_len: int = 0            # host bound on the other rows' context (0: not known)
 
 
 @dataclass

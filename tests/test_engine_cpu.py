@@ -318,3 +318,25 @@ def test_every_weight_of_a_product_is_at_rest(cpu_kernels, monkeypatch, tmp_path
                      SamplingParams(temperature=0.0, max_tokens=2, ignore_eos=True))
     assert seen and all(ops.kernels._at_rest(w) for w in seen)
     assert not ops.kernels._at_rest(torch.zeros(2, 2)) and not ops.kernels._at_rest(seen[0][:1])
+
+
+def test_a_step_says_how_long_its_prompts_contexts_are(cpu_kernels, model_dirs):
+    """The plan of a step that runs kernel by kernel has the longest context of the rows that bring several tokens; a graph's
+    has the bound of its class."""
+    from liteinfer_b200 import LLM
+    from liteinfer_b200.engine.runner import StepEntry
+    from liteinfer_b200.ops import kernels
+
+    _, _, page = tiny_configs.ALL["tiny_a"]
+    with LLM(str(model_dirs["tiny_a"]), dtype="float32", device="cpu", block_size=page, max_num_seqs=4, max_model_len=64) as llm:
+        runner = llm.engine.runner
+        runner.step([StepEntry("a", list(range(1, 12)), (10,)), StepEntry("b", [1, 2, 3], (2,))])
+        entries = [StepEntry("a", [5], (0,)), StepEntry("b", [4, 5], (1,))]
+        runner.cache.reserve(["a", "b"], [12, 5])
+        plan = runner.build_context(entries).plan
+        assert (plan.max_prefill_context_len, plan.max_decode_context_len) == (5, 12)
+        runner.cache.rollback(["a", "b"])
+        assert runner.build_context([StepEntry("a", [5], (0,))]).plan.max_prefill_context_len == 0
+    bounds = [kernels.context_class(n, 4096) for n in (1, 448, 449, 576, 577, 4096)]
+    assert bounds == [448, 448, 576, 576, 4096, 4096]
+    assert [kernels.context_class(n, 448) for n in (5, 448)] == [448, 448] and kernels.context_class(500, 520) == 520

@@ -257,6 +257,31 @@ def test_prompt_attention_with_shared_keys(heads, kv_heads, head_dim, q_lens, ct
     assert ops.gemm_error_flag("cuda:0") == 0
 
 
+# Grids on both sides of the numbers of blocks up to which a launch goes out in pairs (74 and 148 at head size 64, 74 at 128),
+# contexts that are known, unknown and those of a padded shape, whose grid has blocks without queries.
+@pytest.mark.parametrize("head_dim,n,q_len", [(64, 1, 444), (64, 1, 570), (64, 1, 580), (64, 1, 1184), (64, 1, 1200), (64, 2, 1184), (64, 4, 592), (64, 3, 790),
+                                                (128, 2, 1184), (128, 2, 1200)])
+@pytest.mark.parametrize("extra", [0, 5, 300])
+def test_prompt_attention_in_pairs_where_the_grid_has_room(head_dim, n, q_len, extra):
+    from liteinfer_b200 import ops
+
+    heads, kv_heads = 8, 1                                  # 16 queries a tile of rows
+    q_lens, ctx_lens = [q_len] + [q_len // 2] * (n - 1), [q_len + extra] + [q_len // 2 + extra] * (n - 1)
+    case = _paged_case(torch.bfloat16, heads, kv_heads, head_dim, 16, q_lens, ctx_lens)
+    qkv, k_pool, v_pool = case["qkv"], case["k_pool"], case["v_pool"]
+    ops.rope_kv_write(qkv, case["positions"], case["seq_of"], case["table"], k_pool, v_pool, None, heads, kv_heads, head_dim, 0)
+    common = (case["table"], case["qsl"], case["ctx"])
+    want = torch.empty(case["T"], heads * head_dim, dtype=torch.bfloat16, device="cuda")
+    ref.paged_attention(qkv, qkv.shape[1], want, k_pool, v_pool, *common, n, q_len, heads, kv_heads, head_dim, head_dim ** -0.5, 0)
+    places = torch.tensor([*range(n), -1], dtype=torch.int32, device="cuda")
+    for places_n, longest, context in ((n, q_len, max(ctx_lens)), (n, q_len, 0), (n + 1, q_len * 5 // 4, 4096)):
+        out = torch.empty_like(want)
+        ops.paged_attention_tcgen05(qkv, qkv.stride(0), out, k_pool, v_pool, *common, places, places_n, longest, heads, kv_heads,
+                                    head_dim, head_dim ** -0.5, max_context_len=context)
+        torch.testing.assert_close(out.float(), want.float(), **_tol(torch.bfloat16))
+    assert ops.gemm_error_flag("cuda:0") == 0
+
+
 # Rows walked by one warp and by teams, one unit of keys and several rounds of them, every width of values.
 @pytest.mark.parametrize("heads,kv_heads,head_dim,page_size", [(3, 1, 64, 16), (9, 1, 20, 16), (2, 2, 128, 16), (6, 3, 256, 8),
                                                                (2, 1, 320, 16), (34, 2, 33, 5)])
