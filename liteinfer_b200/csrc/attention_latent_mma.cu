@@ -627,8 +627,12 @@ LI_EXPORT int li_latent_attention_mma(const void* q_lat, long q_lat_head_stride,
     t.rot_dims = rot_dims; t.page_size = page_size; t.page_shift = 0; t.num_pages = num_pages;
     while ((1 << t.page_shift) < page_size) ++t.page_shift;
     t.scale_log2 = scale * kLog2e; t.window = window; t.cs_scale = cos_sin_scale; t.error_flag = error_flag;
+    // The tcgen05 kernel gives a row of a latent of 512 to two blocks, each of which reads all of its query and writes half of its
+    // output: not where the output lies over the queries.  (The mma.sync kernel has a row's query in before it writes.)
+    const uintptr_t from = reinterpret_cast<uintptr_t>(q_lat), to = reinterpret_cast<uintptr_t>(out);
+    const bool in_place = (from < to ? to - from : from - to) < (uintptr_t)heads * tokens * kv_rank * sizeof(bf16);
     CUtensorMap map;
-    if (latent_tc::takes(t, pool, num_seqs, max_q_len, kv_rank, rot_dim) &&
+    if (!in_place && latent_tc::takes(t, pool, num_seqs, max_q_len, kv_rank, rot_dim) &&
         latent_tc::make_entry_map(&map, pool, (long)num_pages * page_size, page_size < 32 ? page_size : 32, kv_rank + rot_dim)) {
       if (kv_rank == 128) return latent_tc::launch<128>(t, map, num_seqs, max_q_len, stream);
       if (kv_rank == 256) return latent_tc::launch<256>(t, map, num_seqs, max_q_len, stream);

@@ -1929,7 +1929,8 @@ def latent_attention(q_lat: torch.Tensor, q_raw: torch.Tensor, q_head_stride: in
                      plan=None, window: int = 0, cos_sin_scale: float = 1.0) -> torch.Tensor:
     """Causal multi-query attention of every head over the shared cache entries [latent | rotated key part]:
     score = (q_lat . latent + rotate(q_rot) . key part) * scale, out = sum_j p_j latent_j, with exp(sink[h]) as one
-    more term of the softmax's denominator (sink float32 [heads] or None).  q_lat, out: [heads, tokens, kv_rank];
+    more term of the softmax's denominator (sink float32 [heads] or None).  q_lat, out: [heads, tokens, kv_rank], which may
+    be one tensor;
     q_raw [tokens, columns]: the part of head h that turns lies at columns h * q_head_stride + q_rot_off (rot_dim
     numbers, rotated here by the query's position).  pool [pages, 1, page_size, kv_rank + rot_dim].  `window` > 0:
     a query at position p reads the keys at p - window + 1 ... p.  `cos_sin_scale` multiplies every cosine and

@@ -258,6 +258,25 @@ def test_latent_prompts_by_rows_of_128(heads, c, dims, page, window):
     assert ops.gemm_error_flag(DEV) == 0
 
 
+@pytest.mark.parametrize("heads,c", [(16, 512), (8, 256), (128, 512)])
+def test_latent_attention_over_its_own_queries(heads, c):
+    """The output may be the tensor of the absorbed queries, for prompts and single tokens alike."""
+    from liteinfer_b200 import ops
+
+    dtype, d, r, page = torch.bfloat16, 8, 64, 16
+    query_lens, context_lens = [300, 1, 41], [300, 200, 600]
+    pages = sum(-(-n // page) for n in context_lens) + 3
+    table, qsl, ctxl, pool, q_lat, q_raw = _attention_inputs(dtype, heads, c, r, d, query_lens, context_lens, page, pages, 7)
+    inv_freq = (1000.0 ** (-torch.arange(r // 2, dtype=torch.float64) * 2 / r)).float().to(DEV)
+    rest = (pool, table, qsl, ctxl, inv_freq, None, len(query_lens), 300, heads, c, r, r, 0.09)
+    want = ref.latent_attention(q_lat, q_raw, d + r, d, torch.empty_like(q_lat), *rest)
+    for plan in (None, _plan(query_lens, context_lens)):
+        own = q_lat.clone()
+        assert ops.latent_attention(own, q_raw, d + r, d, own, *rest, plan=plan) is own
+        torch.testing.assert_close(own.float(), want.float(), **_tol(dtype))
+    assert ops.gemm_error_flag(DEV) == 0
+
+
 @pytest.mark.parametrize("dtype,c,r", [(torch.float32, 48, 8), (torch.bfloat16, 48, 8), (torch.bfloat16, 64, 32)])
 @pytest.mark.parametrize("decode", [False, True])
 def test_latent_key_just_inside_and_just_outside_the_window(dtype, c, r, decode):
