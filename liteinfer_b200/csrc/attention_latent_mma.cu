@@ -21,7 +21,7 @@
 // warps (rounds of 64 keys from five stages of 32), their keys split over `num_splits`
 // blocks whose partial results (normalised, with the logarithm of their denominators) a second kernel merges,
 // sink included.  Sequences that bring more run on the kernel of attention_latent_tcgen05.cuh where it takes
-// their sizes, else with MT = 4, KT = 32 and three stages: four consecutive queries share every tile of keys.
+// their sizes and their contexts are not known to be short, else with MT = 4, KT = 32 and three stages: four consecutive queries share every tile of keys.
 #include "attention_latent_tcgen05.cuh"
 #include "attention_mma.cuh"
 #include "tcgen05.cuh"
@@ -601,7 +601,8 @@ LI_EXPORT int li_latent_attention_mma_supports(int kv_rank, int rot_dim, int rot
 // `num_splits` blocks share (partial_out [splits, heads, tokens, kv_rank] and partial_lse [splits, heads, tokens]
 // float; `tokens`: the step's token rows; `two_blocks`: the single-token form as two blocks of eight warps per SM).  error_flag (device int, zero; may be null): set to 31 if a wait for a
 // tile of entries ever gave up.  window > 0: a query sees the newest `window` keys up to its own; cos_sin_scale
-// multiplies every cosine and sine of the query's rotation.
+// multiplies every cosine and sine of the query's rotation.  max_context (0: not known): no sequence that brings several tokens
+// holds more.
 LI_EXPORT int li_latent_attention_mma(const void* q_lat, long q_lat_head_stride, int q_lat_token_stride,
                                       const void* q_raw, int q_raw_token_stride, int q_raw_head_stride, int q_rot_off,
                                       void* out, long out_head_stride, int out_token_stride, const void* pool,
@@ -611,7 +612,7 @@ LI_EXPORT int li_latent_attention_mma(const void* q_lat, long q_lat_head_stride,
                                       int rot_dim, int rot_dims, int page_size, int num_pages, float scale,
                                       int num_splits, float* partial_out, float* partial_lse, int tokens,
                                       int two_blocks, int* error_flag, int window, float cos_sin_scale,
-                                      cudaStream_t stream) {
+                                      int max_context, cudaStream_t stream) {
   if (num_seqs == 0 || max_q_len == 0) return 0;
   if (!li_latent_attention_mma_supports(kv_rank, rot_dim, rot_dims) || num_seqs > 65535) return LI_ERR_UNSUPPORTED;
   if (!aligned16(q_lat) || !aligned16(pool) || (q_lat_token_stride % 8) || (q_lat_head_stride % 8) || (out_token_stride % 2) ||
@@ -633,6 +634,7 @@ LI_EXPORT int li_latent_attention_mma(const void* q_lat, long q_lat_head_stride,
     const bool in_place = (from < to ? to - from : from - to) < (uintptr_t)heads * tokens * kv_rank * sizeof(bf16);
     CUtensorMap map;
     if (!in_place && latent_tc::takes(t, pool, num_seqs, max_q_len, kv_rank, rot_dim) &&
+        latent_tc::worth(t, num_seqs, max_q_len, kv_rank, max_context) &&
         latent_tc::make_entry_map(&map, pool, (long)num_pages * page_size, page_size < 32 ? page_size : 32, kv_rank + rot_dim)) {
       if (kv_rank == 128) return latent_tc::launch<128>(t, map, num_seqs, max_q_len, stream);
       if (kv_rank == 256) return latent_tc::launch<256>(t, map, num_seqs, max_q_len, stream);

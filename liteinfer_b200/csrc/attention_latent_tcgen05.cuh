@@ -24,8 +24,8 @@
 // of P E: 1.57 us a tile.  (A pair of CTAs would halve them: tiles of 64 keys at the same shared memory.)  Measured on B200
 // beside the mma.sync kernel, 16 heads, latent 512: prompts of 1,300, 910, 520 and 130 within a window of 1,024 197 against
 // 367 us; 2,048 causal 230 against 462; 256 queries over 8,000 keys 393 against 903; portions of 5, 2 and 9 behind contexts of
-// up to 1,300 60 against 125; latent 256, twice 1,000: 59 against 174.  Prompts of a tile or less, which the host cannot tell
-// from short portions of long contexts: 5 tokens 13.9 against 14.7, eight of 30 17.9 against 15.5.  The products issued by the whole
+// up to 1,300 60 against 125; latent 256, twice 1,000: 59 against 174.  What it does before its first tile takes longer, though:
+// see `worth`.  The products issued by the whole
 // warp with one lane's predicate: 269 to 209 us together with the rotated parts asked for all at once.
 #pragma once
 
@@ -472,6 +472,20 @@ inline bool takes(const Params& p, const void* pool, int num_seqs, int max_q_len
          (p.page_size == 16 || p.page_size == 32 || p.page_size == 64) && max_q_len > 1 &&
          max_q_len / (kRows / p.heads) < 65535 && num_seqs <= 65535 && (p.out_token_stride % 8) == 0 &&
          (p.out_head_stride % 8) == 0 && aligned16(p.out) && aligned16(pool);
+}
+
+// Whether it is the faster one there.  Contexts of at most two tiles (`max_context`, 0: not known) it has no use for its faster
+// walk: 16 heads of a latent of 512 over one prompt of 16 tokens take 16.0 us here and 13.9 on the mma.sync kernel, eight of 30
+// 17.4 and 15.1, sixteen of 33 30.2 and 15.9; 8 heads and eight prompts of 30 18.0 and 11.7; 64 tokens are even.  Unless the
+// mma.sync kernel's blocks, of four queries and sixteen heads, need more rounds of the device's SMs: 8 heads and sixteen prompts
+// of 64 18.5 and 29.3.
+constexpr int kShortContext = 2 * kKeys;
+inline bool worth(const Params& p, int num_seqs, int max_q_len, int kv_rank, int max_context) {
+  if (max_context <= 0 || max_context > kShortContext) return true;
+  const int tq = kRows / p.heads;
+  const long here = (long)num_seqs * ((max_q_len + tq - 1) / tq) * (kv_rank > 256 ? 2 : 1);
+  const long there = (long)num_seqs * ((max_q_len + 3) / 4) * ((p.heads + 15) / 16);
+  return (here + 147) / 148 < (there + 147) / 148;
 }
 
 template <int C>

@@ -173,7 +173,7 @@ _SIGNATURES = {
     "li_latent_attention_mma": ("attention_latent_mma", [
         c_void_p, c_long, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_long, c_int, c_void_p, c_void_p, c_int,
         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-        c_float, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_float, c_void_p]),
+        c_float, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_float, c_int, c_void_p]),
     "li_latent_attention_mma_supports": ("attention_latent_mma", [c_int, c_int, c_int]),
     "li_gate_heads": ("attention_latent", [c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p]),
     "li_argmax": ("sampling", [c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
@@ -1153,14 +1153,16 @@ def tensor_core_sizes(key_dim: int, value_dim: int, heads: int, kv_heads: int) -
 MASKED_ON_MMA = os.environ.get("LITEINFER_TCGEN05_ATTN", "1") == "0"
 
 
-# Up to these contexts kernels for prompts are chosen differently (the shortest that two blocks of the tcgen05 attention share,
-# with few blocks and with more), so a step that is replayed from a graph keeps the class that its prompts' contexts lie in.
-CONTEXT_CLASSES = (448, 576)
+# Up to these contexts the kernels for prompts are chosen differently (the shortest that two blocks of the tcgen05 attention
+# share, with few blocks and with more; the longest that the tcgen05 latent attention leaves to the other kernel), so a step that
+# is replayed from a graph keeps the class that its prompts' contexts lie in.
+ATTENTION_CONTEXTS = (448, 576)
+LATENT_CONTEXTS = (64,)
 
 
-def context_class(longest: int, most: int) -> int:
+def context_class(longest: int, most: int, bounds: tuple[int, ...]) -> int:
     """The bound of the class that a context of `longest` tokens lies in, where none is longer than `most`."""
-    return next((bound for bound in CONTEXT_CLASSES if longest <= bound < most), most)
+    return next((bound for bound in bounds if longest <= bound < most), most)
 
 
 # In a step that has both, the attention of the single tokens runs on a second stream beside that of the portions, which
@@ -1958,8 +1960,8 @@ def latent_attention(q_lat: torch.Tensor, q_raw: torch.Tensor, q_head_stride: in
                 block_table.stride(0), query_start_loc.data_ptr(), context_lens.data_ptr(), _ptr(seq_index),
                 inv_freq.data_ptr(), _ptr(sink), count, q_len, heads, kv_rank, rot_dim, rot_dims, page_size, pages,
                 float(scale), splits, _ptr(partial_out), _ptr(partial_lse), tokens, int(two_blocks),
-                scratch_for(out.device).gemm_error.data_ptr(), int(window), float(cos_sin_scale), _stream()),
-                "latent_attention_mma")
+                scratch_for(out.device).gemm_error.data_ptr(), int(window), float(cos_sin_scale),
+                0 if plan is None else plan.max_prefill_context_len, _stream()), "latent_attention_mma")
 
         if plan is None:
             run(None, num_seqs, max(max_q_len, 2))

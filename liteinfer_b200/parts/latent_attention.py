@@ -38,6 +38,8 @@ def _sink_init(shape, generator):
 
 
 class LatentAttention:
+    context_bounds = ops.LATENT_CONTEXTS
+
     def __init__(self, hidden_size: int, heads: int, dim: int, rot_dim: int, vdim: int, q_rank: int | None,
                  kv_rank: int, scale: float, norm_eps: float, position: PartSpec, dtype: torch.dtype,
                  device: torch.device, sink: bool = True, gate: bool = True, own_kv: bool = True,

@@ -134,6 +134,12 @@ class Model:
         A part that reads device values on the host in `forward` sets `graph_safe = False`."""
         return all(getattr(part, "graph_safe", True) for _, part, _ in self._named_parts())
 
+    def context_bounds(self) -> tuple[int, ...]:
+        """The contexts, ascending, up to which the kernels of some part are chosen differently for prompts."""
+        bounds = {bound for _, part, _ in self._named_parts() for one in (part, *getattr(part, "members", ()))
+                  for bound in getattr(one, "context_bounds", ())}
+        return tuple(sorted(bounds)) if self.dtype == torch.bfloat16 else ()
+
     def weight_bytes(self) -> int:
         seen: dict[int, int] = {}
         for _, part, _ in self._named_parts():

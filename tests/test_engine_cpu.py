@@ -337,6 +337,23 @@ def test_a_step_says_how_long_its_prompts_contexts_are(cpu_kernels, model_dirs):
         assert (plan.max_prefill_context_len, plan.max_decode_context_len) == (5, 12)
         runner.cache.rollback(["a", "b"])
         assert runner.build_context([StepEntry("a", [5], (0,))]).plan.max_prefill_context_len == 0
-    bounds = [kernels.context_class(n, 4096) for n in (1, 448, 449, 576, 577, 4096)]
-    assert bounds == [448, 448, 576, 576, 4096, 4096]
-    assert [kernels.context_class(n, 448) for n in (5, 448)] == [448, 448] and kernels.context_class(500, 520) == 520
+    classes = [kernels.context_class(n, 4096, (64, 448)) for n in (1, 64, 65, 448, 449, 4096)]
+    assert classes == [64, 64, 448, 448, 4096, 4096]
+    assert [kernels.context_class(n, 64, (64, 448)) for n in (5, 64)] == [64, 64] and kernels.context_class(100, 300, (64, 448)) == 300
+    assert kernels.context_class(5, 300, ()) == 300
+
+
+def test_a_model_names_the_contexts_that_its_kernels_turn_at():
+    import kutolix_configs
+
+    from liteinfer_b200.config.registry import resolve
+    from liteinfer_b200.ops import kernels
+    from liteinfer_b200.parts.model import Model
+
+    def bounds(config, dtype):
+        arch, typed = resolve(config)
+        return Model(arch.build_spec(typed), dtype, torch.device("cpu")).context_bounds()
+
+    assert bounds(tiny_configs.ALL["tiny_a"][0], torch.bfloat16) == kernels.ATTENTION_CONTEXTS
+    assert bounds(kutolix_configs.ALL["kut_a"][0], torch.bfloat16) == kernels.LATENT_CONTEXTS + kernels.ATTENTION_CONTEXTS
+    assert bounds(kutolix_configs.ALL["kut_a"][0], torch.float32) == ()

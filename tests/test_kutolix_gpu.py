@@ -258,6 +258,27 @@ def test_latent_prompts_by_rows_of_128(heads, c, dims, page, window):
     assert ops.gemm_error_flag(DEV) == 0
 
 
+# Prompts of one tile of keys and of two, one token more; one round of blocks of either kernel, and of one of them only.
+@pytest.mark.parametrize("heads,c,n", [(8, 512, 1), (8, 512, 17), (16, 512, 16), (16, 256, 17), (24, 128, 2)])
+@pytest.mark.parametrize("longest", [7, 32, 64, 65])
+def test_latent_prompts_of_known_short_contexts(heads, c, n, longest):
+    from liteinfer_b200 import ops
+
+    dtype, d, r, page = torch.bfloat16, 8, 64, 16
+    query_lens = [max(2, longest - i) for i in range(n)]
+    table, qsl, ctxl, pool, q_lat, q_raw = _attention_inputs(dtype, heads, c, r, d, query_lens, query_lens, page,
+                                                             sum(-(-x // page) for x in query_lens) + 1, 3)
+    inv_freq = (1000.0 ** (-torch.arange(r // 2, dtype=torch.float64) * 2 / r)).float().to(DEV)
+    rest = (pool, table, qsl, ctxl, inv_freq, _randn(heads, seed=9), n, longest, heads, c, r, r, 0.09)
+    want = ref.latent_attention(q_lat, q_raw, d + r, d, torch.empty_like(q_lat), *rest)
+    plan = _plan(query_lens, query_lens)
+    for known in (0, longest, 4096):
+        plan.max_prefill_context_len = known
+        got = ops.latent_attention(q_lat, q_raw, d + r, d, torch.full_like(q_lat, 7.0), *rest, plan=plan)
+        torch.testing.assert_close(got.float(), want.float(), **_tol(dtype))
+    assert ops.gemm_error_flag(DEV) == 0
+
+
 @pytest.mark.parametrize("heads,c", [(16, 512), (8, 256), (128, 512)])
 def test_latent_attention_over_its_own_queries(heads, c):
     """The output may be the tensor of the absorbed queries, for prompts and single tokens alike."""
