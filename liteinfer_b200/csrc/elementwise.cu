@@ -342,16 +342,17 @@ __global__ void scatter_tokens_kernel(int* __restrict__ tokens, const int* __res
 // then the late tokens into theirs: one launch instead of a copy and a launch.  Bound by the bus: a thread has one read of
 // 16 bytes, all of them on their way at once over as many blocks as that takes (48 sequences
 // of 256 pages: 3.8 us against 19.6 for one block that read word by word).  Each block places the late tokens
-// that fall among the words it has copied; where they go it reads from the host's copy, since another block may bring that.
+// that fall among the words it has copied; where they go it reads from the host's copy, since another block may bring that
+// (so the lists of places lie in the batch, at dst_at and src_at, as the tokens do).  `vec`: both copies lie on 16 bytes.
 constexpr int kStageThreads = 256;
 __global__ void __launch_bounds__(kStageThreads) stage_batch_kernel(int* __restrict__ device, const int* __restrict__ host, int words,
                                                                     int tokens_at, int dst_at, int src_at,
-                                                                    const int* __restrict__ source, int n_late) {
+                                                                    const int* __restrict__ source, int n_late, bool vec) {
   const int first = blockIdx.x * kStageThreads * 4, last = min(first + kStageThreads * 4, words), i = first + threadIdx.x * 4;
-  if (i + 4 <= last) {
+  if (vec && i + 4 <= last) {
     *reinterpret_cast<int4*>(device + i) = *reinterpret_cast<const int4*>(host + i);
   } else {
-    for (int k = i; k < last; ++k) device[k] = host[k];
+    for (int k = i; k < min(last, i + 4); ++k) device[k] = host[k];
   }
   if (n_late <= 0 || source == nullptr) return;
   __syncthreads();
@@ -381,21 +382,23 @@ __global__ void __launch_bounds__(256) zero_slots_kernel(const unsigned long lon
 
 using namespace li;
 
-// device[0 .. words) = host[0 .. words), then tokens[dst[i]] = source[src[i]] wherever dst[i] >= 0 (tokens, dst and
-// src lie inside `device`; source may be null: nothing is placed then).  `host` must be page-locked memory that the
-// device can read in place; where it cannot, LI_ERR_UNSUPPORTED is returned and nothing is launched.
-LI_EXPORT int li_stage_batch(int* device, const int* host, int words, int* tokens, const int* dst, const int* src,
-                             const int* source, int n_late, cudaStream_t stream) {
+// device[0 .. words) = host[0 .. words), then device[tokens_at + dst[i]] = source[src[i]] wherever dst[i] >= 0, i < n_late,
+// dst = device + dst_at and src = device + src_at, n_late entries each, inside `device` (source may be null: nothing is placed
+// then).  `host` must be page-locked memory that the device can read in place; where it cannot, LI_ERR_UNSUPPORTED is returned and
+// nothing is launched.
+LI_EXPORT int li_stage_batch(int* device, const int* host, int words, int tokens_at, int dst_at, int src_at, const int* source,
+                             int n_late, cudaStream_t stream) {
   if (words <= 0) return 0;
+  if (n_late > 0 && source && (tokens_at < 0 || dst_at < 0 || src_at < 0 || n_late > words - dst_at || n_late > words - src_at))
+    return LI_ERR_UNSUPPORTED;
   void* mapped = nullptr;
   if (cudaHostGetDevicePointer(&mapped, const_cast<int*>(host), 0) != cudaSuccess || mapped == nullptr) {
     cudaGetLastError();
     return LI_ERR_UNSUPPORTED;
   }
-  if (!aligned16(device) || !aligned16(mapped)) return LI_ERR_UNSUPPORTED;
   const int blocks = (words + kStageThreads * 4 - 1) / (kStageThreads * 4);
-  stage_batch_kernel<<<blocks, kStageThreads, 0, stream>>>(device, static_cast<const int*>(mapped), words, (int)(tokens - device),
-                                                           (int)(dst - device), (int)(src - device), source, n_late);
+  stage_batch_kernel<<<blocks, kStageThreads, 0, stream>>>(device, static_cast<const int*>(mapped), words, tokens_at, dst_at, src_at,
+                                                           source, n_late, aligned16(device) && aligned16(mapped));
   LI_LAUNCH_CHECK();
 }
 

@@ -42,7 +42,7 @@ _SIGNATURES = {
     "li_embedding": ("elementwise", [c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]),
     "li_scatter_tokens": ("elementwise", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
     "li_zero_slots": ("elementwise", [c_void_p, c_void_p, c_int, c_longlong, c_void_p, c_int, c_void_p]),
-    "li_stage_batch": ("elementwise", [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
+    "li_stage_batch": ("elementwise", [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p]),
     "li_rmsnorm": ("elementwise", [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float,
                                    c_int, c_void_p]),
     "li_add": ("elementwise", [c_int, c_void_p, c_void_p, c_size_t, c_void_p]),
@@ -427,22 +427,34 @@ def scatter_tokens(tokens: torch.Tensor, dst: torch.Tensor, src: torch.Tensor, s
 STAGE_KERNEL_MAX_WORDS = 16384
 
 
+def _at_words(part: torch.Tensor, whole: torch.Tensor) -> int | None:
+    """Where `part` lies in `whole` (both int32), in words; None if it is not inside."""
+    at = part.data_ptr() - whole.data_ptr()
+    return at // 4 if at >= 0 and at % 4 == 0 and at // 4 + part.numel() <= whole.numel() else None
+
+
 def stage_batch(device: torch.Tensor, host: torch.Tensor, tokens: torch.Tensor, dst: torch.Tensor, src: torch.Tensor,
                 source: torch.Tensor | None) -> bool:
     """device[:] = host[:] (int32; `host` pinned), then tokens[dst[i]] = source[src[i]] wherever dst[i] >= 0, in one
-    launch.  False (and nothing done) where the buffer is too large for that or the device cannot read `host` in
+    launch where `tokens`, `dst` and `src` are slices of `device` (the kernel then reads the latter two in `host`), else
+    in two.  False (and nothing done) where the buffer is too large for that or the device cannot read `host` in
     place: the caller then copies and scatters."""
     _on_gpu(device, tokens, dst, src, source)
     for t, what in ((device, "device"), (host, "host"), (tokens, "tokens"), (dst, "dst"), (src, "src")):
         _int32(t, what)
-    words = device.numel()
+    words, late = device.numel(), 0 if source is None else dst.numel()
     if words > STAGE_KERNEL_MAX_WORDS or host.numel() != words or not host.is_pinned():
         return False
-    code = _fn("li_stage_batch")(device.data_ptr(), host.data_ptr(), words, tokens.data_ptr(), dst.data_ptr(),
-                                 src.data_ptr(), _ptr(source), dst.numel() if source is not None else 0, _stream())
+    places = [_at_words(t, device) for t in (tokens, dst, src)]
+    assert src.numel() >= late
+    apart = late > 0 and None in places
+    code = _fn("li_stage_batch")(device.data_ptr(), host.data_ptr(), words, *(at or 0 for at in places),
+                                 _ptr(source), 0 if apart else late, _stream())
     if code == 100001:        # LI_ERR_UNSUPPORTED: the device cannot read this host memory in place
         return False
     _check(code, "stage_batch")
+    if apart:
+        scatter_tokens(tokens, dst, src[:late], source)
     return True
 
 

@@ -682,6 +682,34 @@ def test_stage_batch_equals_copy_and_scatter(words, n_late):
         assert torch.equal(device, want)
 
 
+@pytest.mark.parametrize("apart", [(), ("tokens",), ("dst",), ("src",), ("tokens", "dst", "src")])
+@pytest.mark.parametrize("words,off", [(3000, 0), (3001, 1), (1025, 3)])
+def test_stage_batch_with_tensors_of_their_own(apart, words, off):
+    """Tokens and the lists of places may be tensors outside the batch, and the batch may start anywhere."""
+    from liteinfer_b200 import ops
+
+    g = torch.Generator().manual_seed(words)
+    n = 40
+    host = torch.randint(0, 1000, (words + off,), generator=g, dtype=torch.int32)
+    host[off + 400:off + 400 + n] = torch.randperm(300, generator=g)[:n].to(torch.int32)
+    host[off + 400:off + 400 + n:3] = -1
+    host[off + 500:off + 500 + n] = torch.randint(0, 32, (n,), generator=g, dtype=torch.int32)
+    host = host.pin_memory()[off:]
+    source = torch.randint(0, 50000, (32,), generator=g, dtype=torch.int32).cuda()
+    device = torch.full((words + off,), -7, dtype=torch.int32, device="cuda")[off:]
+    at = {"tokens": slice(0, 300), "dst": slice(400, 400 + n), "src": slice(500, 500 + n)}
+    parts = {name: host[place].cuda() if name in apart else device[place] for name, place in at.items()}
+    assert ops.stage_batch(device, host, parts["tokens"], parts["dst"], parts["src"], source)
+    tokens = host[:300].clone()
+    for d, s in zip(host[400:400 + n].tolist(), host[500:500 + n].tolist()):
+        if d >= 0:
+            tokens[d] = int(source[s])
+    want = host.clone()
+    if "tokens" not in apart:
+        want[:300] = tokens
+    assert torch.equal(parts["tokens"].cpu(), tokens) and torch.equal(device.cpu(), want)
+
+
 @pytest.mark.parametrize("shapes", [[(3, 5)], [(16, 128, 128), (7,), (4, 1000)], [(1,)] * 40])
 def test_zeroed_slots(shapes):
     """The slots named, and no others, are zero in every state tensor, whatever a slot's size and alignment."""
