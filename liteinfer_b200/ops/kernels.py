@@ -2113,7 +2113,8 @@ EXPERT_TILE_ROWS = 256
 
 def moe_tile_rows(dtype: torch.dtype, hidden: int, ff: int, pairs: int | None = None) -> int:
     """Rows of a tile of an expert's products: 128 where the tcgen05 kernel takes them (bfloat16, sizes in eights, a
-    step of many pairs), 64 where both run on mma.sync tiles, else 32 (FFMA tiles)."""
+    step of many pairs; it takes tiles of up to `EXPERT_TILE_ROWS`, which `moe_expert_rows` makes for it), 64 where both run on
+    mma.sync tiles, else 32 (FFMA tiles)."""
     if not torch.cuda.is_available():
         return 32
     code = _DTYPE_CODE[dtype]
@@ -2158,12 +2159,13 @@ def moe_grouped_tcgen05(mode: str, a: torch.Tensor, weight: torch.Tensor, out: t
                         activation: str = "swiglu", limit: float = 0.0, alpha: float = 1.0,
                         pair_weights: torch.Tensor | None = None) -> torch.Tensor:
     """`moe_grouped` on the tcgen05 kernel (bfloat16): `a` [pairs, K] and `out` hold their rows in the order of the
-    experts' runs (`plan.order`), the plan's tiles are `EXPERT_TILE_ROWS` rows, and in mode "gate_up" an expert's gate and up rows lie
-    interleaved in eights.  mode "down" multiplies row m by pair_weights[plan.order[m]]; mode "up": experts without a gate."""
+    experts' runs (`plan.order`), the plan's tiles are of 128 rows or, which reads the weights fewer times, `EXPERT_TILE_ROWS`,
+    and in mode "gate_up" an expert's gate and up rows lie interleaved in eights.  mode "down" multiplies row m by pair_weights[plan.order[m]]; mode "up": experts without a gate."""
     _on_gpu(a, weight, out, pair_weights)
     experts, rows, K = weight.shape
     pairs = plan.order.numel()
-    assert plan.tile_rows == EXPERT_TILE_ROWS and mode in ("gate_up", "down", "up") and a.dtype == weight.dtype == out.dtype == torch.bfloat16
+    assert plan.tile_rows in (128, EXPERT_TILE_ROWS) and mode in ("gate_up", "down", "up")
+    assert a.dtype == weight.dtype == out.dtype == torch.bfloat16
     assert a.shape == (pairs, K) and out.shape == (pairs, rows // 2 if mode == "gate_up" else rows)
     act = {"down": -1, "up": -2}.get(mode)
     if act is None:

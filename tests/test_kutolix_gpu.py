@@ -492,6 +492,27 @@ def test_expert_tiles_of_every_height(hidden, ff, counts, mode):
     assert ops.gemm_error_flag(DEV) == 0
 
 
+@pytest.mark.parametrize("counts", [[300, 0, 128, 1, 40], [129, 127, 256, 257, 512]])
+def test_expert_products_of_a_plan_in_tiles_of_128(counts):
+    """A plan of the rows that `moe_tile_rows` names gives the same rows as one of the kernel's own tiles."""
+    from liteinfer_b200 import ops
+
+    dtype, hidden, ff, pairs, experts = torch.bfloat16, 264, 136, sum(counts), len(counts)
+    assert ops.moe_tile_rows(dtype, hidden, ff, pairs) == 128
+    x, w = _randn(pairs, hidden, seed=1, dtype=dtype), _randn(experts, 2 * ff, hidden, seed=2, scale=hidden ** -0.5, dtype=dtype)
+    down = _randn(experts, hidden, ff, seed=3, scale=ff ** -0.5, dtype=dtype)
+    ids = torch.repeat_interleave(torch.arange(experts), torch.tensor(counts))[torch.randperm(pairs, generator=torch.Generator().manual_seed(6))]
+    ids, weights = ids.to(torch.int32).to(DEV), _randn(pairs, seed=7).abs()
+    got = []
+    for tile in (128, ops.kernels.EXPERT_TILE_ROWS):
+        plan = ops.moe_sort(ids, experts, tile)
+        rows = ops.moe_gather(x, plan, 1, torch.empty_like(x))
+        act = ops.moe_grouped_tcgen05("gate_up", rows, w, torch.empty(pairs, ff, dtype=dtype, device=DEV), plan)
+        each = ops.moe_grouped_tcgen05("down", act, down, torch.empty_like(x), plan, pair_weights=weights)
+        got.append(torch.empty_like(x).index_copy_(0, plan.order.long(), each))
+    assert torch.equal(*got) and ops.gemm_error_flag(DEV) == 0
+
+
 def test_router_gives_every_row_an_expert_whatever_it_holds():
     """A row of padding may hold anything (what an attention that found no work left in its output): NaN and
     infinities still choose experts inside the table, so that nothing behind the router reads out of bounds."""
