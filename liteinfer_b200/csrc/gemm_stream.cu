@@ -13,10 +13,12 @@
 // Because w depends on no earlier kernel, a block fills its rings before it waits for the kernel ahead of it
 // (programmatic dependent launch), and it lets the kernel behind it start at once: with at most one block of 97 KB
 // per SM, two such kernels fit on an SM side by side, so the next product's first 14 MB are on their way while
-// this one still runs, and a chain of products reads memory without the pause that a launch otherwise costs.
+// this one still runs, and a chain of products reads memory without the pause that a launch otherwise costs.  (Not beside the
+// blocks of 160 KB that a weight of many long rows gets: see plan_and_launch.)
 //
-// The warps of a block split a tile's k among them (chunk c goes to warp c mod 8) and add their partial tiles
-// through shared memory in warp order at the end of each tile; the order of every sum is fixed by the shapes.
+// The warps of a block, six or eight by the plan, split a tile's k among them (chunk c goes to warp c mod 8, or 6) and add
+// their partial tiles through shared memory in warp order at the end of each tile; the order of every sum is fixed by the
+// shapes, the number of rows of x among them.
 // Epilogues: bias; act(gate) * up on weights whose rows are interleaved in eights; or the residual sum
 // (out += product) with the new rows' sums of squares per tile.
 //
@@ -342,6 +344,21 @@ static int launch_stream_gemm(const CUtensorMap& map, const StreamParams& p, int
                                  dim3(kWarps * 32), stream_gemm_smem<kWarps, kRing>(), stream, map, p);
 }
 
+// Rows of 19 to 32 chunks of k, whose x does not fit the registers of two blocks of six warps an SM: one block of eight warps with
+// deep rings, at most three or four chunks a warp, keeps it there all the same.  Without, every warp reads its share of x again
+// for every tile.  Measured on B200 over weights that no cache holds, the six-warp form in brackets: 4,800 x 4096 7.7 us (10.0)
+// at one row, 7.9 (12.1) at eight; 9,440 x 4096 12.2 (13.3) and 12.8 (14.4); 38,400 x 3072 36.4 (36.9) and 37.8 (39.5).  What it
+// loses is the second block's start of a tile while the first ends one, so one row, which has little of x to read, and the
+// shortest of these rows need a reason in the rounds that the tiles take, one block an SM against two: 9,440 x 2312 8.8 us with
+// six warps at one row and 9.4 with eight (four rounds either way), 5,920 x 2312 7.2 and 6.6 (three rounds against four);
+// 14,208 x 2432 at four rows 1.01 times the six-warp form's.  A weight of very many tiles gains nothing:
+// 128256 x 4096 152 us with six warps, 158 with eight.
+static bool worth_one_block(int tiles, int sms, int chunks, int M) {
+  if (tiles > 24 * sms) return false;
+  const int rounds = (tiles + sms - 1) / sms, two_blocks = 2 * ((tiles + 2 * sms - 1) / (2 * sms));
+  return chunks >= 22 || (M > 1 && chunks >= 20) || (rounds < two_blocks && (M > 1 || rounds <= 5));
+}
+
 // A weight of few tiles (at most two for every SM: the projections around the attention, the down projection) gives
 // every tile a block of eight warps that split k.  A weight of more tiles gets two blocks of six warps per SM, which
 // walk over the tiles; the smaller blocks leave a level-one cache that holds x.  Measured on B200 at 8 rows
@@ -360,17 +377,14 @@ static int plan_and_launch(const CUtensorMap& map, const StreamParams& p, cudaSt
     case 'f': return launch_stream_gemm<NT, 12, 3, false>(map, p, tiles <= 2 * sms ? tiles : sms, stream);
     case 'd': return launch_stream_gemm<NT, 6, 3, true>(map, p, min(2 * sms, (tiles + 5) / 6), stream);
     case 'c':
-      // (with at most three chunks of k a warp and one tile of rows, a warp keeps its share of x in registers)
-      if (NT == 1 && (p.K + kChunkK - 1) / kChunkK <= 18 && !getenv("LITEINFER_STREAM_NO_X_CACHE"))
-        return launch_stream_gemm<1, 6, 3, false, 3>(map, p, min(tiles, 2 * sms), stream);
-      // Longer rows, whose x does not fit those registers: one block of eight warps per SM with deep rings, at most three or
-      // four chunks of k a warp, so that x stays in registers all the same.  Without, every warp reads its share of x again
-      // for every tile.  Measured on B200 at 3 rows: 28672 x 4096 with its activation 34.4 us (39.8), 6144 x 4096 8.5 (11.8),
-      // at 8 rows 16384 x 3072 16.1 (18.5); a decode step of three sequences at the 8B sizes 3,243 us (3,439).  A weight of
-      // very many tiles gains more from two blocks' rings than from x at hand: 128256 x 4096 152 us with them, 158 without.
-      if (NT == 1 && tiles <= 24 * sms) {
-        if ((p.K + kChunkK - 1) / kChunkK <= 24) return launch_stream_gemm<1, 8, 5, false, 3>(map, p, min(tiles, sms), stream);
-        if ((p.K + kChunkK - 1) / kChunkK <= 32) return launch_stream_gemm<1, 8, 5, false, 4>(map, p, min(tiles, sms), stream);
+      if constexpr (NT == 1) {
+        static const bool keep_x = !getenv("LITEINFER_STREAM_NO_X_CACHE");
+        const int chunks = (p.K + kChunkK - 1) / kChunkK;
+        // (with at most three chunks of k a warp and one tile of rows, a warp keeps its share of x in registers)
+        if (keep_x && chunks <= 18) return launch_stream_gemm<1, 6, 3, false, 3>(map, p, min(tiles, 2 * sms), stream);
+        if (keep_x && chunks <= 32 && worth_one_block(tiles, sms, chunks, p.M))
+          return chunks <= 24 ? launch_stream_gemm<1, 8, 5, false, 3>(map, p, min(tiles, sms), stream)
+                              : launch_stream_gemm<1, 8, 5, false, 4>(map, p, min(tiles, sms), stream);
       }
       return launch_stream_gemm<NT, 6, 3, false>(map, p, min(tiles, 2 * sms), stream);
     default: return launch_stream_gemm<NT, 8, 3, false>(map, p, tiles <= 2 * sms ? tiles : sms, stream);

@@ -1005,9 +1005,11 @@ def test_fused_decode_layer_chain_matches_the_unfused_one(monkeypatch):
     torch.testing.assert_close(s2.sumsq.sum(0), b.float().pow(2).sum(-1), rtol=1e-5, atol=1e-5)
 
 
-# More tiles than two for every SM with rows of 19 to 24 chunks of 128 k, of 25 to 32 and of more; and very many tiles.
+# More tiles than two for every SM with rows of 19 to 24 chunks of 128 k, of 25 to 32 and of more; and very many tiles; short rows
+# in rounds of tiles that one block of eight warps and two of six take alike, and that they do not.
 @pytest.mark.parametrize("M", [1, 8, 9])
-@pytest.mark.parametrize("N,K", [(4752, 2312), (6144, 3072), (5001, 3080), (9000, 4096), (4752, 4104), (57000, 2440)])
+@pytest.mark.parametrize("N,K", [(4752, 2312), (6144, 3072), (5001, 3080), (9000, 4096), (4752, 4104), (57000, 2440),
+                                 (8000, 2312), (14208, 2560), (17600, 2440), (8000, 2816)])
 def test_gemm_stream_of_long_rows(M, N, K):
     from liteinfer_b200 import ops
 
