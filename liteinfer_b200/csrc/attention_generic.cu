@@ -34,6 +34,7 @@ constexpr int kMaxKeyDim = 1024;
 constexpr int kQueriesPerBlock = 8;
 constexpr int kUnit = 32;
 constexpr int kMostWarps = 16;
+constexpr int kSms = 148;
 
 template <typename T>
 struct GenericParams {
@@ -300,14 +301,20 @@ LI_EXPORT int li_paged_attention_generic(int dtype, const void* q, int q_row_str
   if (head_dim < 1 || head_dim > kMaxKeyDim || kv_heads < 1 || heads % kv_heads) return LI_ERR_UNSUPPORTED;
   if (v_dim < 1 || v_dim > 32 * 32) return LI_ERR_UNSUPPORTED;
   if (kv_heads > 65535 || num_seqs > 65535) return LI_ERR_UNSUPPORTED;
-  // Few rows a block (decode): more warps share a row's units.  Single tokens of few sequences: a block for every row, whose
-  // warps then walk sixteen units at once (12 sequences of 19 to 190 keys, 12 heads on 4: 9.2 us a launch, 12.9 with the three
-  // rows of a KV head in a block; 64 sequences of 500, whose keys every row's block would fetch again: 72 and 52).
+  // Single tokens of few sequences: a block for every row, whose warps then walk many units at once (12 sequences of 19 to 190
+  // keys, 12 heads on 4: 9.2 us a launch, 12.9 with the three rows of a KV head in a block; 64 sequences of 500, whose keys
+  // every row's block would fetch again: 72 and 52).
   const int groups = heads / kv_heads;
-  const bool row_blocks = max_q_len == 1 && groups > 1 && (long)num_seqs * heads <= 2 * 148;
+  const bool row_blocks = max_q_len == 1 && groups > 1 && (long)num_seqs * heads <= 2 * kSms;
   const int rows = row_blocks ? 1 : (max_q_len < kQueriesPerBlock ? max_q_len : kQueriesPerBlock) * groups;
-  const int threads = rows >= 8 || v_dim > 256 ? 256 : 32 * kMostWarps;
   const dim3 grid(row_blocks ? groups : (max_q_len + kQueriesPerBlock - 1) / kQueriesPerBlock, kv_heads, num_seqs);
+  // Few rows a block (decode): as many warps share a row's units as keep an SM busy with the blocks that it gets.  Sixteen warps
+  // for every block, however many there are, had most of them wait at the barriers of rows of a unit or two: 256
+  // sequences of 16 keys at 16 heads took 120 us (55 with a warp a row; now 22), of 500 keys 383 (248), while 8 sequences of
+  // 1,500 keys take 37 us with sixteen warps, 53 with eight and 69 with four.
+  const long blocks = (long)grid.x * grid.y * grid.z;
+  const int warps = blocks <= kSms ? kMostWarps : blocks <= 2 * kSms ? kMostWarps / 2 : blocks <= 4 * kSms ? kMostWarps / 4 : kMostWarps / 8;
+  const int threads = rows >= 8 ? 256 : 32 * (v_dim > 256 && warps > 8 ? 8 : warps);
   const auto run = [&](auto p) {
     p.block_table = block_table, p.query_start_loc = query_start_loc, p.context_lens = context_lens, p.sink = sink;
     p.q_row_stride = q_row_stride, p.out_row_stride = out_row_stride, p.table_stride = table_stride;

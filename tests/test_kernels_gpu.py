@@ -326,6 +326,32 @@ def test_generic_attention_cuts_agree_bit_for_bit(heads, kv_heads, head_dim, pag
         assert torch.equal(attend(start, count), whole[start:start + count]), (start, count)
 
 
+# As many sequences as give a block sixteen warps, eight, four and two, at rows of less than a unit of keys and of many.
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(16, 16, 64), (12, 4, 128), (8, 8, 300)])
+def test_generic_attention_of_any_number_of_sequences(heads, kv_heads, head_dim):
+    from liteinfer_b200 import ops
+
+    lengths = [1, 31, 33, 400]
+    case = _paged_case(torch.float32, heads, kv_heads, head_dim, 16, [1] * 4, lengths)
+    case["k_pool"].copy_(_randn(*case["k_pool"].shape, dtype=torch.float32, seed=5))
+    case["v_pool"].copy_(_randn(*case["v_pool"].shape, dtype=torch.float32, seed=6))
+
+    def attend(n):
+        qkv = case["qkv"][:4].repeat(n // 4, 1)
+        out = torch.empty(n, heads * head_dim, device="cuda")
+        return ops.paged_attention_generic(qkv, qkv.stride(0), out, case["k_pool"], case["v_pool"], case["table"].repeat(n // 4, 1),
+                                           torch.arange(n + 1, dtype=torch.int32, device="cuda"), case["ctx"].repeat(n // 4), n, 1,
+                                           heads, kv_heads, head_dim, head_dim ** -0.5)
+
+    few = attend(4)
+    want = torch.empty_like(few)
+    ref.paged_attention(case["qkv"], case["qkv"].shape[1], want, case["k_pool"], case["v_pool"], case["table"], case["qsl"], case["ctx"],
+                        4, 1, heads, kv_heads, head_dim, head_dim ** -0.5, 0)
+    torch.testing.assert_close(few, want, **_tol(torch.float32))
+    for n in (8, 12, 20, 36, 40, 80, 152):
+        assert torch.equal(attend(n), few.repeat(n // 4, 1)), n
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_attention_finds_one_far_key(dtype):
     """One key among hundreds is made to dominate: the output must be that key's value, wherever its page lies."""
