@@ -41,14 +41,20 @@ __device__ __forceinline__ void copy16_async(float* dst, const float* src, int b
                "r"(bytes));
 }
 
-// Four neighbours along k, `left` of which exist: to shared memory, asynchronously where `vec` (the row lies on 16 bytes).
+__device__ __forceinline__ void copy4_async(float* dst, const float* src, int bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes));
+}
+
+// Four neighbours along k, `left` of which exist, to shared memory: at once where `vec` (the row lies on 16 bytes).  (What does not
+// exist is filled with zeros; the address is then the row's last number's.)  32-bit numbers go asynchronously either way: 3,000 rows
+// of 5000 x 770 740 us, 859 when a thread waited for its four, 300 rows of 3072 x 2049 171 and 209.
 __device__ __forceinline__ void stage_four(float* dst, const float* src, int left, bool vec) {
   if (vec) {
     copy16_async(dst, left > 0 ? src : src - (4 - left) / 4 * 4, left > 0 ? 16 : 0);   // K is a multiple of four
     return;
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) dst[i] = i < left ? src[i] : 0.f;
+  for (int i = 0; i < 4; ++i) copy4_async(dst + i, src + min(i, left - 1), i < left ? 4 : 0);
 }
 __device__ __forceinline__ void stage_four(float* dst, const bf16* src, int left, bool vec) {
   if (vec && left > 0) {
