@@ -126,6 +126,12 @@ struct Share {
   }
 };
 
+// The barrier of a row's blocks; a row that is one block's has no use for a cluster's.
+__device__ __forceinline__ void row_sync(const cg::cluster_group& cluster) {
+  if (cluster.num_blocks() > 1) cluster.sync();
+  else __syncthreads();
+}
+
 __device__ __forceinline__ unsigned long long warp_inclusive(unsigned long long v, int lane) {
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -144,7 +150,7 @@ __device__ void find_boundary(SampleSmem& sm, int buf, bool wide, unsigned long 
   cg::cluster_group cluster = cg::this_cluster();
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   if (t == 0) sm.chosen = -1;
-  cluster.sync();
+  row_sync(cluster);
   static_assert(kBins == 2 * kSampleThreads, "two bins a thread");
   unsigned long long a = 0, b = 0;
   const int ranks = (int)cluster.num_blocks();
@@ -307,7 +313,7 @@ __device__ Keep select_prefix(Share<S>& share, bool all_in, Keep within, unsigne
       sm.exchange[slot] = all;
       sm.exchange[slot + 1] = (unsigned long long)vocab;
     }
-    cluster.sync();
+    row_sync(cluster);
     unsigned long long before = 0;
     for (unsigned r = 0; r < cluster.block_rank(); ++r) before += *cluster.map_shared_rank(&sm.exchange[slot], r);
     for (int k = 0; k < w; ++k) before += sm.warp[k];
@@ -330,7 +336,7 @@ __device__ Keep select_prefix(Share<S>& share, bool all_in, Keep within, unsigne
         left -= here;
       }
     }
-    cluster.sync();
+    row_sync(cluster);
     int cut = vocab;
     for (unsigned r = 0; r < cluster.num_blocks(); ++r) cut = min(cut, (int)*cluster.map_shared_rank(&sm.exchange[slot + 1], r));
     out.tie_cut = cut;
@@ -400,13 +406,13 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, bool stag
   }
   const ArgMax block_top = block_argmax(mine, sm.warp_best);
   if (threadIdx.x == 0) sm.best = block_top;
-  cluster.sync();
+  row_sync(cluster);
   ArgMax top = *cluster.map_shared_rank(&sm.best, 0);
   for (int k = 1; k < ranks; ++k) top = better(top, *cluster.map_shared_rank(&sm.best, k));
 
   if (greedy) {
     if (rank == 0 && threadIdx.x == 0) out[r] = top.i;
-    cluster.sync();          // the others may still read this block's maximum
+    row_sync(cluster);          // the others may still read this block's maximum
     return;
   }
   const int part_size = (share.n + kSampleWarps - 1) / kSampleWarps;
@@ -438,6 +444,7 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, bool stag
   // Draw: the first index (ascending) at which the running weight passes uniform * total.
   const int from = share.from, to = share.to;
   unsigned long long part = 0;
+#pragma unroll 4
   for (int j = from + lane; j < to; j += 32) {
     const int i = share.column(j);
     const float x = share.value(i);
@@ -453,7 +460,7 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, bool stag
     for (int i = 0; i < kSampleWarps; ++i) all += sm.warp[i];
     sm.exchange[slot] = all;
   }
-  cluster.sync();
+  row_sync(cluster);
   unsigned long long before = 0, total = 0;
   for (int i = 0; i < ranks; ++i) {
     const unsigned long long v = *cluster.map_shared_rank(&sm.exchange[slot], i);
@@ -468,24 +475,39 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, bool stag
   if (total == 0) {                      // the maximum weighs 2^32: only a row without finite values comes here
     if (rank == 0 && threadIdx.x == 0) out[r] = top.i;
   } else if (part > 0 && before <= target && target < before + part) {
-    for (int j = from; j < to; j += 32) {
-      int i = 0;
-      unsigned long long weight = 0;
-      if (j + lane < to) {
-        i = share.column(j + lane);
-        const float x = share.value(i);
-        if (keep.has(ordered_key(x), share.base + i)) weight = share.weight(x);
+    // Four neighbouring columns a lane at a time: the walk is one warp's, so what it takes is its steps one after the other.
+    for (int j = from; j < to; j += 128) {
+      unsigned long long each[4], sum = 0;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int at = j + lane * 4 + e;
+        each[e] = 0;
+        if (at < to) {
+          const int i = share.column(at);
+          const float x = share.value(i);
+          if (keep.has(ordered_key(x), share.base + i)) each[e] = share.weight(x);
+        }
+        sum += each[e];
       }
-      const unsigned long long upto = before + warp_inclusive(weight, lane);
+      const unsigned long long upto = before + warp_inclusive(sum, lane);
       const unsigned passed = __ballot_sync(0xffffffffu, upto > target);
       if (passed) {
-        if (lane == __ffs(passed) - 1) out[r] = share.base + i;
+        if (lane == __ffs(passed) - 1) {
+          int e = 0;
+          unsigned long long run = upto - sum;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            run += each[k];
+            e += run <= target;
+          }
+          out[r] = share.base + share.column(j + lane * 4 + e);
+        }
         break;
       }
       before = __shfl_sync(0xffffffffu, upto, 31);
     }
   }
-  cluster.sync();            // nobody leaves while another block reads
+  row_sync(cluster);            // nobody leaves while another block reads
 }
 
 template <typename T, typename S>
