@@ -126,10 +126,11 @@ struct Share {
   }
 };
 
-// The barrier of a row's blocks; a row that is one block's has no use for a cluster's.
+// The barrier of a row's blocks; a row that is one block's (kAlone) has no use for a cluster's.
+template <bool kAlone>
 __device__ __forceinline__ void row_sync(const cg::cluster_group& cluster) {
-  if (cluster.num_blocks() > 1) cluster.sync();
-  else __syncthreads();
+  if constexpr (kAlone) __syncthreads();
+  else cluster.sync();
 }
 
 __device__ __forceinline__ unsigned long long warp_inclusive(unsigned long long v, int lane) {
@@ -144,13 +145,13 @@ __device__ __forceinline__ unsigned long long warp_inclusive(unsigned long long 
 // Sums the blocks' histograms `buf` and finds the last non-empty bin whose preceding weight is within the limit
 // (`whole`: the limit is the share `top_p` of the whole sum, and is left in `limit`).  Every thread returns with the bin,
 // the weight before it and its own weight.
-template <bool unit>
+template <bool unit, bool kAlone>
 __device__ void find_boundary(SampleSmem& sm, int buf, bool wide, unsigned long long above, bool whole, float top_p,
                               unsigned long long& limit, int& chosen, unsigned long long& before, unsigned long long& mass) {
   cg::cluster_group cluster = cg::this_cluster();
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   if (t == 0) sm.chosen = -1;
-  row_sync(cluster);
+  row_sync<kAlone>(cluster);
   static_assert(kBins == 2 * kSampleThreads, "two bins a thread");
   unsigned long long a = 0, b = 0;
   const int ranks = (int)cluster.num_blocks();
@@ -203,7 +204,7 @@ __device__ void find_boundary(SampleSmem& sm, int buf, bool wide, unsigned long 
 // whose preceding weight sum is within the limit.  `unit` weights count elements (top-k with limit k - 1); otherwise the
 // weight is exp(x - row_max) in 2^-32 fixed point (top-p with limit p * total).  `turn`: the histogram to use next;
 // `slot`: the next free exchange.  Lists what survives the first histogram.
-template <typename S, bool unit>
+template <typename S, bool unit, bool kAlone>
 __device__ Keep select_prefix(Share<S>& share, bool all_in, Keep within, unsigned long long limit, float top_p, int vocab,
                               int& turn, int& slot, SampleSmem& sm) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -244,7 +245,7 @@ __device__ Keep select_prefix(Share<S>& share, bool all_in, Keep within, unsigne
       }
     }
     int chosen;
-    find_boundary<unit>(sm, turn, wide, above, !unit && level == 0, top_p, limit, chosen, above, mass);
+    find_boundary<unit, kAlone>(sm, turn, wide, above, !unit && level == 0, top_p, limit, chosen, above, mass);
     turn ^= 1;
     if (chosen < 0) return within;
     if (level == 0) {
@@ -313,7 +314,7 @@ __device__ Keep select_prefix(Share<S>& share, bool all_in, Keep within, unsigne
       sm.exchange[slot] = all;
       sm.exchange[slot + 1] = (unsigned long long)vocab;
     }
-    row_sync(cluster);
+    row_sync<kAlone>(cluster);
     unsigned long long before = 0;
     for (unsigned r = 0; r < cluster.block_rank(); ++r) before += *cluster.map_shared_rank(&sm.exchange[slot], r);
     for (int k = 0; k < w; ++k) before += sm.warp[k];
@@ -336,7 +337,7 @@ __device__ Keep select_prefix(Share<S>& share, bool all_in, Keep within, unsigne
         left -= here;
       }
     }
-    row_sync(cluster);
+    row_sync<kAlone>(cluster);
     int cut = vocab;
     for (unsigned r = 0; r < cluster.num_blocks(); ++r) cut = min(cut, (int)*cluster.map_shared_rank(&sm.exchange[slot + 1], r));
     out.tie_cut = cut;
@@ -347,7 +348,7 @@ __device__ Keep select_prefix(Share<S>& share, bool all_in, Keep within, unsigne
 
 // Grid: rows x (cluster size) blocks, a row's in one cluster.  `staged`: a block's share lies in its shared memory behind
 // `sm`, as S: the logits as they are, or as float, divided by the temperature.
-template <typename T, typename S>
+template <typename T, typename S, bool kAlone>
 __global__ void __launch_bounds__(kSampleThreads, sizeof(S) == 2 ? 3 : 2)
 sample_kernel(const T* __restrict__ logits, int vocab, int share_size, bool staged, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ uniform,
@@ -406,13 +407,13 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, bool stag
   }
   const ArgMax block_top = block_argmax(mine, sm.warp_best);
   if (threadIdx.x == 0) sm.best = block_top;
-  row_sync(cluster);
+  row_sync<kAlone>(cluster);
   ArgMax top = *cluster.map_shared_rank(&sm.best, 0);
   for (int k = 1; k < ranks; ++k) top = better(top, *cluster.map_shared_rank(&sm.best, k));
 
   if (greedy) {
     if (rank == 0 && threadIdx.x == 0) out[r] = top.i;
-    row_sync(cluster);          // the others may still read this block's maximum
+    row_sync<kAlone>(cluster);          // the others may still read this block's maximum
     return;
   }
   const int part_size = (share.n + kSampleWarps - 1) / kSampleWarps;
@@ -438,13 +439,12 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, bool stag
   const bool by_count = k > 0 && k < vocab;
   int turn = 0, slot = 0;
   Keep keep{0u, vocab};  // every finite value has a key > 0
-  if (by_count) keep = select_prefix<S, true>(share, true, keep, (unsigned long long)(k - 1), 0.f, vocab, turn, slot, sm);
-  if (p > 0.f && p < 1.f) keep = select_prefix<S, false>(share, !by_count, keep, 0, p, vocab, turn, slot, sm);
+  if (by_count) keep = select_prefix<S, true, kAlone>(share, true, keep, (unsigned long long)(k - 1), 0.f, vocab, turn, slot, sm);
+  if (p > 0.f && p < 1.f) keep = select_prefix<S, false, kAlone>(share, !by_count, keep, 0, p, vocab, turn, slot, sm);
 
   // Draw: the first index (ascending) at which the running weight passes uniform * total.
   const int from = share.from, to = share.to;
   unsigned long long part = 0;
-#pragma unroll 4
   for (int j = from + lane; j < to; j += 32) {
     const int i = share.column(j);
     const float x = share.value(i);
@@ -460,7 +460,7 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, bool stag
     for (int i = 0; i < kSampleWarps; ++i) all += sm.warp[i];
     sm.exchange[slot] = all;
   }
-  row_sync(cluster);
+  row_sync<kAlone>(cluster);
   unsigned long long before = 0, total = 0;
   for (int i = 0; i < ranks; ++i) {
     const unsigned long long v = *cluster.map_shared_rank(&sm.exchange[slot], i);
@@ -475,47 +475,50 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, bool stag
   if (total == 0) {                      // the maximum weighs 2^32: only a row without finite values comes here
     if (rank == 0 && threadIdx.x == 0) out[r] = top.i;
   } else if (part > 0 && before <= target && target < before + part) {
-    // Four neighbouring columns a lane at a time: the walk is one warp's, so what it takes is its steps one after the other.
-    for (int j = from; j < to; j += 128) {
-      unsigned long long each[4], sum = 0;
+    // The walk is one warp's, so what it takes is its steps one after the other: in a short row where nothing is listed, first
+    // 128 columns a step.
+    int at = from;
+    if (kAlone && !share.listed) {
+      for (; at + 128 < to; at += 128) {
+        unsigned long long sum = 0;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int at = j + lane * 4 + e;
-        each[e] = 0;
-        if (at < to) {
-          const int i = share.column(at);
+        for (int e = 0; e < 4; ++e) {
+          const int i = at + e * 32 + lane;
           const float x = share.value(i);
-          if (keep.has(ordered_key(x), share.base + i)) each[e] = share.weight(x);
+          if (keep.has(ordered_key(x), share.base + i)) sum += share.weight(x);
         }
-        sum += each[e];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (before + sum > target) break;
+        before += sum;
       }
-      const unsigned long long upto = before + warp_inclusive(sum, lane);
+    }
+    for (int j = at; j < to; j += 32) {
+      int i = 0;
+      unsigned long long weight = 0;
+      if (j + lane < to) {
+        i = share.column(j + lane);
+        const float x = share.value(i);
+        if (keep.has(ordered_key(x), share.base + i)) weight = share.weight(x);
+      }
+      const unsigned long long upto = before + warp_inclusive(weight, lane);
       const unsigned passed = __ballot_sync(0xffffffffu, upto > target);
       if (passed) {
-        if (lane == __ffs(passed) - 1) {
-          int e = 0;
-          unsigned long long run = upto - sum;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            run += each[k];
-            e += run <= target;
-          }
-          out[r] = share.base + share.column(j + lane * 4 + e);
-        }
+        if (lane == __ffs(passed) - 1) out[r] = share.base + i;
         break;
       }
       before = __shfl_sync(0xffffffffu, upto, 31);
     }
   }
-  row_sync(cluster);            // nobody leaves while another block reads
+  row_sync<kAlone>(cluster);            // nobody leaves while another block reads
 }
 
-template <typename T, typename S>
+template <typename T, typename S, bool kAlone>
 int launch_sample(const T* logits, int rows, int vocab, int ranks, int share, bool staged, const float* temperature,
                   const int* top_k, const float* top_p, const float* uniform, int* out, cudaStream_t stream) {
   const size_t smem = (sizeof(SampleSmem) + 15) / 16 * 16 + (staged ? (size_t)share * sizeof(S) : 0);
   const cudaError_t status =
-      cudaFuncSetAttribute(sample_kernel<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleMostSmem);
+      cudaFuncSetAttribute(sample_kernel<T, S, kAlone>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleMostSmem);
   if (status != cudaSuccess) return (int)status;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(rows * ranks);
@@ -529,7 +532,7 @@ int launch_sample(const T* logits, int rows, int vocab, int ranks, int share, bo
   attribute[0].val.clusterDim.z = 1;
   config.attrs = attribute;
   config.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&config, sample_kernel<T, S>, logits, vocab, share, staged, temperature, top_k, top_p,
+  return (int)cudaLaunchKernelEx(&config, sample_kernel<T, S, kAlone>, logits, vocab, share, staged, temperature, top_k, top_p,
                                  uniform, out);
 }
 
@@ -546,9 +549,12 @@ int sample_rows(const T* logits, int rows, int vocab, const float* temperature, 
   if ((long long)rows * ranks > 0x7fffffffll) return LI_ERR_UNSUPPORTED;
   const size_t room = kSampleMostSmem - (sizeof(SampleSmem) + 15) / 16 * 16;
   const bool raw = (size_t)share * sizeof(T) <= room;
-  if (sizeof(T) == 4 || ((size_t)share * 4 <= room / 2 && rows * ranks <= 2 * 148))
-    return launch_sample<T, float>(logits, rows, vocab, ranks, share, raw, temperature, top_k, top_p, uniform, out, stream);
-  return launch_sample<T, T>(logits, rows, vocab, ranks, share, raw, temperature, top_k, top_p, uniform, out, stream);
+  const bool floats = sizeof(T) == 4 || ((size_t)share * 4 <= room / 2 && rows * ranks <= 2 * 148);
+  const auto launch = [&](auto kernel) {
+    return kernel(logits, rows, vocab, ranks, share, raw, temperature, top_k, top_p, uniform, out, stream);
+  };
+  if (ranks == 1) return floats ? launch(launch_sample<T, float, true>) : launch(launch_sample<T, T, true>);
+  return floats ? launch(launch_sample<T, float, false>) : launch(launch_sample<T, T, false>);
 }
 
 template <typename T>
