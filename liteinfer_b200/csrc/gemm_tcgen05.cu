@@ -449,8 +449,8 @@ __device__ __forceinline__ float grouped_value(float v, float scale, int gated_a
 // Bound by the second-level cache: a step of 64 k brings 16 KB of w and up to 16 KB of x to each CTA for 512 cycles of
 // products, 64 bytes a cycle, about what an SM gets.  Single CTAs on 128 x 256 tiles took in 96 (and 25 % padding with 256
 // rows an expert).  Measured on B200 (32 experts
-// of 2,048 x 2,048 with a capped gate, four a token, both products): 2,048 tokens 250 us against 278, 2,048 tokens of eight experts
-// half as wide, two a token, with all around it 123 against 169, 8 tokens 130 against 148.  The activations, a row of w and a
+// of 2,048 x 2,048 with a capped gate, four a token; router, sort, gather and combine included): 2,048 tokens 284 us against 337,
+// 64 162 against 169, 8 124 against 135.  The activations, a row of w and a
 // row of x a lane, bound it with eight warps that computed each twice (378 us).
 //
 // Way out: a warp has 32 rows of w by 32 rows of x in its registers, turns them in shared memory and stores, a lane a row of
