@@ -337,7 +337,7 @@ class ModelRunner:
         self._graphs: dict[int, _DecodeGraph] = {}
         self._padded_graphs: dict[tuple, _PaddedGraph] = {}
         self._graph_limits: tuple[int, int] | None = None
-        self._context_bounds = model.context_bounds()
+        self._context_bounds: dict[tuple[int, int], tuple[int, ...]] = {}     # of the model, by prompts and their longest
         self._padded_limit = 0      # most tokens of a step that is replayed from a padded graph
         self.graph_pool = None
         self.graph_launches = 0     # launches of this package's kernels replayed from graphs
@@ -450,7 +450,10 @@ class ModelRunner:
         # launch sized for it a quarter too large); several share the step's.
         brought = [(len(e.tokens), total) for e, total in zip(entries, totals) if len(e.tokens) > 1]
         portion = _token_bucket(brought[0][0] if len(brought) == 1 else tokens)
-        context = kernels.context_class(max((total for _, total in brought), default=max_len), max_len, self._context_bounds)
+        bounds = self._context_bounds.get((prefill, portion))
+        if bounds is None:
+            bounds = self._context_bounds[prefill, portion] = self.model.context_bounds(prefill, portion)
+        context = kernels.context_class(max((total for _, total in brought), default=max_len), max_len, bounds)
         key = (_token_bucket(tokens), seqs, n_decode > 0, prefill, portion, context, rows)
         graph = self._padded_graphs.get(key)
         if graph is None:

@@ -1172,6 +1172,22 @@ ATTENTION_CONTEXTS = (448, 576)
 LATENT_CONTEXTS = (64,)
 
 
+def attention_contexts(heads: int, kv_heads: int, head_dim: int, prompts: int, longest: int) -> tuple[int, ...]:
+    """The bound of `ATTENTION_CONTEXTS` that decides a launch over `prompts` sequences of up to `longest` queries: the first while
+    its blocks and their seconds have an SM each, the second while they have a place each, and none in a launch of more blocks,
+    which is never in pairs (nor one at sizes that the tcgen05 attention does not take)."""
+    groups = heads // kv_heads
+    if head_dim not in (64, 128) or groups > 128:
+        return ()
+    rows = 128 // groups
+    if head_dim == 128 and longest > rows:
+        rows *= 2                   # two tiles of queries a block
+    blocks = 2 * kv_heads * prompts * -(-longest // rows)
+    if blocks <= NUM_SMS:
+        return ATTENTION_CONTEXTS[:1]
+    return ATTENTION_CONTEXTS[1:] if head_dim == 64 and blocks <= 2 * NUM_SMS else ()
+
+
 def context_class(longest: int, most: int, bounds: tuple[int, ...]) -> int:
     """The bound of the class that a context of `longest` tokens lies in, where none is longer than `most`."""
     return next((bound for bound in bounds if longest <= bound < most), most)

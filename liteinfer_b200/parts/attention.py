@@ -232,7 +232,10 @@ class Attention:
 
     takes_pending_norm = True       # x may be an ops.PendingNorm: the qkv product folds the norm in
     adds_to_residual = True         # the output projection adds into the residual stream where its kernel can
-    context_bounds = ops.ATTENTION_CONTEXTS
+
+    def context_bounds(self, prompts: int, longest: int) -> tuple[int, ...]:
+        """The contexts up to which the kernels for `prompts` prompts of up to `longest` tokens are chosen differently."""
+        return ops.attention_contexts(self.heads, self.kv_heads, self.head_dim, prompts, longest)
 
     def forward(self, x, ctx: StepContext, cache: LayerCache, residual: torch.Tensor | None = None):
         qkv = torch.empty((x.shape[0], self.qkv_weight.shape[0]), dtype=x.dtype, device=x.device)

@@ -38,8 +38,6 @@ def _sink_init(shape, generator):
 
 
 class LatentAttention:
-    context_bounds = ops.LATENT_CONTEXTS
-
     def __init__(self, hidden_size: int, heads: int, dim: int, rot_dim: int, vdim: int, q_rank: int | None,
                  kv_rank: int, scale: float, norm_eps: float, position: PartSpec, dtype: torch.dtype,
                  device: torch.device, sink: bool = True, gate: bool = True, own_kv: bool = True,
@@ -124,6 +122,10 @@ class LatentAttention:
 
     def cache_needs(self) -> tuple:
         return (KVNeed(1, self.kv_rank + self.rot_dim, self.window, name=self.cache_name, v_head_dim=0),)
+
+    def context_bounds(self, prompts: int, longest: int) -> tuple[int, ...]:
+        """The contexts up to which the kernels for `prompts` prompts of up to `longest` tokens are chosen differently."""
+        return ops.LATENT_CONTEXTS
 
     def forward(self, x: torch.Tensor, ctx: StepContext, cache: LayerCache) -> torch.Tensor:
         if self.own_kv == cache.read_only:

@@ -134,11 +134,13 @@ class Model:
         A part that reads device values on the host in `forward` sets `graph_safe = False`."""
         return all(getattr(part, "graph_safe", True) for _, part, _ in self._named_parts())
 
-    def context_bounds(self) -> tuple[int, ...]:
-        """The contexts, ascending, up to which the kernels of some part are chosen differently for prompts."""
-        bounds = {bound for _, part, _ in self._named_parts() for one in (part, *getattr(part, "members", ()))
-                  for bound in getattr(one, "context_bounds", ())}
-        return tuple(sorted(bounds)) if self.dtype == torch.bfloat16 else ()
+    def context_bounds(self, prompts: int, longest: int) -> tuple[int, ...]:
+        """The contexts, ascending, up to which the kernels of some part are chosen differently for `prompts` prompts of up to
+        `longest` tokens."""
+        if self.dtype != torch.bfloat16 or prompts == 0:
+            return ()
+        return tuple(sorted({bound for _, part, _ in self._named_parts() for one in (part, *getattr(part, "members", ()))
+                             if hasattr(one, "context_bounds") for bound in one.context_bounds(prompts, longest)}))
 
     def weight_bytes(self) -> int:
         seen: dict[int, int] = {}

@@ -350,10 +350,37 @@ def test_a_model_names_the_contexts_that_its_kernels_turn_at():
     from liteinfer_b200.ops import kernels
     from liteinfer_b200.parts.model import Model
 
-    def bounds(config, dtype):
+    def bounds(config, dtype, prompts=1, longest=16):
         arch, typed = resolve(config)
-        return Model(arch.build_spec(typed), dtype, torch.device("cpu")).context_bounds()
+        return Model(arch.build_spec(typed), dtype, torch.device("cpu")).context_bounds(prompts, longest)
 
-    assert bounds(tiny_configs.ALL["tiny_a"][0], torch.bfloat16) == kernels.ATTENTION_CONTEXTS
-    assert bounds(kutolix_configs.ALL["kut_a"][0], torch.bfloat16) == kernels.LATENT_CONTEXTS + kernels.ATTENTION_CONTEXTS
+    plain = dict(tiny_configs.ALL["tiny_a"][0], head_dim=64, num_attention_heads=8, num_key_value_heads=2)
+    few, more = kernels.ATTENTION_CONTEXTS
+    assert bounds(plain, torch.bfloat16) == (few,) and bounds(plain, torch.bfloat16, 4, 512) == (more,)
+    assert bounds(plain, torch.bfloat16, 8, 512) == () and bounds(plain, torch.bfloat16, 0, 512) == ()
+    assert kernels.LATENT_CONTEXTS[0] in bounds(kutolix_configs.ALL["kut_a"][0], torch.bfloat16)
     assert bounds(kutolix_configs.ALL["kut_a"][0], torch.float32) == ()
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(32, 8, 64), (24, 8, 128), (8, 1, 64), (128, 1, 128), (4, 4, 96), (6, 2, 64)])
+def test_a_graph_launches_prompt_attention_as_its_steps_would(heads, kv_heads, head_dim):
+    """Whether blocks go out in pairs is the same for a step's contexts and for the bound of their class, and a launch whose form
+    no context decides has one class."""
+    from liteinfer_b200.ops import kernels
+
+    def in_pairs(prompts, longest, context):            # the launch's own rule
+        rows = 128 // (heads // kv_heads)
+        rows *= 2 if head_dim == 128 and longest > rows else 1
+        blocks = kv_heads * prompts * -(-longest // rows)
+        return (head_dim in (64, 128) and 2 * blocks <= (296 if head_dim == 64 else 148)
+                and context > 64 * (9 if 2 * blocks > 148 else 7))
+
+    for prompts in (1, 2, 4, 16):
+        for longest in (16, 112, 448, 512, 576, 640, 1024, 2048):
+            bounds = kernels.attention_contexts(heads, kv_heads, head_dim, prompts, longest)
+            assert len(bounds) <= 1
+            for context in (2, 447, 448, 449, 576, 577, 4000, 4096):
+                stated = kernels.context_class(context, 4096, bounds)
+                assert in_pairs(prompts, longest, context) == in_pairs(prompts, longest, stated)
+            forms = {in_pairs(prompts, longest, context) for context in (2, 4096)}
+            assert len(forms) == 1 + len(bounds)
