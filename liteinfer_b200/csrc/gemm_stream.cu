@@ -378,7 +378,7 @@ static int plan_and_launch(const CUtensorMap& map, const StreamParams& p, cudaSt
     case 'd': return launch_stream_gemm<NT, 6, 3, true>(map, p, min(2 * sms, (tiles + 5) / 6), stream);
     case 'c':
       if constexpr (NT == 1) {
-        static const bool keep_x = !getenv("LITEINFER_STREAM_NO_X_CACHE");
+        const bool keep_x = !getenv("LITEINFER_STREAM_NO_X_CACHE");
         const int chunks = (p.K + kChunkK - 1) / kChunkK;
         // (with at most three chunks of k a warp and one tile of rows, a warp keeps its share of x in registers)
         if (keep_x && chunks <= 18) return launch_stream_gemm<1, 6, 3, false, 3>(map, p, min(tiles, 2 * sms), stream);
