@@ -58,16 +58,19 @@ __device__ ArgMax block_argmax(ArgMax mine, ArgMax* scratch /* 32 */) {
 //
 // Top-k and top-p are the same selection: in descending order, keep the elements whose preceding weight (1 each, or
 // the probability) is within a limit.  The first histogram bins by the distance below the row's maximum, in steps of
-// 1/46 up to where probabilities in 2^-32 vanish: the interesting values spread over hundreds of bins, so the atomics
-// rarely meet.  Elements above the boundary bin are in, those below are out; the others are told apart by histograms over
-// ever narrower ranges of their keys (two more, as a rule).  What can still be chosen is listed after the first histogram,
-// in the order of the columns, so the passes behind it walk a few hundred columns instead of the vocabulary.
+// 1/73 for 14 units: the interesting values spread over hundreds of bins, so the atomics rarely meet, and the last bin takes
+// the rest, whose weight is added up in registers.  Elements above the boundary bin are in, those below are out.  The walk
+// behind the histogram lists what can still be chosen, in the order of the columns, and picks out what has to be told apart:
+// the boundary bin, or for a top-k that leaves no more than kCandidates, everything.  Those few are sorted, by every block for
+// itself (top-p), or by one block that then finishes the row alone, top-p and draw included (top-k).  Where they are more (equal
+// values, a flat row, a share of 2^16 columns) histograms over ever narrower ranges of keys tell them apart, each a meeting of the blocks.
 //
-// Bound by the instructions of the passes over the whole row (load and maximum, histogram, listing) and by the
-// barriers between the others (a pass over 16,000 columns with a division and an exponential each takes a block some 10 us
-// when three share an SM).  Measured on B200, 48 rows of 128,256 bfloat16 logits, all kinds of parameters: 83 us, against
-// 2,075 for a block of 1,024 threads a row that read the row from L2 a dozen times, with 64-bit atomics into 256 bins of
-// the key's bits, most of them into the same bin, and one thread that walked the bins; one row with top-k and top-p: 50 us.
+// Bound by the walks over the whole row (load and maximum 6,400 cycles, histogram 5,000 to 16,000, listing 5,000 to 12,000 for
+// 16,000 columns a block) and by what a meeting costs: a cluster barrier and the reads of eight blocks' memory behind it, 2,000
+// to 6,000 cycles.  Walks take four columns a lane, so that one trip's latencies cover four columns and what is kept of them is
+// placed by three ballots; all that a lane needs from other blocks is asked for before the first of it is used.
+// Measured on B200, 128,256 bfloat16 columns, 48 rows: all kinds of parameters 55.9 us (85.2 with a histogram per level of keys,
+// one column a lane), top-k 50 37.1 (47.4), top-p 0.9 68.9 (98.5), both 45.7 (86.9); one row 22.8 (33.0), 37.1 (47.4), 28.7 (49.4).
 constexpr int kSampleThreads = 512, kSampleWarps = kSampleThreads / 32;
 constexpr int kMostRanks = 8;      // blocks of a row's cluster
 // A row of no more columns is one block's, and so on.  The passes over a share get longer, but there are fewer blocks to meet at
@@ -76,8 +79,9 @@ constexpr int kMostRanks = 8;      // blocks of a row's cluster
 constexpr int kRankColumns = 8192;
 constexpr int kBins = 1024;
 constexpr int kListed = 512;       // columns that a warp can list; where one has more its block goes on walking its whole share
+constexpr int kCandidates = 1024;  // elements of a row that are sorted at once, two a thread
 constexpr int kSampleMostSmem = 200 << 10;
-constexpr float kBinsPerUnit = 46.f;   // (kBins - 1) / 46 = 22.24 > 32 ln 2: a value in the last bin has no probability left
+constexpr float kBinsPerUnit = 73.f;   // the last bin holds all that lies 14 and more below the maximum
 
 struct Keep {        // the surviving set: key > beta, or key == beta and index <= tie_cut
   uint32_t beta;
@@ -92,38 +96,64 @@ struct SampleSmem {
   unsigned long long exchange[8];           // what other blocks of the cluster read, one slot per exchange
   unsigned long long warp[kSampleWarps];
   ArgMax warp_best[32];
-  ArgMax best;
+  ArgMax best[kMostRanks];                  // of every block of the row
   unsigned long long before, mass;          // of the boundary bin
   int chosen;
+  int found;                                // entries of `cand`, or more where it did not hold them all
+  Keep keep;
   uint16_t list[kSampleWarps][kListed];
+  unsigned long long cand[kCandidates];     // this block's elements of the boundary bin (top-k: and of those above it)
 };
 
 // One block's share of a row: columns [base, base + n) of it, whose element i lies at data[i] (in shared memory, or the row
 // itself where a share does not fit).  The walks over a share go warp by warp: each warp has a run of columns, and once
 // `listed` is set a list of those of its columns that still count, so a walk is in the order of the columns.
-template <typename S>
+template <typename S, bool kStaged>
 struct Share {
   const S* data;
   const uint16_t* list;      // this warp's list
   int n, base;
   int from, to;              // this warp's columns, or the length of its list (from 0)
-  bool listed, divided;      // divided: data holds value / temperature
+  bool listed;
+  bool undivided;            // data holds value, not value / temperature
   bool wide;                 // the row's shares have 2^16 columns or more
   float temp, row_max;
   float bin_max, bin_scale;  // the maximum as it is stored in `data`, and bins per unit of what is stored there
   uint32_t max_key;
   __device__ __forceinline__ int column(int j) const { return listed ? list[j] : j; }
-  __device__ __forceinline__ float value(int i) const { return divided ? to_float(data[i]) : to_float(data[i]) / temp; }
-  __device__ __forceinline__ unsigned long long weight(float x) const {
-    return (unsigned long long)(expf(x - row_max) * 4294967296.0f);
+  // Four neighbours as they are stored, i a multiple of four (what lies behind the share's end has no meaning).
+  __device__ __forceinline__ void four(int i, float (&f)[4]) const {
+    if constexpr (kStaged) {
+      if constexpr (sizeof(S) == 4) {
+        const float4 v = *reinterpret_cast<const float4*>(data + i);
+        f[0] = v.x, f[1] = v.y, f[2] = v.z, f[3] = v.w;
+      } else {
+        const uint2 v = *reinterpret_cast<const uint2*>(data + i);
+        f[0] = __uint_as_float(v.x << 16), f[1] = __uint_as_float(v.x & 0xffff0000u);
+        f[2] = __uint_as_float(v.y << 16), f[3] = __uint_as_float(v.y & 0xffff0000u);
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) f[e] = i + e < n ? to_float(data[i + e]) : 0.f;
+    }
   }
-  // Never rises with the value, and equal values divided by the temperature are in one bin.  A difference that is no
+  __device__ __forceinline__ float quotient(float stored) const {
+    if constexpr (kStaged && sizeof(S) == 4) return stored;
+    else return undivided ? stored / temp : stored;
+  }
+  __device__ __forceinline__ float value(int i) const { return quotient(to_float(data[i])); }
+  __device__ __forceinline__ unsigned long long weight(float x) const {
+    const float scaled = expf(x - row_max) * 4294967296.0f;
+    return scaled < 4294967296.0f ? (unsigned long long)(uint32_t)scaled : (unsigned long long)scaled;
+  }
+  // The bin never rises with the value, and equal values divided by the temperature are in one bin.  A difference that is no
   // number (infinities, NaN) goes by the key.
-  __device__ __forceinline__ int bin(int i) const {
-    const float stored = to_float(data[i]), d = bin_max - stored;
-    if (!(d >= 0.f)) return ordered_key(divided ? stored : stored / temp) >= max_key ? 0 : kBins - 1;
+  __device__ __forceinline__ int bin_of(float stored) const {
+    const float d = bin_max - stored;
+    if (!(d >= 0.f)) return ordered_key(quotient(stored)) >= max_key ? 0 : kBins - 1;
     return (int)fminf(d * bin_scale, (float)(kBins - 1));
   }
+  __device__ __forceinline__ int bin(int i) const { return bin_of(to_float(data[i])); }
 };
 
 // The barrier of a row's blocks; a row that is one block's (kAlone) has no use for a cluster's.
@@ -142,6 +172,127 @@ __device__ __forceinline__ unsigned long long warp_inclusive(unsigned long long 
   return v;
 }
 
+// A candidate: its key above its index counted down, so that descending order is the selection's (equal values by ascending
+// index).  Zero is none: it sorts last.
+__device__ __forceinline__ unsigned long long candidate(uint32_t key, int i) {
+  return (unsigned long long)key << 32 | (0xffffffffu - (uint32_t)i);
+}
+__device__ __forceinline__ float key_value(uint32_t key) {
+  return __uint_as_float((key & 0x80000000u) ? key & 0x7fffffffu : ~key);
+}
+
+// Sorts a block's numbers in descending order: thread t holds the t-th and, H = 2, the (t + 512)-th of the first `many` (a power
+// of two, 32 or more).  A bitonic network; steps within a warp are shuffles, the others meet in `a`.
+template <int H>
+__device__ __forceinline__ void sort_down_by(unsigned long long (&v)[2], int many, unsigned long long* a) {
+  const int t = threadIdx.x;
+  const bool active = H == 2 || t < many;            // whole warps
+  const auto step = [&](int size, int stride, const unsigned long long (&other)[2]) {
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const bool greater = (((t + h * kSampleThreads) & size) == 0) == ((t & stride) == 0);
+      v[h] = (v[h] > other[h]) == greater ? v[h] : other[h];
+    }
+  };
+#pragma unroll 1
+  for (int size = 2; size <= many; size <<= 1) {
+#pragma unroll 1
+    for (int stride = size >> 1; stride >= 32; stride >>= 1) {
+      if (H == 2 && stride == kSampleThreads) {
+        const unsigned long long hi = max(v[0], v[1]), lo = min(v[0], v[1]);
+        v[0] = hi;
+        v[1] = lo;
+        continue;
+      }
+      unsigned long long other[2];
+      if (active) {
+#pragma unroll
+        for (int h = 0; h < H; ++h) a[t + h * kSampleThreads] = v[h];
+      }
+      __syncthreads();
+      if (active) {
+#pragma unroll
+        for (int h = 0; h < H; ++h) other[h] = a[(t ^ stride) + h * kSampleThreads];
+      }
+      __syncthreads();
+      if (active) step(size, stride, other);
+    }
+    if (active) {
+#pragma unroll
+      for (int stride = 16; stride > 0; stride >>= 1) {
+        if (stride >= size) continue;
+        unsigned long long other[2];
+#pragma unroll
+        for (int h = 0; h < H; ++h) other[h] = __shfl_xor_sync(0xffffffffu, v[h], stride);
+        step(size, stride, other);
+      }
+    }
+  }
+}
+__device__ __noinline__ void sort_down(unsigned long long (&v)[2], int many, unsigned long long* a) {
+  if (many > kSampleThreads) sort_down_by<2>(v, many, a);
+  else sort_down_by<1>(v, many, a);
+}
+
+// Inclusive sums over the first `many` of a block's 1,024 numbers (those behind are zero), thread t holding the t-th and the
+// (t + 512)-th; returns the sum of all.
+__device__ unsigned long long scan_both(unsigned long long (&v)[2], int many, SampleSmem& sm) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned long long all = 0;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    if (h * kSampleThreads >= many) break;
+    v[h] = warp_inclusive(v[h], lane);
+    __syncthreads();
+    if (lane == 31) sm.warp[w] = v[h];
+    __syncthreads();
+    unsigned long long start = all;
+#pragma unroll
+    for (int i = 0; i < kSampleWarps; ++i) {
+      const unsigned long long part = sm.warp[i];
+      if (i < w) start += part;
+      all += part;
+    }
+    v[h] += start;
+  }
+  return all;
+}
+
+__device__ __forceinline__ int power_above(int n) { return n <= 32 ? 32 : 1 << (32 - __clz(n - 1)); }
+
+// The candidates of all blocks of a row, thread t taking the t-th and the (t + 512)-th.  Behind a barrier of the row.
+// Returns how many there are, or more than kCandidates where a block did not hold all of its own.
+__device__ int gather_candidates(unsigned long long (&v)[2], SampleSmem& sm) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int ranks = (int)cluster.num_blocks();
+  int count[kMostRanks], all = 0;
+  bool whole = true;
+#pragma unroll
+  for (int r = 0; r < kMostRanks; ++r) count[r] = r < ranks ? *cluster.map_shared_rank(&sm.found, r) : 0;
+#pragma unroll
+  for (int r = 0; r < kMostRanks; ++r) {
+    whole = whole && count[r] <= kCandidates;
+    all += min(count[r], kCandidates);
+  }
+  v[0] = v[1] = 0;
+  if (!whole || all > kCandidates) return kCandidates + 1;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    int at = threadIdx.x + h * kSampleThreads;
+    if (at >= all) break;
+    int r = 0;
+#pragma unroll
+    for (int i = 0; i < kMostRanks - 1; ++i) {
+      if (r == i && at >= count[i]) {
+        at -= count[i];
+        ++r;
+      }
+    }
+    v[h] = cluster.map_shared_rank(sm.cand, r)[at];
+  }
+  return all;
+}
+
 // Sums the blocks' histograms `buf` and finds the last non-empty bin whose preceding weight is within the limit
 // (`whole`: the limit is the share `top_p` of the whole sum, and is left in `limit`).  Every thread returns with the bin,
 // the weight before it and its own weight.
@@ -155,22 +306,32 @@ __device__ void find_boundary(SampleSmem& sm, int buf, bool wide, unsigned long 
   static_assert(kBins == 2 * kSampleThreads, "two bins a thread");
   unsigned long long a = 0, b = 0;
   const int ranks = (int)cluster.num_blocks();
-#pragma unroll
-  for (int r = 0; r < kMostRanks; ++r) {
-    if (r >= ranks) break;
-    if (!unit && wide) {
+  if (!unit && wide) {
+    for (int r = 0; r < ranks; ++r) {
       const ulonglong2 both = *reinterpret_cast<const ulonglong2*>(cluster.map_shared_rank(&sm.bins[buf][4 * t], r));
       a += both.x;
       b += both.y;
-      continue;
     }
-    const uint2 lo = *reinterpret_cast<const uint2*>(cluster.map_shared_rank(&sm.bins[buf][2 * t], r));
-    a += lo.x;
-    b += lo.y;
-    if (!unit) {
-      const uint2 hi = *reinterpret_cast<const uint2*>(cluster.map_shared_rank(&sm.bins[buf][kBins + 2 * t], r));
-      a += (unsigned long long)hi.x << 16;
-      b += (unsigned long long)hi.y << 16;
+  } else {
+    // (Four blocks' sums are asked for before the first is used.)
+#pragma unroll
+    for (int first = 0; first < kMostRanks; first += 4) {
+      if (first >= ranks) break;
+      uint2 lo[4], hi[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = first + i;
+        lo[i] = hi[i] = make_uint2(0, 0);
+        if (r < ranks) {
+          lo[i] = *reinterpret_cast<const uint2*>(cluster.map_shared_rank(&sm.bins[buf][2 * t], r));
+          if (!unit) hi[i] = *reinterpret_cast<const uint2*>(cluster.map_shared_rank(&sm.bins[buf][kBins + 2 * t], r));
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        a += lo[i].x + ((unsigned long long)hi[i].x << 16);
+        b += lo[i].y + ((unsigned long long)hi[i].y << 16);
+      }
     }
   }
   const unsigned long long incl = warp_inclusive(a + b, lane);
@@ -200,15 +361,60 @@ __device__ void find_boundary(SampleSmem& sm, int buf, bool wide, unsigned long 
   mass = sm.mass;
 }
 
+// The last selections and the draw of a row whose top-k leaves few elements, by one block: the candidates, all that top-k
+// keeps among them, lie over the blocks.  Returns the column.
+template <typename S, bool kStaged>
+__device__ int draw_from_candidates(const Share<S, kStaged>& share, int k, float top_p, double u, int fallback, SampleSmem& sm) {
+  const int t = threadIdx.x;
+  unsigned long long* table = reinterpret_cast<unsigned long long*>(sm.bins[0]);
+  unsigned long long v[2];
+  const int many = gather_candidates(v, sm);
+  sort_down(v, power_above(many), table);
+  k = min(k, many);
+  unsigned long long weight[2], upto[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    weight[h] = t + h * kSampleThreads < k ? share.weight(key_value((uint32_t)(v[h] >> 32))) : 0;
+    upto[h] = weight[h];
+  }
+  if (top_p > 0.f && top_p < 1.f) {
+    const unsigned long long total = scan_both(upto, k, sm);
+    const unsigned long long limit = (unsigned long long)((double)top_p * (double)total);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (upto[h] - weight[h] > limit) weight[h] = 0;
+  }
+  // In the order of the columns: the index, counted down, above the key.
+#pragma unroll
+  for (int h = 0; h < 2; ++h) v[h] = weight[h] ? v[h] << 32 | v[h] >> 32 : 0;
+  __syncthreads();
+  sort_down(v, power_above(k), table);
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    upto[h] = weight[h] = v[h] && t + h * kSampleThreads < k ? share.weight(key_value((uint32_t)v[h])) : 0;
+  const unsigned long long total = scan_both(upto, k, sm);
+  unsigned long long target = (unsigned long long)(u * (double)total);
+  if (target >= total) target = total ? total - 1 : 0;
+  if (t == 0) sm.chosen = fallback;
+  __syncthreads();
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    if (upto[h] > target && upto[h] - weight[h] <= target) sm.chosen = (int)(0xffffffffu - (uint32_t)(v[h] >> 32));
+  __syncthreads();
+  return sm.chosen;
+}
+
 // Among the elements of `within`, in descending order of value (equal values by ascending index), keeps each element
 // whose preceding weight sum is within the limit.  `unit` weights count elements (top-k with limit k - 1); otherwise the
 // weight is exp(x - row_max) in 2^-32 fixed point (top-p with limit p * total).  `turn`: the histogram to use next;
-// `slot`: the next free exchange.  Lists what survives the first histogram.
-template <typename S, bool unit, bool kAlone>
-__device__ Keep select_prefix(Share<S>& share, bool all_in, Keep within, unsigned long long limit, float top_p, int vocab,
-                              int& turn, int& slot, SampleSmem& sm) {
+// `slot`: the next free exchange.  Lists what survives the first histogram.  `few` (top-k): set where what it keeps lies among
+// that many candidates, which one block is to finish with; nothing else is then returned.
+template <bool unit, bool kAlone, typename S, bool kStaged>
+__device__ Keep select_prefix(Share<S, kStaged>& share, bool all_in, Keep within, unsigned long long limit, float top_p, int vocab,
+                              int& turn, int& slot, int& few, SampleSmem& sm) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const bool wide = share.wide;
+  cg::cluster_group cluster = cg::this_cluster();
   int first_bin = -1;
   uint32_t low_key = 0, high_key = 0xffffffffu;
   unsigned long long above = 0, mass = 0;
@@ -217,31 +423,61 @@ __device__ Keep select_prefix(Share<S>& share, bool all_in, Keep within, unsigne
     const int shift = level == 0 ? 32 : max(0, 32 - __clz(range) - 10);
     uint32_t* bins = sm.bins[turn];
     for (int i = threadIdx.x; i < 2 * kBins; i += kSampleThreads) bins[i] = 0;
+    if (level == 0 && threadIdx.x == 0) sm.found = 0;
     __syncthreads();
-#pragma unroll 4
-    for (int j = share.from + lane; j < share.to; j += 32) {
-      const int i = share.column(j);
-      int bin = share.bin(i);
-      float x = 0.f;
-      if (!all_in || level > 0) {
-        x = share.value(i);
+    const auto add = [&](int bin, unsigned long long weight) {
+      if (unit) {
+        atomicAdd(bins + bin, 1u);
+      } else if (wide) {
+        atomicAdd(reinterpret_cast<unsigned long long*>(bins) + bin, weight);
+      } else {
+        const uint32_t high = (uint32_t)(weight >> 16);
+        atomicAdd(bins + bin, (uint32_t)weight & 0xffffu);
+        if (high) atomicAdd(bins + kBins + bin, high);
+      }
+    };
+    if (all_in && level == 0) {
+      unsigned long long far = 0;      // the last bin's weight: what many columns have is not added one by one
+#pragma unroll 1
+      for (int j = share.from + 4 * lane; j < share.to; j += 128) {
+        float f[4];
+        share.four(j, f);
+        int bin[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) bin[e] = share.bin_of(f[e]);
+        if (unit) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (j + e < share.to) atomicAdd(bins + bin[e], 1u);
+        } else {
+          unsigned long long weight[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) weight[e] = j + e < share.to ? share.weight(share.quotient(f[e])) : 0;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if (bin[e] == kBins - 1) far += weight[e];
+            else add(bin[e], weight[e]);
+          }
+        }
+      }
+      if (!unit) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) far += __shfl_xor_sync(0xffffffffu, far, o);
+        if (lane == 0) add(kBins - 1, far);
+      }
+    } else {
+#pragma unroll 2
+      for (int j = share.from + lane; j < share.to; j += 32) {
+        const int i = share.column(j);
+        int bin = share.bin(i);
+        const float x = share.value(i);
         const uint32_t key = ordered_key(x);
         if (!all_in && !within.has(key, share.base + i)) continue;
         if (level > 0) {
           if (bin != first_bin || key < low_key || key > high_key) continue;
           bin = (int)((high_key - key) >> shift);
         }
-      }
-      if (unit) {
-        atomicAdd(bins + bin, 1u);
-      } else if (bin < kBins - 1 || level > 0) {   // what weighs nothing lies behind every limit
-        const unsigned long long weight = share.weight(all_in && level == 0 ? share.value(i) : x);
-        if (!wide) {
-          atomicAdd(bins + bin, (uint32_t)weight & 0xffffu);
-          atomicAdd(bins + kBins + bin, (uint32_t)(weight >> 16));
-        } else {
-          atomicAdd(reinterpret_cast<unsigned long long*>(bins) + bin, weight);
-        }
+        add(bin, unit ? 1ull : share.weight(x));
       }
     }
     int chosen;
@@ -255,39 +491,115 @@ __device__ Keep select_prefix(Share<S>& share, bool all_in, Keep within, unsigne
       if (chosen > 0) high_key = ordered_key(share.row_max - near + slack);
       if (chosen < kBins - 1) low_key = ordered_key(share.row_max - far - slack);
       if (!(fabsf(share.row_max) < 3.0e38f)) low_key = 0, high_key = 0xffffffffu;
-      if (!share.listed && !wide) {   // list what the boundary bin and those above it hold
-        int listed = 0;
-        bool fits = true;
-        for (int j = share.from; j < share.to; j += 32) {
-          const int i = j + lane;
-          bool in = i < share.to && share.bin(i) <= first_bin;
-          if (in && !all_in) in = within.has(ordered_key(share.value(i)), share.base + i);
-          const unsigned votes = __ballot_sync(0xffffffffu, in);
-          const int many = __popc(votes);
-          if (listed + many > kListed) {
-            fits = false;
-            break;
-          }
-          if (in) sm.list[w][listed + __popc(votes & ((1u << lane) - 1))] = (uint16_t)i;
-          listed += many;
+      if (wide) continue;
+      // List what the boundary bin and those above it hold, and put what has to be told apart where the other blocks find it.
+      const bool collect = !unit || above + mass <= kCandidates;
+      bool fits = !share.listed;
+      int listed = 0;
+      const auto put = [&](bool taken, int i, float x) {       // a warp's elements that have to be told apart
+        const unsigned votes = __ballot_sync(0xffffffffu, taken);
+        if (!votes) return;
+        int at = 0;
+        if (lane == 0) at = atomicAdd(&sm.found, __popc(votes));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(votes & ((1u << lane) - 1));
+        if (taken && at < kCandidates) sm.cand[at] = candidate(ordered_key(x), share.base + i);
+      };
+      if (share.listed) {
+        for (int j = share.from; j < share.to && collect; j += 32) {
+          const int i = j + lane < share.to ? share.column(j + lane) : 0;
+          const int bin = j + lane < share.to ? share.bin(i) : kBins;
+          const float x = share.value(i);
+          put((unit ? bin <= first_bin : bin == first_bin) && (all_in || within.has(ordered_key(x), share.base + i)), i, x);
         }
-        if (__syncthreads_and(fits)) {
-          share.listed = true;
-          share.list = sm.list[w];
-          share.from = 0;
-          share.to = listed;
+      } else {
+        // For a difference that is a number two comparisons are as good as its bin.
+        const float lowest = first_bin == kBins - 1 ? INFINITY : (float)(first_bin + 1), boundary = (float)first_bin;
+#pragma unroll 1
+        for (int j = share.from; j < share.to && (fits || collect); j += 128) {
+          const int i = j + 4 * lane;
+          float f[4];
+          unsigned in = 0, taken = 0;
+          bool odd = false;
+          share.four(min(i, share.n - 1) & ~3, f);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float d = share.bin_max - f[e], t = fminf(d * share.bin_scale, (float)(kBins - 1));
+            const bool here = i + e < share.to;
+            odd = odd || (here && !(d >= 0.f));
+            in |= (unsigned)(here && t < lowest) << e;
+            taken |= (unsigned)(here && t < lowest && (unit || t >= boundary)) << e;
+          }
+          if (__any_sync(0xffffffffu, odd) || !all_in) {
+            in = taken = 0;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              if (i + e >= share.to) continue;
+              const int bin = share.bin_of(f[e]);
+              if (bin > first_bin || !(all_in || within.has(ordered_key(share.quotient(f[e])), share.base + i + e))) continue;
+              in |= 1u << e;
+              if (unit || bin == first_bin) taken |= 1u << e;
+            }
+          }
+          if (!__any_sync(0xffffffffu, in != 0)) continue;
+          if (fits) {
+            // The lanes' counts, 0 to 4, are added up bit by bit.
+            const int many = __popc(in);
+            const unsigned below = (1u << lane) - 1, ones = __ballot_sync(0xffffffffu, many & 1),
+                           twos = __ballot_sync(0xffffffffu, many & 2), fours = __ballot_sync(0xffffffffu, many & 4);
+            const int all = __popc(ones) + 2 * __popc(twos) + 4 * __popc(fours);
+            fits = listed + all <= kListed;
+            if (fits) {
+              int at = listed + __popc(ones & below) + 2 * __popc(twos & below) + 4 * __popc(fours & below);
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                if (in >> e & 1) sm.list[w][at++] = (uint16_t)(i + e);
+              listed += all;
+            }
+          }
+          if (collect && __any_sync(0xffffffffu, taken != 0)) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) put(taken >> e & 1, i + e, share.quotient(f[e]));
+          }
         }
       }
-      continue;
+      if (!share.listed && __syncthreads_and(fits)) {
+        share.listed = true;
+        share.list = sm.list[w];
+        share.from = 0;
+        share.to = listed;
+      }
+      if (!collect) continue;
+      row_sync<kAlone>(cluster);
+      if (unit) {
+        few = (int)(above + mass);
+        return within;
+      }
+      // The few elements of the boundary bin, sorted, tell where the cut falls; every block sorts them for itself.
+      unsigned long long v[2], upto[2], weight[2];
+      const int many = gather_candidates(v, sm);
+      if (many > kCandidates) continue;
+      sort_down(v, power_above(many), reinterpret_cast<unsigned long long*>(sm.bins[0]));
+#pragma unroll
+      for (int h = 0; h < 2; ++h) upto[h] = weight[h] = v[h] ? share.weight(key_value((uint32_t)(v[h] >> 32))) : 0;
+      scan_both(upto, many, sm);
+      int kept = 0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        kept += __syncthreads_count((int)threadIdx.x + h * kSampleThreads < many && above + upto[h] - weight[h] <= limit);
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if ((int)threadIdx.x + h * kSampleThreads == kept - 1)
+          sm.keep = Keep{(uint32_t)(v[h] >> 32), (int)(0xffffffffu - (uint32_t)v[h])};
+      __syncthreads();
+      return sm.keep;
     }
     high_key -= (uint32_t)chosen << shift;
     if (shift == 0) break;
     const uint32_t width = (1u << shift) - 1;
     if (high_key - low_key > width) low_key = high_key - width;
   }
-  cg::cluster_group cluster = cg::this_cluster();
   const uint32_t beta = high_key;
-  const float beta_value = __uint_as_float((beta & 0x80000000u) ? beta & 0x7fffffffu : ~beta);
+  const float beta_value = key_value(beta);
   const unsigned long long each = unit ? 1ull : share.weight(beta_value);
   const unsigned long long count = each ? mass / each : 1ull;
   const unsigned long long ties = each ? min(count, (limit - above) / each + 1) : 1ull;   // above <= limit
@@ -348,9 +660,9 @@ __device__ Keep select_prefix(Share<S>& share, bool all_in, Keep within, unsigne
 
 // Grid: rows x (cluster size) blocks, a row's in one cluster.  `staged`: a block's share lies in its shared memory behind
 // `sm`, as S: the logits as they are, or as float, divided by the temperature.
-template <typename T, typename S, bool kAlone>
+template <typename T, typename S, bool kAlone, bool kStaged>
 __global__ void __launch_bounds__(kSampleThreads, sizeof(S) == 2 ? 3 : 2)
-sample_kernel(const T* __restrict__ logits, int vocab, int share_size, bool staged, const float* __restrict__ temperature,
+sample_kernel(const T* __restrict__ logits, int vocab, int share_size, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ uniform,
               int* __restrict__ out) {
   extern __shared__ __align__(16) char sample_smem[];
@@ -362,18 +674,19 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, bool stag
   const T* row = logits + (size_t)r * vocab;
   const float temp = temperature ? temperature[r] : 0.f;
   const bool greedy = !(temp > 0.f) || (top_k && top_k[r] == 1);
-  Share<S> share;
+  Share<S, kStaged> share;
   share.base = min(vocab, rank * share_size);
   share.n = min(vocab, share.base + share_size) - share.base;
   const T* mine_row = row + share.base;
-  share.divided = staged && sizeof(S) == 4 && !greedy;
 
+  if constexpr (!kAlone) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");   // this block runs: its memory may be written
+  const bool divide = temp != 1.f;
   ArgMax mine{-INFINITY, 0x7fffffff};
   constexpr int N = Vec16<T>::N;
   int done = 0;
   if (aligned16(mine_row)) {
     done = share.n / N * N;
-#pragma unroll 2
+#pragma unroll 4
     for (int i = threadIdx.x * N; i < done; i += kSampleThreads * N) {
       const Vec16<T> v = load16(mine_row + i);
       float f[N];
@@ -385,7 +698,7 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, bool stag
 #pragma unroll
         for (int k = 0; k < N; ++k) mine = better(mine, ArgMax{f[k], share.base + i + k});
       }
-      if (staged && !greedy) {
+      if (kStaged && !greedy) {
         if constexpr (sizeof(S) == sizeof(T) && sizeof(T) == 2) {
           store16(reinterpret_cast<T*>(stage) + i, v);
         } else {
@@ -393,7 +706,7 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, bool stag
           for (int k = 0; k < N; k += 4) {
             Vec16<float> d;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) d.set(e, f[k + e] / temp);
+            for (int e = 0; e < 4; ++e) d.set(e, divide ? f[k + e] / temp : f[k + e]);
             store16(reinterpret_cast<float*>(stage) + i + k, d);
           }
         }
@@ -402,53 +715,74 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, bool stag
   }
   for (int i = done + threadIdx.x; i < share.n; i += kSampleThreads) {
     const T v = mine_row[i];
-    if (staged && !greedy) stage[i] = from_float<S>(sizeof(S) == 4 ? to_float(v) / temp : to_float(v));
+    if (kStaged && !greedy) stage[i] = from_float<S>(sizeof(S) == 4 ? to_float(v) / temp : to_float(v));
     mine = better(mine, ArgMax{to_float(v), share.base + i});
   }
   const ArgMax block_top = block_argmax(mine, sm.warp_best);
-  if (threadIdx.x == 0) sm.best = block_top;
+  if constexpr (!kAlone) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  if (threadIdx.x < ranks) cluster.map_shared_rank(sm.best, threadIdx.x)[rank] = block_top;
   row_sync<kAlone>(cluster);
-  ArgMax top = *cluster.map_shared_rank(&sm.best, 0);
-  for (int k = 1; k < ranks; ++k) top = better(top, *cluster.map_shared_rank(&sm.best, k));
+  ArgMax top = sm.best[0];
+  for (int k = 1; k < ranks; ++k) top = better(top, sm.best[k]);
 
   if (greedy) {
     if (rank == 0 && threadIdx.x == 0) out[r] = top.i;
-    row_sync<kAlone>(cluster);          // the others may still read this block's maximum
-    return;
+    return;                             // nothing of this block's is read any more
   }
-  const int part_size = (share.n + kSampleWarps - 1) / kSampleWarps;
+  const int part_size = (share.n + 4 * kSampleWarps - 1) / (4 * kSampleWarps) * 4;
   share.from = min(share.n, w * part_size);
   share.to = min(share.n, share.from + part_size);
   share.listed = false;
+  share.undivided = !(kStaged && sizeof(S) == 4) && temp != 1.f;
   share.wide = share_size >= 1 << 16;
   share.list = nullptr;
   share.temp = temp;
   share.row_max = top.v / temp;
-  share.bin_max = share.divided ? share.row_max : top.v;
-  share.bin_scale = share.divided ? kBinsPerUnit : kBinsPerUnit / temp;
+  share.bin_max = share.undivided ? top.v : share.row_max;
+  share.bin_scale = share.undivided ? kBinsPerUnit / temp : kBinsPerUnit;
   share.max_key = ordered_key(share.row_max);
 
-  if constexpr (sizeof(S) == sizeof(T)) {
-    if (!staged) reinterpret_cast<const T*&>(share.data) = mine_row;
-    else share.data = stage;
-  } else {
-    share.data = stage;
-  }
+  if constexpr (kStaged) share.data = stage;
+  else share.data = mine_row;
   const int k = top_k ? top_k[r] : -1;
   const float p = top_p ? top_p[r] : 1.f;
   const bool by_count = k > 0 && k < vocab;
-  int turn = 0, slot = 0;
+  double u = uniform ? (double)uniform[r] : 0.5;
+  u = u < 0.0 ? 0.0 : (u >= 1.0 ? 0.99999994 : u);
+  int turn = 0, slot = 0, few = 0;
   Keep keep{0u, vocab};  // every finite value has a key > 0
-  if (by_count) keep = select_prefix<S, true, kAlone>(share, true, keep, (unsigned long long)(k - 1), 0.f, vocab, turn, slot, sm);
-  if (p > 0.f && p < 1.f) keep = select_prefix<S, false, kAlone>(share, !by_count, keep, 0, p, vocab, turn, slot, sm);
+  if (by_count) {
+    keep = select_prefix<true, kAlone>(share, true, keep, (unsigned long long)(k - 1), 0.f, vocab, turn, slot, few, sm);
+    if (few) {
+      if (rank == 0) {
+        const int column = draw_from_candidates(share, k, p, u, top.i, sm);
+        if (threadIdx.x == 0) out[r] = column;
+      }
+      row_sync<kAlone>(cluster);        // the others' candidates stay until they have been read
+      return;
+    }
+  }
+  if (p > 0.f && p < 1.f) keep = select_prefix<false, kAlone>(share, !by_count, keep, 0, p, vocab, turn, slot, few, sm);
 
   // Draw: the first index (ascending) at which the running weight passes uniform * total.
   const int from = share.from, to = share.to;
   unsigned long long part = 0;
-  for (int j = from + lane; j < to; j += 32) {
-    const int i = share.column(j);
-    const float x = share.value(i);
-    if (keep.has(ordered_key(x), share.base + i)) part += share.weight(x);
+  const auto kept_weight = [&](float x, int i) { return keep.has(ordered_key(x), share.base + i) ? share.weight(x) : 0ull; };
+  const auto four_weights = [&](int i, unsigned long long (&weight)[4]) {
+    float f[4];
+    share.four(i, f);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) weight[e] = i + e < to ? kept_weight(share.quotient(f[e]), i + e) : 0;
+  };
+  if (share.listed) {
+    for (int j = from + lane; j < to; j += 32) part += kept_weight(share.value(share.column(j)), share.column(j));
+  } else {
+#pragma unroll 2
+    for (int j = from + 4 * lane; j < to; j += 128) {
+      unsigned long long weight[4];
+      four_weights(j, weight);
+      part += weight[0] + weight[1] + weight[2] + weight[3];
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
@@ -468,57 +802,56 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, bool stag
     total += v;
   }
   for (int i = 0; i < w; ++i) before += sm.warp[i];
-  double u = uniform ? (double)uniform[r] : 0.5;
-  u = u < 0.0 ? 0.0 : (u >= 1.0 ? 0.99999994 : u);
   unsigned long long target = (unsigned long long)(u * (double)total);
   if (target >= total) target = total ? total - 1 : 0;
   if (total == 0) {                      // the maximum weighs 2^32: only a row without finite values comes here
     if (rank == 0 && threadIdx.x == 0) out[r] = top.i;
   } else if (part > 0 && before <= target && target < before + part) {
-    // The walk is one warp's, so what it takes is its steps one after the other: in a short row where nothing is listed, first
-    // 128 columns a step.
-    int at = from;
-    if (kAlone && !share.listed) {
-      for (; at + 128 < to; at += 128) {
-        unsigned long long sum = 0;
+    if (!share.listed) {
+      for (int j = from; j < to; j += 128) {
+        unsigned long long weight[4] = {0, 0, 0, 0};
+        if (j + 4 * lane < to) four_weights(j + 4 * lane, weight);
+        const unsigned long long mine = weight[0] + weight[1] + weight[2] + weight[3];
+        unsigned long long upto = before + warp_inclusive(mine, lane);
+        const unsigned passed = __ballot_sync(0xffffffffu, upto > target);
+        if (passed) {
+          if (lane == __ffs(passed) - 1) {
+            upto -= mine;
+            int e = 0;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int i = at + e * 32 + lane;
-          const float x = share.value(i);
-          if (keep.has(ordered_key(x), share.base + i)) sum += share.weight(x);
+            for (; e < 3; ++e) {
+              upto += weight[e];
+              if (upto > target) break;
+            }
+            out[r] = share.base + j + 4 * lane + e;
+          }
+          break;
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (before + sum > target) break;
-        before += sum;
+        before = __shfl_sync(0xffffffffu, upto, 31);
       }
-    }
-    for (int j = at; j < to; j += 32) {
-      int i = 0;
-      unsigned long long weight = 0;
-      if (j + lane < to) {
-        i = share.column(j + lane);
-        const float x = share.value(i);
-        if (keep.has(ordered_key(x), share.base + i)) weight = share.weight(x);
+    } else {
+      for (int j = from; j < to; j += 32) {
+        const int i = j + lane < to ? share.column(j + lane) : 0;
+        const unsigned long long weight = j + lane < to ? kept_weight(share.value(i), i) : 0;
+        const unsigned long long upto = before + warp_inclusive(weight, lane);
+        const unsigned passed = __ballot_sync(0xffffffffu, upto > target);
+        if (passed) {
+          if (lane == __ffs(passed) - 1) out[r] = share.base + i;
+          break;
+        }
+        before = __shfl_sync(0xffffffffu, upto, 31);
       }
-      const unsigned long long upto = before + warp_inclusive(weight, lane);
-      const unsigned passed = __ballot_sync(0xffffffffu, upto > target);
-      if (passed) {
-        if (lane == __ffs(passed) - 1) out[r] = share.base + i;
-        break;
-      }
-      before = __shfl_sync(0xffffffffu, upto, 31);
     }
   }
   row_sync<kAlone>(cluster);            // nobody leaves while another block reads
 }
 
-template <typename T, typename S, bool kAlone>
-int launch_sample(const T* logits, int rows, int vocab, int ranks, int share, bool staged, const float* temperature,
+template <typename T, typename S, bool kAlone, bool kStaged>
+int launch_sample(const T* logits, int rows, int vocab, int ranks, int share, const float* temperature,
                   const int* top_k, const float* top_p, const float* uniform, int* out, cudaStream_t stream) {
-  const size_t smem = (sizeof(SampleSmem) + 15) / 16 * 16 + (staged ? (size_t)share * sizeof(S) : 0);
+  const size_t smem = (sizeof(SampleSmem) + 15) / 16 * 16 + (kStaged ? (size_t)share * sizeof(S) : 0);
   const cudaError_t status =
-      cudaFuncSetAttribute(sample_kernel<T, S, kAlone>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleMostSmem);
+      cudaFuncSetAttribute(sample_kernel<T, S, kAlone, kStaged>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleMostSmem);
   if (status != cudaSuccess) return (int)status;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(rows * ranks);
@@ -532,12 +865,12 @@ int launch_sample(const T* logits, int rows, int vocab, int ranks, int share, bo
   attribute[0].val.clusterDim.z = 1;
   config.attrs = attribute;
   config.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&config, sample_kernel<T, S, kAlone>, logits, vocab, share, staged, temperature, top_k, top_p,
+  return (int)cudaLaunchKernelEx(&config, sample_kernel<T, S, kAlone, kStaged>, logits, vocab, share, temperature, top_k, top_p,
                                  uniform, out);
 }
 
 // Shares in shared memory where they fit.  bfloat16 is staged as divided floats while all of the launch's blocks are resident
-// at once that way, two an SM (64 KB of floats beside 33 KB): the passes then divide nothing.  A wider launch stages the
+// at once that way, two an SM (64 KB of floats beside 41 KB): the passes then divide nothing.  A wider launch stages the
 // logits as they are, three blocks an SM, and divides again in the passes that need the quotient, so that 48 rows of
 // 128,256 (384 blocks) still are one wave; two waves would cost each row's chain of barriers twice.
 template <typename T>
@@ -551,10 +884,11 @@ int sample_rows(const T* logits, int rows, int vocab, const float* temperature, 
   const bool raw = (size_t)share * sizeof(T) <= room;
   const bool floats = sizeof(T) == 4 || ((size_t)share * 4 <= room / 2 && rows * ranks <= 2 * 148);
   const auto launch = [&](auto kernel) {
-    return kernel(logits, rows, vocab, ranks, share, raw, temperature, top_k, top_p, uniform, out, stream);
+    return kernel(logits, rows, vocab, ranks, share, temperature, top_k, top_p, uniform, out, stream);
   };
-  if (ranks == 1) return floats ? launch(launch_sample<T, float, true>) : launch(launch_sample<T, T, true>);
-  return floats ? launch(launch_sample<T, float, false>) : launch(launch_sample<T, T, false>);
+  if (!raw) return launch(launch_sample<T, T, false, false>);
+  if (ranks == 1) return floats ? launch(launch_sample<T, float, true, true>) : launch(launch_sample<T, T, true, true>);
+  return floats ? launch(launch_sample<T, float, false, true>) : launch(launch_sample<T, T, false, true>);
 }
 
 template <typename T>

@@ -491,6 +491,33 @@ def test_sample_splits_a_row_over_blocks(dtype, vocab, rows):
             assert any(bool((keep == int(got[r])).any()) for _, keep in rules), f"row {r}: {int(got[r])} is not in what is kept"
 
 
+# What is told apart by sorting: a top-k at and around the 1,024 candidates that are sorted at most; boundary bins of a handful and of
+# thousands of columns (scale 0.02: the whole row lies in a few bins); one block a row and eight.
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("vocab", [2048, 8192, 50257])
+@pytest.mark.parametrize("scale", [0.02, 0.5, 3.0])
+def test_sample_among_few_and_many_candidates(dtype, vocab, scale):
+    from liteinfer_b200 import ops
+
+    g = torch.Generator().manual_seed(vocab + int(100 * scale))
+    ks, ps, rows = [2, 32, 33, 512, 513, 1023, 1024, 1025, 0, 0, 0, 0], [1.0, 0.3, 0.999], 36
+    logits = (torch.randn(rows, vocab, generator=g) * scale).to(dtype)
+    temps = torch.tensor([1.0, 0.6, 1.7] * (rows // 3))
+    top_k, top_p = torch.tensor([k for k in ks for _ in ps], dtype=torch.int32), torch.tensor(ps * len(ks))
+    u = torch.rand(rows, generator=g)
+    got = ops.sample(logits.cuda(), temps.cuda(), top_k.cuda(), top_p.cuda(), u.cuda(),
+                     torch.empty(rows, dtype=torch.int32, device="cuda")).cpu()
+    off = 2.0 ** -22 + vocab * 2.0 ** -32          # as in the test above
+    for r in range(rows):
+        x = logits[r].float() / temps[r]
+        k, p, v = int(top_k[r]), float(top_p[r]), float(u[r])
+        rules = [_sample_rule(x, k, p + dp, min(max(v + du, 0.0), 0.9999999)) for du in (-2 * off, 0.0, 2 * off)
+                 for dp in ((-2 * off, 0.0, 2 * off) if p < 1 else (0.0,))]
+        low, high = min(at for at, _ in rules), max(at for at, _ in rules)
+        assert low <= int(got[r]) <= high, f"row {r}: got {int(got[r])}, the rule gives {low} to {high}"
+        assert any(bool((keep == int(got[r])).any()) for _, keep in rules), f"row {r}: {int(got[r])} is not in what is kept"
+
+
 def test_sample_distribution():
     """Many draws of one row follow softmax(logits / T) restricted to the top-k."""
     from liteinfer_b200 import ops
