@@ -658,12 +658,22 @@ __device__ Keep select_prefix(Share<S, kStaged>& share, bool all_in, Keep within
   return out;
 }
 
+// What a row is sampled with.  A launch of few rows brings it along: no buffer to be pinned and no copy on the stream before
+// the kernel (48 rows of 128,256 bfloat16 columns: 66 us a call behind a pinned copy, 55 with it, the time of the kernel).
+constexpr int kBroughtAlong = 128;
+struct RowParams {
+  const float *temperature, *top_p, *uniform;      // on the device; null: the values below
+  const int* top_k;
+  bool along;
+  float values[3][kBroughtAlong];                  // temperature, top_p, uniform
+  int counts[kBroughtAlong];                       // top_k
+};
+
 // Grid: rows x (cluster size) blocks, a row's in one cluster.  `staged`: a block's share lies in its shared memory behind
 // `sm`, as S: the logits as they are, or as float, divided by the temperature.
 template <typename T, typename S, bool kAlone, bool kStaged>
 __global__ void __launch_bounds__(kSampleThreads, sizeof(S) == 2 ? 3 : 2)
-sample_kernel(const T* __restrict__ logits, int vocab, int share_size, const float* __restrict__ temperature,
-              const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ uniform,
+sample_kernel(const T* __restrict__ logits, int vocab, int share_size, const __grid_constant__ RowParams params,
               int* __restrict__ out) {
   extern __shared__ __align__(16) char sample_smem[];
   SampleSmem& sm = *reinterpret_cast<SampleSmem*>(sample_smem);
@@ -672,8 +682,12 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, const flo
   const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks(), r = blockIdx.x / ranks;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const T* row = logits + (size_t)r * vocab;
-  const float temp = temperature ? temperature[r] : 0.f;
-  const bool greedy = !(temp > 0.f) || (top_k && top_k[r] == 1);
+  const bool along = params.along;
+  grid_dependency_wait();
+  const float temp = along ? params.values[0][r] : params.temperature ? params.temperature[r] : 0.f;
+  const int k = along ? params.counts[r] : params.top_k ? params.top_k[r] : -1;
+  const float p = along ? params.values[1][r] : params.top_p ? params.top_p[r] : 1.f;
+  const bool greedy = !(temp > 0.f) || k == 1;
   Share<S, kStaged> share;
   share.base = min(vocab, rank * share_size);
   share.n = min(vocab, share.base + share_size) - share.base;
@@ -744,10 +758,8 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, const flo
 
   if constexpr (kStaged) share.data = stage;
   else share.data = mine_row;
-  const int k = top_k ? top_k[r] : -1;
-  const float p = top_p ? top_p[r] : 1.f;
   const bool by_count = k > 0 && k < vocab;
-  double u = uniform ? (double)uniform[r] : 0.5;
+  double u = along ? (double)params.values[2][r] : params.uniform ? (double)params.uniform[r] : 0.5;
   u = u < 0.0 ? 0.0 : (u >= 1.0 ? 0.99999994 : u);
   int turn = 0, slot = 0, few = 0;
   Keep keep{0u, vocab};  // every finite value has a key > 0
@@ -847,8 +859,8 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, const flo
 }
 
 template <typename T, typename S, bool kAlone, bool kStaged>
-int launch_sample(const T* logits, int rows, int vocab, int ranks, int share, const float* temperature,
-                  const int* top_k, const float* top_p, const float* uniform, int* out, cudaStream_t stream) {
+int launch_sample(const T* logits, int rows, int vocab, int ranks, int share, const RowParams& params, int* out,
+                  cudaStream_t stream) {
   const size_t smem = (sizeof(SampleSmem) + 15) / 16 * 16 + (kStaged ? (size_t)share * sizeof(S) : 0);
   const cudaError_t status =
       cudaFuncSetAttribute(sample_kernel<T, S, kAlone, kStaged>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleMostSmem);
@@ -858,15 +870,16 @@ int launch_sample(const T* logits, int rows, int vocab, int ranks, int share, co
   config.blockDim = dim3(kSampleThreads);
   config.dynamicSmemBytes = smem;
   config.stream = stream;
-  cudaLaunchAttribute attribute[1];
-  attribute[0].id = cudaLaunchAttributeClusterDimension;
-  attribute[0].val.clusterDim.x = ranks;
-  attribute[0].val.clusterDim.y = 1;
-  attribute[0].val.clusterDim.z = 1;
-  config.attrs = attribute;
-  config.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&config, sample_kernel<T, S, kAlone, kStaged>, logits, vocab, share, temperature, top_k, top_p,
-                                 uniform, out);
+  cudaLaunchAttribute attributes[2];
+  attributes[0].id = cudaLaunchAttributeClusterDimension;
+  attributes[0].val.clusterDim.x = ranks;
+  attributes[0].val.clusterDim.y = 1;
+  attributes[0].val.clusterDim.z = 1;
+  attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[1].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attributes;
+  config.numAttrs = pdl_enabled(rows) ? 2 : 1;
+  return (int)cudaLaunchKernelEx(&config, sample_kernel<T, S, kAlone, kStaged>, logits, vocab, share, params, out);
 }
 
 // Shares in shared memory where they fit.  bfloat16 is staged as divided floats while all of the launch's blocks are resident
@@ -874,8 +887,7 @@ int launch_sample(const T* logits, int rows, int vocab, int ranks, int share, co
 // logits as they are, three blocks an SM, and divides again in the passes that need the quotient, so that 48 rows of
 // 128,256 (384 blocks) still are one wave; two waves would cost each row's chain of barriers twice.
 template <typename T>
-int sample_rows(const T* logits, int rows, int vocab, const float* temperature, const int* top_k, const float* top_p,
-                const float* uniform, int* out, cudaStream_t stream) {
+int sample_rows(const T* logits, int rows, int vocab, const RowParams& params, int* out, cudaStream_t stream) {
   int ranks = 1;
   while (ranks < kMostRanks && ranks * kRankColumns < vocab) ranks *= 2;
   const int share = ((vocab + ranks - 1) / ranks + 7) / 8 * 8;
@@ -884,7 +896,7 @@ int sample_rows(const T* logits, int rows, int vocab, const float* temperature, 
   const bool raw = (size_t)share * sizeof(T) <= room;
   const bool floats = sizeof(T) == 4 || ((size_t)share * 4 <= room / 2 && rows * ranks <= 2 * 148);
   const auto launch = [&](auto kernel) {
-    return kernel(logits, rows, vocab, ranks, share, temperature, top_k, top_p, uniform, out, stream);
+    return kernel(logits, rows, vocab, ranks, share, params, out, stream);
   };
   if (!raw) return launch(launch_sample<T, T, false, false>);
   if (ranks == 1) return floats ? launch(launch_sample<T, float, true, true>) : launch(launch_sample<T, T, true, true>);
@@ -981,6 +993,28 @@ LI_EXPORT int li_argmax(int dtype, const void* logits, int rows, int vocab, int*
 LI_EXPORT int li_sample(int dtype, const void* logits, int rows, int vocab, const float* temperature,
                         const int* top_k, const float* top_p, const float* uniform, int* out, cudaStream_t stream) {
   if (rows == 0) return 0;
-  if (dtype == kFloat32) return sample_rows((const float*)logits, rows, vocab, temperature, top_k, top_p, uniform, out, stream);
-  return sample_rows((const bf16*)logits, rows, vocab, temperature, top_k, top_p, uniform, out, stream);
+  RowParams params = {};
+  params.temperature = temperature;
+  params.top_p = top_p;
+  params.uniform = uniform;
+  params.top_k = top_k;
+  if (dtype == kFloat32) return sample_rows((const float*)logits, rows, vocab, params, out, stream);
+  return sample_rows((const bf16*)logits, rows, vocab, params, out, stream);
+}
+
+// The same with the parameters in host memory, which is read before this returns; at most kBroughtAlong rows.
+LI_EXPORT int li_sample_from_host(int dtype, const void* logits, int rows, int vocab, const float* temperature, const int* top_k,
+                                  const float* top_p, const float* uniform, int* out, cudaStream_t stream) {
+  if (rows == 0) return 0;
+  if (rows > kBroughtAlong) return LI_ERR_UNSUPPORTED;
+  RowParams params = {};
+  params.along = true;
+  for (int r = 0; r < rows; ++r) {
+    params.values[0][r] = temperature[r];
+    params.values[1][r] = top_p[r];
+    params.values[2][r] = uniform[r];
+    params.counts[r] = top_k[r];
+  }
+  if (dtype == kFloat32) return sample_rows((const float*)logits, rows, vocab, params, out, stream);
+  return sample_rows((const bf16*)logits, rows, vocab, params, out, stream);
 }

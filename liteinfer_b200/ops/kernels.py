@@ -180,6 +180,8 @@ _SIGNATURES = {
                                c_void_p]),
     "li_sample": ("sampling", [c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                c_void_p]),
+    "li_sample_from_host": ("sampling", [c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                         c_void_p]),
 }
 
 
@@ -2289,4 +2291,22 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
         assert t.dtype == torch.float32 and t.numel() == rows
     _check(_fn("li_sample")(_code(logits), logits.data_ptr(), rows, vocab, temperature.data_ptr(), top_k.data_ptr(),
                             top_p.data_ptr(), uniform.data_ptr(), out.data_ptr(), _stream()), "sample")
+    return out
+
+
+# Rows whose sampling parameters a launch brings along (kBroughtAlong of sampling.cu).
+SAMPLE_FROM_HOST = 128
+
+
+def sample_from_host(logits: torch.Tensor, params: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+    """`sample` with its parameters in host memory, [4, rows] float32: temperature, top_p, uniform and the bits of an int32
+    top_k.  They are read before this returns and travel with the launch; at most SAMPLE_FROM_HOST rows."""
+    _on_gpu(logits, out)
+    _int32(out, "out")
+    rows, vocab = logits.shape
+    if params.is_cuda or params.dtype != torch.float32 or params.shape != (4, rows) or not params.is_contiguous():
+        raise KernelLibraryError("sample_from_host: params is a contiguous float32 tensor [4, rows] on the host")
+    at = params.data_ptr()
+    _check(_fn("li_sample_from_host")(_code(logits), logits.data_ptr(), rows, vocab, at, at + 12 * rows, at + 4 * rows,
+                                      at + 8 * rows, out.data_ptr(), _stream()), "sample_from_host")
     return out

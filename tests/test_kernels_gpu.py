@@ -4,6 +4,8 @@ odd group sizes, pages of odd length."""
 
 from __future__ import annotations
 
+import random
+
 import pytest
 import torch
 
@@ -516,6 +518,24 @@ def test_sample_among_few_and_many_candidates(dtype, vocab, scale):
         low, high = min(at for at, _ in rules), max(at for at, _ in rules)
         assert low <= int(got[r]) <= high, f"row {r}: got {int(got[r])}, the rule gives {low} to {high}"
         assert any(bool((keep == int(got[r])).any()) for _, keep in rules), f"row {r}: {int(got[r])} is not in what is kept"
+
+
+# Parameters that travel with the launch, up to as many rows as it takes, and one row more through the pinned copy.
+@pytest.mark.parametrize("rows", [1, 3, 128, 129])
+def test_sampler_brings_its_parameters_along(rows):
+    from liteinfer_b200 import SamplingParams, ops
+    from liteinfer_b200.sampling.sampler import Sampler
+
+    g = torch.Generator().manual_seed(rows)
+    logits = (torch.randn(rows, 3000, generator=g) * 2.5).cuda()
+    kinds = [dict(temperature=0.8, top_k=40), dict(temperature=0.0), dict(temperature=1.3, top_p=0.8), dict(temperature=1.0)]
+    params = [SamplingParams(seed=i, **kinds[i % 4]) for i in range(rows)]
+    got = Sampler(0)(logits, params)
+    uniform = torch.tensor([0.0 if p.greedy else random.Random(p.seed).random() for p in params]).cuda()
+    want = ops.sample(logits, torch.tensor([p.temperature for p in params]).cuda(),
+                      torch.tensor([max(p.top_k, 0) for p in params], dtype=torch.int32).cuda(),
+                      torch.tensor([p.top_p for p in params]).cuda(), uniform, torch.empty(rows, dtype=torch.int32, device="cuda"))
+    assert torch.equal(got, want)
 
 
 def test_sample_distribution():
