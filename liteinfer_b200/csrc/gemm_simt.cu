@@ -4,9 +4,10 @@
 // for shapes the tensor-core kernels refuse.
 //
 // Every output element adds its K products in the same order whatever M and N are, so a row's result does not depend on
-// which other rows are in the batch: chunks of 128 k, each one chain of fused multiply-adds in ascending order from zero,
-// and the chunks' sums in ascending order.  Both kernels keep that order; the chunks are what lets the narrow one give
-// each to a warp of its own (and the sum of short chains is nearer to the exact one than a single long chain was).
+// which other rows are in the batch: chunks of 128 k, each two chains of fused multiply-adds in ascending order from zero, of its
+// even and its odd k, which one instruction takes side by side; their sum; and the chunks' sums in ascending order.  Both kernels
+// keep that order; the chunks are what lets the narrow one give each to a warp of its own (and the sum of short chains is nearer to
+// the exact one: relative error of a product over 768 k 1.55e-7, 2.1e-7 with one chain a chunk).
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -17,6 +18,16 @@ namespace li {
 
 constexpr int kChunk = 128;
 
+// Two sums side by side, of the even and of the odd k: one instruction multiplies and adds for both.
+typedef unsigned long long Pair;
+__device__ __forceinline__ Pair multiply_add(Pair a, Pair b, Pair sums) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sums) : "l"(a), "l"(b));
+  return sums;
+}
+__device__ __forceinline__ float both(Pair sums) {
+  return __uint_as_float((unsigned)sums) + __uint_as_float((unsigned)(sums >> 32));
+}
+
 struct SimtProduct {
   const void *x, *w, *bias;
   void* out;
@@ -25,14 +36,16 @@ struct SimtProduct {
   bool w_at_rest;       // nothing that is still under way writes w
 };
 
-// ---- many rows of x: 128 x 64 tiles, 8 x 4 outputs a thread ------------------------------------------------------
-// Bound by the FFMA pipe: four k are 128 multiply-adds a thread on 12 vector loads from shared memory, rows along k in
-// both operands (threads have rows 16 apart, which with rows of 36 words keeps the reads off one another's banks).  Three
-// steps of 32 k are on their way (cp.async) while a fourth is multiplied, so a grid of few tiles does not wait for every
-// step's loads.
-// Measured on B200, 1,250 rows: 3072 x 2048 488 us (32 TFLOP/s), 16384 x 2048 2,170 us (39), 1280 x 768 98 us; the tiles of
-// 64 x 64 before them (4 x 4 a thread, scalar loads between two barriers of every 16 k) took 833, 4,073 and 141 us.
-constexpr int BN = 64, BK = 32, kTileThreads = 256, kTileStages = 4;
+// ---- many rows of x: 64 x 64 tiles, 8 x 4 outputs a thread -------------------------------------------------------
+// Bound by shared memory's reads: four k are 64 two-wide multiply-adds a thread on 12 vector loads, and a warp's vector load takes four
+// cycles where its multiply-adds take 32 in all.  Rows lie along k in both operands (threads have rows 8 and 16 apart, which with
+// rows of 36 words keeps the reads off one another's banks), so two neighbours along k are a pair as they are loaded.  Three steps
+// of 32 k are on their way (cp.async) while a fourth is multiplied.  Three blocks of four warps an SM: blocks of this size spread a
+// grid of a few hundred over the SMs more evenly than 128 x 64 (1,250 rows of 1280 x 768: 79 us, 97), and half the
+// multiply-adds' instructions leave the issue slots to the loads.
+// Measured on B200, 1,250 rows: 3072 x 2048 437 us (36 TFLOP/s; 486 in tiles of 128 x 64 with one-wide multiply-adds), 4096 x 768
+// 213 (232); 400 rows of 2048 x 8192 443 (595), of 1280 x 768 35 (44).
+constexpr int BN = 64, BK = 32, kTileThreads = 128, kTileStages = 4;
 constexpr int kTileRow = BK + 4;
 template <int BM> constexpr size_t kTileSmem = (size_t)kTileStages * (BM + BN) * kTileRow * sizeof(float);
 
@@ -68,7 +81,7 @@ __device__ __forceinline__ void stage_four(float* dst, const bf16* src, int left
 }
 
 template <typename T, int BM>
-__global__ void __launch_bounds__(kTileThreads, 2) gemm_simt_tile_kernel(SimtProduct p, bool vec) {
+__global__ void __launch_bounds__(kTileThreads, 3) gemm_simt_tile_kernel(SimtProduct p, bool vec) {
   extern __shared__ __align__(16) float tile_smem[];      // [stage][x rows, then w rows][kTileRow]
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN, K = p.K;
   const T* x = static_cast<const T*>(p.x) + blockIdx.z * p.x_batch;
@@ -94,11 +107,12 @@ __global__ void __launch_bounds__(kTileThreads, 2) gemm_simt_tile_kernel(SimtPro
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
-  float acc[BM / 16][4], total[BM / 16][4];
+  Pair acc[BM / 8][4];
+  float total[BM / 8][4];
 #pragma unroll
-  for (int i = 0; i < BM / 16; ++i)
+  for (int i = 0; i < BM / 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = total[i][j] = 0.f;
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0, total[i][j] = 0.f;
 
   for (int step = 0; step < kTileStages - 1; ++step) fill(step);
   for (int step = 0; step < steps; ++step) {
@@ -110,31 +124,32 @@ __global__ void __launch_bounds__(kTileThreads, 2) gemm_simt_tile_kernel(SimtPro
     const float* wr = stage + (BM + tx) * kTileRow;
 #pragma unroll 2
     for (int k = 0; k < BK; k += 4) {
-      float4 b[4];
+      ulonglong2 b[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(wr + j * 16 * kTileRow + k);
+      for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(wr + j * 16 * kTileRow + k);
 #pragma unroll
-      for (int i = 0; i < BM / 16; ++i) {
-        const float4 a = *reinterpret_cast<const float4*>(xr + i * 16 * kTileRow + k);
+      for (int i = 0; i < BM / 8; ++i) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(xr + i * 8 * kTileRow + k);
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          acc[i][j] = fmaf(a.w, b[j].w, fmaf(a.z, b[j].z, fmaf(a.y, b[j].y, fmaf(a.x, b[j].x, acc[i][j]))));
+        for (int j = 0; j < 4; ++j) acc[i][j] = multiply_add(a.x, b[j].x, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = multiply_add(a.y, b[j].y, acc[i][j]);
       }
     }
     if ((step + 1) * BK % kChunk == 0 || step + 1 == steps) {
 #pragma unroll
-      for (int i = 0; i < BM / 16; ++i)
+      for (int i = 0; i < BM / 8; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          total[i][j] += acc[i][j];
-          acc[i][j] = 0.f;
+          total[i][j] += both(acc[i][j]);
+          acc[i][j] = 0;
         }
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < BM / 16; ++i) {
-    const int m = m0 + ty + 16 * i;
+  for (int i = 0; i < BM / 8; ++i) {
+    const int m = m0 + ty + 8 * i;
     if (m >= p.M) continue;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -199,27 +214,27 @@ __global__ void __launch_bounds__(32 * kMostChunks * G) gemm_simt_rows_kernel(Si
     }
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    float acc[R][2];
+    Pair acc[R][2];
 #pragma unroll
-    for (int r = 0; r < R; ++r) acc[r][0] = acc[r][1] = 0.f;
-    const float4* w0 = reinterpret_cast<const float4*>(wt + lane * kRowStride);
-    const float4* w1 = reinterpret_cast<const float4*>(wt + (lane + 32) * kRowStride);
-    const float4* xr = reinterpret_cast<const float4*>(xt + part * R * kChunk);
+    for (int r = 0; r < R; ++r) acc[r][0] = acc[r][1] = 0;
+    const ulonglong2* w0 = reinterpret_cast<const ulonglong2*>(wt + lane * kRowStride);
+    const ulonglong2* w1 = reinterpret_cast<const ulonglong2*>(wt + (lane + 32) * kRowStride);
+    const ulonglong2* xr = reinterpret_cast<const ulonglong2*>(xt + part * R * kChunk);
 #pragma unroll 2
     for (int f = 0; f < fours; ++f) {
-      const float4 b0 = w0[f], b1 = w1[f];
+      const ulonglong2 b0 = w0[f], b1 = w1[f];
 #pragma unroll
       for (int r = 0; r < R; ++r) {        // rows beyond x or w hold what the memory held: their sums are not stored
-        const float4 a = xr[r * (kChunk / 4) + f];
-        acc[r][0] = fmaf(a.w, b0.w, fmaf(a.z, b0.z, fmaf(a.y, b0.y, fmaf(a.x, b0.x, acc[r][0]))));
-        acc[r][1] = fmaf(a.w, b1.w, fmaf(a.z, b1.z, fmaf(a.y, b1.y, fmaf(a.x, b1.x, acc[r][1]))));
+        const ulonglong2 a = xr[r * (kChunk / 4) + f];
+        acc[r][0] = multiply_add(a.y, b0.y, multiply_add(a.x, b0.x, acc[r][0]));
+        acc[r][1] = multiply_add(a.y, b1.y, multiply_add(a.x, b1.x, acc[r][1]));
       }
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       float* mine_sums = sums + (place * (R * G) + part * R + r) * kRowsN + lane;
-      mine_sums[0] = acc[r][0];
-      mine_sums[32] = acc[r][1];
+      mine_sums[0] = both(acc[r][0]);
+      mine_sums[32] = both(acc[r][1]);
     }
   }
   cluster.sync();
@@ -300,18 +315,19 @@ int launch_tiles(const SimtProduct& p, bool vec, int batch, cudaStream_t stream)
   LI_LAUNCH_CHECK();
 }
 
-// Which kernel, by what each was measured to take (B200, microseconds, float32).  The narrow one: 4 and 2.2 for every million
-// weights of a group of 16 rows (16384 x 2048: 73 for 12 rows; 1280 x 768: 10.2 for 64).  Tiles of 32 rows: 26 per 768 k
-// while each SM has one or none, then 0.15 a tile (1280 x 768: 26 for 192 rows, 120 for 1,250); tiles of 128 rows: 54 per 768 k
-// up to one an SM, 98 up to two, then 0.37 a tile (1280 x 768: 54 for 256 rows, 98 for 1,250; 4096 x 768: 239 for 1,250).
+// Which kernel, by what each was measured to take (B200, microseconds, float32).  The narrow one: 4 and 2.1 for every million
+// weights of a group of 16 rows (16384 x 2048: 70 for 12 rows; 1280 x 768: 11.3 for 64).  Tiles of 32 rows: 24 per 768 k
+// while each SM has one or none, 35 up to some 250, then 12 and 0.094 a tile (1280 x 768: 24.7 for 192 rows, 87 for 1,250); tiles of
+// 64 rows: 35.5 per 768 k up to one an SM, 58 up to two, then 12 and 0.155 a tile (1280 x 768: 35.6 for 256 rows, 79 for 1,250; 4096 x
+// 768: 213 for 1,250).
 constexpr int kMostRows = 256;
 inline float rows_cost(const SimtProduct& p, int batch) {
-  return 4.f + 2.2e-6f * (float)p.N * p.K * ((p.M + 15) / 16) * batch;
+  return 4.f + 2.1e-6f * (float)p.N * p.K * ((p.M + 15) / 16) * batch;
 }
 inline float tiles_cost(const SimtProduct& p, int batch, int rows) {
   const float tiles = (float)((p.N + BN - 1) / BN) * ((p.M + rows - 1) / rows) * batch, depth = p.K / 768.f;
-  if (rows == 32) return depth * fmaxf(26.f, 0.15f * tiles);
-  return depth * (tiles <= 148.f ? 54.f : fmaxf(98.f, 0.37f * tiles));
+  if (rows == 32) return depth * (tiles <= 148.f ? 24.f : fmaxf(35.f, 12.f + 0.094f * tiles));
+  return depth * (tiles <= 148.f ? 35.5f : fmaxf(58.f, 12.f + 0.155f * tiles));
 }
 
 int launch_product(int dtype, const SimtProduct& p, int batch, cudaStream_t stream) {
@@ -319,7 +335,7 @@ int launch_product(int dtype, const SimtProduct& p, int batch, cudaStream_t stre
   // Loads of four k at once: every row of x and w starts on their size.
   const bool vec = p.K % 4 == 0 && p.ldx % 4 == 0 && p.x_batch % 4 == 0 && p.w_batch % 4 == 0 &&
                    reinterpret_cast<uintptr_t>(p.x) % four == 0 && reinterpret_cast<uintptr_t>(p.w) % four == 0;
-  const float small = tiles_cost(p, batch, 32), large = tiles_cost(p, batch, 128);
+  const float small = tiles_cost(p, batch, 32), large = tiles_cost(p, batch, 64);
   if (dtype == kFloat32 && vec && p.K > 0 && p.M <= kMostRows && p.K <= kMostEach * kMostCluster * kChunk &&
       batch <= 65535 && rows_cost(p, batch) < fminf(small, large)) {
     if (p.M == 1) return launch_rows<1, 1>(p, batch, stream);
@@ -330,8 +346,8 @@ int launch_product(int dtype, const SimtProduct& p, int batch, cudaStream_t stre
   }
   const bool narrow = small < large && (p.M + 31) / 32 <= 65535;
   if (dtype == kFloat32)
-    return narrow ? launch_tiles<float, 32>(p, vec, batch, stream) : launch_tiles<float, 128>(p, vec, batch, stream);
-  return narrow ? launch_tiles<bf16, 32>(p, vec, batch, stream) : launch_tiles<bf16, 128>(p, vec, batch, stream);
+    return narrow ? launch_tiles<float, 32>(p, vec, batch, stream) : launch_tiles<float, 64>(p, vec, batch, stream);
+  return narrow ? launch_tiles<bf16, 32>(p, vec, batch, stream) : launch_tiles<bf16, 64>(p, vec, batch, stream);
 }
 
 }  // namespace li
