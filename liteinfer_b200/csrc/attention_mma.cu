@@ -379,7 +379,7 @@ attention_mma_kernel(const AttnParams p) {
       }
     }
     __syncthreads();
-    combine_warps<D>(p, os, ms, ls, rows_used, groups, q_begin, q0, kvh, part, split);
+    combine_warps<D>(p, os, ms, ls, rows_used, groups, q_begin, q0, kvh, part, split, p.num_splits);
   } else {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -406,7 +406,7 @@ attention_mma_kernel(const AttnParams p) {
   }
   if (p.num_splits == 1) return;
 
-  merge_splits<D>(p, smem_raw, &is_last, rows_used, groups, q_begin, q0, kvh, part, qtile);
+  merge_splits<D>(p, smem_raw, &is_last, rows_used, groups, q_begin, q0, kvh, part, qtile, p.num_splits);
 }
 
 template <int D, bool kDecode, int kStages>

@@ -103,11 +103,12 @@ template <int D> __device__ __forceinline__ bf16* tile_ptr(bf16* base, int row, 
 
 // Decode: the four warps of a block each saw a quarter of the keys and left (accumulator, maximum, sum) in
 // shared memory (os [4][16][D], ms and ls [4][16]); their combination is the block's result: the output itself,
-// or with several splits this split's partial result and its log-sum-exp.
+// or with several splits this split's partial result and its log-sum-exp.  (`splits`: how many there are, at most the p.num_splits that
+// the partial results are laid out for.)
 template <int D>
 __device__ __forceinline__ void combine_warps(const AttnParams& p, const float* os, const float* ms, const float* ls,
                                               int rows_used, int groups, int q_begin, int q0, int kvh, int part,
-                                              int split) {
+                                              int split, int splits) {
   for (int e = threadIdx.x; e < rows_used * D; e += kWarps * 32) {
     const int row = e / D, d = e % D;
     float mx = -INFINITY;
@@ -122,9 +123,9 @@ __device__ __forceinline__ void combine_warps(const AttnParams& p, const float* 
       acc += wgt * os[((size_t)w * 16 + row) * D + d];
     }
     const int qi = q0 + row / groups, head = kvh * groups + row % groups;
-    if (p.num_splits == 1 && p.sink != nullptr) denom += exp2f(p.sink[head] * kLog2e - mx);
+    if (splits == 1 && p.sink != nullptr) denom += exp2f(p.sink[head] * kLog2e - mx);
     const float value = denom > 0.f ? acc / denom : 0.f;
-    if (p.num_splits == 1) {
+    if (splits == 1) {
       p.out[(size_t)(q_begin + qi) * p.out_row_stride + (size_t)out_head(p, head, part) * D + d] = __float2bfloat16_rn(value);
     } else {
       const size_t slot = ((size_t)(q_begin + qi) * p.heads * p.v_parts + out_head(p, head, part)) * p.num_splits + split;
@@ -140,14 +141,14 @@ __device__ __forceinline__ void combine_warps(const AttnParams& p, const float* 
 template <int D>
 __device__ __forceinline__ void merge_splits(const AttnParams& p, unsigned char* smem_raw, bool* is_last_flag,
                                              int rows_used, int groups, int q_begin, int q0, int kvh, int v_part,
-                                             int qtile) {
+                                             int qtile, int splits) {
   // ---- the block that arrives last merges the splits of this (sequence, KV head, query tile).
   __threadfence();
   __syncthreads();
   const unsigned counter_index = ((unsigned)blockIdx.z * gridDim.y + blockIdx.y) * (gridDim.x / p.num_splits) + qtile;
   if (threadIdx.x == 0) {
     const unsigned arrived = atomicAdd(&p.counters[counter_index], 1u);
-    *is_last_flag = arrived == (unsigned)p.num_splits - 1;
+    *is_last_flag = arrived == (unsigned)splits - 1;
   }
   __syncthreads();
   if (!*is_last_flag) return;
@@ -157,7 +158,7 @@ __device__ __forceinline__ void merge_splits(const AttnParams& p, unsigned char*
   // log-sum-exp seen so far, as a softmax over blocks of keys would be.  Where the block has more threads than such
   // items, P neighbouring lanes share an item (lane j takes the splits j, j + P, ...) and merge their running
   // results by shuffles at the end.  No shared memory, no barrier.
-  const int S = p.num_splits;
+  const int S = splits;
   const int items = rows_used * (D / 4);
   const int P = items * 4 <= kWarps * 32 ? 4 : (items * 2 <= kWarps * 32 ? 2 : 1);
   for (int e0 = 0; e0 < items * P; e0 += kWarps * 32) {
@@ -166,7 +167,7 @@ __device__ __forceinline__ void merge_splits(const AttnParams& p, unsigned char*
     const int item = live ? e / P : 0, part = e % P;
     const int row = item / (D / 4), d4 = item % (D / 4);
     const int qi = q0 + row / groups, head = kvh * groups + row % groups;
-    const size_t first = ((size_t)(q_begin + qi) * p.heads * p.v_parts + out_head(p, head, v_part)) * S;
+    const size_t first = ((size_t)(q_begin + qi) * p.heads * p.v_parts + out_head(p, head, v_part)) * p.num_splits;
     const float* lse = p.partial_lse + first;
     const float4* src = reinterpret_cast<const float4*>(p.partial_out + first * D) + d4;
     float mx = -INFINITY, denom = 0.f;

@@ -141,10 +141,33 @@ __device__ __noinline__ void merge_in_cluster(const AttnParams& p, const float* 
   cluster_sync_all();                                    // nobody leaves while the first block reads
 }
 
+// ceil(a / b) for 0 < a, b < 2^20, in few instructions: every block starts with it, and its first keys wait for it.  (The half keeps the
+// quotient away from whole numbers by more than the division's error.)
+__device__ __forceinline__ int ceil_quotient(int a, int b) {
+  return (int)__fdividef((float)(a + b - 1) + 0.5f, (float)b);
+}
+
+// The splits that a sequence with this many tiles of keys has in a launch that gives it `most` at most (the host, which may replay
+// the launch for contexts of any length, knows no better).  A merge costs some 2 us, and more the more parts it reads and the more
+// sequences do it at once, a tile 0.65 us (0.9 at head size 128): up to four tiles are one block's, seven where several sequences share
+// the device (`most` below 16), whose blocks then have three tiles at least; alone a sequence has a block a tile up to 16, and
+// 32 blocks only from 97 tiles on.  Measured on B200, 8 KV heads of 64, all splits that the host allows, then so: one sequence of 60 keys 7.6 us
+// and 3.0, of 250 7.5 and 5.0, of 611 7.8 and 6.5, of 1,500 8.5 and 7.4, of 8,000 12.0 and 11.4; eight of 120 7.6 and 4.4, of
+// 440 8.8 and 7.2, of 700 9.2 and 8.4; at head size 128 one of 60 11.2 and 4.1, of 611 11.7 and 9.1, of 1,500 12.5 and 10.6.
+__device__ __forceinline__ int splits_of(int tiles, int most) {
+  const bool shared = most < 16;
+  if (tiles <= (shared ? 7 : 4)) return 1;
+  const int wanted = min(min(most, shared ? (tiles + 2) / 3 : tiles), tiles <= 96 ? 16 : 32);
+  return wanted <= 1 ? 1 : ceil_quotient(tiles, ceil_quotient(tiles, wanted));
+}
+
+// kWide: a form in fewer registers, three blocks of head size 128 an SM instead of two, for launches of more blocks than two an SM.  It is
+// some 4 % slower a block.  Measured on B200, 8 KV heads of 128: 48 sequences of 1,500 keys 48 us (65.5), 40 of 2,000 55 (81), 24 of
+// 3,000, in two splits each then, 52 (63); 32 of 2,000, which are one wave either way, 47.4 (45).
 // kRing: slots per warp; up to kRing - 1 groups are on their way while one is multiplied.
 // kCapped: scores are capped (p.cap_in, p.cap_out); a form of its own, so that the plain one stays what it was.
-template <int D, int kRing, bool kCluster, bool kCapped = false>
-__global__ void __launch_bounds__(kWarps * 32, D == 64 ? 5 : 2)   // blocks per SM that the rings leave room for
+template <int D, int kRing, bool kCluster, bool kCapped = false, bool kWide = false>
+__global__ void __launch_bounds__(kWarps * 32, D == 64 ? 5 : kWide ? 3 : 2)   // blocks per SM that the rings leave room for
 attention_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                         const AttnParams p) {
   constexpr unsigned kHalfBytes = kGroupKeys * D * 2;      // K or V of one group
@@ -157,7 +180,6 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   __shared__ float rope_cos[D / 2], rope_sin[D / 2];
   __shared__ __align__(16) bf16 newest[2 * D];             // the rotated key and the value of the newest token
   __shared__ __align__(8) unsigned long long ring_bars[kWarps * kMaxRing];
-  __shared__ int slot_filled[kWarps * kMaxRing];           // whether the slot's current group was fetched at all
 
   const int seq = p.seq_index ? p.seq_index[blockIdx.z] : blockIdx.z;
   if (seq < 0) return;        // a place of padding in the list of sequences
@@ -170,7 +192,9 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   const int qpos = ctx - 1, hi = ctx;
   const int lo = first_visible(qpos, p.window);
   const int tile_lo = lo / kBlockN, tile_hi = (hi + kBlockN - 1) / kBlockN;
-  const int per_split = (tile_hi - tile_lo + p.num_splits - 1) / p.num_splits;
+  const int splits = kCluster ? p.num_splits : splits_of(tile_hi - tile_lo, p.num_splits);
+  if (split >= splits) return;
+  const int per_split = splits == 1 ? tile_hi - tile_lo : ceil_quotient(tile_hi - tile_lo, splits);
   const int my_lo = tile_lo + split * per_split, my_hi = min(tile_hi, my_lo + per_split);
   const int my_groups = max(0, my_hi - my_lo);             // groups of this warp: one per tile of the block
   const bool fused = p.rope_inv_freq != nullptr;
@@ -200,13 +224,20 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     if (page < 0 || page >= p.num_pages) return -1;
     return ((long)page * p.kv_heads + kvh) * p.page_size + (kpos0 - block * p.page_size);
   };
+  // The rows of 32 groups at a time, a lane each: a group's request then waits for no trip to the block table, and the warp, which
+  // waits for its requesting lane, neither.  (One block over 4,000 keys: 42 us at head size 64, 53 with a look at the table per
+  // group; 57 and 67 at 128.)
+  int rows = -1;
+  unsigned filled = 0;                                      // a bit for every group (modulo 32) that was fetched at all
   // One lane asks for group i's boxes, or just arrives where there is nothing to fetch (the slot's phase moves on
   // either way).  The slot's last reader has finished: the warp synchronised after reading it.
   auto request = [&](int i) {
-    if (lane != 0 || i >= my_groups) return;
+    if (i >= my_groups) return;
+    if ((i & 31) == 0) rows = (int)group_row(i + lane);
+    const int row = __shfl_sync(0xffffffffu, rows, i & 31);
+    filled = row >= 0 ? filled | 1u << (i & 31) : filled & ~(1u << (i & 31));
+    if (lane != 0) return;
     const unsigned slot = ring + (unsigned)(i % kRing) * kSlotBytes, bar = bars + 8u * (i % kRing);
-    const long row = group_row(i);
-    slot_filled[warp * kMaxRing + i % kRing] = row >= 0;      // read by the warp after its wait on the barrier below
     if (row < 0) {
       mbar_arrive(bar);
       return;
@@ -214,8 +245,8 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     mbar_expect_tx(bar, kSlotBytes);
 #pragma unroll
     for (int b = 0; b < kBoxes; ++b) {
-      tma_load_2d(slot + b * 2048, &map_k, bar, b * 64, (int)row);
-      tma_load_2d(slot + kHalfBytes + b * 2048, &map_v, bar, part * D + b * 64, (int)row);
+      tma_load_2d(slot + b * 2048, &map_k, bar, b * 64, row);
+      tma_load_2d(slot + kHalfBytes + b * 2048, &map_v, bar, part * D + b * 64, row);
     }
   };
   // The pages hold nothing that the kernel before this one wrote when the cache write is fused in here; otherwise
@@ -318,7 +349,7 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         break;
       }
       const unsigned slot = ring + (unsigned)(i % kRing) * kSlotBytes;
-      const bool filled = slot_filled[warp * kMaxRing + i % kRing] != 0;
+      const bool present = filled >> (i & 31) & 1;
       if (owns_newest && qpos >= kpos0 && qpos < kpos0 + kGroupKeys) {
         // This group holds the newest token: its row of the slot is replaced by what this kernel computed.
         const int row = qpos - kpos0;
@@ -331,7 +362,7 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         }
         __syncwarp();
       }
-      if (filled) {
+      if (present) {
         // S = Q K^T: two tiles of eight keys.
         float s[2][4];
 #pragma unroll
@@ -463,9 +494,9 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   }
   __syncthreads();
   if (!kCluster) {
-    combine_warps<D>(p, os, ms, ls, groups, groups, q_begin, 0, kvh, part, split);
-    if (p.num_splits == 1) return;
-    merge_splits<D>(p, generic_base, &is_last, groups, groups, q_begin, 0, kvh, part, 0);
+    combine_warps<D>(p, os, ms, ls, groups, groups, q_begin, 0, kvh, part, split, splits);
+    if (splits == 1) return;
+    merge_splits<D>(p, generic_base, &is_last, groups, groups, q_begin, 0, kvh, part, 0, splits);
     return;
   }
   merge_in_cluster<D>(p, os, ms, ls, groups, q_begin, kvh, part, split);
@@ -506,32 +537,58 @@ static bool make_group_map(CUtensorMap* map, const void* pool, long rows, int he
   return true;
 }
 
+// Blocks of the kernel that the current device holds at once; 0 if the query fails.
+template <int D, int kRing, bool kWide>
+int stream_capacity() {
+  static int capacity = -1;
+  if (capacity >= 0) return capacity;
+  int device = 0, sms = 0, per_sm = 0;
+  if (cudaGetDevice(&device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+      cudaFuncSetAttribute(attention_stream_kernel<D, kRing, false, false, kWide>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)stream_smem<D, kRing>()) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attention_stream_kernel<D, kRing, false, false, kWide>, kWarps * 32,
+                                                    stream_smem<D, kRing>()) != cudaSuccess)
+    return 0;
+  capacity = per_sm * sms;
+  return capacity;
+}
+
+// Blocks that walk a sequence's splits one by one, without a cluster.
+template <int D, int kRing, bool kCapped, bool kWide>
+int launch_blocks(const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams& p, dim3 grid, cudaStream_t stream) {
+  static bool ready = false;
+  if (!ready) {
+    cudaError_t e = cudaFuncSetAttribute(attention_stream_kernel<D, kRing, false, kCapped, kWide>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stream_smem<D, kRing>());
+    if (e != cudaSuccess) return (int)e;
+    ready = true;
+  }
+  return (int)launch_pdl(grid.z, attention_stream_kernel<D, kRing, false, kCapped, kWide>, grid, dim3(kWarps * 32),
+                         stream_smem<D, kRing>(), stream, mk, mv, p);
+}
+
 template <int D, int kRing>
 int launch_stream(const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams& p, int num_seqs, cudaStream_t stream) {
+  const dim3 grid(p.num_splits, p.kv_heads * p.v_parts, num_seqs);
+  if (!p.cluster_merge) {
+    if constexpr (D == 128) {
+      const int narrow = stream_capacity<D, kRing, false>();
+      if (narrow > 0 && (long)grid.x * grid.y * grid.z > narrow) {
+        return p.cap_out > 0.f ? launch_blocks<D, kRing, true, true>(mk, mv, p, grid, stream)
+                               : launch_blocks<D, kRing, false, true>(mk, mv, p, grid, stream);
+      }
+    }
+    return p.cap_out > 0.f ? launch_blocks<D, kRing, true, false>(mk, mv, p, grid, stream)
+                           : launch_blocks<D, kRing, false, false>(mk, mv, p, grid, stream);
+  }
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_stream_kernel<D, kRing, false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stream_smem<D, kRing>());
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(attention_stream_kernel<D, kRing, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)stream_smem<D, kRing>());
+    cudaError_t e = cudaFuncSetAttribute(attention_stream_kernel<D, kRing, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)stream_smem<D, kRing>());
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  const dim3 grid(p.num_splits, p.kv_heads * p.v_parts, num_seqs);
-  if (p.cap_out > 0.f) {
-    static bool ready = false;
-    if (!ready) {
-      cudaError_t e = cudaFuncSetAttribute(attention_stream_kernel<D, kRing, false, true>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stream_smem<D, kRing>());
-      if (e != cudaSuccess) return (int)e;
-      ready = true;
-    }
-    return (int)launch_pdl(num_seqs, attention_stream_kernel<D, kRing, false, true>, grid, dim3(kWarps * 32),
-                           stream_smem<D, kRing>(), stream, mk, mv, p);
-  }
-  if (!p.cluster_merge)
-    return (int)launch_pdl(num_seqs, attention_stream_kernel<D, kRing, false>, grid, dim3(kWarps * 32), stream_smem<D, kRing>(), stream, mk, mv, p);
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
   config.blockDim = dim3(kWarps * 32);
@@ -581,23 +638,6 @@ int stream_cluster_capacity(int splits) {
   return clusters;
 }
 
-// Blocks of the kernel that the current device holds at once; 0 if the query fails.
-template <int D, int kRing>
-int stream_capacity() {
-  static int capacity = -1;
-  if (capacity >= 0) return capacity;
-  int device = 0, sms = 0, per_sm = 0;
-  if (cudaGetDevice(&device) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-      cudaFuncSetAttribute(attention_stream_kernel<D, kRing, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)stream_smem<D, kRing>()) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attention_stream_kernel<D, kRing, false>, kWarps * 32,
-                                                    stream_smem<D, kRing>()) != cudaSuccess)
-    return 0;
-  capacity = per_sm * sms;
-  return capacity;
-}
-
 // Slots per warp: a slot is 4 KB at head size 64 and 8 KB at 128; with these, three blocks fit on an SM.
 constexpr int kRing64 = RING64, kRing128 = 2;
 
@@ -618,11 +658,16 @@ LI_EXPORT int li_paged_attention_stream_cluster_capacity(int head_dim, int split
 }
 
 LI_EXPORT int li_paged_attention_stream_capacity(int head_dim) {
-  return head_dim == 64 ? stream_capacity<64, kRing64>() : (head_dim == 128 ? stream_capacity<128, kRing128>() : 0);
+  return head_dim == 64 ? stream_capacity<64, kRing64, false>() : (head_dim == 128 ? stream_capacity<128, kRing128, false>() : 0);
+}
+
+// The same of the form that takes launches of more blocks than that.
+LI_EXPORT int li_paged_attention_stream_wide_capacity(int head_dim) {
+  return head_dim == 128 ? stream_capacity<128, kRing128, true>() : li_paged_attention_stream_capacity(head_dim);
 }
 
 // Every launched sequence brings exactly one token.  Arguments as li_paged_attention_mma (its counters export
-// says how many counters a split launch needs); sizes as li_paged_attention_stream_supports allows.
+// says how many counters a split launch needs; num_splits is the most that a sequence gets, see splits_of); sizes as li_paged_attention_stream_supports allows.
 // error_flag (device int, zero; may be null): set to 21 if a wait for a group of keys ever gave up.
 // sink (optional, [heads] float32): exp(sink[h]) is one more term of head h's denominator.  v_dim: the size of a value,
 // a multiple of head_dim.  softcap > 0: a scaled score s becomes softcap * tanh(s / softcap).

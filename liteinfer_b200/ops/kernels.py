@@ -136,6 +136,7 @@ _SIGNATURES = {
         c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_float, c_void_p]),
     "li_paged_attention_stream_supports": ("attention_stream", [c_int, c_int, c_int, c_int]),
     "li_paged_attention_stream_capacity": ("attention_stream", [c_int]),
+    "li_paged_attention_stream_wide_capacity": ("attention_stream", [c_int]),
     "li_paged_attention_stream_cluster_capacity": ("attention_stream", [c_int, c_int]),
     "li_paged_attention_mma_counters": ("attention_mma", [c_int, c_int, c_int, c_int]),
     "li_paged_attention_mma_decode_capacity": ("attention_mma", [c_int]),
@@ -993,6 +994,18 @@ def decode_capacity(head_dim: int, streaming: bool = False) -> int:
     return _decode_capacity[key]
 
 
+_wide_capacity = 0
+
+
+def decode_wide_capacity() -> int:
+    """`decode_capacity` of the streaming kernel's form for more blocks of head size 128 than two an SM."""
+    global _wide_capacity
+    if not _wide_capacity:
+        blocks = int(_fn("li_paged_attention_stream_wide_capacity")(128)) if torch.cuda.is_available() else 0
+        _wide_capacity = blocks or 3 * NUM_SMS
+    return _wide_capacity
+
+
 def decode_splits_for(num_decode: int, kv_heads: int, max_context_len: int, head_dim: int = 64,
                       streaming: bool = False) -> int:
     """Blocks that share one sequence's keys in a decode launch: as many as still run as one wave when the
@@ -1002,7 +1015,10 @@ def decode_splits_for(num_decode: int, kv_heads: int, max_context_len: int, head
     if tiles < 4:
         return 1
     pairs = max(1, num_decode * kv_heads)
-    splits = max(1, min(decode_capacity(head_dim, streaming) // pairs, tiles // 2, 32))
+    fitting = decode_capacity(head_dim, streaming) // pairs
+    if streaming and head_dim == 128 and fitting == 1:
+        fitting = max(1, min(2, decode_wide_capacity() // pairs))       # the form of three blocks an SM, where it gives a second split
+    splits = max(1, min(fitting, tiles // 2, 32))
     if streaming and cluster_merge_wanted() and splits > 1:
         # The streaming kernel can merge the splits of a sequence through distributed shared memory when they are
         # one thread-block cluster (16 blocks at most) and every cluster of the launch is resident at once: then a

@@ -659,6 +659,30 @@ def test_tensor_core_attention_against_the_plain_kernel(heads, kv_heads, head_di
     torch.testing.assert_close(got.float(), want.float(), rtol=2 ** -6, atol=2 ** -6)
 
 
+# Contexts at the edges of one block's tiles, of sixteen blocks' and of one tile a block, together in a launch; many sequences, whose
+# blocks at head size 128 are more than two an SM (320 of them) and as many again behind a second split.
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("ctx_lens,splits", [([1, 64, 256, 257, 320, 1024, 1025, 6144, 6145], 32), ([1, 256, 257, 448, 704, 6145], 7),
+                                             ([70 + 5 * i for i in range(40)], None), ([300 + 9 * i for i in range(40)], 2)])
+@pytest.mark.parametrize("window,softcap,sink", [(0, 0.0, False), (300, 0.0, True), (0, 20.0, False)])
+def test_decode_splits_follow_the_context(head_dim, ctx_lens, splits, window, softcap, sink):
+    from liteinfer_b200 import ops
+
+    heads, kv_heads, q_lens = 16, 8, [1] * len(ctx_lens)
+    case = _paged_case(torch.bfloat16, heads, kv_heads, head_dim, 16, q_lens, ctx_lens)
+    qkv, k_pool, v_pool = case["qkv"], case["k_pool"], case["v_pool"]
+    ops.rope_kv_write(qkv, case["positions"], case["seq_of"], case["table"], k_pool, v_pool, None, heads, kv_heads,
+                      head_dim, 0)
+    args = (qkv, qkv.shape[1])
+    rest = (k_pool, v_pool, case["table"], case["qsl"], case["ctx"], case["B"], 1, heads, kv_heads, head_dim, head_dim ** -0.5, window)
+    extra = dict(softcap=softcap, sink=_randn(heads, dtype=torch.float32, seed=9) if sink else None)
+    want = ref.paged_attention(*args, torch.empty(case["T"], heads * head_dim, dtype=torch.bfloat16, device="cuda"), *rest, **extra)
+    got = ops.paged_attention(*args, torch.full((case["T"], heads * head_dim), float("nan"), dtype=torch.bfloat16, device="cuda"),
+                              *rest, plan=_plan_for(q_lens, ctx_lens), decode_splits=splits, **extra)
+    torch.testing.assert_close(got.float(), want.float(), rtol=2 ** -6, atol=2 ** -6)
+    assert ops.gemm_error_flag("cuda:0") == 0
+
+
 @pytest.mark.parametrize("heads,kv_heads,head_dim,page_size", [(32, 8, 64, 16), (8, 8, 64, 8), (16, 1, 128, 16),
                                                                (6, 2, 128, 5), (5, 1, 64, 32)])
 @pytest.mark.parametrize("window", [0, 100])
