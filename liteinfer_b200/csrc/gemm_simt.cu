@@ -5,7 +5,7 @@
 //
 // Every output element adds its K products in the same order whatever M and N are, so a row's result does not depend on
 // which other rows are in the batch: chunks of 128 k, each two chains of fused multiply-adds in ascending order from zero, of its
-// even and its odd k, which one instruction takes side by side; their sum; and the chunks' sums in ascending order.  Both kernels
+// even and its odd k, (which the wide kernel's instruction takes side by side); their sum; and the chunks' sums in ascending order.  Both kernels
 // keep that order; the chunks are what lets the narrow one give each to a warp of its own (and the sum of short chains is nearer to
 // the exact one: relative error of a product over 768 k 1.55e-7, 2.1e-7 with one chain a chunk).
 #include <cooperative_groups.h>
@@ -214,27 +214,30 @@ __global__ void __launch_bounds__(32 * kMostChunks * G) gemm_simt_rows_kernel(Si
     }
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    Pair acc[R][2];
+    float acc[R][2][2];
 #pragma unroll
-    for (int r = 0; r < R; ++r) acc[r][0] = acc[r][1] = 0;
-    const ulonglong2* w0 = reinterpret_cast<const ulonglong2*>(wt + lane * kRowStride);
-    const ulonglong2* w1 = reinterpret_cast<const ulonglong2*>(wt + (lane + 32) * kRowStride);
-    const ulonglong2* xr = reinterpret_cast<const ulonglong2*>(xt + part * R * kChunk);
+    for (int r = 0; r < R; ++r) acc[r][0][0] = acc[r][0][1] = acc[r][1][0] = acc[r][1][1] = 0.f;
+    const float4* w0 = reinterpret_cast<const float4*>(wt + lane * kRowStride);
+    const float4* w1 = reinterpret_cast<const float4*>(wt + (lane + 32) * kRowStride);
+    const float4* xr = reinterpret_cast<const float4*>(xt + part * R * kChunk);
+    // (One k at a time here: two-wide multiply-adds made a step of 12 sequences at six layers of 768 2 % longer.)
 #pragma unroll 2
     for (int f = 0; f < fours; ++f) {
-      const ulonglong2 b0 = w0[f], b1 = w1[f];
+      const float4 b0 = w0[f], b1 = w1[f];
 #pragma unroll
-      for (int r = 0; r < R; ++r) {        // rows beyond x or w hold what the memory held: their sums are not stored
-        const ulonglong2 a = xr[r * (kChunk / 4) + f];
-        acc[r][0] = multiply_add(a.y, b0.y, multiply_add(a.x, b0.x, acc[r][0]));
-        acc[r][1] = multiply_add(a.y, b1.y, multiply_add(a.x, b1.x, acc[r][1]));
+      for (int r = 0; r < R; ++r) {
+        const float4 a = xr[r * (kChunk / 4) + f];
+        acc[r][0][0] = fmaf(a.z, b0.z, fmaf(a.x, b0.x, acc[r][0][0]));
+        acc[r][0][1] = fmaf(a.w, b0.w, fmaf(a.y, b0.y, acc[r][0][1]));
+        acc[r][1][0] = fmaf(a.z, b1.z, fmaf(a.x, b1.x, acc[r][1][0]));
+        acc[r][1][1] = fmaf(a.w, b1.w, fmaf(a.y, b1.y, acc[r][1][1]));
       }
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       float* mine_sums = sums + (place * (R * G) + part * R + r) * kRowsN + lane;
-      mine_sums[0] = both(acc[r][0]);
-      mine_sums[32] = both(acc[r][1]);
+      mine_sums[0] = acc[r][0][0] + acc[r][0][1];
+      mine_sums[32] = acc[r][1][0] + acc[r][1][1];
     }
   }
   cluster.sync();
@@ -317,7 +320,7 @@ int launch_tiles(const SimtProduct& p, bool vec, int batch, cudaStream_t stream)
 
 // Which kernel, by what each was measured to take (B200, microseconds, float32).  The narrow one: 4 and 2.1 for every million
 // weights of a group of 16 rows (16384 x 2048: 70 for 12 rows; 1280 x 768: 11.3 for 64).  Tiles of 32 rows: 24 per 768 k
-// while each SM has one or none, 35 up to some 250, then 12 and 0.094 a tile (1280 x 768: 24.7 for 192 rows, 87 for 1,250); tiles of
+// while each SM has one or none, 35 up to some 250, then 12 and 0.104 a tile (1280 x 768: 24.7 for 192 rows, 87 for 1,250); tiles of
 // 64 rows: 35.5 per 768 k up to one an SM, 58 up to two, then 12 and 0.155 a tile (1280 x 768: 35.6 for 256 rows, 79 for 1,250; 4096 x
 // 768: 213 for 1,250).
 constexpr int kMostRows = 256;
@@ -326,7 +329,7 @@ inline float rows_cost(const SimtProduct& p, int batch) {
 }
 inline float tiles_cost(const SimtProduct& p, int batch, int rows) {
   const float tiles = (float)((p.N + BN - 1) / BN) * ((p.M + rows - 1) / rows) * batch, depth = p.K / 768.f;
-  if (rows == 32) return depth * (tiles <= 148.f ? 24.f : fmaxf(35.f, 12.f + 0.094f * tiles));
+  if (rows == 32) return depth * (tiles <= 148.f ? 24.f : fmaxf(35.f, 12.f + 0.104f * tiles));
   return depth * (tiles <= 148.f ? 35.5f : fmaxf(58.f, 12.f + 0.155f * tiles));
 }
 
