@@ -284,6 +284,31 @@ def test_prompt_attention_in_pairs_where_the_grid_has_room(head_dim, n, q_len, e
     assert ops.gemm_error_flag("cuda:0") == 0
 
 
+# Prompts, portions and single tokens of 32-bit numbers in one launch: tiles of one query and of eight, groups of 1 to 8 heads, units of
+# keys that only some of a tile's queries see, pages that are not there (NaN wherever no request owns a slot).
+@pytest.mark.parametrize("heads,kv_heads,head_dim,page_size", [(4, 4, 64, 16), (4, 2, 20, 5), (12, 4, 64, 16), (8, 2, 128, 8), (16, 2, 100, 16),
+                                                               (9, 1, 64, 16)])
+@pytest.mark.parametrize("window,keep_first,softcap,sink", [(0, 0, 0.0, False), (70, 0, 0.0, True), (100, 68, 20.0, False),
+                                                            (-96, 0, 0.0, False)])
+def test_prompts_in_32_bit_share_their_keys(heads, kv_heads, head_dim, page_size, window, keep_first, softcap, sink):
+    from liteinfer_b200 import ops
+
+    q_lens, ctx_lens = [9, 1, 33, 2, 8, 1, 150, 7], [9, 200, 33, 130, 264, 1, 301, 64]
+    case = _paged_case(torch.float32, heads, kv_heads, head_dim, page_size, q_lens, ctx_lens)
+    sinks = _randn(heads, dtype=torch.float32, seed=9) if sink else None
+    ops.rope_kv_write(case["qkv"], case["positions"], case["seq_of"], case["table"], case["k_pool"], case["v_pool"], None,
+                      heads, kv_heads, head_dim, 0)
+    args = (case["qkv"], case["qkv"].shape[1])
+    rest = (case["k_pool"], case["v_pool"], case["table"], case["qsl"], case["ctx"], case["B"], max(q_lens), heads, kv_heads,
+            head_dim, head_dim ** -0.5)
+    options = dict(window=max(window, 0), chunk=max(-window, 0), keep_first=keep_first, softcap=softcap, sink=sinks)
+    out = lambda: torch.full((case["T"], heads * head_dim), float("nan"), device="cuda")
+    want = ref.paged_attention(*args, out(), *rest, **options)
+    for plan in (None, _plan_for(q_lens, ctx_lens)):
+        got = ops.paged_attention(*args, out(), *rest, plan=plan, **options)
+        torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-5)
+
+
 # Rows walked by one warp and by teams, one unit of keys and several rounds of them, every width of values.
 @pytest.mark.parametrize("heads,kv_heads,head_dim,page_size", [(3, 1, 64, 16), (9, 1, 20, 16), (2, 2, 128, 16), (6, 3, 256, 8),
                                                                (2, 1, 320, 16), (34, 2, 33, 5)])
