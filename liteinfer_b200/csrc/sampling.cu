@@ -74,8 +74,9 @@ __device__ ArgMax block_argmax(ArgMax mine, ArgMax* scratch /* 32 */) {
 constexpr int kSampleThreads = 512, kSampleWarps = kSampleThreads / 32;
 constexpr int kMostRanks = 8;      // blocks of a row's cluster
 // A row of no more columns is one block's, and so on.  The passes over a share get longer, but there are fewer blocks to meet at
-// every barrier, and more rows at once: 12 rows of 16,000 columns take 27.7 us in two blocks each and 35.8 in eight, 64 rows of
-// 32,000 42 in four and 74 in eight; with twice as many columns a block 34.7 and 40.
+// every barrier, and more rows at once: 48 rows of 32,000 columns, top-p 0.9, take 27 us in four blocks each and 43 in eight.  Where the
+// launch's blocks have an SM each all the same, half as many columns: 12 rows of 16,000, top-p 0.9, 22.0 us in two blocks each
+// and 17.2 in four, of 32,000 23.5 in four and 19.7 in eight.
 constexpr int kRankColumns = 8192;
 constexpr int kBins = 1024;
 constexpr int kListed = 512;       // columns that a warp can list; where one has more its block goes on walking its whole share
@@ -890,6 +891,7 @@ template <typename T>
 int sample_rows(const T* logits, int rows, int vocab, const RowParams& params, int* out, cudaStream_t stream) {
   int ranks = 1;
   while (ranks < kMostRanks && ranks * kRankColumns < vocab) ranks *= 2;
+  if (ranks > 1 && ranks < kMostRanks && 2LL * ranks * rows <= 148) ranks *= 2;
   const int share = ((vocab + ranks - 1) / ranks + 7) / 8 * 8;
   if ((long long)rows * ranks > 0x7fffffffll) return LI_ERR_UNSUPPORTED;
   const size_t room = kSampleMostSmem - (sizeof(SampleSmem) + 15) / 16 * 16;
