@@ -17,6 +17,8 @@
 // tokens are in flight while one is computed.  Whole prompts, portions and single tokens run
 // the same code from the state the step before left, in the same order, so the result does not depend on how a
 // sequence was cut.  Tokens of padding (sequence -1) and sequences that bring no token touch nothing.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace li {
@@ -128,15 +130,23 @@ __device__ __forceinline__ float sum_over_column_lanes(float v) {   // the eight
   return v;
 }
 
+__device__ __forceinline__ float4 load_piece(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load_piece(const bf16* p) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  return make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16),
+                     __uint_as_float(raw.y & 0xffff0000u));
+}
+
 // What of a token does not depend on the state, once per (token, head) instead of once per column of S:
 // units [tokens][kv_heads][2][dim] = (q dim^-0.5 / |q|, k / |k|) in float with |x| = sqrt(sum x^2 + 1e-6), and
 // gates [tokens][heads][2] = (beta, g) = (sigmoid(raw_b), exp(-exp(A_log) * softplus(raw_a + dt_bias))).  One warp
-// a (token, head or kv head).
+// a (token, head or kv head).  `products` (optional, [tokens][kv_heads][4]): (q . k, k . k', q . k', 0) of the unit vectors, k' the
+// token's before (the launch's first has none); dim is then 4, 8, ... or 128 in whole pieces of four, the rows on their size.
 template <typename T>
 __global__ void delta_gates_kernel(const T* __restrict__ qkv, size_t row_width, const T* __restrict__ ab,
                                    size_t ab_stride, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
-                                   float* __restrict__ scales, float* __restrict__ gates, int tokens, int heads,
-                                   int kv_heads, int dim) {
+                                   float* __restrict__ scales, float* __restrict__ gates, float* __restrict__ products, int tokens,
+                                   int heads, int kv_heads, int dim) {
   grid_dependency_wait();
   const int lane = threadIdx.x & 31;
   const int per_token = kv_heads + (heads + 31) / 32;
@@ -148,6 +158,28 @@ __global__ void delta_gates_kernel(const T* __restrict__ qkv, size_t row_width, 
     const T* q = qkv + t * row_width + (size_t)what * dim;
     const T* k = q + (size_t)kv_heads * dim;
     float qq = 0.f, kk = 0.f;
+    if (products != nullptr) {
+      // A lane's four dimensions at once (dim <= 128).
+      const bool mine = 4 * lane < dim;
+      const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 a = mine ? load_piece(q + 4 * lane) : none, b = mine ? load_piece(k + 4 * lane) : none;
+      const float4 c = mine && t > 0 ? load_piece(k + 4 * lane - (ptrdiff_t)row_width) : none;
+      const auto dot = [](const float4& x, const float4& y) { return fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, x.x * y.x))); };
+      qq = warp_sum(dot(a, a));
+      kk = warp_sum(dot(b, b));
+      const float pp = warp_sum(dot(c, c)), qk = warp_sum(dot(a, b)), kp = warp_sum(dot(b, c)), qp = warp_sum(dot(a, c));
+      const float q_inv = (1.0f / sqrtf((float)dim)) / sqrtf(qq + 1e-6f), k_inv = 1.0f / sqrtf(kk + 1e-6f);
+      const float p_inv = 1.0f / sqrtf(pp + 1e-6f);
+      float* unit = scales + (t * kv_heads + what) * 2 * (size_t)dim;
+      if (mine) {
+        *reinterpret_cast<float4*>(unit + 4 * lane) = make_float4(a.x * q_inv, a.y * q_inv, a.z * q_inv, a.w * q_inv);
+        *reinterpret_cast<float4*>(unit + dim + 4 * lane) = make_float4(b.x * k_inv, b.y * k_inv, b.z * k_inv, b.w * k_inv);
+      }
+      if (lane == 0)
+        *reinterpret_cast<float4*>(products + (t * kv_heads + what) * 4) =
+            make_float4(qk * (q_inv * k_inv), kp * (k_inv * p_inv), qp * (q_inv * p_inv), 0.f);
+      return;
+    }
     for (int i = lane; i < dim; i += 32) {
       const float a = to_float(q[i]), b = to_float(k[i]);
       qq = fmaf(a, a, qq);
@@ -175,13 +207,6 @@ __global__ void delta_gates_kernel(const T* __restrict__ qkv, size_t row_width, 
 // Which entries of a column of 8 R a lane keeps, where everything is vectors: pieces of four, the eight lanes' pieces side by
 // side, so that the lanes of a column read 128 neighbouring bytes at once.
 __device__ __forceinline__ int piece_at(int c, int part) { return (c * 8 + part) * 4; }
-
-__device__ __forceinline__ float4 load_piece(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 load_piece(const bf16* p) {
-  const uint2 raw = *reinterpret_cast<const uint2*>(p);
-  return make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16),
-                     __uint_as_float(raw.y & 0xffff0000u));
-}
 
 // A lane's R values of a row as floats: its pieces of the row at p (16-byte aligned) when kVector, else the `live` first of
 // the R that start at p.
@@ -388,13 +413,12 @@ __device__ __forceinline__ float sum_pair(pair32 a) {
 // for the ones just asked for, and a token cost a whole trip to the second-level cache (0.5 us, whatever the head
 // size).  Here a block copies eight tokens at a time (unit q and k in float, gates, the block's values of v)
 // with cp.async, whose groups are waited for in order, two chunks in flight, and reads them with shared-memory
-// loads.  For dim == 8 R, vdim a multiple of 16 and 16-byte aligned rows.
+// loads.  For heads of 256, vdim a multiple of 16 and 16-byte aligned rows (the kernel behind this one takes the smaller heads).
 //
 // Bound by instructions: a token is about 90 a warp of four columns, one after the other in a launch of a few hundred warps
 // (a prompt or two: each waits for the one before, some 3.5 cycles), and one of several warps' on every scheduler in a wide
 // one.  So a multiply-add works on two numbers, a chunk's tokens lie at places known to the compiler, and what a thread copies
-// comes from pointers that move on by a constant.  Measured on B200, 16 heads of 128 x 128: one prompt of 512 tokens 98 us
-// (148 before these three), eight 304 (404).  Two columns a lane, which share the reads of q and k: 119 and 309.
+// comes from pointers that move on by a constant.
 constexpr int kStageTokens = 8;
 
 template <typename T, int R>
@@ -530,6 +554,278 @@ gated_delta_rule_staged_kernel(const T* __restrict__ qkv, const float* __restric
     *reinterpret_cast<ulonglong2*>(mine + piece_at(c, part)) = make_ulonglong2(S[c][0], S[c][1]);
 }
 
+// The same for head sizes up to 128: two tokens at a time, C columns a lane (1, or 2 where a launch has blocks enough).  With S the state before a pair of
+// tokens, S2 = g1 g2 S + k1 (g2 c1)^T + k2 c2^T, where c1 = beta1 (v1 - g1 S^T k1) and c2 = beta2 (v2 - g2 (g1 S^T k2 + (k1 . k2) c1)):
+// all four products with S (k1, k2, q1, q2) are taken at once, what the second token meets of the first is three products of the
+// pair's vectors that the kernel in front has made, and the sums over a column's eight lanes are one exchange of eight values
+// (seven shuffles, each lane ending with one of them; of four where a lane has one column) instead of four of two.  Two columns share the
+// reads of q and k.
+//
+// Bound by the multiply-adds and shared memory's reads side by side where a launch is wide (56 and 64 cycles of an SM for two tokens of eight
+// columns), by the chain of a pair's sums where it is not.  Measured on B200, 16 heads of 128 x 128, the kernel in front included: one
+// prompt of 512 tokens 79 us (94 a token at a time in one column a lane; 98 in two), eight of 512 272 (303), eight of 67 to 450 157 (181);
+// 8 heads, one of 1,400 198 (240).
+template <typename T, int R, int C>
+__global__ void __launch_bounds__(128)
+gated_delta_rule_pairs_kernel(const T* __restrict__ qkv, const float* __restrict__ units, const float* __restrict__ gates,
+                              const float* __restrict__ products, float* __restrict__ state, const int* __restrict__ query_start_loc,
+                              const int* __restrict__ state_slots, float* __restrict__ out, int heads, int kv_heads, int vdim) {
+  extern __shared__ __align__(16) unsigned char staged[];
+  constexpr int dim = 8 * R, kColumns = 16 * C, kPieces = R / 4;
+  constexpr int kUnitBytes = 8 * dim, kValueBytes = kColumns * (int)sizeof(T);
+  constexpr int kGatesAt = kUnitBytes, kProductsAt = kUnitBytes + 16, kValuesAt = kUnitBytes + 32;
+  constexpr int kTokenBytes = kValuesAt + kValueBytes;          // units | gates (8 bytes, padded) | products | v
+  grid_dependency_wait();
+  const int seq = blockIdx.z, head = blockIdx.y;
+  const int begin = query_start_loc[seq], end = query_start_loc[seq + 1];
+  if (end <= begin) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int part = lane >> 2;                                   // which eighth of the columns
+  const int local_column = (warp * 4 + (lane & 3)) * C;         // of C
+  const int qk_width = kv_heads * dim;
+  const size_t row_width = 2 * (size_t)qk_width + (size_t)heads * vdim;
+  const int kv_head = head / (heads / kv_heads);
+  const size_t v_at = 2 * (size_t)qk_width + (size_t)head * vdim + (size_t)blockIdx.x * kColumns;
+  float* mine = state + (((size_t)state_slots[seq] * heads + head) * vdim + blockIdx.x * kColumns + local_column) * dim;
+
+  pair32 S[C][kPieces][2];
+#pragma unroll
+  for (int j = 0; j < C; ++j)
+#pragma unroll
+    for (int c = 0; c < kPieces; ++c) {
+      const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(mine + j * dim + piece_at(c, part));
+      S[j][c][0] = v.x;
+      S[j][c][1] = v.y;
+    }
+
+  // A thread's copies of a chunk, as in the kernel above.
+  constexpr int kUnitPieces = kUnitBytes / 16, kRound = 128 / kUnitPieces > 0 ? 128 / kUnitPieces : 1;
+  constexpr int kValuePieces = kValueBytes / 16;
+  static_assert(128 % kUnitPieces == 0 && kStageTokens * kValuePieces <= 128, "a chunk's copies");
+  const size_t unit_row = (size_t)kv_heads * 2 * dim;
+  const int unit_token = threadIdx.x / kUnitPieces, unit_piece = threadIdx.x % kUnitPieces;
+  const float* unit_src = units + ((size_t)(begin + unit_token) * kv_heads + kv_head) * 2 * dim + unit_piece * 4;
+  const int value_token = threadIdx.x / kValuePieces, value_piece = threadIdx.x % kValuePieces;
+  const T* value_src = qkv + (size_t)(begin + value_token) * row_width + v_at + value_piece * (16 / (int)sizeof(T));
+  const int small_token = threadIdx.x & 31;                     // warp 0: gates; warp 1: products
+  const float* small_src = threadIdx.x < 32 ? gates + ((size_t)(begin + small_token) * heads + head) * 2
+                                            : products + ((size_t)(begin + small_token) * kv_heads + kv_head) * 4;
+  const size_t small_step = threadIdx.x < 32 ? (size_t)kStageTokens * heads * 2 : (size_t)kStageTokens * kv_heads * 4;
+  const unsigned stage = (unsigned)__cvta_generic_to_shared(staged);
+  auto copy_chunk = [&](int chunk) {
+    const unsigned buffer = stage + (unsigned)(chunk & 1) * (kStageTokens * kTokenBytes);
+    const int left = end - begin - chunk * kStageTokens;
+#pragma unroll
+    for (int j = 0; j < kStageTokens; j += kRound)
+      if (unit_token + j < left && unit_token + j < kStageTokens)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(buffer + (unit_token + j) * kTokenBytes + unit_piece * 16),
+                     "l"(unit_src + j * unit_row));
+    if (value_token < kStageTokens && value_token < left)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(buffer + value_token * kTokenBytes + kValuesAt + value_piece * 16),
+                   "l"(value_src));
+    if (threadIdx.x < 64 && small_token < kStageTokens && small_token < left) {
+      if (threadIdx.x < 32)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(buffer + small_token * kTokenBytes + kGatesAt), "l"(small_src));
+      else
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(buffer + small_token * kTokenBytes + kProductsAt), "l"(small_src));
+    }
+    asm volatile("cp.async.commit_group;" ::);
+    unit_src += kStageTokens * unit_row;
+    value_src += kStageTokens * row_width;
+    small_src += small_step;
+  };
+
+  const size_t out_row = (size_t)heads * vdim;
+  // A lane of the last four eighths (one column: of two of them) stores one of the pair's read-outs: of the first or the second token, of
+  // its first or second column.
+  const bool second_token = C == 2 ? part & 1 : part & 2, second_column = C == 2 && (part & 2);
+  const bool stores = C == 2 ? part >= 4 : part == 4 || part == 6;
+  float* out_at = out + (size_t)(begin + second_token) * out_row + (size_t)head * vdim + blockIdx.x * kColumns + local_column + second_column;
+  const auto column_values = [&](const unsigned char* tok, float (&v)[C]) {
+    const T* at = reinterpret_cast<const T*>(tok + kValuesAt) + local_column;
+#pragma unroll
+    for (int j = 0; j < C; ++j) v[j] = widen(at[j]);
+  };
+  // Sums over the eight lanes of a column group: lane `part` returns with the sum of v[part], or with one column of v[part / 2].
+  const auto exchange = [&](float (&v)[4 * C]) {
+    const bool high = part & 4, mid = part & 2, low = part & 1;
+    if constexpr (C == 1) {
+      float a[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) a[i] = (high ? v[i + 2] : v[i]) + __shfl_xor_sync(0xffffffffu, high ? v[i] : v[i + 2], 16);
+      const float b = (mid ? a[1] : a[0]) + __shfl_xor_sync(0xffffffffu, mid ? a[0] : a[1], 8);
+      return b + __shfl_xor_sync(0xffffffffu, b, 4);
+    } else {
+    float a[4], b[2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = (high ? v[i + 4] : v[i]) + __shfl_xor_sync(0xffffffffu, high ? v[i] : v[i + 4], 16);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) b[i] = (mid ? a[i + 2] : a[i]) + __shfl_xor_sync(0xffffffffu, mid ? a[i] : a[i + 2], 8);
+    return (low ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, low ? b[0] : b[1], 4);
+    }
+  };
+  // Which lane has the sums of S^T k of the first or second token, column j.
+  const auto holder = [&](int j, int token) { return (C == 2 ? 8 * j + 4 * token : 8 * token) + (lane & 3); };
+  // Two tokens whose inputs lie at `tok` and behind it.
+  const auto step_two = [&](const unsigned char* tok) {
+    const unsigned char *one = tok + part * 16, *two = one + kTokenBytes;
+    pair32 k1[kPieces][2], k2[kPieces][2], sum[C][4];
+#pragma unroll
+    for (int c = 0; c < kPieces; ++c) {
+      const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(one + dim * 4 + c * 128);
+      const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(two + dim * 4 + c * 128);
+      const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(one + c * 128), r = *reinterpret_cast<const ulonglong2*>(two + c * 128);
+      k1[c][0] = a.x, k1[c][1] = a.y, k2[c][0] = b.x, k2[c][1] = b.y;
+#pragma unroll
+      for (int j = 0; j < C; ++j) {
+        sum[j][0] = c == 0 ? mul_pair(S[j][c][0], a.x) : fma_pair(S[j][c][0], a.x, sum[j][0]);
+        sum[j][1] = c == 0 ? mul_pair(S[j][c][0], b.x) : fma_pair(S[j][c][0], b.x, sum[j][1]);
+        sum[j][2] = c == 0 ? mul_pair(S[j][c][0], q.x) : fma_pair(S[j][c][0], q.x, sum[j][2]);
+        sum[j][3] = c == 0 ? mul_pair(S[j][c][0], r.x) : fma_pair(S[j][c][0], r.x, sum[j][3]);
+        sum[j][0] = fma_pair(S[j][c][1], a.y, sum[j][0]);
+        sum[j][1] = fma_pair(S[j][c][1], b.y, sum[j][1]);
+        sum[j][2] = fma_pair(S[j][c][1], q.y, sum[j][2]);
+        sum[j][3] = fma_pair(S[j][c][1], r.y, sum[j][3]);
+      }
+    }
+    const float2 gate1 = *reinterpret_cast<const float2*>(tok + kGatesAt), gate2 = *reinterpret_cast<const float2*>(tok + kTokenBytes + kGatesAt);
+    const float own1 = *reinterpret_cast<const float*>(tok + kProductsAt);
+    const float4 met = *reinterpret_cast<const float4*>(tok + kTokenBytes + kProductsAt);      // q2 . k2, k2 . k1, q2 . k1
+    float v1[C], v2[C];
+    column_values(tok, v1);
+    column_values(tok + kTokenBytes, v2);
+    // By lane: S^T k1 and S^T k2 of the first column, of the second, then S^T q1 and S^T q2 of the first, of the second.
+    float parts[4 * C];
+#pragma unroll
+    for (int j = 0; j < C; ++j)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        parts[2 * j + i] = sum_pair(sum[j][i]);
+        parts[2 * C + 2 * j + i] = sum_pair(sum[j][2 + i]);
+      }
+    const float held = exchange(parts);
+    const float g1 = gate1.y, g2 = gate2.y, both_decays = g1 * g2;
+    float c1[C], c2[C];
+#pragma unroll
+    for (int j = 0; j < C; ++j) {
+      const float d1 = __shfl_sync(0xffffffffu, held, holder(j, 0)), d2 = __shfl_sync(0xffffffffu, held, holder(j, 1));
+      c1[j] = gate1.x * (v1[j] - g1 * d1);
+      c2[j] = gate2.x * (v2[j] - g2 * fmaf(met.y, c1[j], g1 * d2));
+    }
+    if (stores) {
+      const float first = second_column ? c1[C - 1] : c1[0], second = second_column ? c2[C - 1] : c2[0];
+      *out_at = second_token ? fmaf(met.x, second, fmaf(met.z, g2 * first, both_decays * held)) : fmaf(own1, first, g1 * held);
+    }
+    out_at += 2 * out_row;
+    const pair32 decay = both(both_decays);
+#pragma unroll
+    for (int j = 0; j < C; ++j) {
+      const pair32 e1 = both(g2 * c1[j]), e2 = both(c2[j]);
+#pragma unroll
+      for (int c = 0; c < kPieces; ++c) {
+        S[j][c][0] = fma_pair(S[j][c][0], decay, fma_pair(k2[c][0], e2, mul_pair(k1[c][0], e1)));
+        S[j][c][1] = fma_pair(S[j][c][1], decay, fma_pair(k2[c][1], e2, mul_pair(k1[c][1], e1)));
+      }
+    }
+  };
+  // The last token of an odd number.
+  const auto step_one = [&](const unsigned char* tok) {
+    const unsigned char* one = tok + part * 16;
+    pair32 k1[kPieces][2], sum[C][2];
+#pragma unroll
+    for (int c = 0; c < kPieces; ++c) {
+      const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(one + dim * 4 + c * 128), q = *reinterpret_cast<const ulonglong2*>(one + c * 128);
+      k1[c][0] = a.x, k1[c][1] = a.y;
+#pragma unroll
+      for (int j = 0; j < C; ++j) {
+        sum[j][0] = c == 0 ? mul_pair(S[j][c][0], a.x) : fma_pair(S[j][c][0], a.x, sum[j][0]);
+        sum[j][1] = c == 0 ? mul_pair(S[j][c][0], q.x) : fma_pair(S[j][c][0], q.x, sum[j][1]);
+        sum[j][0] = fma_pair(S[j][c][1], a.y, sum[j][0]);
+        sum[j][1] = fma_pair(S[j][c][1], q.y, sum[j][1]);
+      }
+    }
+    const float2 gate = *reinterpret_cast<const float2*>(tok + kGatesAt);
+    const float own = *reinterpret_cast<const float*>(tok + kProductsAt);
+    float v[C];
+    column_values(tok, v);
+    float parts[4 * C];
+#pragma unroll
+    for (int j = 0; j < C; ++j) {
+      parts[2 * j] = sum_pair(sum[j][0]);
+      parts[2 * C + 2 * j] = sum_pair(sum[j][1]);
+      parts[2 * j + 1] = parts[2 * C + 2 * j + 1] = 0.f;
+    }
+    const float held = exchange(parts);
+    float c1[C];
+#pragma unroll
+    for (int j = 0; j < C; ++j) c1[j] = gate.x * (v[j] - gate.y * __shfl_sync(0xffffffffu, held, holder(j, 0)));
+    if (stores && !second_token) *out_at = fmaf(own, second_column ? c1[C - 1] : c1[0], gate.y * held);
+    const pair32 decay = both(gate.y);
+#pragma unroll
+    for (int j = 0; j < C; ++j) {
+      const pair32 e1 = both(c1[j]);
+#pragma unroll
+      for (int c = 0; c < kPieces; ++c) {
+        S[j][c][0] = fma_pair(S[j][c][0], decay, mul_pair(k1[c][0], e1));
+        S[j][c][1] = fma_pair(S[j][c][1], decay, mul_pair(k1[c][1], e1));
+      }
+    }
+  };
+
+  const int chunks = (end - begin + kStageTokens - 1) / kStageTokens;
+  copy_chunk(0);
+  for (int chunk = 0; chunk < chunks; ++chunk) {
+    if (chunk + 1 < chunks) {
+      copy_chunk(chunk + 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const unsigned char* tok = staged + (size_t)(chunk & 1) * kStageTokens * kTokenBytes;
+    const int count = min(kStageTokens, end - begin - chunk * kStageTokens);
+    if (count == kStageTokens) {           // at places known when this is compiled
+#pragma unroll
+      for (int j = 0; j < kStageTokens; j += 2) step_two(tok + j * kTokenBytes);
+    } else {
+#pragma unroll 1
+      for (int j = 0; j + 1 < count; j += 2) step_two(tok + j * kTokenBytes);
+    }
+    if (count & 1) step_one(tok + (count - 1) * kTokenBytes);
+    __syncthreads();     // the buffer is written again two chunks on
+  }
+#pragma unroll
+  for (int j = 0; j < C; ++j)
+#pragma unroll
+    for (int c = 0; c < kPieces; ++c)
+      *reinterpret_cast<ulonglong2*>(mine + j * dim + piece_at(c, part)) = make_ulonglong2(S[j][c][0], S[j][c][1]);
+}
+
+// Whether a launch's prompts go two tokens at a time: the sizes and alignments that the kernel above takes.
+template <typename T>
+bool in_pairs(int dim, int vdim, int heads, int kv_heads, const T* qkv, const float* state, const float* scales) {
+  const size_t row_bytes = (2 * (size_t)kv_heads * dim + (size_t)heads * vdim) * sizeof(T);
+  return (dim == 32 || dim == 64 || dim == 128) && vdim % 16 == 0 && row_bytes % 16 == 0 && aligned16(qkv) && aligned16(state) &&
+         aligned16(scales) && ((size_t)heads * vdim * sizeof(T)) % 16 == 0 && (2 * (size_t)kv_heads * dim * sizeof(T)) % 16 == 0;
+}
+
+template <typename T, int R, int C>
+int launch_pairs(int tokens, dim3 grid, cudaStream_t stream, const T* qkv, const float* scales, const float* gates, const float* products,
+                 float* state, const int* qsl, const int* slots, float* out, int heads, int kv_heads, int vdim) {
+  constexpr size_t smem = 2 * (size_t)kStageTokens * (8 * 8 * R + 32 + 16 * C * sizeof(T));
+  return (int)launch_pdl(tokens, gated_delta_rule_pairs_kernel<T, R, C>, dim3(vdim / (16 * C), grid.y, grid.z), dim3(128), smem, stream, qkv, scales,
+                         gates, products, state, qsl, slots, out, heads, kv_heads, vdim);
+}
+
+// Two columns a lane where that still makes more than two blocks an SM; one where the chain is what a launch waits for.
+template <typename T, int R>
+int launch_pairs(int tokens, dim3 grid, cudaStream_t stream, const T* qkv, const float* scales, const float* gates, const float* products,
+                 float* state, const int* qsl, const int* slots, float* out, int heads, int kv_heads, int vdim) {
+  const bool wide = vdim % 32 == 0 && (long)(vdim / 32) * grid.y * grid.z > 2 * 148;
+  return wide ? launch_pairs<T, R, 2>(tokens, grid, stream, qkv, scales, gates, products, state, qsl, slots, out, heads, kv_heads, vdim)
+              : launch_pairs<T, R, 1>(tokens, grid, stream, qkv, scales, gates, products, state, qsl, slots, out, heads, kv_heads, vdim);
+}
+
 template <typename T, int R>
 int launch_delta_r(bool single, bool vector, int tokens, dim3 grid, cudaStream_t stream, const T* qkv, const float* scales,
                    const float* gates, float* state, const int* qsl, const int* slots, float* out, int heads,
@@ -544,11 +840,13 @@ int launch_delta_r(bool single, bool vector, int tokens, dim3 grid, cudaStream_t
     if (vector) LI_DELTA(1, true);
     LI_DELTA(1, false);
   }
-  if (vector && vdim % 16 == 0 && aligned16(scales) && (((size_t)heads * vdim) * sizeof(T)) % 16 == 0) {
-    constexpr size_t smem = 2 * (size_t)kStageTokens * (8 * 8 * R + 16 + (16 * sizeof(T) + 15) / 16 * 16);
-    const dim3 staged_grid(vdim / 16, grid.y, grid.z);
-    return (int)launch_pdl(tokens, gated_delta_rule_staged_kernel<T, R>, staged_grid, dim3(128), smem, stream, qkv, scales, gates,
-                           state, qsl, slots, out, heads, kv_heads, vdim);
+  if constexpr (R == 32) {      // (smaller heads go two tokens at a time)
+    if (vector && vdim % 16 == 0 && aligned16(scales) && (((size_t)heads * vdim) * sizeof(T)) % 16 == 0) {
+      constexpr size_t smem = 2 * (size_t)kStageTokens * (8 * 8 * R + 16 + (16 * sizeof(T) + 15) / 16 * 16);
+      const dim3 staged_grid(vdim / 16, grid.y, grid.z);
+      return (int)launch_pdl(tokens, gated_delta_rule_staged_kernel<T, R>, staged_grid, dim3(128), smem, stream, qkv, scales, gates,
+                             state, qsl, slots, out, heads, kv_heads, vdim);
+    }
   }
   if (vector) LI_DELTA(kDeep, true);
   LI_DELTA(kDeep, false);
@@ -623,7 +921,7 @@ LI_EXPORT int li_short_conv_update(int dtype, const void* x, size_t x_stride, vo
 
 // qkv [tokens, 2 * kv_heads * dim + heads * vdim]; ab [tokens, >= 2 * heads] with `ab_stride` elements a row; state
 // [slots, heads, vdim, dim] (column by column); out [tokens, heads * vdim]; scratch: 2 * tokens * (kv_heads * dim +
-// heads) floats.  max_q_len: the most tokens a sequence brings (1 chooses the variant without tokens in flight).
+// heads) + 4 * tokens * kv_heads + 4 floats.  max_q_len: the most tokens a sequence brings (1 chooses the variant without tokens in flight).
 LI_EXPORT int li_gated_delta_rule(int dtype, const void* qkv, const void* ab, size_t ab_stride, int tokens, int num_seqs,
                                   const float* a_log, const float* dt_bias, float* state, const int* query_start_loc,
                                   const int* state_slots, float* out, int heads, int kv_heads, int dim, int vdim,
@@ -634,27 +932,28 @@ LI_EXPORT int li_gated_delta_rule(int dtype, const void* qkv, const void* ab, si
     return LI_ERR_UNSUPPORTED;
   float* scales = scratch;
   float* gates = scratch + 2 * (size_t)tokens * kv_heads * dim;
+  float* room = gates + ((2 * (size_t)tokens * heads + 3) & ~(size_t)3);      // products of neighbouring tokens
   const size_t row_width = 2 * (size_t)kv_heads * dim + (size_t)heads * vdim;
   const size_t items = (size_t)tokens * (kv_heads + (heads + 31) / 32);
   const dim3 gates_grid((unsigned)((items + 7) / 8));
   const dim3 grid((vdim + 31) / 32, heads, num_seqs);
   const bool single = max_q_len == 1;     // the recurrence kernel then works out scales and gates itself
-  int code = 0;
-  if (dtype == kFloat32) {
-    if (!single)
-      code = (int)launch_pdl(tokens, delta_gates_kernel<float>, gates_grid, dim3(256), 0, stream, (const float*)qkv,
-                             row_width, (const float*)ab, ab_stride, a_log, dt_bias, scales, gates, tokens, heads,
-                             kv_heads, dim);
-    if (code) return code;
-    return launch_delta<float>(dim, single, tokens, grid, stream, (const float*)qkv, scales, gates, state,
-                               query_start_loc, state_slots, out, heads, kv_heads, vdim, (const float*)ab, ab_stride,
-                               a_log, dt_bias);
-  }
-  if (!single)
-    code = (int)launch_pdl(tokens, delta_gates_kernel<bf16>, gates_grid, dim3(256), 0, stream, (const bf16*)qkv,
-                           row_width, (const bf16*)ab, ab_stride, a_log, dt_bias, scales, gates, tokens, heads, kv_heads,
-                           dim);
-  if (code) return code;
-  return launch_delta<bf16>(dim, single, tokens, grid, stream, (const bf16*)qkv, scales, gates, state, query_start_loc,
-                            state_slots, out, heads, kv_heads, vdim, (const bf16*)ab, ab_stride, a_log, dt_bias);
+  const auto run = [&](auto* typed) {
+    using T = std::remove_cv_t<std::remove_pointer_t<decltype(typed)>>;
+    const T* rows = (const T*)qkv;
+    const bool pairs = !single && in_pairs(dim, vdim, heads, kv_heads, rows, state, scales);
+    if (!single) {
+      const int code = (int)launch_pdl(tokens, delta_gates_kernel<T>, gates_grid, dim3(256), 0, stream, rows, row_width, (const T*)ab,
+                                       ab_stride, a_log, dt_bias, scales, gates, pairs ? room : (float*)nullptr, tokens, heads, kv_heads, dim);
+      if (code) return code;
+    }
+    if (pairs) {
+      if (dim == 32) return launch_pairs<T, 4>(tokens, grid, stream, rows, scales, gates, room, state, query_start_loc, state_slots, out, heads, kv_heads, vdim);
+      if (dim == 64) return launch_pairs<T, 8>(tokens, grid, stream, rows, scales, gates, room, state, query_start_loc, state_slots, out, heads, kv_heads, vdim);
+      return launch_pairs<T, 16>(tokens, grid, stream, rows, scales, gates, room, state, query_start_loc, state_slots, out, heads, kv_heads, vdim);
+    }
+    return launch_delta<T>(dim, single, tokens, grid, stream, rows, scales, gates, state, query_start_loc, state_slots, out, heads, kv_heads,
+                           vdim, (const T*)ab, ab_stride, a_log, dt_bias);
+  };
+  return dtype == kFloat32 ? run((float*)nullptr) : run((bf16*)nullptr);
 }

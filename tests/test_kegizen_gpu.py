@@ -214,6 +214,32 @@ def test_gated_delta_rule_in_portions_equals_whole(dtype, heads, kv_heads, dim, 
     assert not state_parts[[1, 2]].any()
 
 
+# Two tokens at a time: sequences of one token, of an odd and an even number, around the eight that are staged at once; one column a lane and
+# (40 sequences x 4 heads x 2 blocks of columns) two.
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("kv_heads,dim,vdim,lengths", [(1, 128, 48, [1, 2, 3, 7, 8, 9, 17]), (4, 32, 16, [16, 1, 15]),
+                                                       (2, 64, 64, [1 + i % 19 for i in range(40)])])
+def test_gated_delta_rule_two_tokens_at_a_time(dtype, kv_heads, dim, vdim, lengths):
+    from liteinfer_b200 import ops
+
+    heads, tokens = 4, sum(lengths)
+    qkv = _randn(tokens, 2 * kv_heads * dim + heads * vdim, seed=1, dtype=dtype)
+    ab = _randn(tokens, 2 * heads, seed=2, scale=2.0, dtype=dtype)
+    a_log, dt_bias = torch.log(1 + 3 * torch.rand(heads, device=DEV)), _randn(heads, seed=5)
+    qsl = [0]
+    for n in lengths:
+        qsl.append(qsl[-1] + n)
+    slots = _ints(torch.randperm(len(lengths), generator=torch.Generator().manual_seed(3)).tolist())
+    got = []
+    for impl in (ops, ref):
+        state = _randn(len(lengths), heads, vdim, dim, seed=7, scale=0.1)
+        out = torch.zeros(tokens, heads * vdim, device=DEV)
+        impl.gated_delta_rule(qkv, ab, a_log, dt_bias, state, _ints(qsl), slots, len(lengths), heads, kv_heads, dim, vdim, out, max(lengths))
+        got.append((out, state))
+    for a, b in zip(*got):
+        torch.testing.assert_close(a, b, rtol=1e-4, atol=1e-5)
+
+
 def test_gated_delta_rule_recalls_a_far_key():
     """One key written 300 tokens back with decay 1 is read out exactly; with a decay below 1 it has faded."""
     from liteinfer_b200 import ops
