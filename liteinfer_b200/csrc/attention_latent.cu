@@ -212,6 +212,27 @@ __global__ void gate_heads_kernel(const T* __restrict__ v, const T* __restrict__
   }
 }
 
+// The same, 16 bytes of a head's output a thread (vdim and gate_stride whole vectors, 16-byte aligned pointers): element by element a
+// prompt's threads did little but divide for their place, 25 us for 2,860 tokens of 16 heads of 128, 4.6 now.
+template <typename T>
+__global__ void gate_heads_vec_kernel(const T* __restrict__ v, const T* __restrict__ gate, int gate_stride, T* __restrict__ out,
+                                      int tokens, int heads, int pieces) {
+  constexpr int N = Vec16<T>::N;
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const int per_token = heads * pieces, i = blockIdx.y * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x;
+  if (i >= per_token) return;
+  const int h = i / pieces, piece = i - h * pieces;
+  float x[N], g[N];
+  unpack16(load16(v + (((size_t)h * tokens + t) * pieces + piece) * N), x);
+  if (gate) unpack16(load16(gate + (size_t)t * gate_stride + (size_t)i * N), g);
+  Vec16<T> result;
+#pragma unroll
+  for (int e = 0; e < N; ++e) result.set(e, x[e] * (gate ? 1.0f / (1.0f + expf(-g[e])) : 1.0f));
+  store16(out + ((size_t)t * per_token + i) * N, result);
+}
+
 }  // namespace li
 
 using namespace li;
@@ -283,6 +304,17 @@ LI_EXPORT int li_gate_heads(int dtype, const void* v, const void* gate, int gate
                             int heads, int vdim, cudaStream_t stream) {
   const size_t n = (size_t)tokens * heads * vdim;
   if (n == 0) return 0;
+  const int lanes = dtype == kFloat32 ? 4 : 8;
+  if (vdim % lanes == 0 && (gate == nullptr || gate_stride % lanes == 0) && aligned16(v) && aligned16(gate) && aligned16(out)) {
+    const int pieces = vdim / lanes, items = heads * pieces, threads = items < 256 ? (items + 31) / 32 * 32 : 256;
+    const dim3 grid(tokens, (items + threads - 1) / threads);
+    if (grid.y <= 65535)
+      return (int)(dtype == kFloat32
+                       ? launch_pdl(tokens, gate_heads_vec_kernel<float>, grid, dim3(threads), 0, stream, (const float*)v,
+                                    (const float*)gate, gate_stride, (float*)out, tokens, heads, pieces)
+                       : launch_pdl(tokens, gate_heads_vec_kernel<bf16>, grid, dim3(threads), 0, stream, (const bf16*)v,
+                                    (const bf16*)gate, gate_stride, (bf16*)out, tokens, heads, pieces));
+  }
   const int blocks = (int)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);
   cudaError_t e;
   if (dtype == kFloat32)

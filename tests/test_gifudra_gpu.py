@@ -113,6 +113,19 @@ def test_squared_relu_and_gate(dtype):
     assert torch.equal(plain, v.transpose(0, 1).reshape(9, 60))
 
 
+# Heads of whole vectors: fewer of them in a token than a block has threads, and more; one token and several.
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("tokens,heads,vdim", [(1, 1, 8), (5, 3, 24), (7, 40, 128)])
+def test_gate_heads_by_vectors(dtype, tokens, heads, vdim):
+    from liteinfer_b200 import ops
+
+    v, wide = _randn(heads, tokens, vdim, seed=1, dtype=dtype), _randn(tokens, heads * vdim + 16, seed=2, dtype=dtype)
+    gate, out = wide[:, 8:8 + heads * vdim], lambda: torch.empty(tokens, heads * vdim, dtype=dtype, device=DEV)
+    plain = v.transpose(0, 1).reshape(tokens, heads * vdim)
+    torch.testing.assert_close(ops.gate_heads(v, gate, out()).float(), plain.float() * torch.sigmoid(gate.float()), **_tol(dtype))
+    assert torch.equal(ops.gate_heads(v, None, out()), plain)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("M,N,K", [(1, 264, 96), (5, 4096, 512), (8, 200, 1024), (12, 328, 96), (16, 8192, 256), (40, 264, 96)])
 @pytest.mark.parametrize("name", ["relu_squared", "silu", "gelu_tanh"])
