@@ -103,6 +103,75 @@ __global__ void short_conv_vec_kernel(const T* __restrict__ x, size_t x_stride, 
   store16(out + (size_t)t * channels + c, result);
 }
 
+// The same for prompts, kRunTokens neighbouring tokens a thread: the taps of its channels stay in registers, and so do the K - 1 inputs
+// before the token at hand, so every input is read once and a half instead of K times, and all of a run's are asked for at once.  2,070
+// tokens of 6,144 channels, four taps: 15.9 us (23).
+constexpr int kRunTokens = 8;
+template <typename T, int K>
+__global__ void __launch_bounds__(128)
+short_conv_run_kernel(const T* __restrict__ x, size_t x_stride, const T* __restrict__ taps, const T* __restrict__ tail,
+                      const int* __restrict__ seq_of_token, const int* __restrict__ query_start_loc,
+                      const int* __restrict__ state_slots, T* __restrict__ out, int tokens, int channels, int act,
+                      const float* __restrict__ bias) {
+  constexpr int N = Vec16<T>::N;
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * N;
+  if (c >= channels) return;
+  grid_dependency_wait();
+  const int first = blockIdx.x * kRunTokens;
+  Vec16<T> input[kRunTokens];
+#pragma unroll
+  for (int i = 0; i < kRunTokens; ++i) input[i] = load16(x + (size_t)min(first + i, tokens - 1) * x_stride + c);
+  float w[K][N], b[N];
+#pragma unroll
+  for (int m = 0; m < K; ++m) unpack16(load16(taps + (size_t)m * channels + c), w[m]);
+#pragma unroll
+  for (int e = 0; e < N; ++e) b[e] = bias != nullptr ? bias[c + e] : 0.f;
+  Vec16<T> before[K - 1];       // the inputs K - 1, ..., 1 tokens back
+  int current = -1;
+#pragma unroll
+  for (int i = 0; i < kRunTokens; ++i) {
+    const int t = first + i;
+    if (t >= tokens) return;
+    const int seq = seq_of_token[t];
+    Vec16<T> result;
+    if (seq < 0) {
+#pragma unroll
+      for (int e = 0; e < N; ++e) result.set(e, 0.f);
+      store16(out + (size_t)t * channels + c, result);
+      current = -1;
+      continue;
+    }
+    if (seq != current) {       // a run's first token, or the first of the next sequence
+      const int j = t - query_start_loc[seq];
+      const T* old = tail + (size_t)state_slots[seq] * (K - 1) * channels;
+#pragma unroll
+      for (int m = 0; m < K - 1; ++m) {
+        const int back = K - 1 - m;
+        before[m] = back <= j ? load16(x + (size_t)(t - back) * x_stride + c) : load16(old + (size_t)(K - 1 + j - back) * channels + c);
+      }
+      current = seq;
+    }
+    float acc[N], v[N];
+#pragma unroll
+    for (int e = 0; e < N; ++e) acc[e] = b[e];
+#pragma unroll
+    for (int m = 0; m < K; ++m) {
+      unpack16(m < K - 1 ? before[m < K - 1 ? m : 0] : input[i], v);
+#pragma unroll
+      for (int e = 0; e < N; ++e) acc[e] = fmaf(w[m][e], v[e], acc[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+      const float sig = sizeof(T) == 2 ? __fdividef(1.0f, 1.0f + __expf(-acc[e])) : 1.0f / (1.0f + expf(-acc[e]));
+      result.set(e, act ? acc[e] * sig : acc[e]);
+    }
+    store16(out + (size_t)t * channels + c, result);
+#pragma unroll
+    for (int m = 0; m + 1 < K - 1; ++m) before[m] = before[m + 1];
+    before[K - 2] = input[i];
+  }
+}
+
 template <typename T>
 __global__ void short_conv_update_kernel(const T* __restrict__ x, size_t x_stride, T* __restrict__ tail,
                                          const int* __restrict__ query_start_loc, const int* __restrict__ state_slots,
@@ -888,6 +957,17 @@ LI_EXPORT int li_short_conv(int dtype, const void* x, size_t x_stride, const voi
       (K == 1 || aligned16(tail))) {
     const int vectors = channels / lanes;
     const dim3 vgrid(tokens, (vectors + 127) / 128);
+    // Four taps, and tokens enough that every SM still has a few blocks.
+    if (K == 4 && !move_tail && (long)(tokens / kRunTokens) * vgrid.y >= 2 * 148) {
+      const dim3 rgrid((tokens + kRunTokens - 1) / kRunTokens, vgrid.y);
+      if (dtype == kFloat32)
+        return (int)launch_pdl(tokens, short_conv_run_kernel<float, 4>, rgrid, dim3(128), 0, stream, (const float*)x, x_stride,
+                               (const float*)taps, (const float*)tail, seq_of_token, query_start_loc, state_slots, (float*)out, tokens,
+                               channels, act, bias);
+      return (int)launch_pdl(tokens, short_conv_run_kernel<bf16, 4>, rgrid, dim3(128), 0, stream, (const bf16*)x, x_stride,
+                             (const bf16*)taps, (const bf16*)tail, seq_of_token, query_start_loc, state_slots, (bf16*)out, tokens, channels,
+                             act, bias);
+    }
     if (dtype == kFloat32)
       return (int)launch_pdl(tokens, short_conv_vec_kernel<float>, vgrid, dim3(128), 0, stream, (const float*)x, x_stride,
                              (const float*)taps, (const float*)tail, seq_of_token, query_start_loc, state_slots,

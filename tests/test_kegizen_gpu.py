@@ -161,6 +161,34 @@ def test_short_conv_in_portions_equals_whole(dtype, taps):
     assert not tail_parts[[0, 1, 3, 4, 6, 7]].any()
 
 
+# Tokens in runs of eight: sequences that end anywhere in a run and several in one, tokens of padding behind them, to the bit what each
+# sequence gives alone.
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_short_conv_in_runs_of_tokens(dtype):
+    from liteinfer_b200 import ops
+
+    channels, lengths = 2056, [1, 2, 5, 700, 3, 89, 400, 11]
+    tokens = sum(lengths) + 5
+    wide = _randn(tokens, channels + 8, seed=1, dtype=dtype)
+    x, w = wide[:, 8:], _randn(4, channels, seed=3, scale=0.5, dtype=dtype)
+    tail = _randn(len(lengths) + 1, 3, channels, seed=4, dtype=dtype)
+    bias = _randn(channels, seed=5)
+    slots = torch.randperm(len(lengths), generator=torch.Generator().manual_seed(2)).tolist()
+    qsl = [0]
+    for n in lengths:
+        qsl.append(qsl[-1] + n)
+    seq_of = [i for i, n in enumerate(lengths) for _ in range(n)] + [-1] * 5
+    out = lambda n: torch.empty(n, channels, dtype=dtype, device=DEV)
+    got = ops.short_conv(x, w, tail, _ints(seq_of), _ints(qsl), _ints(slots), out(tokens), "silu", bias=bias)
+    for i, n in enumerate(lengths):
+        part = x[qsl[i]:qsl[i] + min(n, 60)]        # (a launch of few tokens has a token a block)
+        alone = ops.short_conv(part, w, tail, _ints([0] * len(part)), _ints([0, len(part)]), _ints([slots[i]]), out(len(part)), "silu",
+                               bias=bias)
+        assert torch.equal(got[qsl[i]:qsl[i] + len(part)], alone)
+    want = ref.short_conv(x, w, tail, _ints(seq_of), _ints(qsl), _ints(slots), out(tokens), "silu", bias=bias)
+    torch.testing.assert_close(got.float(), want.float(), **_tol(dtype))
+
+
 def test_short_conv_skips_padding():
     from liteinfer_b200 import ops
 
