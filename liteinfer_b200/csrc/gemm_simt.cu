@@ -41,10 +41,10 @@ struct SimtProduct {
 // cycles where its multiply-adds take 32 in all.  Rows lie along k in both operands (threads have rows 8 and 16 apart, which with
 // rows of 36 words keeps the reads off one another's banks), so two neighbours along k are a pair as they are loaded.  Three steps
 // of 32 k are on their way (cp.async) while a fourth is multiplied.  Three blocks of four warps an SM: blocks of this size spread a
-// grid of a few hundred over the SMs more evenly than 128 x 64 (1,250 rows of 1280 x 768: 79 us, 97), and half the
+// grid of a few hundred over the SMs more evenly than 128 x 64 (1,250 rows of 1280 x 768: 78 us, 97), and half the
 // multiply-adds' instructions leave the issue slots to the loads.
-// Measured on B200, 1,250 rows: 3072 x 2048 437 us (36 TFLOP/s; 486 in tiles of 128 x 64 with one-wide multiply-adds), 4096 x 768
-// 213 (232); 400 rows of 2048 x 8192 443 (595), of 1280 x 768 35 (44).
+// Measured on B200, 1,250 rows: 768 x 2048 132 us (145 with reads just ahead of their use), 4096 x 768 204 us (39 TFLOP/s; 232 in
+// tiles of 128 x 64 with one-wide multiply-adds); 400 rows of 768 x 768 33 (37), 256 of 16000 x 768 160 (169).
 constexpr int BN = 64, BK = 32, kTileThreads = 128, kTileStages = 4;
 constexpr int kTileRow = BK + 4;
 template <int BM> constexpr size_t kTileSmem = (size_t)kTileStages * (BM + BN) * kTileRow * sizeof(float);
@@ -122,19 +122,30 @@ __global__ void __launch_bounds__(kTileThreads, 3) gemm_simt_tile_kernel(SimtPro
     const float* stage = tile_smem + (step % kTileStages) * ((BM + BN) * kTileRow);
     const float* xr = stage + ty * kTileRow;
     const float* wr = stage + (BM + tx) * kTileRow;
-#pragma unroll 2
-    for (int k = 0; k < BK; k += 4) {
-      ulonglong2 b[4];
+    // (The next four k are read while these are multiplied.)
+    const auto read = [&](int k, ulonglong2 (&a)[BM / 8], ulonglong2 (&b)[4]) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(wr + j * 16 * kTileRow + k);
 #pragma unroll
+      for (int i = 0; i < BM / 8; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xr + i * 8 * kTileRow + k);
+    };
+    ulonglong2 a[BM / 8], b[4];
+    read(0, a, b);
+#pragma unroll
+    for (int k = 0; k < BK; k += 4) {
+      ulonglong2 next_a[BM / 8], next_b[4];
+      if (k + 4 < BK) read(k + 4, next_a, next_b);
+#pragma unroll
       for (int i = 0; i < BM / 8; ++i) {
-        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(xr + i * 8 * kTileRow + k);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = multiply_add(a.x, b[j].x, acc[i][j]);
+        for (int j = 0; j < 4; ++j) acc[i][j] = multiply_add(a[i].x, b[j].x, acc[i][j]);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = multiply_add(a.y, b[j].y, acc[i][j]);
+        for (int j = 0; j < 4; ++j) acc[i][j] = multiply_add(a[i].y, b[j].y, acc[i][j]);
       }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) b[j] = next_b[j];
+#pragma unroll
+      for (int i = 0; i < BM / 8; ++i) a[i] = next_a[i];
     }
     if ((step + 1) * BK % kChunk == 0 || step + 1 == steps) {
 #pragma unroll
