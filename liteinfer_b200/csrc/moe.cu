@@ -190,8 +190,10 @@ moe_route_kernel(const float* __restrict__ logits, int tokens, const RouteRule r
 // The router's product and the routing in one launch: logits[e] = sum_k x[k] * w[e][k] in 32-bit (lane l adds up
 // its k in order, then the lanes' sums meet in a fixed tree: the same bits whatever else is in the step), then
 // `route_token`.  A block takes TOK tokens; a warp takes EXP experts at a time, so that a value of x serves EXP products
-// and one of w TOK: eight tokens by four experts in a wide step; in a narrow one, where a warp's chain of loads is what
-// the launch waits for, one token and two experts of as many warps as there are.
+// and one of w TOK: eight tokens by four experts in a wide step, which reading w once a block bounds (2,048 tokens of 2,048 by 32
+// experts: 14.3 us, 67 MB from the second-level cache; 15.8 with 160 exchanges instead of 31 for 32 sums; sixteen tokens a block leave
+// too few warps: 18 to 36); four tokens where that leaves SMs idle; in a narrow step, where a warp's chain of loads is what the
+// launch waits for, one token and two experts of as many warps as there are.
 //
 // `gated`: w has one more row, whose logit's sigmoid is a number per token for an expert that every token runs.  It goes
 // to gate[token] (where given) and is the weight of the slots behind the chosen experts, which hold the experts
@@ -221,7 +223,7 @@ moe_router_kernel(const T* __restrict__ x, size_t x_stride, const float* __restr
 #pragma unroll
     for (int t = 0; t < TOK; ++t) xr[t] = x + (size_t)min(t0 + t, tokens - 1) * x_stride;
     if (wide) {
-#pragma unroll(TOK == 1 ? 8 : 2)
+#pragma unroll(TOK == 1 ? 8 : TOK == 4 ? 4 : 2)
       for (int k = lane * 4; k < K; k += 128) {
         float4 wv[EXP];
 #pragma unroll
@@ -252,13 +254,39 @@ moe_router_kernel(const T* __restrict__ x, size_t x_stride, const float* __restr
         }
       }
     }
-#pragma unroll
-    for (int i = 0; i < EXP; ++i) {
+    const auto put = [&](int i, int t, float sum) {
       const int e = e0 + i * warps;
+      if (e < rows) route_smem[t * per_token + (e < experts ? e : per_token - 1)] = sum;
+    };
+    if constexpr (TOK == 1) {
 #pragma unroll
-      for (int t = 0; t < TOK; ++t) {
-        const float sum = warp_sum(acc[i][t]);
-        if (lane == 0 && e < rows) route_smem[t * per_token + (e < experts ? e : per_token - 1)] = sum;
+      for (int i = 0; i < EXP; ++i) {
+        const float sum = warp_sum(acc[i][0]);
+        if (lane == 0) put(i, 0, sum);
+      }
+    } else {
+      // The lanes' sums meet in the tree of `warp_sum`, but a lane keeps half of what it holds at every step and gives the other
+      // half away: 31 exchanges for 32 sums instead of 160.
+      constexpr int kSums = EXP * TOK < 32 ? EXP * TOK : 32, kShared = 32 / kSums;      // lanes that end up with the same sum
+      static_assert(EXP * TOK % kSums == 0 && kSums % TOK == 0, "whole experts at a time");
+#pragma unroll
+      for (int i0 = 0; i0 < EXP; i0 += kSums / TOK) {
+        float v[kSums];
+#pragma unroll
+        for (int n = 0; n < kSums; ++n) v[n] = acc[i0 + n / TOK][n % TOK];
+#pragma unroll
+        for (int o = 16, held = kSums; o >= kShared; o >>= 1, held >>= 1) {
+          const bool upper = (lane & o) != 0;
+#pragma unroll
+          for (int n = 0; n < held / 2; ++n) {
+            const float keep = upper ? v[n + held / 2] : v[n], give = upper ? v[n] : v[n + held / 2];
+            v[n] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+          }
+        }
+#pragma unroll
+        for (int o = kShared >> 1; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        const int n = lane / kShared;
+        if (lane % kShared == 0) put(i0 + n / TOK, n % TOK, v[0]);
       }
     }
   }
@@ -344,18 +372,29 @@ moe_sort_kernel(const int* __restrict__ ids, int pairs, int experts, int tile_ro
   for (int i = threadIdx.x + kHeld * blockDim.x; i < pairs; i += blockDim.x) put(i, ids[i]);
 }
 
-// out[m] = x[order[m] / top]: every pair's token row, in the order of the experts' runs.
+// out[m] = x[order[m] / top]: every pair's token row, in the order of the experts' runs.  A block copies one piece of
+// `kGatherRows` rows, a vector of each a thread, so that a thread looks its rows up and has them all on their way at once.
+// 2,048 tokens of 2,048, four experts a token: 7.5 us (8.9 a vector at a time), 8,000 of 1,024, eight: 24.5 (32.6; 144 MB).
+constexpr int kGatherRows = 4;
+
 template <typename T>
-__global__ void moe_gather_kernel(const T* __restrict__ x, size_t x_stride, const int* __restrict__ order, int top,
-                                  T* __restrict__ out, const int* __restrict__ count, int width) {
+__global__ void __launch_bounds__(256)
+moe_gather_kernel(const T* __restrict__ x, size_t x_stride, const int* __restrict__ order, int top, T* __restrict__ out,
+                  const int* __restrict__ count, int pieces) {
   constexpr int N = Vec16<T>::N;
+  const int m0 = blockIdx.x * kGatherRows, piece = blockIdx.y * blockDim.x + threadIdx.x;
   grid_dependency_wait();
-  const int per_row = width / N;
-  const size_t total = (size_t)*count * per_row;       // pairs of identity experts are in no run
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const int m = (int)(i / per_row), c = (int)(i - (size_t)m * per_row) * N;
-    store16(out + (size_t)m * width + c, load16(x + (size_t)(order[m] / top) * x_stride + c));
-  }
+  const int rows = min(kGatherRows, *count - m0);       // pairs of identity experts are in no run
+  if (piece >= pieces) return;
+  const T* from = x + (size_t)piece * N;
+  T* to = out + ((size_t)m0 * pieces + piece) * N;
+  Vec16<T> v[kGatherRows];
+#pragma unroll
+  for (int r = 0; r < kGatherRows; ++r)
+    if (r < rows) v[r] = load16(from + (size_t)(order[m0 + r] / top) * x_stride);
+#pragma unroll
+  for (int r = 0; r < kGatherRows; ++r)
+    if (r < rows) store16(to + (size_t)r * pieces * N, v[r]);
 }
 
 // --------------------------------------------------------------------------------- grouped, FFMA
@@ -664,16 +703,21 @@ LI_EXPORT int li_moe_router(int dtype, const void* x, size_t x_stride, const flo
   if (identity_experts < 0 || (identity_experts > 0) != (identity != nullptr) || (identity_experts > 0 && gated))
     return LI_ERR_UNSUPPORTED;
   const bool wide = tokens > 128;
-  const size_t smem = (size_t)(wide ? 8 : 1) * (route_floats(experts, groups) + 1) * sizeof(float);
+  const size_t smem = (size_t)(wide ? 8 : 1) * (route_floats(experts, groups) + 1) * sizeof(float);      // (four tokens: half)
   if (smem > 48 * 1024) return LI_ERR_UNSUPPORTED;
   const int rows = experts + (gated ? 1 : 0);
   const int most = wide ? 16 : 32;
   const int wanted = wide ? (rows + 3) / 4 : rows;     // a narrow step: a warp a row as far as they go, then two
   const int warps = wanted < most ? wanted : most;
+  // Four tokens a block where all such blocks have a place at once (sixteen of these warps an SM): what counts then is how long a block
+  // takes.  In more than one wave of blocks eight read w half as often.  500 tokens of 2,048 by 32 experts 7.9 us (10.6 by eight),
+  // 300 of 4,096 by 128 26.5 (50); just beyond the line 1,500 by 32 16.7 (14.3), 700 by 128 32.3 (28.9).
+  const bool four = wide && (tokens + 3) / 4 <= 148 * (16 / warps);
 #define LI_ROUTER(T, TOK, EXP)                                                                                        \
   return (int)launch_pdl(tokens, moe_router_kernel<T, TOK, EXP>, dim3((tokens + TOK - 1) / TOK), dim3(warps * 32),     \
                          smem, stream, (const T*)x, x_stride, w, tokens, K, rule, gated ? 1 : 0, ids, weights, gate)
-  if (dtype == kFloat32) { if (wide) LI_ROUTER(float, 8, 4); LI_ROUTER(float, 1, 2); }
+  if (dtype == kFloat32) { if (four) LI_ROUTER(float, 4, 4); if (wide) LI_ROUTER(float, 8, 4); LI_ROUTER(float, 1, 2); }
+  if (four) LI_ROUTER(bf16, 4, 4);
   if (wide) LI_ROUTER(bf16, 8, 4);
   LI_ROUTER(bf16, 1, 2);
 #undef LI_ROUTER
@@ -685,13 +729,13 @@ LI_EXPORT int li_moe_gather(int dtype, const void* x, size_t x_stride, const int
   if (pairs == 0 || width == 0) return 0;
   const int n = dtype == kFloat32 ? 4 : 8;
   if (width % n || x_stride % n || !aligned16(x) || !aligned16(out)) return LI_ERR_ALIGNMENT;
-  const size_t total = (size_t)pairs * (width / n);
-  const dim3 grid((unsigned)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16));
+  const int pieces = width / n, threads = pieces < 256 ? (pieces + 31) / 32 * 32 : 256;
+  const dim3 grid((pairs + kGatherRows - 1) / kGatherRows, (pieces + threads - 1) / threads);
   if (dtype == kFloat32)
-    return (int)launch_pdl(pairs, moe_gather_kernel<float>, grid, dim3(256), 0, stream, (const float*)x, x_stride, order,
-                           top, (float*)out, count, width);
-  return (int)launch_pdl(pairs, moe_gather_kernel<bf16>, grid, dim3(256), 0, stream, (const bf16*)x, x_stride, order, top,
-                         (bf16*)out, count, width);
+    return (int)launch_pdl(pairs, moe_gather_kernel<float>, grid, dim3(threads), 0, stream, (const float*)x, x_stride, order,
+                           top, (float*)out, count, pieces);
+  return (int)launch_pdl(pairs, moe_gather_kernel<bf16>, grid, dim3(threads), 0, stream, (const bf16*)x, x_stride, order, top,
+                         (bf16*)out, count, pieces);
 }
 
 // mode 0: out[pair, 0:N] = act(W_gate,e x[pair / top], W_up,e x[pair / top]), w [experts, 2N, K] (gate rows, then up).

@@ -513,6 +513,40 @@ def test_expert_products_of_a_plan_in_tiles_of_128(counts):
     assert torch.equal(*got) and ops.gemm_error_flag(DEV) == 0
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("experts,K,top", [(5, 40, 2), (32, 264, 4), (61, 130, 3), (128, 512, 8)])
+def test_router_has_the_same_bits_at_every_width_of_block(dtype, experts, K, top):
+    """A step of up to 128 tokens takes one a block, of more four where all blocks have a place at once, else eight."""
+    from liteinfer_b200 import ops
+
+    x, w = _randn(5003, K, seed=7, dtype=dtype), _randn(experts, K, seed=8, scale=K ** -0.5)
+    results = {}
+    for tokens in (5003, 2365, 597, 593, 589, 301, 129, 128, 7, 1):
+        ids, weights = torch.empty(tokens, top, dtype=torch.int32, device=DEV), torch.empty(tokens, top, device=DEV)
+        ops.moe_router(x[:tokens], w, top, 1, 1, False, ids, weights)
+        results[tokens] = ids, weights
+    ids, weights = results[5003]
+    for tokens, (i, v) in results.items():
+        assert torch.equal(i, ids[:tokens]) and torch.equal(v, weights[:tokens])
+    # A softmax's weight moves by at most itself times twice what a logit does: K products of numbers that sum to a few units.
+    exact = (x.double() @ w.double().t()).softmax(-1).gather(1, ids.long())
+    torch.testing.assert_close(weights.double(), exact, rtol=K * 2.0 ** -22, atol=1e-7)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("tokens,width,top", [(1, 8, 1), (3, 264, 3), (5, 2056, 1), (130, 512, 4)])
+def test_gather_brings_the_pairs_that_have_an_expert(dtype, tokens, width, top):
+    from liteinfer_b200 import ops
+
+    ids = torch.randint(0, 7, (tokens, top), generator=torch.Generator().manual_seed(tokens), dtype=torch.int32).to(DEV)
+    plan = ops.moe_sort(ids, 5, 32)             # (5 and 6: no expert's, in no run)
+    count = int((ids < 5).sum())
+    x = _randn(tokens, 2 * width, seed=9, dtype=dtype)[:, :width]
+    out = ops.moe_gather(x, plan, top, torch.full((tokens * top, width), 7.0, dtype=dtype, device=DEV))
+    assert torch.equal(out[:count], x[(plan.order[:count] // top).long()])
+    assert bool((out[count:] == 7.0).all())
+
+
 def test_router_gives_every_row_an_expert_whatever_it_holds():
     """A row of padding may hold anything (what an attention that found no work left in its output): NaN and
     infinities still choose experts inside the table, so that nothing behind the router reads out of bounds."""
