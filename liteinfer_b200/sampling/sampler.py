@@ -74,6 +74,8 @@ class Sampler:
             temperatures.append(temperature)
             stream = streams.get((p._serial, key)) or self._new_stream(p, key)
             uniforms.append(stream.random())
+        if len(uniforms) != rows:
+            raise ValueError(f"keys length {len(uniforms)} != batch size {rows}")
         # Temperature, top_p, uniform (float32) and top_k (the bits of int32).
         along = logits.is_cuda and rows <= ops.SAMPLE_FROM_HOST
         host = torch.empty((4, rows), dtype=torch.float32, pin_memory=logits.is_cuda and not along)

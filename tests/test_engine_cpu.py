@@ -196,6 +196,16 @@ def test_sampler_streams_do_not_depend_on_the_batch(cpu_kernels):
         s(logits, [p])
 
 
+@pytest.mark.parametrize("keys", [["a"], ["a", "b"]])
+def test_sampler_refuses_fewer_keys_than_rows(cpu_kernels, keys):
+    """One key for three rows is not the first row's parameters for all of them."""
+    from liteinfer_b200 import SamplingParams
+    from liteinfer_b200.sampling.sampler import Sampler
+
+    with pytest.raises(ValueError):
+        Sampler(5)(torch.zeros(3, 50), [SamplingParams(temperature=t) for t in (0.0, 1.0, 2.0)], keys)
+
+
 def test_sample_rule_properties():
     """The row-by-row rule the kernel is tested against: top-k keeps exactly k, the entry crossing p is kept."""
     from torch_kernels import sample_row
