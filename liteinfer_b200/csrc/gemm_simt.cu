@@ -318,15 +318,27 @@ int launch_rows(const SimtProduct& p, int batch, cudaStream_t stream) {
   return (int)cudaLaunchKernelEx(&config, gemm_simt_rows_kernel<R, G>, p, chunks, rounds, all_chunks);
 }
 
+constexpr int kMostTileRows = 65535 * 128;
+
 template <typename T, int BM>
 int launch_tiles(const SimtProduct& p, bool vec, int batch, cudaStream_t stream) {
-  const dim3 grid((p.N + BN - 1) / BN, (p.M + BM - 1) / BM, batch);
-  if (grid.y > 65535 || batch > 65535) return LI_ERR_UNSUPPORTED;
+  if (p.M > kMostTileRows || batch > 65535) return LI_ERR_UNSUPPORTED;
   const cudaError_t status =
       cudaFuncSetAttribute(gemm_simt_tile_kernel<T, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem<BM>);
   if (status != cudaSuccess) return (int)status;
-  gemm_simt_tile_kernel<T, BM><<<grid, kTileThreads, kTileSmem<BM>, stream>>>(p, vec);
-  LI_LAUNCH_CHECK();
+  // A grid has at most 65,535 tiles along the rows; more of them are another launch's.
+  constexpr int kRowsOfGrid = 65535 * BM;
+  for (int first = 0; first < p.M; first += kRowsOfGrid) {
+    SimtProduct part = p;
+    part.M = p.M - first < kRowsOfGrid ? p.M - first : kRowsOfGrid;
+    part.x = static_cast<const T*>(p.x) + (size_t)first * p.ldx;
+    part.out = static_cast<T*>(p.out) + (size_t)first * p.ldo;
+    const dim3 grid((p.N + BN - 1) / BN, (part.M + BM - 1) / BM, batch);
+    gemm_simt_tile_kernel<T, BM><<<grid, kTileThreads, kTileSmem<BM>, stream>>>(part, vec);
+    const cudaError_t launched = cudaGetLastError();
+    if (launched != cudaSuccess) return (int)launched;
+  }
+  return 0;
 }
 
 // Which kernel, by what each was measured to take (B200, microseconds, float32).  The narrow one: 4 and 2.1 for every million

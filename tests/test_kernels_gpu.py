@@ -121,6 +121,19 @@ def test_gemm_simt_widths_agree_bit_for_bit(N, K):
             assert torch.equal(batched[i], one)
 
 
+# More rows than a grid has tiles of 64 for: the first launch's last rows and the second's.
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_gemm_simt_of_more_rows_than_a_grid_takes(dtype):
+    from liteinfer_b200 import ops
+
+    M, N, K = 65535 * 64 + 70, 3, 8
+    x, w, b = _randn(M, K, dtype=dtype), _randn(N, K, dtype=dtype, seed=1), _randn(N, dtype=dtype, seed=2)
+    got = ops.gemm_simt(x, w, torch.full((M, N), float("nan"), dtype=dtype, device="cuda"), b)
+    # Eight products, their sum and the bias, each rounding by 2^-24 of what it has, and the result's own rounding.
+    want, size = x.double() @ w.double().t() + b.double(), x.double().abs() @ w.double().abs().t() + b.double().abs()
+    assert bool(((got.double() - want).abs() <= size * (9 * 2.0 ** -24 + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0))).all())
+
+
 # As many rows as the narrow kernel takes at once and one more, at a k that is the last of twelve chunks a block, the first of
 # thirteen, between, the narrow kernel's last and the first beyond it.
 @pytest.mark.parametrize("K", [12288, 12292, 14336, 16384, 16388])
