@@ -161,6 +161,11 @@ __device__ __forceinline__ int splits_of(int tiles, int most) {
   return wanted <= 1 ? 1 : ceil_quotient(tiles, ceil_quotient(tiles, wanted));
 }
 
+// How many groups a warp has asked for when it waits for group `i`: `ring` - 1 before the first, and one more in each round before its wait.
+__host__ __device__ constexpr int asked_for(int i, int ring, int groups) { return i + ring < groups ? i + ring : groups; }
+static_assert(asked_for(0, 2, 9) == 2 && asked_for(3, 4, 9) == 7 && asked_for(7, 2, 9) == 9 && asked_for(8, 2, 9) == 9 && asked_for(0, 4, 1) == 1,
+              "the newest request is among those that are waited for");
+
 // kWide: a form in fewer registers, three blocks of head size 128 an SM instead of two, for launches of more blocks than two an SM.  It is
 // some 4 % slower a block.  Measured on B200, 8 KV heads of 128: 48 sequences of 1,500 keys 48 us (65.5), 40 of 2,000 55 (81), 24 of
 // 3,000, in two splits each then, 52 (63); 32 of 2,000, which are one wave either way, 47.4 (45).
@@ -344,7 +349,7 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       if (!mbar_wait(bars + 8u * (i % kRing), (unsigned)(i / kRing) & 1, p.error_flag, 21)) {
         // Gave up: before the ring's memory is used for anything else, give the copies still on their way one
         // more (bounded) chance to land.
-        for (int r = i + 1; r < my_groups && r < i + kRing - 1; ++r)
+        for (int r = i + 1; r < asked_for(i, kRing, my_groups); ++r)
           mbar_wait(bars + 8u * (r % kRing), (unsigned)(r / kRing) & 1, nullptr, 0);
         break;
       }
