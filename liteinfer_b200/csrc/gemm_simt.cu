@@ -7,7 +7,10 @@
 // which other rows are in the batch: chunks of 128 k, each two chains of fused multiply-adds in ascending order from zero, of its
 // even and its odd k, (which the wide kernel's instruction takes side by side); their sum; and the chunks' sums in ascending order.  Both kernels
 // keep that order; the chunks are what lets the narrow one give each to a warp of its own (and the sum of short chains is nearer to
-// the exact one: relative error of a product over 768 k 1.55e-7, 2.1e-7 with one chain a chunk).
+// the exact one: relative error of a product over 768 k 1.55e-7, 2.1e-7 with one chain a chunk).  In bfloat16, where there is the wide
+// kernel only, a chunk is one chain.
+#include <type_traits>
+
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -27,6 +30,7 @@ __device__ __forceinline__ Pair multiply_add(Pair a, Pair b, Pair sums) {
 __device__ __forceinline__ float both(Pair sums) {
   return __uint_as_float((unsigned)sums) + __uint_as_float((unsigned)(sums >> 32));
 }
+__device__ __forceinline__ float both(float sum) { return sum; }
 
 struct SimtProduct {
   const void *x, *w, *bias;
@@ -45,7 +49,13 @@ struct SimtProduct {
 // multiply-adds' instructions leave the issue slots to the loads.
 // Measured on B200, 1,250 rows: 768 x 2048 132 us (145 with reads just ahead of their use), 4096 x 768 204 us (39 TFLOP/s; 232 in
 // tiles of 128 x 64 with one-wide multiply-adds); 400 rows of 768 x 768 33 (37), 256 of 16000 x 768 160 (169).
-constexpr int BN = 64, BK = 32, kTileThreads = 128, kTileStages = 4;
+//
+// bfloat16 is widened on its way to shared memory, by loads that a thread waits for: what counts is how many threads do that, and a
+// launch's tiles are 128 x 64 (or 32 x 64) by eight warps, with one-wide multiply-adds in fewer registers, two blocks an SM.  100 rows
+// of 4096 x 4096 238 us, 390 by blocks of four warps as above; 12 rows of 2048 x 2048 94 and 99.
+constexpr int BN = 64, BK = 32, kTileStages = 4;
+template <typename T> constexpr int kTileThreads = sizeof(T) == 4 ? 128 : 256;
+template <typename T> constexpr int kLargeTile = sizeof(T) == 4 ? 64 : 128;        // rows
 constexpr int kTileRow = BK + 4;
 template <int BM> constexpr size_t kTileSmem = (size_t)kTileStages * (BM + BN) * kTileRow * sizeof(float);
 
@@ -81,7 +91,8 @@ __device__ __forceinline__ void stage_four(float* dst, const bf16* src, int left
 }
 
 template <typename T, int BM>
-__global__ void __launch_bounds__(kTileThreads, 3) gemm_simt_tile_kernel(SimtProduct p, bool vec) {
+__global__ void __launch_bounds__(kTileThreads<T>, sizeof(T) == 4 ? 3 : 2) gemm_simt_tile_kernel(SimtProduct p, bool vec) {
+  constexpr int kThreads = kTileThreads<T>, kApart = kThreads / 16, kRows = BM / kApart;      // a thread's rows of x: kRows, kApart apart
   extern __shared__ __align__(16) float tile_smem[];      // [stage][x rows, then w rows][kTileRow]
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN, K = p.K;
   const T* x = static_cast<const T*>(p.x) + blockIdx.z * p.x_batch;
@@ -98,19 +109,20 @@ __global__ void __launch_bounds__(kTileThreads, 3) gemm_simt_tile_kernel(SimtPro
       float* dst = tile_smem + (step % kTileStages) * ((BM + BN) * kTileRow) + lr * kTileRow + lk;
       const int k = step * BK + lk, left = K - k;
 #pragma unroll
-      for (int r = 0; r < BM; r += kTileThreads / 8)
+      for (int r = 0; r < BM; r += kThreads / 8)
         stage_four(dst + r * kTileRow, x + (size_t)min(m0 + lr + r, p.M - 1) * p.ldx + k, left, vec);
 #pragma unroll
-      for (int r = 0; r < BN; r += kTileThreads / 8)
+      for (int r = 0; r < BN; r += kThreads / 8)
         stage_four(dst + (BM + r) * kTileRow, w + (size_t)min(n0 + lr + r, p.N - 1) * K + k, left, vec);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
-  Pair acc[BM / 8][4];
-  float total[BM / 8][4];
+  using Sum = std::conditional_t<sizeof(T) == 4, Pair, float>;
+  Sum acc[kRows][4];
+  float total[kRows][4];
 #pragma unroll
-  for (int i = 0; i < BM / 8; ++i)
+  for (int i = 0; i < kRows; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0, total[i][j] = 0.f;
 
@@ -122,34 +134,50 @@ __global__ void __launch_bounds__(kTileThreads, 3) gemm_simt_tile_kernel(SimtPro
     const float* stage = tile_smem + (step % kTileStages) * ((BM + BN) * kTileRow);
     const float* xr = stage + ty * kTileRow;
     const float* wr = stage + (BM + tx) * kTileRow;
-    // (The next four k are read while these are multiplied.)
-    const auto read = [&](int k, ulonglong2 (&a)[BM / 8], ulonglong2 (&b)[4]) {
+    if constexpr (sizeof(T) == 4) {
+      // (The next four k are read while these are multiplied.)
+      const auto read = [&](int k, ulonglong2 (&a)[kRows], ulonglong2 (&b)[4]) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(wr + j * 16 * kTileRow + k);
+        for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(wr + j * 16 * kTileRow + k);
 #pragma unroll
-      for (int i = 0; i < BM / 8; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xr + i * 8 * kTileRow + k);
-    };
-    ulonglong2 a[BM / 8], b[4];
-    read(0, a, b);
+        for (int i = 0; i < kRows; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(xr + i * kApart * kTileRow + k);
+      };
+      ulonglong2 a[kRows], b[4];
+      read(0, a, b);
 #pragma unroll
-    for (int k = 0; k < BK; k += 4) {
-      ulonglong2 next_a[BM / 8], next_b[4];
-      if (k + 4 < BK) read(k + 4, next_a, next_b);
+      for (int k = 0; k < BK; k += 4) {
+        ulonglong2 next_a[kRows], next_b[4];
+        if (k + 4 < BK) read(k + 4, next_a, next_b);
 #pragma unroll
-      for (int i = 0; i < BM / 8; ++i) {
+        for (int i = 0; i < kRows; ++i) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = multiply_add(a[i].x, b[j].x, acc[i][j]);
+          for (int j = 0; j < 4; ++j) acc[i][j] = multiply_add(a[i].x, b[j].x, acc[i][j]);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = multiply_add(a[i].y, b[j].y, acc[i][j]);
+          for (int j = 0; j < 4; ++j) acc[i][j] = multiply_add(a[i].y, b[j].y, acc[i][j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) b[j] = next_b[j];
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) a[i] = next_a[i];
       }
+    } else {
+#pragma unroll 2
+      for (int k = 0; k < BK; k += 4) {
+        float4 b[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = next_b[j];
+        for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(wr + j * 16 * kTileRow + k);
 #pragma unroll
-      for (int i = 0; i < BM / 8; ++i) a[i] = next_a[i];
+        for (int i = 0; i < kRows; ++i) {
+          const float4 a = *reinterpret_cast<const float4*>(xr + i * kApart * kTileRow + k);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            acc[i][j] = fmaf(a.w, b[j].w, fmaf(a.z, b[j].z, fmaf(a.y, b[j].y, fmaf(a.x, b[j].x, acc[i][j]))));
+        }
+      }
     }
     if ((step + 1) * BK % kChunk == 0 || step + 1 == steps) {
 #pragma unroll
-      for (int i = 0; i < BM / 8; ++i)
+      for (int i = 0; i < kRows; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           total[i][j] += both(acc[i][j]);
@@ -159,8 +187,8 @@ __global__ void __launch_bounds__(kTileThreads, 3) gemm_simt_tile_kernel(SimtPro
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < BM / 8; ++i) {
-    const int m = m0 + ty + 8 * i;
+  for (int i = 0; i < kRows; ++i) {
+    const int m = m0 + ty + kApart * i;
     if (m >= p.M) continue;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -334,7 +362,7 @@ int launch_tiles(const SimtProduct& p, bool vec, int batch, cudaStream_t stream)
     part.x = static_cast<const T*>(p.x) + (size_t)first * p.ldx;
     part.out = static_cast<T*>(p.out) + (size_t)first * p.ldo;
     const dim3 grid((p.N + BN - 1) / BN, (part.M + BM - 1) / BM, batch);
-    gemm_simt_tile_kernel<T, BM><<<grid, kTileThreads, kTileSmem<BM>, stream>>>(part, vec);
+    gemm_simt_tile_kernel<T, BM><<<grid, kTileThreads<T>, kTileSmem<BM>, stream>>>(part, vec);
     const cudaError_t launched = cudaGetLastError();
     if (launched != cudaSuccess) return (int)launched;
   }
@@ -345,13 +373,14 @@ int launch_tiles(const SimtProduct& p, bool vec, int batch, cudaStream_t stream)
 // weights of a group of 16 rows (16384 x 2048: 70 for 12 rows; 1280 x 768: 11.3 for 64).  Tiles of 32 rows: 24 per 768 k
 // while each SM has one or none, 35 up to some 250, then 12 and 0.104 a tile (1280 x 768: 24.7 for 192 rows, 87 for 1,250); tiles of
 // 64 rows: 35.5 per 768 k up to one an SM, 58 up to two, then 12 and 0.155 a tile (1280 x 768: 35.6 for 256 rows, 79 for 1,250; 4096 x
-// 768: 213 for 1,250).
+// 768: 213 for 1,250).  bfloat16: tiles of 32 rows 26, then 0.15 a tile; of 128 rows 54, up to two an SM 98, then 0.37 a tile.
 constexpr int kMostRows = 256;
 inline float rows_cost(const SimtProduct& p, int batch) {
   return 4.f + 2.1e-6f * (float)p.N * p.K * ((p.M + 15) / 16) * batch;
 }
-inline float tiles_cost(const SimtProduct& p, int batch, int rows) {
+inline float tiles_cost(int dtype, const SimtProduct& p, int batch, int rows) {
   const float tiles = (float)((p.N + BN - 1) / BN) * ((p.M + rows - 1) / rows) * batch, depth = p.K / 768.f;
+  if (dtype != kFloat32) return depth * (rows == 32 ? fmaxf(26.f, 0.15f * tiles) : tiles <= 148.f ? 54.f : fmaxf(98.f, 0.37f * tiles));
   if (rows == 32) return depth * (tiles <= 148.f ? 24.f : fmaxf(35.f, 12.f + 0.104f * tiles));
   return depth * (tiles <= 148.f ? 35.5f : fmaxf(58.f, 12.f + 0.155f * tiles));
 }
@@ -361,7 +390,7 @@ int launch_product(int dtype, const SimtProduct& p, int batch, cudaStream_t stre
   // Loads of four k at once: every row of x and w starts on their size.
   const bool vec = p.K % 4 == 0 && p.ldx % 4 == 0 && p.x_batch % 4 == 0 && p.w_batch % 4 == 0 &&
                    reinterpret_cast<uintptr_t>(p.x) % four == 0 && reinterpret_cast<uintptr_t>(p.w) % four == 0;
-  const float small = tiles_cost(p, batch, 32), large = tiles_cost(p, batch, 64);
+  const float small = tiles_cost(dtype, p, batch, 32), large = tiles_cost(dtype, p, batch, dtype == kFloat32 ? kLargeTile<float> : kLargeTile<bf16>);
   if (dtype == kFloat32 && vec && p.K > 0 && p.M <= kMostRows && p.K <= kMostEach * kMostCluster * kChunk &&
       batch <= 65535 && rows_cost(p, batch) < fminf(small, large)) {
     if (p.M == 1) return launch_rows<1, 1>(p, batch, stream);
@@ -372,8 +401,8 @@ int launch_product(int dtype, const SimtProduct& p, int batch, cudaStream_t stre
   }
   const bool narrow = small < large && (p.M + 31) / 32 <= 65535;
   if (dtype == kFloat32)
-    return narrow ? launch_tiles<float, 32>(p, vec, batch, stream) : launch_tiles<float, 64>(p, vec, batch, stream);
-  return narrow ? launch_tiles<bf16, 32>(p, vec, batch, stream) : launch_tiles<bf16, 64>(p, vec, batch, stream);
+    return narrow ? launch_tiles<float, 32>(p, vec, batch, stream) : launch_tiles<float, kLargeTile<float>>(p, vec, batch, stream);
+  return narrow ? launch_tiles<bf16, 32>(p, vec, batch, stream) : launch_tiles<bf16, kLargeTile<bf16>>(p, vec, batch, stream);
 }
 
 }  // namespace li
