@@ -213,16 +213,19 @@ __global__ void gate_heads_kernel(const T* __restrict__ v, const T* __restrict__
 }
 
 // The same, 16 bytes of a head's output a thread (vdim and gate_stride whole vectors, 16-byte aligned pointers): element by element a
-// prompt's threads did little but divide for their place, 25 us for 2,860 tokens of 16 heads of 128, 4.6 now.
-template <typename T>
+// prompt's threads did little but divide for their place, 25 us for 2,860 tokens of 16 heads of 128, 4.6 now.  A block has a token, or
+// neighbouring ones where a token is a few vectors (`kShared`).
+template <typename T, bool kShared>
 __global__ void gate_heads_vec_kernel(const T* __restrict__ v, const T* __restrict__ gate, int gate_stride, T* __restrict__ out,
                                       int tokens, int heads, int pieces) {
   constexpr int N = Vec16<T>::N;
   grid_dependency_wait();
   grid_launch_dependents();
-  const int per_token = heads * pieces, i = blockIdx.y * blockDim.x + threadIdx.x;
-  const int t = blockIdx.x;
-  if (i >= per_token) return;
+  const int per_token = heads * pieces, tokens_a_block = kShared ? (int)blockDim.x / per_token : 1;
+  const int row = kShared ? (int)threadIdx.x / per_token : 0;
+  const int i = kShared ? (int)threadIdx.x - row * per_token : (int)(blockIdx.y * blockDim.x + threadIdx.x);
+  const int t = blockIdx.x * tokens_a_block + row;
+  if (i >= per_token || row >= tokens_a_block || t >= tokens) return;
   const int h = i / pieces, piece = i - h * pieces;
   float x[N], g[N];
   unpack16(load16(v + (((size_t)h * tokens + t) * pieces + piece) * N), x);
@@ -305,14 +308,29 @@ LI_EXPORT int li_gate_heads(int dtype, const void* v, const void* gate, int gate
   const size_t n = (size_t)tokens * heads * vdim;
   if (n == 0) return 0;
   const int lanes = dtype == kFloat32 ? 4 : 8;
-  if (vdim % lanes == 0 && (gate == nullptr || gate_stride % lanes == 0) && aligned16(v) && aligned16(gate) && aligned16(out)) {
-    const int pieces = vdim / lanes, items = heads * pieces, threads = items < 256 ? (items + 31) / 32 * 32 : 256;
+  // In bfloat16 a thread has eight exponentials one after the other, which up to two blocks an SM of the kernel above takes longer than
+  // its divisions do: 1 token of 16 x 128 1.66 us by elements and 1.89 by vectors, 32 1.76 and 1.94, 64 2.13 and 1.95 (float32: 1.66 and 1.61).
+  const bool few = dtype != kFloat32 && n <= 2 * 148 * 256;
+  if (!few && vdim % lanes == 0 && (gate == nullptr || gate_stride % lanes == 0) && aligned16(v) && aligned16(gate) && aligned16(out)) {
+    // Tokens of up to 64 vectors share blocks where there are many of them: a block each, 8,000 tokens of 1 x 8 took 8.7 us, of
+    // 2 x 64 8.6 (1.9 and 2.6 now); a few hundred are as fast either way.
+    const int pieces = vdim / lanes, items = heads * pieces;
+    if (items <= 64 && tokens >= 512) {
+      const int rows = 256 / items;
+      const dim3 grid((tokens + rows - 1) / rows);
+      return (int)(dtype == kFloat32
+                       ? launch_pdl(tokens, gate_heads_vec_kernel<float, true>, grid, dim3(256), 0, stream, (const float*)v,
+                                    (const float*)gate, gate_stride, (float*)out, tokens, heads, pieces)
+                       : launch_pdl(tokens, gate_heads_vec_kernel<bf16, true>, grid, dim3(256), 0, stream, (const bf16*)v,
+                                    (const bf16*)gate, gate_stride, (bf16*)out, tokens, heads, pieces));
+    }
+    const int threads = items < 256 ? (items + 31) / 32 * 32 : 256;
     const dim3 grid(tokens, (items + threads - 1) / threads);
     if (grid.y <= 65535)
       return (int)(dtype == kFloat32
-                       ? launch_pdl(tokens, gate_heads_vec_kernel<float>, grid, dim3(threads), 0, stream, (const float*)v,
+                       ? launch_pdl(tokens, gate_heads_vec_kernel<float, false>, grid, dim3(threads), 0, stream, (const float*)v,
                                     (const float*)gate, gate_stride, (float*)out, tokens, heads, pieces)
-                       : launch_pdl(tokens, gate_heads_vec_kernel<bf16>, grid, dim3(threads), 0, stream, (const bf16*)v,
+                       : launch_pdl(tokens, gate_heads_vec_kernel<bf16, false>, grid, dim3(threads), 0, stream, (const bf16*)v,
                                     (const bf16*)gate, gate_stride, (bf16*)out, tokens, heads, pieces));
   }
   const int blocks = (int)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);

@@ -126,6 +126,14 @@ def test_gate_heads_by_vectors(dtype, tokens, heads, vdim):
     assert torch.equal(ops.gate_heads(v, None, out()), plain)
 
 
+# More elements than a launch takes one by one in bfloat16: a block a token, several, and blocks that tokens share (a vector each, three
+# heads of three, 64 in all; the last block not full).
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("tokens,heads,vdim", [(15, 40, 128), (80, 3, 320), (9600, 1, 8), (1301, 3, 24), (513, 4, 128)])
+def test_gate_heads_of_many_tokens(dtype, tokens, heads, vdim):
+    test_gate_heads_by_vectors(dtype, tokens, heads, vdim)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("M,N,K", [(1, 264, 96), (5, 4096, 512), (8, 200, 1024), (12, 328, 96), (16, 8192, 256), (40, 264, 96)])
 @pytest.mark.parametrize("name", ["relu_squared", "silu", "gelu_tanh"])
