@@ -374,8 +374,21 @@ moe_sort_kernel(const int* __restrict__ ids, int pairs, int experts, int tile_ro
 
 // out[m] = x[order[m] / top]: every pair's token row, in the order of the experts' runs.  A block copies one piece of
 // `kGatherRows` rows, a vector of each a thread, so that a thread looks its rows up and has them all on their way at once.
-// 2,048 tokens of 2,048, four experts a token: 7.5 us (8.9 a vector at a time), 8,000 of 1,024, eight: 24.5 (32.6; 144 MB).
+// 2,048 tokens of 2,048, four experts a token: 7.5 us (8.9 a vector at a time), 8,000 of 1,024, eight: 24.5 (32.6; 144 MB).  Up to
+// kFewVectors, which have their threads at once, a vector a thread is the faster: 16 of 1,024 by two 1.45 us (1.9 by rows), 128 of 2,048 by four
+// 1.9 (2.1).
 constexpr int kGatherRows = 4;
+constexpr long kFewVectors = 148 * 2400;
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+moe_gather_few_kernel(const T* __restrict__ x, size_t x_stride, const int* __restrict__ order, int top, T* __restrict__ out,
+                      const int* __restrict__ count, int pieces) {
+  constexpr int N = Vec16<T>::N;
+  const unsigned at = blockIdx.x * blockDim.x + threadIdx.x, m = at / pieces, piece = at - m * pieces;
+  grid_dependency_wait();
+  if ((int)m < *count) store16(out + (size_t)at * N, load16(x + (size_t)(order[m] / top) * x_stride + (size_t)piece * N));
+}
 
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -729,7 +742,17 @@ LI_EXPORT int li_moe_gather(int dtype, const void* x, size_t x_stride, const int
   if (pairs == 0 || width == 0) return 0;
   const int n = dtype == kFloat32 ? 4 : 8;
   if (width % n || x_stride % n || !aligned16(x) || !aligned16(out)) return LI_ERR_ALIGNMENT;
-  const int pieces = width / n, threads = pieces < 256 ? (pieces + 31) / 32 * 32 : 256;
+  const int pieces = width / n;
+  const long vectors = (long)pairs * pieces;
+  if (vectors <= kFewVectors) {
+    const dim3 few((unsigned)((vectors + 255) / 256));
+    if (dtype == kFloat32)
+      return (int)launch_pdl(pairs, moe_gather_few_kernel<float>, few, dim3(256), 0, stream, (const float*)x, x_stride, order, top,
+                             (float*)out, count, pieces);
+    return (int)launch_pdl(pairs, moe_gather_few_kernel<bf16>, few, dim3(256), 0, stream, (const bf16*)x, x_stride, order, top,
+                           (bf16*)out, count, pieces);
+  }
+  const int threads = pieces < 256 ? (pieces + 31) / 32 * 32 : 256;
   const dim3 grid((pairs + kGatherRows - 1) / kGatherRows, (pieces + threads - 1) / threads);
   if (dtype == kFloat32)
     return (int)launch_pdl(pairs, moe_gather_kernel<float>, grid, dim3(threads), 0, stream, (const float*)x, x_stride, order,

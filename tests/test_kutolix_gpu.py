@@ -547,6 +547,13 @@ def test_gather_brings_the_pairs_that_have_an_expert(dtype, tokens, width, top):
     assert bool((out[count:] == 7.0).all())
 
 
+# More vectors than a launch has a thread each for: four rows a block, the last of them not full.
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("tokens,width,top", [(701, 2056, 3), (23001, 128, 1)])
+def test_gather_of_many_rows(dtype, tokens, width, top):
+    test_gather_brings_the_pairs_that_have_an_expert(dtype, tokens, width, top)
+
+
 def test_router_gives_every_row_an_expert_whatever_it_holds():
     """A row of padding may hold anything (what an attention that found no work left in its output): NaN and
     infinities still choose experts inside the table, so that nothing behind the router reads out of bounds."""
