@@ -886,11 +886,19 @@ int launch_pairs(int tokens, dim3 grid, cudaStream_t stream, const T* qkv, const
                          gates, products, state, qsl, slots, out, heads, kv_heads, vdim);
 }
 
-// Two columns a lane where that still makes more than two blocks an SM; one where the chain is what a launch waits for.
+// Two columns a lane where a launch has blocks enough for that; one where it waits for the chain over its longest sequence's tokens.  What
+// counts as a block is a longest sequence's worth of tokens (`tokens` / `max_q_len` of them); a sequence beside those that brings one token
+// reads and writes its state and is done, a twelfth of one.  By the number of sequences alone 20 single tokens beside a prompt of 300, 16
+// heads of 64 x 64, took 52 us in two columns (43 in one, 49 a token at a time).  The line, by head size: 16 heads of 128 x 128, 4
+// prompts of 512 163 us in one and 149 in two, of 32 heads 261 and 250, 8 heads and 300 beside 20 single tokens 50 and 59; 64 x 64, 16 heads, 8 of
+// 512 122 and 126, 30 of 64 50 and 48.  At head size 32,
+// where the chain is short, 16 heads in float32, 4 of 512 72.5 and 73.2, 8 of 512 89 and 84, 20 single tokens beside 300 39 and 40.
 template <typename T, int R>
-int launch_pairs(int tokens, dim3 grid, cudaStream_t stream, const T* qkv, const float* scales, const float* gates, const float* products,
-                 float* state, const int* qsl, const int* slots, float* out, int heads, int kv_heads, int vdim) {
-  const bool wide = vdim % 32 == 0 && (long)(vdim / 32) * grid.y * grid.z > 2 * 148;
+int launch_pairs(int tokens, int max_q_len, dim3 grid, cudaStream_t stream, const T* qkv, const float* scales, const float* gates,
+                 const float* products, float* state, const int* qsl, const int* slots, float* out, int heads, int kv_heads, int vdim) {
+  const float sequences = (float)grid.z, whole = max_q_len > 1 ? fminf((float)tokens / (float)max_q_len, sequences) : sequences;
+  const float blocks = (float)(vdim / 32 * grid.y) * (R == 4 ? sequences : whole + (sequences - whole) / 12.f);
+  const bool wide = vdim % 32 == 0 && blocks > (R == 8 ? 576.f : R == 16 ? 320.f : 64.f);
   return wide ? launch_pairs<T, R, 2>(tokens, grid, stream, qkv, scales, gates, products, state, qsl, slots, out, heads, kv_heads, vdim)
               : launch_pairs<T, R, 1>(tokens, grid, stream, qkv, scales, gates, products, state, qsl, slots, out, heads, kv_heads, vdim);
 }
@@ -1028,9 +1036,9 @@ LI_EXPORT int li_gated_delta_rule(int dtype, const void* qkv, const void* ab, si
       if (code) return code;
     }
     if (pairs) {
-      if (dim == 32) return launch_pairs<T, 4>(tokens, grid, stream, rows, scales, gates, room, state, query_start_loc, state_slots, out, heads, kv_heads, vdim);
-      if (dim == 64) return launch_pairs<T, 8>(tokens, grid, stream, rows, scales, gates, room, state, query_start_loc, state_slots, out, heads, kv_heads, vdim);
-      return launch_pairs<T, 16>(tokens, grid, stream, rows, scales, gates, room, state, query_start_loc, state_slots, out, heads, kv_heads, vdim);
+      if (dim == 32) return launch_pairs<T, 4>(tokens, max_q_len, grid, stream, rows, scales, gates, room, state, query_start_loc, state_slots, out, heads, kv_heads, vdim);
+      if (dim == 64) return launch_pairs<T, 8>(tokens, max_q_len, grid, stream, rows, scales, gates, room, state, query_start_loc, state_slots, out, heads, kv_heads, vdim);
+      return launch_pairs<T, 16>(tokens, max_q_len, grid, stream, rows, scales, gates, room, state, query_start_loc, state_slots, out, heads, kv_heads, vdim);
     }
     return launch_delta<T>(dim, single, tokens, grid, stream, rows, scales, gates, state, query_start_loc, state_slots, out, heads, kv_heads,
                            vdim, (const T*)ab, ab_stride, a_log, dt_bias);

@@ -135,3 +135,9 @@ class StepContext:
     @property
     def is_decode_only(self) -> bool:
         return self.max_query_len == 1
+
+    @property
+    def longest_portion(self) -> int:
+        """The most tokens that a sequence brings, as closely as the host knows it: in a step of a padded shape `max_query_len` is
+        all of its tokens."""
+        return self.plan.max_prefill_query_len if self.plan is not None and self.plan.num_prefill else self.max_query_len

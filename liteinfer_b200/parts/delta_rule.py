@@ -89,7 +89,7 @@ class GatedDeltaRule:
         read = torch.empty((tokens, v), dtype=torch.float32, device=x.device)
         ops.gated_delta_rule(conved, proj[:, c + v:c + v + 2 * self.heads], self.a_log, self.dt_bias, state,
                              ctx.query_start_loc, ctx.state_slots, ctx.num_seqs, self.heads, self.kv_heads, self.dim,
-                             self.vdim, read, ctx.max_query_len)
+                             self.vdim, read, ctx.longest_portion)
         gated = torch.empty((tokens, v), dtype=x.dtype, device=x.device)
         ops.gated_rmsnorm(read, proj[:, c:c + v], self.norm_weight, self.norm_eps, gated, self.heads)
         return ops.linear(gated, self.o_weight, None)

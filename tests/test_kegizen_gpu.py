@@ -268,6 +268,32 @@ def test_gated_delta_rule_two_tokens_at_a_time(dtype, kv_heads, dim, vdim, lengt
         torch.testing.assert_close(a, b, rtol=1e-4, atol=1e-5)
 
 
+# A sequence's bits, alone (one column a lane) and beside others (two), every other argument the same.
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("dim", [32, 64, 128])
+def test_gated_delta_rule_has_the_same_bits_beside_others(dtype, dim):
+    from liteinfer_b200 import ops
+
+    heads, vdim, lengths = 8, 64, [37] * 60 + [1] * 40
+    tokens, first = sum(lengths), 37
+    qkv = _randn(tokens, (2 * heads) * dim + heads * vdim, seed=1, dtype=dtype)
+    ab = _randn(tokens, 2 * heads, seed=2, scale=2.0, dtype=dtype)
+    a_log, dt_bias = torch.log(1 + 3 * torch.rand(heads, device=DEV)), _randn(heads, seed=5)
+    start = _randn(len(lengths), heads, vdim, dim, seed=7, scale=0.1)
+    qsl = [0]
+    for n in lengths:
+        qsl.append(qsl[-1] + n)
+    got = []
+    for seqs, longest in ((1, first), (len(lengths), first), (len(lengths), 0), (len(lengths), tokens)):
+        rows, state = qsl[seqs], start.clone()
+        out = torch.zeros(rows, heads * vdim, device=DEV)
+        ops.gated_delta_rule(qkv[:rows], ab[:rows], a_log, dt_bias, state, _ints(qsl[:seqs + 1]), _ints(list(range(seqs))), seqs, heads,
+                             heads, dim, vdim, out, longest)
+        got.append((out[:first], state[0]))
+    for out, state in got[1:]:
+        assert torch.equal(out, got[0][0]) and torch.equal(state, got[0][1])
+
+
 def test_gated_delta_rule_recalls_a_far_key():
     """One key written 300 tokens back with decay 1 is read out exactly; with a decay below 1 it has faded."""
     from liteinfer_b200 import ops
