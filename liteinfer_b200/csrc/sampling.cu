@@ -82,6 +82,7 @@ constexpr int kBins = 1024;
 constexpr int kListed = 512;       // columns that a warp can list; where one has more its block goes on walking its whole share
 constexpr int kCandidates = 1024;  // elements of a row that are sorted at once, two a thread
 constexpr int kSampleMostSmem = 200 << 10;
+constexpr size_t kSmemOfSm = 228 << 10, kReservedSmem = 1 << 10;      // an SM's shared memory, and what it keeps of it for a block
 constexpr float kBinsPerUnit = 73.f;   // the last bin holds all that lies 14 and more below the maximum
 
 struct Keep {        // the surviving set: key > beta, or key == beta and index <= tie_cut
@@ -92,7 +93,8 @@ struct Keep {        // the surviving set: key > beta, or key == beta and index 
 
 struct SampleSmem {
   // Two histograms in turn: kBins counts, or the sums of the weights' lower 16 bits and, behind them, of the bits above;
-  // for a share of 2^16 columns or more, where those could overflow, kBins 64-bit sums.
+  // for a share of 2^16 columns or more, where those could overflow, kBins 64-bit sums.  Behind the row's barrier that follows, the one just
+  // summed is read by nobody any more, and the other one has been free since the barrier before: see `candidates`.
   alignas(16) uint32_t bins[2][2 * kBins];
   unsigned long long exchange[8];           // what other blocks of the cluster read, one slot per exchange
   unsigned long long warp[kSampleWarps];
@@ -103,8 +105,12 @@ struct SampleSmem {
   int found;                                // entries of `cand`, or more where it did not hold them all
   Keep keep;
   uint16_t list[kSampleWarps][kListed];
-  unsigned long long cand[kCandidates];     // this block's elements of the boundary bin (top-k: and of those above it)
+  // This block's elements of the boundary bin (top-k: and of those above it), in the histogram whose turn is next: every block has read
+  // what it held before it came to the barrier in front of the sums that found the boundary.  In 8 KB of their own they left an SM
+  // room for one block of a row of 151,936 columns where there had been two.
+  __device__ __forceinline__ unsigned long long* candidates(int turn) { return reinterpret_cast<unsigned long long*>(bins[turn]); }
 };
+static_assert(sizeof(uint32_t[2 * kBins]) == kCandidates * sizeof(unsigned long long), "candidates lie in a histogram");
 
 // One block's share of a row: columns [base, base + n) of it, whose element i lies at data[i] (in shared memory, or the row
 // itself where a share does not fit).  The walks over a share go warp by warp: each warp has a run of columns, and once
@@ -263,7 +269,7 @@ __device__ __forceinline__ int power_above(int n) { return n <= 32 ? 32 : 1 << (
 
 // The candidates of all blocks of a row, thread t taking the t-th and the (t + 512)-th.  Behind a barrier of the row.
 // Returns how many there are, or more than kCandidates where a block did not hold all of its own.
-__device__ int gather_candidates(unsigned long long (&v)[2], SampleSmem& sm) {
+__device__ int gather_candidates(unsigned long long (&v)[2], int turn, SampleSmem& sm) {
   cg::cluster_group cluster = cg::this_cluster();
   const int ranks = (int)cluster.num_blocks();
   int count[kMostRanks], all = 0;
@@ -289,7 +295,7 @@ __device__ int gather_candidates(unsigned long long (&v)[2], SampleSmem& sm) {
         ++r;
       }
     }
-    v[h] = cluster.map_shared_rank(sm.cand, r)[at];
+    v[h] = cluster.map_shared_rank(sm.candidates(turn), r)[at];
   }
   return all;
 }
@@ -365,11 +371,11 @@ __device__ void find_boundary(SampleSmem& sm, int buf, bool wide, unsigned long 
 // The last selections and the draw of a row whose top-k leaves few elements, by one block: the candidates, all that top-k
 // keeps among them, lie over the blocks.  Returns the column.
 template <typename S, bool kStaged>
-__device__ int draw_from_candidates(const Share<S, kStaged>& share, int k, float top_p, double u, int fallback, SampleSmem& sm) {
+__device__ int draw_from_candidates(const Share<S, kStaged>& share, int k, float top_p, double u, int fallback, int turn, SampleSmem& sm) {
   const int t = threadIdx.x;
-  unsigned long long* table = reinterpret_cast<unsigned long long*>(sm.bins[0]);
+  unsigned long long* table = sm.candidates(turn ^ 1);      // what was summed last
   unsigned long long v[2];
-  const int many = gather_candidates(v, sm);
+  const int many = gather_candidates(v, turn, sm);
   sort_down(v, power_above(many), table);
   k = min(k, many);
   unsigned long long weight[2], upto[2];
@@ -503,7 +509,7 @@ __device__ Keep select_prefix(Share<S, kStaged>& share, bool all_in, Keep within
         int at = 0;
         if (lane == 0) at = atomicAdd(&sm.found, __popc(votes));
         at = __shfl_sync(0xffffffffu, at, 0) + __popc(votes & ((1u << lane) - 1));
-        if (taken && at < kCandidates) sm.cand[at] = candidate(ordered_key(x), share.base + i);
+        if (taken && at < kCandidates) sm.candidates(turn)[at] = candidate(ordered_key(x), share.base + i);
       };
       if (share.listed) {
         for (int j = share.from; j < share.to && collect; j += 32) {
@@ -577,9 +583,9 @@ __device__ Keep select_prefix(Share<S, kStaged>& share, bool all_in, Keep within
       }
       // The few elements of the boundary bin, sorted, tell where the cut falls; every block sorts them for itself.
       unsigned long long v[2], upto[2], weight[2];
-      const int many = gather_candidates(v, sm);
+      const int many = gather_candidates(v, turn, sm);
       if (many > kCandidates) continue;
-      sort_down(v, power_above(many), reinterpret_cast<unsigned long long*>(sm.bins[0]));
+      sort_down(v, power_above(many), sm.candidates(turn ^ 1));
 #pragma unroll
       for (int h = 0; h < 2; ++h) upto[h] = weight[h] = v[h] ? share.weight(key_value((uint32_t)(v[h] >> 32))) : 0;
       scan_both(upto, many, sm);
@@ -768,7 +774,7 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, const __g
     keep = select_prefix<true, kAlone>(share, true, keep, (unsigned long long)(k - 1), 0.f, vocab, turn, slot, few, sm);
     if (few) {
       if (rank == 0) {
-        const int column = draw_from_candidates(share, k, p, u, top.i, sm);
+        const int column = draw_from_candidates(share, k, p, u, top.i, turn, sm);
         if (threadIdx.x == 0) out[r] = column;
       }
       row_sync<kAlone>(cluster);        // the others' candidates stay until they have been read
@@ -884,9 +890,9 @@ int launch_sample(const T* logits, int rows, int vocab, int ranks, int share, co
 }
 
 // Shares in shared memory where they fit.  bfloat16 is staged as divided floats while all of the launch's blocks are resident
-// at once that way, two an SM (64 KB of floats beside 41 KB): the passes then divide nothing.  A wider launch stages the
+// at once that way, two an SM (64 KB of floats beside 33 KB) or, of wide rows, one: the passes then divide nothing.  A wider launch stages the
 // logits as they are, three blocks an SM, and divides again in the passes that need the quotient, so that 48 rows of
-// 128,256 (384 blocks) still are one wave; two waves would cost each row's chain of barriers twice.
+// 128,256 (384 blocks) still are one wave; two waves would cost each row's chain of barriers twice (24 rows of 151,936, top-k 50: 44 us, in one wave 30).
 template <typename T>
 int sample_rows(const T* logits, int rows, int vocab, const RowParams& params, int* out, cudaStream_t stream) {
   int ranks = 1;
@@ -894,9 +900,10 @@ int sample_rows(const T* logits, int rows, int vocab, const RowParams& params, i
   if (ranks > 1 && ranks < kMostRanks && 2LL * ranks * rows <= 148) ranks *= 2;
   const int share = ((vocab + ranks - 1) / ranks + 7) / 8 * 8;
   if ((long long)rows * ranks > 0x7fffffffll) return LI_ERR_UNSUPPORTED;
-  const size_t room = kSampleMostSmem - (sizeof(SampleSmem) + 15) / 16 * 16;
+  const size_t fixed = (sizeof(SampleSmem) + 15) / 16 * 16, room = kSampleMostSmem - fixed;
+  const bool two = 2 * (fixed + (size_t)share * 4 + kReservedSmem) <= kSmemOfSm;      // blocks of floats an SM
   const bool raw = (size_t)share * sizeof(T) <= room;
-  const bool floats = sizeof(T) == 4 || ((size_t)share * 4 <= room / 2 && rows * ranks <= 2 * 148);
+  const bool floats = sizeof(T) == 4 || ((size_t)share * 4 <= room / 2 && rows * ranks <= (two ? 2 : 1) * 148);
   const auto launch = [&](auto kernel) {
     return kernel(logits, rows, vocab, ranks, share, params, out, stream);
   };
