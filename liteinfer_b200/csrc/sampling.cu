@@ -58,10 +58,10 @@ __device__ ArgMax block_argmax(ArgMax mine, ArgMax* scratch /* 32 */) {
 //
 // Top-k and top-p are the same selection: in descending order, keep the elements whose preceding weight (1 each, or
 // the probability) is within a limit.  The first histogram bins by the distance below the row's maximum, in steps of
-// 1/73 for 14 units: the interesting values spread over hundreds of bins, so the atomics rarely meet, and the last bin takes
-// the rest, whose weight is added up in registers.  Elements above the boundary bin are in, those below are out.  The walk
+// 1/73 for 14 units (counts: see kCountsPerUnit): the interesting values spread over hundreds of bins, so the atomics rarely meet, and the
+// last bin takes the rest, whose weight is added up in registers.  Elements above the boundary bin are in, those below are out.  The walk
 // behind the histogram lists what can still be chosen, in the order of the columns, and picks out what has to be told apart:
-// the boundary bin, or for a top-k that leaves no more than kCandidates, everything.  Those few are sorted, by every block for
+// the boundary bin, or for a top-k that leaves few (most_sorted), everything.  Those few are sorted, by every block for
 // itself (top-p), or by one block that then finishes the row alone, top-p and draw included (top-k).  Where they are more (equal
 // values, a flat row, a share of 2^16 columns) histograms over ever narrower ranges of keys tell them apart, each a meeting of the blocks.
 //
@@ -83,7 +83,19 @@ constexpr int kListed = 512;       // columns that a warp can list; where one ha
 constexpr int kCandidates = 1024;  // elements of a row that are sorted at once, two a thread
 constexpr int kSampleMostSmem = 200 << 10;
 constexpr size_t kSmemOfSm = 228 << 10, kReservedSmem = 1 << 10;      // an SM's shared memory, and what it keeps of it for a block
-constexpr float kBinsPerUnit = 73.f;   // the last bin holds all that lies 14 and more below the maximum
+constexpr float kBinsPerUnit = 73.f;   // by weight: the last bin holds all that lies 14 and more below the maximum
+// By count (top-k) what lies far below the maximum counts as much as what is near it, so a bin holds 1/46 of a unit for 14 units and then one
+// unit up to 393: the k-th value of a row with a low temperature or few large values is in a bin of a few columns, too.  With the bins of
+// the weights 24 rows of 262,144 columns, top-k 50 at a temperature of 0.2, took 124 us (36 now), 12 of 1,000 20 (10.7).
+constexpr float kCountsPerUnit = 46.f, kFar = 14.f, kFarFrom = kFar * (kCountsPerUnit - 1.f);      // (where the second line cuts zero)
+static_assert(kFarFrom < kBins - 2, "the lines meet within the histogram");
+// A top-k is finished by sorting where no more than this many columns can be chosen, which costs two sorts and saves the histograms that tell the
+// boundary bin's columns apart and, with a top-p behind it, those of the second selection.  In a row of one block, which meets nobody, a
+// histogram is cheap: 8,192 float32 columns, top-k 50 alone 15.5 us by sorts and 12.4 by histograms, with top-p 0.9 16.3 and 17.6, top-k 200 with
+// it 20.0 and 17.9.  In a cluster's: 32,000 bfloat16, top-k 100 alone 19.3 and 20.3, 200 21.3 and 20.6, 800 41 and 21; with top-p 400 26
+// and 30, 800 42 and 30.
+__host__ __device__ constexpr unsigned most_sorted(bool alone, bool weights_follow) { return alone ? (weights_follow ? 128 : 0) : weights_follow ? 512 : 128; }
+static_assert(most_sorted(false, true) <= kCandidates, "a block holds what is sorted");
 
 struct Keep {        // the surviving set: key > beta, or key == beta and index <= tie_cut
   uint32_t beta;
@@ -153,15 +165,31 @@ struct Share {
     const float scaled = expf(x - row_max) * 4294967296.0f;
     return scaled < 4294967296.0f ? (unsigned long long)(uint32_t)scaled : (unsigned long long)scaled;
   }
+  // Where a difference from the maximum (as it is stored) lies among the bins of counts (`unit`) or weights.
+  template <bool unit>
+  __device__ __forceinline__ float place(float d) const {
+    const float t = d * bin_scale;
+    return fminf(unit ? fminf(t, fmaf(t, 1.f / kCountsPerUnit, kFarFrom)) : t, (float)(kBins - 1));
+  }
   // The bin never rises with the value, and equal values divided by the temperature are in one bin.  A difference that is no
   // number (infinities, NaN) goes by the key.
+  template <bool unit>
   __device__ __forceinline__ int bin_of(float stored) const {
     const float d = bin_max - stored;
     if (!(d >= 0.f)) return ordered_key(quotient(stored)) >= max_key ? 0 : kBins - 1;
-    return (int)fminf(d * bin_scale, (float)(kBins - 1));
+    return (int)place<unit>(d);
   }
-  __device__ __forceinline__ int bin(int i) const { return bin_of(to_float(data[i])); }
+  template <bool unit>
+  __device__ __forceinline__ int bin(int i) const { return bin_of<unit>(to_float(data[i])); }
+  __device__ __forceinline__ void bins_per_unit(float bins) { bin_scale = undivided ? bins / temp : bins; }
 };
+
+// The difference from the maximum, in units, at which a bin begins.
+template <bool unit>
+__device__ __forceinline__ float bin_begin(int bin) {
+  const float b = (float)bin;
+  return unit ? fmaxf(b * (1.f / kCountsPerUnit), b - kFarFrom) : b * (1.f / kBinsPerUnit);
+}
 
 // The barrier of a row's blocks; a row that is one block's (kAlone) has no use for a cluster's.
 template <bool kAlone>
@@ -414,7 +442,7 @@ __device__ int draw_from_candidates(const Share<S, kStaged>& share, int k, float
 // Among the elements of `within`, in descending order of value (equal values by ascending index), keeps each element
 // whose preceding weight sum is within the limit.  `unit` weights count elements (top-k with limit k - 1); otherwise the
 // weight is exp(x - row_max) in 2^-32 fixed point (top-p with limit p * total).  `turn`: the histogram to use next;
-// `slot`: the next free exchange.  Lists what survives the first histogram.  `few` (top-k): set where what it keeps lies among
+// `slot`: the next free exchange.  Lists what survives the first histogram.  `few` (top-k, whose `top_p` is what follows it): set where what it keeps lies among
 // that many candidates, which one block is to finish with; nothing else is then returned.
 template <bool unit, bool kAlone, typename S, bool kStaged>
 __device__ Keep select_prefix(Share<S, kStaged>& share, bool all_in, Keep within, unsigned long long limit, float top_p, int vocab,
@@ -451,7 +479,7 @@ __device__ Keep select_prefix(Share<S, kStaged>& share, bool all_in, Keep within
         share.four(j, f);
         int bin[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) bin[e] = share.bin_of(f[e]);
+        for (int e = 0; e < 4; ++e) bin[e] = share.template bin_of<unit>(f[e]);
         if (unit) {
 #pragma unroll
           for (int e = 0; e < 4; ++e)
@@ -476,7 +504,7 @@ __device__ Keep select_prefix(Share<S, kStaged>& share, bool all_in, Keep within
 #pragma unroll 2
       for (int j = share.from + lane; j < share.to; j += 32) {
         const int i = share.column(j);
-        int bin = share.bin(i);
+        int bin = share.template bin<unit>(i);
         const float x = share.value(i);
         const uint32_t key = ordered_key(x);
         if (!all_in && !within.has(key, share.base + i)) continue;
@@ -493,14 +521,14 @@ __device__ Keep select_prefix(Share<S, kStaged>& share, bool all_in, Keep within
     if (chosen < 0) return within;
     if (level == 0) {
       first_bin = chosen;
-      const float far = (float)(chosen + 1) * (1.0001f / kBinsPerUnit), near = (float)chosen * (0.9999f / kBinsPerUnit);
+      const float far = 1.0001f * bin_begin<unit>(chosen + 1), near = 0.9999f * bin_begin<unit>(chosen);
       const float slack = 1e-5f * (fabsf(share.row_max) + 1.f);
       if (chosen > 0) high_key = ordered_key(share.row_max - near + slack);
       if (chosen < kBins - 1) low_key = ordered_key(share.row_max - far - slack);
       if (!(fabsf(share.row_max) < 3.0e38f)) low_key = 0, high_key = 0xffffffffu;
       if (wide) continue;
       // List what the boundary bin and those above it hold, and put what has to be told apart where the other blocks find it.
-      const bool collect = !unit || above + mass <= kCandidates;
+      const bool collect = !unit || above + mass <= most_sorted(kAlone, top_p > 0.f && top_p < 1.f);
       bool fits = !share.listed;
       int listed = 0;
       const auto put = [&](bool taken, int i, float x) {       // a warp's elements that have to be told apart
@@ -514,7 +542,7 @@ __device__ Keep select_prefix(Share<S, kStaged>& share, bool all_in, Keep within
       if (share.listed) {
         for (int j = share.from; j < share.to && collect; j += 32) {
           const int i = j + lane < share.to ? share.column(j + lane) : 0;
-          const int bin = j + lane < share.to ? share.bin(i) : kBins;
+          const int bin = j + lane < share.to ? share.template bin<unit>(i) : kBins;
           const float x = share.value(i);
           put((unit ? bin <= first_bin : bin == first_bin) && (all_in || within.has(ordered_key(x), share.base + i)), i, x);
         }
@@ -530,7 +558,7 @@ __device__ Keep select_prefix(Share<S, kStaged>& share, bool all_in, Keep within
           share.four(min(i, share.n - 1) & ~3, f);
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            const float d = share.bin_max - f[e], t = fminf(d * share.bin_scale, (float)(kBins - 1));
+            const float d = share.bin_max - f[e], t = share.template place<unit>(d);
             const bool here = i + e < share.to;
             odd = odd || (here && !(d >= 0.f));
             in |= (unsigned)(here && t < lowest) << e;
@@ -541,7 +569,7 @@ __device__ Keep select_prefix(Share<S, kStaged>& share, bool all_in, Keep within
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               if (i + e >= share.to) continue;
-              const int bin = share.bin_of(f[e]);
+              const int bin = share.template bin_of<unit>(f[e]);
               if (bin > first_bin || !(all_in || within.has(ordered_key(share.quotient(f[e])), share.base + i + e))) continue;
               in |= 1u << e;
               if (unit || bin == first_bin) taken |= 1u << e;
@@ -760,7 +788,6 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, const __g
   share.temp = temp;
   share.row_max = top.v / temp;
   share.bin_max = share.undivided ? top.v : share.row_max;
-  share.bin_scale = share.undivided ? kBinsPerUnit / temp : kBinsPerUnit;
   share.max_key = ordered_key(share.row_max);
 
   if constexpr (kStaged) share.data = stage;
@@ -771,7 +798,8 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, const __g
   int turn = 0, slot = 0, few = 0;
   Keep keep{0u, vocab};  // every finite value has a key > 0
   if (by_count) {
-    keep = select_prefix<true, kAlone>(share, true, keep, (unsigned long long)(k - 1), 0.f, vocab, turn, slot, few, sm);
+    share.bins_per_unit(kCountsPerUnit);
+    keep = select_prefix<true, kAlone>(share, true, keep, (unsigned long long)(k - 1), p, vocab, turn, slot, few, sm);
     if (few) {
       if (rank == 0) {
         const int column = draw_from_candidates(share, k, p, u, top.i, turn, sm);
@@ -781,7 +809,10 @@ sample_kernel(const T* __restrict__ logits, int vocab, int share_size, const __g
       return;
     }
   }
-  if (p > 0.f && p < 1.f) keep = select_prefix<false, kAlone>(share, !by_count, keep, 0, p, vocab, turn, slot, few, sm);
+  if (p > 0.f && p < 1.f) {
+    share.bins_per_unit(kBinsPerUnit);
+    keep = select_prefix<false, kAlone>(share, !by_count, keep, 0, p, vocab, turn, slot, few, sm);
+  }
 
   // Draw: the first index (ascending) at which the running weight passes uniform * total.
   const int from = share.from, to = share.to;

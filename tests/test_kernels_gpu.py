@@ -558,6 +558,38 @@ def test_sample_among_few_and_many_candidates(dtype, vocab, scale):
         assert any(bool((keep == int(got[r])).any()) for _, keep in rules), f"row {r}: {int(got[r])} is not in what is kept"
 
 
+# Rows whose k-th value lies far below their maximum: low temperatures, a few large values over many small ones, one value far above all; as
+# many columns as can be chosen and one more than are sorted.  One block a row, a cluster, and a cluster of the most a block's memory holds.
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("vocab", [1000, 8192, 32000, 151936])
+def test_sample_far_below_the_maximum(dtype, vocab):
+    from liteinfer_b200 import ops
+
+    g = torch.Generator().manual_seed(vocab)
+    ks, ps = [2, 50, 127, 129, 511, 513], [1.0, 0.9, 0.999999]
+    kinds = [(0.05, "wide"), (0.2, "wide"), (1.0, "peaked"), (0.02, "peaked"), (1.0, "alone")]
+    cases = [(k, p, t, kind) for k in ks for p in ps for t, kind in kinds]
+    def row(kind):
+        x = torch.randn(vocab, generator=g) * 2.5
+        if kind == "peaked":
+            x = x * 0.6 + 3 * torch.empty(vocab).exponential_(1.0, generator=g)
+        if kind == "alone":
+            x[int(torch.randint(vocab, (1,), generator=g))] = 400.0 + float(torch.rand(1, generator=g))
+        return x
+    logits = torch.stack([row(kind) for *_, kind in cases]).to(dtype)
+    u = torch.rand(len(cases), generator=g)
+    got = ops.sample(logits.cuda(), torch.tensor([t for _, _, t, _ in cases]).cuda(), torch.tensor([k for k, *_ in cases], dtype=torch.int32).cuda(),
+                     torch.tensor([p for _, p, *_ in cases]).cuda(), u.cuda(), torch.empty(len(cases), dtype=torch.int32, device="cuda")).cpu()
+    off = 2.0 ** -22 + vocab * 2.0 ** -32          # as in the tests above
+    for r, (k, p, t, _) in enumerate(cases):
+        x, v = logits[r].float() / t, float(u[r])
+        rules = [_sample_rule(x, k, p + dp, min(max(v + du, 0.0), 0.9999999)) for du in (-2 * off, 0.0, 2 * off)
+                 for dp in ((-2 * off, 0.0, 2 * off) if p < 1 else (0.0,))]
+        low, high = min(at for at, _ in rules), max(at for at, _ in rules)
+        assert low <= int(got[r]) <= high, f"{cases[r]}: got {int(got[r])}, the rule gives {low} to {high}"
+        assert any(bool((keep == int(got[r])).any()) for _, keep in rules), f"{cases[r]}: {int(got[r])} is not in what is kept"
+
+
 # Parameters that travel with the launch, up to as many rows as it takes, and one row more through the pinned copy.
 @pytest.mark.parametrize("rows", [1, 3, 128, 129])
 def test_sampler_brings_its_parameters_along(rows):
