@@ -1,7 +1,8 @@
 // Paged attention for any batch of (sequence, its newest queries), in plain SIMT
 // code: the true 32-bit path, and the path for head sizes and types the tensor-core
 // kernels refuse.  One kernel serves whole prompts, portions of prompts and single
-// decoded tokens in the same launch.
+// decoded tokens in the same launch; in 32-bit prompts and portions of more than a few tokens have
+// a kernel of their own, and the single tokens beside them are a second launch.
 //
 // Rule (liteinfer/models/attention.py:24-27,81-84): a sequence's queries are the
 // last `q_len` positions of its context of `ctx` tokens, so query j has position
@@ -24,8 +25,8 @@
 //
 // Bound by the latency of a unit's loads: a lane asks for 64 numbers of its key at once in 16-byte pieces, and for 32 of the
 // values' numbers, without a branch between the loads.  Measured on B200 (float32, 12 heads
-// on 4, head size 64, generating 24 tokens for 12 sequences of 19 to 190): 24 us a launch on average, prompts included (9 for
-// a decode step), against 238 when a warp walked all of a row's keys one load after another.
+// on 4, head size 64, a decode step of 12 sequences of 19 to 190): 9 us, against 238 when a warp walked all of a row's keys one load
+// after another.
 #include "common.cuh"
 
 namespace li {
@@ -412,6 +413,20 @@ __global__ void __launch_bounds__(32 * kPromptWarps) prompt_attention_kernel(con
   }
 }
 
+// Whether the portions of a launch bring so few queries that the kernel above is the faster for them: it gives a row's units to several warps,
+// where this one has a warp a query, whatever stays idle.  Behind 1,500 keys, microseconds, teams and shared keys: 4 heads on 4 of 64, two
+// queries 53 and 137, five 116 and 140, six 148 and 140; 8 on 4, three 148 and 186, four 193 and 186; 12 on 4, two 148 and 255, three
+// 308 and 254; 8 on 1, two 376 and 433; of 128, 16 on 16, three 127 and 168, four 169 and 169; 8 on 4, three 254 and 280; 16 on 4, two 351 and
+// 350; 16 on 2, two 696 and 580; of 100, 4 on 4, six 171 and 183.  Within one unit of keys groups of one or two heads are
+// faster shared (3 queries of 4 heads on 4 of 64: 4.5 and 3.6), wide ones by teams (2 of 16 on 2 of 128 8.5 and 13.0).
+inline bool few_queries(int queries, int groups, int head_dim, int v_dim, int max_context) {
+  if (max_context > 0 && max_context <= kUnit) return groups > 4 ? queries <= 3 : groups > 2 && queries == 2;
+  const bool narrow = v_dim <= 64;
+  if (groups == 1) return queries <= (narrow ? 5 : head_dim <= 100 ? 6 : 3);
+  if (groups == 2) return queries <= 3;
+  return queries == 2 && (narrow || groups <= 4);
+}
+
 template <int kDimsPerLane, int kRows>
 int launch_prompt(dim3 grid, const GenericParams<float>& p, cudaStream_t stream) {
   const size_t smem = prompt_smem(p.heads / p.kv_heads, p.head_dim, p.v_dim);
@@ -466,12 +481,14 @@ using namespace li;
 // q: [tokens, q_row_stride] with head h of a token at columns [h*head_dim, (h+1)*head_dim).
 // out: [tokens, out_row_stride] with head h at columns [h*v_dim, (h+1)*v_dim).  k_pool: [num_pages, kv_heads,
 // page_size, head_dim]; v_pool likewise with v_dim.  window: see first_visible (common.cuh).  sink: null or [heads].
+// single_tokens: whether sequences may bring one token beside others that bring more.  max_context (0: not known): the most tokens that a
+// sequence which brings more than one holds.
 LI_EXPORT int li_paged_attention_generic(int dtype, const void* q, int q_row_stride, void* out, int out_row_stride,
                                          const void* k_pool, const void* v_pool, const int* block_table,
                                          int table_stride, const int* query_start_loc, const int* context_lens,
                                          int num_seqs, int max_q_len, int heads, int kv_heads, int head_dim,
                                          int v_dim, int page_size, int num_pages, float scale, int window,
-                                         int keep_first, float softcap, const float* sink, int single_tokens,
+                                         int keep_first, float softcap, const float* sink, int single_tokens, int max_context,
                                          cudaStream_t stream) {
   if (num_seqs == 0 || max_q_len == 0) return 0;
   if (head_dim < 1 || head_dim > kMaxKeyDim || kv_heads < 1 || heads % kv_heads) return LI_ERR_UNSUPPORTED;
@@ -480,7 +497,8 @@ LI_EXPORT int li_paged_attention_generic(int dtype, const void* q, int q_row_str
   const int groups = heads / kv_heads;
   int max_q = max_q_len;
   const bool only_single = max_q_len > 1 && dtype == kFloat32 && head_dim % 4 == 0 && v_dim % 4 == 0 && head_dim <= kPromptMostDim &&
-                           v_dim <= kPromptMostDim && groups <= kPromptMostRows && aligned16(k_pool) && aligned16(v_pool);
+                           v_dim <= kPromptMostDim && groups <= kPromptMostRows && aligned16(k_pool) && aligned16(v_pool) &&
+                           !few_queries(max_q_len, groups, head_dim, v_dim, max_context);
   if (only_single) {
     // Prompts and portions by the kernel whose queries share their keys; the single tokens beside them, if any, behind it.
     GenericParams<float> p = typed<float>(q, out, k_pool, v_pool);

@@ -92,7 +92,8 @@ _SIGNATURES = {
                            c_int, c_int, c_void_p]),
     "li_paged_attention_generic": ("attention_generic", [
         c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
-        c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_float, c_void_p, c_int, c_void_p]),
+        c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_float, c_void_p, c_int, c_int,
+        c_void_p]),
     "li_convert": ("layernorm", [c_int, c_void_p, c_size_t, c_int, c_void_p, c_size_t, c_int, c_int, c_void_p]),
     "li_layernorm": ("layernorm", [c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                    c_int, c_int, c_float, c_float, c_int, c_int, c_void_p]),
@@ -1050,11 +1051,12 @@ def cluster_capacity(head_dim: int, splits: int) -> int:
 
 def paged_attention_generic(q, q_row_stride, out, k_pool, v_pool, block_table, query_start_loc, context_lens,
                             num_seqs, max_q_len, heads, kv_heads, head_dim, scale, window=0, keep_first=0,
-                            softcap=0.0, sink=None, single_tokens=True) -> torch.Tensor:
+                            softcap=0.0, sink=None, single_tokens=True, max_context_len=0) -> torch.Tensor:
     """The plain SIMT kernel: any dtype, key and value sizes up to 1,024 (they may differ), any grouping, a window
     that may keep the first `keep_first` keys visible (`window` < 0: chunks of -window positions instead), scores
     capped by softcap * tanh(score / softcap), a sink.  `single_tokens`: whether a sequence may bring just one token (where others
-    bring more, 32-bit prompts go to a kernel of their own)."""
+    bring more than a few, 32-bit prompts go to a kernel of their own).  `max_context_len` (0: not known): the most tokens that a
+    sequence with more than one query holds."""
     _rows2d(q, "q"); _rows2d(out, "out")
     _on_gpu(k_pool, v_pool, block_table, query_start_loc, context_lens, sink)
     pages, kvh, page_size, hd = k_pool.shape
@@ -1062,7 +1064,7 @@ def paged_attention_generic(q, q_row_stride, out, k_pool, v_pool, block_table, q
         _code(q), q.data_ptr(), q_row_stride, out.data_ptr(), out.stride(0), k_pool.data_ptr(), v_pool.data_ptr(),
         block_table.data_ptr(), block_table.stride(0), query_start_loc.data_ptr(), context_lens.data_ptr(),
         num_seqs, max_q_len, heads, kv_heads, head_dim, v_pool.shape[3], page_size, pages, float(scale), int(window),
-        int(keep_first), float(softcap), _ptr(sink), int(single_tokens), _stream()),
+        int(keep_first), float(softcap), _ptr(sink), int(single_tokens), int(max_context_len), _stream()),
         "paged_attention_generic")
     return out
 
@@ -1258,7 +1260,8 @@ def paged_attention(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_poo
         assert newest is None
         return paged_attention_generic(q, q_row_stride, out, k_pool, v_pool, block_table, query_start_loc,
                                        context_lens, num_seqs, max_q_len, heads, kv_heads, head_dim, scale, window,
-                                       keep_first, softcap, sink, plan is None or plan.num_decode > 0)
+                                       keep_first, softcap, sink, plan is None or plan.num_decode > 0,
+                                       plan.max_prefill_context_len if plan is not None else 0)
     common = (q, q_row_stride, out, k_pool, v_pool, block_table, query_start_loc, context_lens)
     # Kept first keys are an option of the tcgen05 kernel (prompts) and of the mma.sync kernel (prompts it takes instead,
     # and single tokens); the streaming decode kernel does not know them.  Capped scores every one of them takes.

@@ -322,6 +322,35 @@ def test_prompts_in_32_bit_share_their_keys(heads, kv_heads, head_dim, page_size
         torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-5)
 
 
+# Portions of few queries on either side of the line between the two kernels, whose sums are the same: as many queries as teams take and
+# one more, each portion also as the end of one of eight queries, which never is theirs.
+@pytest.mark.parametrize("heads,kv_heads,head_dim,few", [(4, 4, 64, 5), (8, 4, 64, 3), (12, 4, 64, 2), (4, 4, 128, 3), (4, 4, 100, 6), (8, 4, 128, 3),
+                                                         (16, 4, 128, 2), (16, 2, 128, 1)])
+@pytest.mark.parametrize("context", [20, 333])
+def test_portions_of_few_queries_in_32_bit(heads, kv_heads, head_dim, few, context):
+    from liteinfer_b200 import ops
+
+    scale = head_dim ** -0.5
+    for queries in (2, few, few + 1):
+        if queries < 2:
+            continue
+        lens = [8, 1, 8]
+        case = _paged_case(torch.float32, heads, kv_heads, head_dim, 16, lens, [context] * 3, poison=False)
+        out = lambda n: torch.full((n, heads * head_dim), float("nan"), device="cuda")
+        ops.rope_kv_write(case["qkv"], case["positions"], case["seq_of"], case["table"], case["k_pool"], case["v_pool"], None,
+                          heads, kv_heads, head_dim, 0)
+        tail = (case["k_pool"], case["v_pool"], case["table"])
+        whole = ops.paged_attention(case["qkv"], case["qkv"].shape[1], out(17), *tail, case["qsl"], case["ctx"], 3, 8, heads, kv_heads,
+                                    head_dim, scale, plan=_plan_for(lens, [context] * 3))
+        short = torch.cat([case["qkv"][8 - queries:9], case["qkv"][17 - queries:]])
+        lens = [queries, 1, queries]
+        qsl = torch.tensor([0, queries, queries + 1, 2 * queries + 1], dtype=torch.int32, device="cuda")
+        for plan in (None, _plan_for(lens, [context] * 3)):
+            got = ops.paged_attention(short, short.shape[1], out(len(short)), *tail, qsl, case["ctx"], 3, queries, heads, kv_heads, head_dim,
+                                      scale, plan=plan)
+            assert torch.equal(got, torch.cat([whole[8 - queries:9], whole[17 - queries:]]))
+
+
 # Rows walked by one warp and by teams, one unit of keys and several rounds of them, every width of values.
 @pytest.mark.parametrize("heads,kv_heads,head_dim,page_size", [(3, 1, 64, 16), (9, 1, 20, 16), (2, 2, 128, 16), (6, 3, 256, 8),
                                                                (2, 1, 320, 16), (34, 2, 33, 5)])
