@@ -10,13 +10,16 @@
 //                         g = exp(-exp(A_log) * softplus(raw + dt_bias))
 //
 // The recurrence is a chain over the tokens of a sequence, but every column of S is a chain of its own:
-// (S^T k)_j, u_j, the update of S[:, j] and o_j touch column j only.  So a block takes 32 columns of one head of
+// (S^T k)_j, u_j, the update of S[:, j] and o_j touch column j only.  So a block takes 16 or 32 columns of one head of
 // one sequence, eight lanes share a column (each keeps dim/8 of its entries in registers for the whole step) and
-// add up their parts of the two dot products with three shuffles.  What does not depend on the state (the unit
+// add up their parts of the dot products with shuffles.  What does not depend on the state (the unit
 // norms, beta, the decay) is computed once per token and head by a kernel in front; the inputs of the next few
-// tokens are in flight while one is computed.  Whole prompts, portions and single tokens run
-// the same code from the state the step before left, in the same order, so the result does not depend on how a
-// sequence was cut.  Tokens of padding (sequence -1) and sequences that bring no token touch nothing.
+// tokens are in flight while one is computed.  Prompts, portions and single tokens go on from the state that the step
+// before left.  Heads of 32, 64 and 128 go two tokens at a time, paired from where the step's portion of a sequence
+// begins: a cut at an odd place pairs other tokens, which rounds differently (in 32-bit, 1e-7 or so of the
+// result), and so does a single token, which is a portion of one beside prompts and another kernel's in a step of
+// its like.  Other heads go a token at a time, in one order however a sequence was cut.  Which other sequences a launch
+// has changes no bit.  Tokens of padding (sequence -1) and sequences that bring no token touch nothing.
 #include <type_traits>
 
 #include "common.cuh"

@@ -235,7 +235,7 @@ def test_gated_delta_rule_in_portions_equals_whole(dtype, heads, kv_heads, dim, 
     parts, state_parts = run(ops, cuts)
     want, state_want = run(ref, cuts)
     for a, b, c in zip(whole, parts, want):
-        torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-6)            # the same chain however it is cut
+        torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-6)            # pairs of tokens or one by one: rounding apart
         torch.testing.assert_close(a, c, rtol=1e-4, atol=1e-5)
     torch.testing.assert_close(state_whole, state_parts, rtol=1e-5, atol=1e-6)
     torch.testing.assert_close(state_parts, state_want, rtol=1e-4, atol=1e-5)
