@@ -393,25 +393,20 @@ int launch_tiles(const SimtProduct& p, bool vec, int batch, cudaStream_t stream)
   return 0;
 }
 
-// Which kernel, by what each was measured to take (B200, microseconds).  float32, the narrow one: 3.6 and 0.12 a row up to 16, and for
-// every million weights 0.72 for one row, 0.85 for four, 1.4 for eight, 1.65 for twelve, 2.1 for every group of 16; a fifth more where k
-// is more than 2,048.  Tiles take their waves of 148, one a whole step each: per 768 k 2 and 12.3 a wave for tiles of 32 rows (a lone wave 17.3),
-// 6.5 and 21 a wave for tiles of 64 (768 k, 140 tiles of 32 18.4, 156 27.7, 288 28.7, 300 39.5, 448 52.7, 640 64; of 64 rows 140 29.3, 156
-// 48.9, 320 70, 448 91).  By a line through these 257 rows of 4096 x 768 went to 320 tiles of 64 rows, 96 us (59 in 576 of 32).
-// Up to 16 rows of one product the narrow kernel is the faster wherever k is not short (16 of 16000 x 768: 29 and 40).
-// bfloat16: tiles of 32 rows 26 per 768 k, then 0.15 a tile; of 128 rows 54, up to two an SM 98, then 0.37 a tile.
+// Which kernel, by what each was measured to take (B200, microseconds, float32).  The narrow one: 4 and 2.1 for every million
+// weights of a group of 16 rows (16384 x 2048: 70 for 12 rows; 1280 x 768: 11.3 for 64).  Tiles of 32 rows: 24 per 768 k
+// while each SM has one or none, 35 up to some 250, then 12 and 0.104 a tile (1280 x 768: 24.7 for 192 rows, 87 for 1,250); tiles of
+// 64 rows: 35.5 per 768 k up to one an SM, 58 up to two, then 12 and 0.155 a tile (1280 x 768: 35.6 for 256 rows, 79 for 1,250; 4096 x
+// 768: 213 for 1,250).  bfloat16: tiles of 32 rows 26, then 0.15 a tile; of 128 rows 54, up to two an SM 98, then 0.37 a tile.
 constexpr int kMostRows = 256;
 inline float rows_cost(const SimtProduct& p, int batch) {
-  if (p.M <= 16 && p.K >= 256 && batch == 1) return 0.f;
-  const float each = p.M == 1 ? 0.72f : p.M <= 4 ? 0.85f : p.M <= 8 ? 1.4f : p.M <= 12 ? 1.65f : 2.1f * ((p.M + 15) / 16);
-  return 3.6f + 0.12f * (p.M < 16 ? p.M : 16) + 1e-6f * each * (p.K > 2048 ? 1.2f : 1.f) * (float)p.N * p.K * batch;
+  return 4.f + 2.1e-6f * (float)p.N * p.K * ((p.M + 15) / 16) * batch;
 }
 inline float tiles_cost(int dtype, const SimtProduct& p, int batch, int rows) {
   const float tiles = (float)((p.N + BN - 1) / BN) * ((p.M + rows - 1) / rows) * batch, depth = p.K / 768.f;
   if (dtype != kFloat32) return depth * (rows == 32 ? fmaxf(26.f, 0.15f * tiles) : tiles <= 148.f ? 54.f : fmaxf(98.f, 0.37f * tiles));
-  const float waves = ceilf(tiles / 148.f);
-  if (rows == 32) return 1.5f + depth * (waves <= 1.f ? 17.3f : 2.f + 12.3f * waves);
-  return 2.f + depth * (6.5f + 21.f * waves);
+  if (rows == 32) return depth * (tiles <= 148.f ? 24.f : fmaxf(35.f, 12.f + 0.104f * tiles));
+  return depth * (tiles <= 148.f ? 35.5f : fmaxf(58.f, 12.f + 0.155f * tiles));
 }
 
 int launch_product(int dtype, const SimtProduct& p, int batch, cudaStream_t stream) {
