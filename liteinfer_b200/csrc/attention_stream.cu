@@ -161,11 +161,6 @@ __device__ __forceinline__ int splits_of(int tiles, int most) {
   return wanted <= 1 ? 1 : ceil_quotient(tiles, ceil_quotient(tiles, wanted));
 }
 
-// How many groups a warp has asked for when it waits for group `i`: `ring` - 1 before the first, and one more in each round before its wait.
-__host__ __device__ constexpr int asked_for(int i, int ring, int groups) { return i + ring < groups ? i + ring : groups; }
-static_assert(asked_for(0, 2, 9) == 2 && asked_for(3, 4, 9) == 7 && asked_for(7, 2, 9) == 9 && asked_for(8, 2, 9) == 9 && asked_for(0, 4, 1) == 1,
-              "the newest request is among those that are waited for");
-
 // kWide: a form in fewer registers, three blocks of head size 128 an SM instead of two, for launches of more blocks than two an SM.  It is
 // some 4 % slower a block.  Measured on B200, 8 KV heads of 128: 48 sequences of 1,500 keys 48 us (65.5), 40 of 2,000 55 (81), 24 of
 // 3,000, in two splits each then, 52 (63); 32 of 2,000, which are one wave either way, 47.4 (45).
@@ -178,6 +173,7 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   constexpr unsigned kHalfBytes = kGroupKeys * D * 2;      // K or V of one group
   constexpr unsigned kSlotBytes = 2 * kHalfBytes;
   constexpr int kBoxes = D / 64;                           // boxes of 64 dimensions per row
+  constexpr int kAhead = kRing - 1;                        // groups that a warp has asked for beyond the one it waits for
   extern __shared__ unsigned char smem_raw[];
   const unsigned base = (smem_addr(smem_raw) + 1023u) & ~1023u;
   unsigned char* generic_base = smem_raw + (base - smem_addr(smem_raw));
@@ -257,10 +253,10 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   // The pages hold nothing that the kernel before this one wrote when the cache write is fused in here; otherwise
   // the newest key and value come from it, and the first requests wait for it too.
   if (fused)
-    for (int i = 0; i < kRing - 1; ++i) request(i);
+    for (int i = 0; i < kAhead; ++i) request(i);
   grid_dependency_wait();
   if (!fused)
-    for (int i = 0; i < kRing - 1; ++i) request(i);
+    for (int i = 0; i < kAhead; ++i) request(i);
 
   const size_t token = (size_t)q_begin * p.q_row_stride;
   // Q: rows g and g+8 of the group (zero beyond it), pieces t, t+4, ...  Asked for before the newest key and value
@@ -343,14 +339,15 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
       v_at[q][c] = kHalfBytes + piece_addr(0, 2 * t + (q & 1) + (q >> 1) * 8, g * (D / 64) + c);
 
   for (int i = 0; i < my_groups; ++i) {
-    request(i + kRing - 1);
+    request(i + kAhead);
     const int kpos0 = (my_lo + i) * kBlockN + warp * kGroupKeys;
     if (kpos0 < hi && kpos0 + kGroupKeys > lo) {
       if (!mbar_wait(bars + 8u * (i % kRing), (unsigned)(i / kRing) & 1, p.error_flag, 21)) {
         // Gave up: before the ring's memory is used for anything else, give the copies still on their way one
         // more (bounded) chance to land.
-        for (int r = i + 1; r < asked_for(i, kRing, my_groups); ++r)
-          mbar_wait(bars + 8u * (r % kRing), (unsigned)(r / kRing) & 1, nullptr, 0);
+#pragma unroll
+        for (int r = 1; r <= kAhead; ++r)
+          if (i + r < my_groups) mbar_wait(bars + 8u * ((i + r) % kRing), (unsigned)((i + r) / kRing) & 1, nullptr, 0);
         break;
       }
       const unsigned slot = ring + (unsigned)(i % kRing) * kSlotBytes;
