@@ -54,8 +54,9 @@ class EngineConfig:
     # Replay decode steps from CUDA graphs.  None: wherever the device is CUDA.
     enable_cuda_graphs: bool | None = None
 
-    # Programs that share one sequence's key loop in decode attention; None lets
-    # the engine choose from the batch width and the context.
+    # Programs that share one sequence's key loop in decode attention, whatever its
+    # context (32 at most); None lets the engine choose from the batch width and the
+    # context.
     paged_decode_splits: int | None = None
 
     collect_stats: bool = True

@@ -50,6 +50,7 @@ struct AttnParams {
   // Values wider than keys: v_parts blocks side by side share a (sequence, KV head, split), each computing the scores
   // and D of the v_parts * D dimensions of the output (blockIdx.y = KV head * v_parts + part).
   int v_parts;
+  bool every_split;       // attention_stream.cu only: num_splits was asked for, and is not just the most that a sequence may have
 };
 
 // Where a head's part of the output (and of the split partials) lies, in units of D.

@@ -193,7 +193,7 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   const int qpos = ctx - 1, hi = ctx;
   const int lo = first_visible(qpos, p.window);
   const int tile_lo = lo / kBlockN, tile_hi = (hi + kBlockN - 1) / kBlockN;
-  const int splits = kCluster ? p.num_splits : splits_of(tile_hi - tile_lo, p.num_splits);
+  const int splits = kCluster || p.every_split ? p.num_splits : splits_of(tile_hi - tile_lo, p.num_splits);
   if (split >= splits) return;
   const int per_split = splits == 1 ? tile_hi - tile_lo : ceil_quotient(tile_hi - tile_lo, splits);
   const int my_lo = tile_lo + split * per_split, my_hi = min(tile_hi, my_lo + per_split);
@@ -669,7 +669,8 @@ LI_EXPORT int li_paged_attention_stream_wide_capacity(int head_dim) {
 }
 
 // Every launched sequence brings exactly one token.  Arguments as li_paged_attention_mma (its counters export
-// says how many counters a split launch needs; num_splits is the most that a sequence gets, see splits_of); sizes as li_paged_attention_stream_supports allows.
+// says how many counters a split launch needs; num_splits is what every sequence gets with every_split, else the most that one gets, see
+// splits_of); sizes as li_paged_attention_stream_supports allows.
 // error_flag (device int, zero; may be null): set to 21 if a wait for a group of keys ever gave up.
 // sink (optional, [heads] float32): exp(sink[h]) is one more term of head h's denominator.  v_dim: the size of a value,
 // a multiple of head_dim.  softcap > 0: a scaled score s becomes softcap * tanh(s / softcap).
@@ -681,7 +682,7 @@ LI_EXPORT int li_paged_attention_stream(const void* q, int q_row_stride, void* o
                                         float* partial_out, float* partial_lse, unsigned* counters,
                                         const float* rope_inv_freq, const void* k_new, const void* v_new,
                                         int store_new, int* error_flag, const float* sink, int v_dim, float softcap,
-                                        cudaStream_t stream) {
+                                        int every_split, cudaStream_t stream) {
   if (num_seqs == 0) return 0;
   if (!li_paged_attention_stream_supports(heads, kv_heads, head_dim, page_size)) return LI_ERR_UNSUPPORTED;
   if (v_dim < head_dim || v_dim % head_dim) return LI_ERR_UNSUPPORTED;
@@ -708,6 +709,7 @@ LI_EXPORT int li_paged_attention_stream(const void* q, int q_row_stride, void* o
   // launch of single blocks does, and the step loses more than the merge gains (1.065 against 0.948 ms).
   const char* cluster_env = getenv("LITEINFER_ATTN_CLUSTER_MERGE");
   p.v_parts = v_parts;
+  p.every_split = every_split != 0;
   p.sink = sink;      // added by the merges of attention_mma.cuh; the merge inside a cluster does not know it
   if (softcap > 0.f) {
     p.cap_in = scale / softcap;

@@ -134,7 +134,7 @@ _SIGNATURES = {
     "li_paged_attention_stream": ("attention_stream", [
         c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
         c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_void_p, c_void_p,
-        c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_float, c_void_p]),
+        c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_float, c_int, c_void_p]),
     "li_paged_attention_stream_supports": ("attention_stream", [c_int, c_int, c_int, c_int]),
     "li_paged_attention_stream_capacity": ("attention_stream", [c_int]),
     "li_paged_attention_stream_wide_capacity": ("attention_stream", [c_int]),
@@ -1072,9 +1072,10 @@ def paged_attention_generic(q, q_row_stride, out, k_pool, v_pool, block_table, q
 def paged_attention_mma(q, q_row_stride, out, k_pool, v_pool, block_table, query_start_loc, context_lens,
                         seq_index, num_seqs, max_q_len, heads, kv_heads, head_dim, scale, window=0,
                         num_splits=1, newest=None, streaming=False, keep_first=0, softcap=0.0,
-                        sink=None) -> torch.Tensor:
+                        sink=None, every_split=True) -> torch.Tensor:
     """The tensor-core kernel (bfloat16, head size 64 or 128); `num_splits` > 1 splits every sequence's keys
-    over that many blocks, the last of which merges the partial results.  `newest` (NewestToken, single-token
+    over that many blocks, the last of which merges the partial results; with `streaming` and not `every_split` that is
+    the most, and a sequence gets as many as its own keys pay for.  `newest` (NewestToken, single-token
     sequences only): q is unrotated and the newest key and value are not in their pages yet; the kernel
     rotates q and the key and stores key and value itself.  `streaming` (single-token sequences, sizes that
     `stream_attention_supports` allows): the kernel that passes K and V through registers only.  `keep_first`
@@ -1104,7 +1105,8 @@ def paged_attention_mma(q, q_row_stride, out, k_pool, v_pool, block_table, query
             block_table.data_ptr(), block_table.stride(0), query_start_loc.data_ptr(), context_lens.data_ptr(),
             _ptr(seq_index), num_seqs, heads, kv_heads, head_dim, page_size, pages, float(scale), int(window),
             int(num_splits), _ptr(partial_out), _ptr(partial_lse), _ptr(counters), *tail,
-            scratch_for(q.device).gemm_error.data_ptr(), _ptr(sink), v_dim, float(softcap), _stream()), "paged_attention_stream")
+            scratch_for(q.device).gemm_error.data_ptr(), _ptr(sink), v_dim, float(softcap), int(every_split), _stream()),
+            "paged_attention_stream")
         return out
     _check(_fn("li_paged_attention_mma")(
         q.data_ptr(), q_row_stride, out.data_ptr(), out.stride(0), k_pool.data_ptr(), v_pool.data_ptr(),
@@ -1233,7 +1235,8 @@ def paged_attention(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_poo
     with `q_row_stride` elements between tokens (the fused qkv buffer is passed as
     it is).  out: [tokens, heads*head_dim].  bfloat16 with head size 64 or 128 runs
     on tensor cores; with a `plan` (AttentionPlan) the sequences that bring one
-    token go through a launch that splits their keys over several blocks, the
+    token go through a launch that splits their keys over several blocks
+    (`decode_splits` of them for every sequence where it is given, 32 at most), the
     others through an unsplit one.  Everything else runs the plain SIMT kernel.
     `newest`: only where `fused_decode_supports` said yes; see `paged_attention_mma`.
     `keep_first` (with a window): the first keys of a sequence stay visible behind the window.  `softcap` > 0:
@@ -1277,7 +1280,7 @@ def paged_attention(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_poo
         streaming = not (keep_first > 0 and window > 0) and stream_attention_supports(q.dtype, heads, kv_heads, head_dim, page_size)
         splits = decode_splits or decode_splits_for(plan.num_decode, kv_heads * parts, bound, head_dim, streaming)
         paged_attention_mma(*common, plan.decode_seqs, plan.num_decode, 1, heads, kv_heads, head_dim, scale,
-                            window, splits, newest, streaming, **options)
+                            window, splits, newest, streaming, every_split=decode_splits is not None, **options)
 
     def portions():
         if tcgen05_attention_supports(q.dtype, heads, kv_heads, head_dim, page_size) and not MASKED_ON_MMA:

@@ -782,6 +782,39 @@ def test_decode_splits_follow_the_context(head_dim, ctx_lens, splits, window, so
     assert ops.gemm_error_flag("cuda:0") == 0
 
 
+# A count that is asked for is every sequence's, also of one with fewer tiles than blocks or as few as one block would take.
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("splits", [1, 2, 5, 8, 32, None])
+def test_splits_that_are_asked_for_are_taken(head_dim, splits, monkeypatch):
+    from liteinfer_b200 import ops
+    from liteinfer_b200.ops import kernels
+
+    heads, kv_heads, ctx_lens = 8, 2, [1, 100, 256, 300, 449, 1000, 3000]
+    case = _paged_case(torch.bfloat16, heads, kv_heads, head_dim, 16, [1] * len(ctx_lens), ctx_lens, poison=False)
+    rest = (case["k_pool"], case["v_pool"], case["table"], case["qsl"], case["ctx"], case["B"], 1, heads, kv_heads, head_dim,
+            head_dim ** -0.5)
+    out = lambda: torch.full((case["T"], heads * head_dim), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.paged_attention(case["qkv"], case["qkv"].shape[1], out(), *rest, plan=_plan_for([1], [64]))        # (what is kept is made)
+    partials = []       # the log-sum-exps of the launch: a split that the kernel wrote holds a number or minus infinity
+    empty = torch.empty
+
+    def marked(*shape, **options):
+        made = empty(*shape, **options)
+        if options.get("dtype") == torch.float32 and made.dim() == 1:
+            made.fill_(float("nan"))
+            partials.append(made)
+        return made
+
+    monkeypatch.setattr(kernels.torch, "empty", marked)
+    got = ops.paged_attention(case["qkv"], case["qkv"].shape[1], out(), *rest, plan=_plan_for([1] * len(ctx_lens), ctx_lens),
+                              decode_splits=splits)
+    monkeypatch.undo()
+    want = ref.paged_attention(case["qkv"], case["qkv"].shape[1], out(), *rest)
+    torch.testing.assert_close(got.float(), want.float(), rtol=2 ** -6, atol=2 ** -6)
+    written = [not bool(torch.isnan(p).any()) for p in partials]
+    assert written == ([] if splits == 1 else [splits is not None])      # None: the short ones have one block, and no partial result
+
+
 @pytest.mark.parametrize("heads,kv_heads,head_dim,page_size", [(32, 8, 64, 16), (8, 8, 64, 8), (16, 1, 128, 16),
                                                                (6, 2, 128, 5), (5, 1, 64, 32)])
 @pytest.mark.parametrize("window", [0, 100])
