@@ -161,7 +161,7 @@ __device__ __forceinline__ int splits_of(int tiles, int most) {
   return wanted <= 1 ? 1 : ceil_quotient(tiles, ceil_quotient(tiles, wanted));
 }
 
-// kWide: a form in fewer registers, three blocks of head size 128 an SM instead of two, for launches of more blocks than two an SM.  It is
+// kWide: a form in fewer registers, three blocks of head size 128 an SM instead of two, for the launches that `wide_form` names.  It is
 // some 4 % slower a block.  Measured on B200, 8 KV heads of 128: 48 sequences of 1,500 keys 48 us (65.5), 40 of 2,000 55 (81), 24 of
 // 3,000, in two splits each then, 52 (63); 32 of 2,000, which are one wave either way, 47.4 (45).
 // kRing: slots per warp; up to kRing - 1 groups are on their way while one is multiplied.
@@ -570,13 +570,22 @@ int launch_blocks(const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams
                          stream_smem<D, kRing>(), stream, mk, mv, p);
 }
 
+// Whether a launch of so many blocks of head size 128 takes the form of three an SM: from the first that does not have a place in the narrow
+// one, except where it would leave a second wave of a few blocks, alone at their latency, while two narrow waves hold all.  8 KV heads,
+// microseconds, narrow and wide: 48 sequences (384 blocks) of 1,500 68 and 50; 56 (448) 69 and 73, 64 (512) 69 and 82, of 60 9.7 and 11.2, of 8,192
+// 319 and 397; 74 (592) 76 and 85; 80 (640) 102 and 85, 96 (768) 104 and 92, 128 138 and 131.  Sequences of many lengths come longest first
+// (decode_longest_first), 64 of 375 to 2,600 62 and 67; as they come 83 and 77.
+bool wide_form(long blocks) {
+  const int narrow = stream_capacity<128, 2, false>(), wide = stream_capacity<128, 2, true>();
+  return narrow > 0 && blocks > narrow && !(blocks > wide && blocks <= 2 * narrow);
+}
+
 template <int D, int kRing>
 int launch_stream(const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams& p, int num_seqs, cudaStream_t stream) {
   const dim3 grid(p.num_splits, p.kv_heads * p.v_parts, num_seqs);
   if (!p.cluster_merge) {
     if constexpr (D == 128) {
-      const int narrow = stream_capacity<D, kRing, false>();
-      if (narrow > 0 && (long)grid.x * grid.y * grid.z > narrow) {
+      if (wide_form((long)grid.x * grid.y * grid.z)) {
         return p.cap_out > 0.f ? launch_blocks<D, kRing, true, true>(mk, mv, p, grid, stream)
                                : launch_blocks<D, kRing, false, true>(mk, mv, p, grid, stream);
       }
@@ -663,7 +672,8 @@ LI_EXPORT int li_paged_attention_stream_capacity(int head_dim) {
   return head_dim == 64 ? stream_capacity<64, kRing64, false>() : (head_dim == 128 ? stream_capacity<128, kRing128, false>() : 0);
 }
 
-// The same of the form that takes launches of more blocks than that.
+// Whether a launch of so many blocks takes the form in fewer registers, and how many blocks of it the device holds at once.
+LI_EXPORT int li_paged_attention_stream_wide(int head_dim, int blocks) { return head_dim == 128 && wide_form(blocks); }
 LI_EXPORT int li_paged_attention_stream_wide_capacity(int head_dim) {
   return head_dim == 128 ? stream_capacity<128, kRing128, true>() : li_paged_attention_stream_capacity(head_dim);
 }

@@ -67,11 +67,11 @@ class StepEntry:
 class _Views:
     """The arrays of one staged batch (slices of one buffer, numpy or torch)."""
 
-    __slots__ = ("tok", "pos", "seq", "qsl", "ctxl", "slots", "rows", "dseq", "dtok", "pseq", "late_dst", "late_src",
-                 "tables")
+    __slots__ = ("tok", "pos", "seq", "qsl", "ctxl", "slots", "rows", "dseq", "dtok", "dlong", "pseq", "late_dst",
+                 "late_src", "tables")
     NAMES = __slots__[:-1]
 
-    def __iter__(self):      # tok, pos, seq, qsl, ctxl, slots, rows, dseq, dtok, pseq, late_dst, late_src, *tables
+    def __iter__(self):      # tok, pos, seq, qsl, ctxl, slots, rows, dseq, dtok, dlong, pseq, late_dst, late_src, *tables
         for name in self.NAMES:
             yield getattr(self, name)
         yield from self.tables
@@ -83,7 +83,7 @@ class _Batch:
     def __init__(self, B: int, T: int, R: int, widths: list[int], n_decode: int, n_prefill: int) -> None:
         self.B, self.T, self.R, self.widths = B, T, R, widths
         self.n_decode, self.n_prefill = n_decode, n_prefill
-        sizes = [T, T, T, B + 1, B, B, R, n_decode, n_decode, n_prefill, B, B] + [B * w for w in widths]
+        sizes = [T, T, T, B + 1, B, B, R, n_decode, n_decode, n_decode, n_prefill, B, B] + [B * w for w in widths]
         # Every array starts on a 16-byte boundary.
         self.sizes = sizes
         self.offsets = []
@@ -103,9 +103,14 @@ class _Batch:
         return v
 
 
+def _longest_first(seqs: np.ndarray, context_lens: np.ndarray) -> np.ndarray:
+    """Sequences by falling context, those of one length in their order."""
+    return seqs[np.argsort(-context_lens[seqs], kind="stable")]
+
+
 def _fill(batch: _Batch, flat: np.ndarray, entries: list[StepEntry], cache: CacheManager,
           starts: list[int]) -> None:
-    tok, pos, seq, qsl, ctxl, slots, rows, dseq, dtok, pseq, late_dst, late_src, *tables = batch.views(flat)
+    tok, pos, seq, qsl, ctxl, slots, rows, dseq, dtok, dlong, pseq, late_dst, late_src, *tables = batch.views(flat)
     cursor = row_cursor = nd = npf = late = 0
     qsl[0] = 0
     late_dst[:] = -1
@@ -132,6 +137,7 @@ def _fill(batch: _Batch, flat: np.ndarray, entries: list[StepEntry], cache: Cach
         qsl[i + 1] = cursor
         ctxl[i] = starts[i] + n
         slots[i] = cache.state_slot(entry.request_id)
+    dlong[:nd] = _longest_first(dseq[:nd], ctxl)
     for g, width in enumerate(batch.widths):
         if not width:
             continue
@@ -143,13 +149,13 @@ def _fill(batch: _Batch, flat: np.ndarray, entries: list[StepEntry], cache: Cach
 
 
 def _context(batch: _Batch, dev: torch.Tensor, device, counts, totals, decode_splits, decode_bound) -> StepContext:
-    tok, pos, seq, qsl, ctxl, slots, rows, dseq, dtok, pseq, _, _, *tables = batch.views(dev)
+    tok, pos, seq, qsl, ctxl, slots, rows, dseq, dtok, dlong, pseq, _, _, *tables = batch.views(dev)
     B = batch.B
     tables = [t.view(B, w) if w else torch.full((B, 1), -1, dtype=torch.int32, device=device)
               for t, w in zip(tables, batch.widths)]
     prefill_lens = [c for c in counts if c > 1]
     plan = AttentionPlan(
-        num_decode=batch.n_decode, decode_seqs=dseq, decode_tokens=dtok, num_prefill=batch.n_prefill,
+        num_decode=batch.n_decode, decode_seqs=dseq, decode_tokens=dtok, decode_longest_first=dlong, num_prefill=batch.n_prefill,
         prefill_seqs=pseq, max_prefill_query_len=max(prefill_lens, default=0), max_decode_context_len=decode_bound,
         max_prefill_context_len=max((t for t, c in zip(totals, counts) if c > 1), default=0))
     return StepContext(
@@ -184,7 +190,7 @@ class _DecodeGraph:
 
     def _write_fixed_parts(self) -> None:
         """What is the same for every batch of this width: sequence i brings token i and wants its logits."""
-        tok, pos, seq, qsl, ctxl, slots, rows, dseq, dtok, pseq, late_dst, late_src, *tables = self.views
+        tok, pos, seq, qsl, ctxl, slots, rows, dseq, dtok, dlong, pseq, late_dst, late_src, *tables = self.views
         width = self.batch.B
         late_dst[:] = -1
         seq[:] = np.arange(width, dtype=np.int32)
@@ -192,6 +198,7 @@ class _DecodeGraph:
         rows[:] = seq
         dseq[:] = seq
         dtok[:] = seq
+        dlong[:] = seq
         for table in tables:
             table.fill(-1)
         self.row_keys = [None] * width
@@ -207,12 +214,13 @@ class _DecodeGraph:
     def stage(self, entries: list[StepEntry], cache: CacheManager, starts: list[int]) -> None:
         """Writes this step's batch (every entry one token, logits wanted) into the pinned buffer."""
         self.copied.synchronize()              # the device has read the batch before this one
-        tok, pos, seq, qsl, ctxl, slots, rows, dseq, dtok, pseq, late_dst, late_src, *tables = self.views
+        tok, pos, seq, qsl, ctxl, slots, rows, dseq, dtok, dlong, pseq, late_dst, late_src, *tables = self.views
         tok[:] = [entry.tokens[0] if entry.late is None else 0 for entry in entries]
         late_dst[:] = [-1 if entry.late is None else i for i, entry in enumerate(entries)]     # token row i is sequence i
         late_src[:] = [entry.late or 0 for entry in entries]
         pos[:] = starts
         np.add(pos, 1, out=ctxl)
+        dlong[:] = _longest_first(dseq, ctxl)
         for i, entry in enumerate(entries):
             key = (entry.request_id, cache.table_version(entry.request_id))
             if self.row_keys[i] == key:
@@ -249,10 +257,10 @@ class _DecodeGraph:
 
 
 def _write_padding(views) -> None:
-    tok, pos, seq, qsl, ctxl, slots, rows, dseq, dtok, pseq, late_dst, late_src, *tables = views
+    tok, pos, seq, qsl, ctxl, slots, rows, dseq, dtok, dlong, pseq, late_dst, late_src, *tables = views
     for array in (tok, pos, qsl, ctxl, slots, rows, dtok, late_src):
         array[:] = 0
-    for array in (seq, dseq, pseq, late_dst, *tables):
+    for array in (seq, dseq, dlong, pseq, late_dst, *tables):
         array[:] = -1
 
 
@@ -278,10 +286,10 @@ class _PaddedGraph:
         n_decode = seqs if decode else 0
         self.batch = batch = _Batch(seqs, tokens, rows, [pages] * len(cache.groups), n_decode, prefill)
         self.device_buffer = torch.zeros(batch.total, dtype=torch.int32, device=runner.device)
-        tok, pos, seq, qsl, ctxl, slots, wanted, dseq, dtok, pseq, _, _, *tables = batch.views(self.device_buffer)
+        tok, pos, seq, qsl, ctxl, slots, wanted, dseq, dtok, dlong, pseq, _, _, *tables = batch.views(self.device_buffer)
         tables = [t.view(seqs, w) for t, w in zip(tables, batch.widths)]
         # The kernels' launch bounds are those of the padded shape; what a step really holds is in the buffers.
-        plan = AttentionPlan(num_decode=n_decode, decode_seqs=dseq, decode_tokens=dtok, num_prefill=prefill,
+        plan = AttentionPlan(num_decode=n_decode, decode_seqs=dseq, decode_tokens=dtok, decode_longest_first=dlong, num_prefill=prefill,
                              prefill_seqs=pseq, max_prefill_query_len=portion if prefill else 0,
                              max_decode_context_len=max_model_len, max_prefill_context_len=prefill_context)
         self.ctx = StepContext(
@@ -300,7 +308,7 @@ class _PaddedGraph:
         """Writes this step's batch and the padding around it into the pinned buffer; returns the wanted rows."""
         self.copied.synchronize()
         _fill(self.batch, self.host.numpy(), entries, cache, starts)
-        tok, pos, seq, qsl, ctxl, slots, wanted, dseq, dtok, pseq, *_ = self.views
+        tok, pos, seq, qsl, ctxl, slots, wanted, dseq, dtok, dlong, pseq, *_ = self.views
         B = len(entries)
         T = int(qsl[B])
         R = sum(len(e.want) for e in entries)
@@ -314,6 +322,7 @@ class _PaddedGraph:
         wanted[R:] = 0
         dseq[n_decode:] = -1    # the attention launches skip these places
         dtok[n_decode:] = 0
+        dlong[n_decode:] = -1
         pseq[B - n_decode:] = -1
         return R
 

@@ -137,6 +137,7 @@ _SIGNATURES = {
         c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_float, c_int, c_void_p]),
     "li_paged_attention_stream_supports": ("attention_stream", [c_int, c_int, c_int, c_int]),
     "li_paged_attention_stream_capacity": ("attention_stream", [c_int]),
+    "li_paged_attention_stream_wide": ("attention_stream", [c_int, c_int]),
     "li_paged_attention_stream_wide_capacity": ("attention_stream", [c_int]),
     "li_paged_attention_stream_cluster_capacity": ("attention_stream", [c_int, c_int]),
     "li_paged_attention_mma_counters": ("attention_mma", [c_int, c_int, c_int, c_int]),
@@ -1011,7 +1012,8 @@ def decode_splits_for(num_decode: int, kv_heads: int, max_context_len: int, head
                       streaming: bool = False) -> int:
     """Blocks that share one sequence's keys in a decode launch: as many as still run as one wave when the
     batch is narrow (a launch a little over one wave takes as long as two), never fewer than two key tiles
-    each, at most 32 (liteinfer/engine/model_runner.py:250-272 and paged_kernels.py:645-693 choose likewise)."""
+    each, at most 32; two of head size 128 where the streaming kernel's form of three blocks an SM has a place for
+    them (19 to 27 sequences of 8 KV heads: 24 of 1,500 keys 31 us, 34 unsplit) (liteinfer/engine/model_runner.py:250-272 and paged_kernels.py:645-693 choose likewise)."""
     tiles = -(-max_context_len // 64)
     if tiles < 4:
         return 1
@@ -1279,7 +1281,11 @@ def paged_attention(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_poo
         bound = min(plan.max_decode_context_len, reach) if reach else plan.max_decode_context_len
         streaming = not (keep_first > 0 and window > 0) and stream_attention_supports(q.dtype, heads, kv_heads, head_dim, page_size)
         splits = decode_splits or decode_splits_for(plan.num_decode, kv_heads * parts, bound, head_dim, streaming)
-        paged_attention_mma(*common, plan.decode_seqs, plan.num_decode, 1, heads, kv_heads, head_dim, scale,
+        sequences = plan.decode_seqs
+        if (streaming and plan.decode_longest_first is not None
+                and plan.num_decode * kv_heads * parts * splits > decode_capacity(head_dim, True)):
+            sequences = plan.decode_longest_first       # more blocks than there are places: what starts last had better be short
+        paged_attention_mma(*common, sequences, plan.num_decode, 1, heads, kv_heads, head_dim, scale,
                             window, splits, newest, streaming, every_split=decode_splits is not None, **options)
 
     def portions():

@@ -103,6 +103,7 @@ class AttentionPlan:
     num_decode: int = 0
     decode_seqs: torch.Tensor | None = None     # [num_decode] int32 batch rows with one query
     decode_tokens: torch.Tensor | None = None   # [num_decode] int32 their token rows
+    decode_longest_first: torch.Tensor | None = None    # `decode_seqs` by falling context, where the host has sorted them
     num_prefill: int = 0
     prefill_seqs: torch.Tensor | None = None    # [num_prefill] int32 batch rows with several queries
     max_prefill_query_len: int = 0

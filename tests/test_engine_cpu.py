@@ -174,6 +174,21 @@ def test_sampling_params_checks():
     assert SamplingParams().id != SamplingParams().id
 
 
+def test_steps_name_their_single_tokens_longest_first():
+    """Of a step's entries and of padding, by falling context, equal ones in their order; a list of its own beside the batch's."""
+    from liteinfer_b200.engine.runner import _Batch, _longest_first, _write_padding
+    import numpy as np
+
+    lengths = np.array([5, 9, 9, 1, 30, 9], dtype=np.int32)
+    assert _longest_first(np.array([0, 1, 2, 3, 4, 5], dtype=np.int32), lengths).tolist() == [4, 1, 2, 5, 0, 3]
+    assert _longest_first(np.array([5, 3, 0], dtype=np.int32), lengths).tolist() == [5, 0, 3]
+    assert _longest_first(np.array([], dtype=np.int32), lengths).tolist() == []
+    batch = _Batch(3, 3, 3, [2], 3, 0)
+    views = batch.views(np.zeros(batch.total, dtype=np.int32))
+    _write_padding(views)
+    assert views.dlong.tolist() == views.dseq.tolist() == [-1] * 3
+
+
 def test_sampler_streams_do_not_depend_on_the_batch(cpu_kernels):
     """A seeded request draws the same tokens alone and beside others; greedy rows are the arg-max."""
     from liteinfer_b200 import SamplingParams

@@ -782,6 +782,46 @@ def test_decode_splits_follow_the_context(head_dim, ctx_lens, splits, window, so
     assert ops.gemm_error_flag("cuda:0") == 0
 
 
+# Blocks of head size 128 (148 SMs): two an SM, three, between one wave of three and two of two, and beyond.
+def test_three_blocks_an_sm_where_they_save_a_wave():
+    from liteinfer_b200.ops import kernels
+
+    narrow, wide = kernels.decode_capacity(128, True), kernels.decode_wide_capacity()
+    assert 2 * wide == 3 * narrow
+    form = lambda blocks: bool(kernels._fn("li_paged_attention_stream_wide")(128, blocks))
+    assert [form(b) for b in (1, narrow, narrow + 1, wide, wide + 1, 2 * narrow, 2 * narrow + 1, 4 * narrow)] == [
+        False, False, True, True, False, False, True, True]
+    assert not kernels._fn("li_paged_attention_stream_wide")(64, wide)
+
+
+# Launches of one wave and of more in every form, contexts of every length, as they come and longest first, some of the places empty.
+@pytest.mark.parametrize("head_dim,n", [(64, 20), (64, 100), (128, 30), (128, 50), (128, 64), (128, 76)])
+def test_decode_longest_first(head_dim, n, monkeypatch):
+    from liteinfer_b200 import ops
+    from liteinfer_b200.ops import kernels
+
+    heads, kv_heads = 16, 8
+    ctx_lens = [1 + (37 * i * i) % 700 for i in range(n)]
+    case = _paged_case(torch.bfloat16, heads, kv_heads, head_dim, 16, [1] * n, ctx_lens, poison=False)
+    rest = (case["k_pool"], case["v_pool"], case["table"], case["qsl"], case["ctx"], case["B"], 1, heads, kv_heads, head_dim,
+            head_dim ** -0.5)
+    out = lambda: torch.full((n, heads * head_dim), float("nan"), dtype=torch.bfloat16, device="cuda")
+    plan, launched = _plan_for([1] * n, ctx_lens), []
+    plain = ops.paged_attention(case["qkv"], case["qkv"].shape[1], out(), *rest, plan=plan)
+    order = sorted(range(n), key=lambda i: -ctx_lens[i])
+    plan.decode_longest_first = torch.tensor(order + [-1] * 3, dtype=torch.int32, device="cuda")
+    plan.decode_seqs = torch.cat([plan.decode_seqs, plan.decode_longest_first[n:]])
+    plan.num_decode += 3
+    kernel = kernels.paged_attention_mma
+    monkeypatch.setattr(kernels, "paged_attention_mma", lambda *args, **options: launched.append(args[8]) or kernel(*args, **options))
+    got = ops.paged_attention(case["qkv"], case["qkv"].shape[1], out(), *rest, plan=plan)
+    assert torch.equal(got, plain) or (n <= 30 and torch.allclose(got.float(), plain.float(), rtol=2 ** -6, atol=2 ** -6))
+    more = (n + 3) * kv_heads > kernels.decode_capacity(head_dim, True)
+    assert launched[0] is (plan.decode_longest_first if more else plan.decode_seqs)
+    want = ref.paged_attention(case["qkv"], case["qkv"].shape[1], out(), *rest)
+    torch.testing.assert_close(got.float(), want.float(), rtol=2 ** -6, atol=2 ** -6)
+
+
 # A count that is asked for is every sequence's, also of one with fewer tiles than blocks or as few as one block would take.
 @pytest.mark.parametrize("head_dim", [64, 128])
 @pytest.mark.parametrize("splits", [1, 2, 5, 8, 32, None])
