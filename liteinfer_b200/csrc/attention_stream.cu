@@ -148,16 +148,18 @@ __device__ __forceinline__ int ceil_quotient(int a, int b) {
 }
 
 // The splits that a sequence with this many tiles of keys has in a launch that gives it `most` at most (the host, which may replay
-// the launch for contexts of any length, knows no better).  A merge costs some 2 us, and more the more parts it reads and the more
-// sequences do it at once, a tile 0.65 us (0.9 at head size 128): up to four tiles are one block's, seven where several sequences share
-// the device (`most` below 16), whose blocks then have three tiles at least; alone a sequence has a block a tile up to 16, and
-// 32 blocks only from 97 tiles on.  Measured on B200, 8 KV heads of 64, all splits that the host allows, then so: one sequence of 60 keys 7.6 us
-// and 3.0, of 250 7.5 and 5.0, of 611 7.8 and 6.5, of 1,500 8.5 and 7.4, of 8,000 12.0 and 11.4; eight of 120 7.6 and 4.4, of
-// 440 8.8 and 7.2, of 700 9.2 and 8.4; at head size 128 one of 60 11.2 and 4.1, of 611 11.7 and 9.1, of 1,500 12.5 and 10.6.
+// the launch for contexts of any length, knows no better).  A merge costs some 2 us however many parts it reads, a tile 0.65 us (0.9 at head
+// size 128) in every block: so a short context is one block's, and any other has as many blocks as there are, a tile each if they suffice.
+// The line lies higher where a sequence has few blocks to gain and many others merge beside it.  Measured on B200, 8 KV heads, all splits
+// that the host allows, 1 block and as many as there are, microseconds: of 64, one sequence of 5 tiles 5.7 and 6.1, 6 6.2 and 6.2, 10 8.8 and 6.5;
+// 12 of 5 7.7 and 7.9, 6 8.9 and 8.1; 16 of 6 8.5 and 9.1, 7 9.3 and 9.1, 8 10.3 and 9.2; 32 of 7 10.2 and 11.3, 10 12.9 and 12.7; of 128, one of 4 6.9
+// and 8.0, 6 8.7 and 8.1; 12 of 4 8.4 and 9.6, 6 10.8 and 9.8.  (With three tiles a block at least, 8 of 611 keys of 64 took 9.3, now 8.2.)
+// Up to 48 tiles 16 blocks are as fast as 32 (one sequence of 32 tiles 7.6 and 7.9), beyond they are not (64 tiles 9.4 and 8.8).
+template <int D>
 __device__ __forceinline__ int splits_of(int tiles, int most) {
-  const bool shared = most < 16;
-  if (tiles <= (shared ? 7 : 4)) return 1;
-  const int wanted = min(min(most, shared ? (tiles + 2) / 3 : tiles), tiles <= 96 ? 16 : 32);
+  const int alone = D == 64 ? (most <= 5 ? 7 : 5) : most <= 4 ? 5 : 4;
+  if (tiles <= alone) return 1;
+  const int wanted = min(min(most, tiles), tiles <= 48 ? 16 : 32);
   return wanted <= 1 ? 1 : ceil_quotient(tiles, ceil_quotient(tiles, wanted));
 }
 
@@ -193,7 +195,7 @@ attention_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   const int qpos = ctx - 1, hi = ctx;
   const int lo = first_visible(qpos, p.window);
   const int tile_lo = lo / kBlockN, tile_hi = (hi + kBlockN - 1) / kBlockN;
-  const int splits = kCluster || p.every_split ? p.num_splits : splits_of(tile_hi - tile_lo, p.num_splits);
+  const int splits = kCluster || p.every_split ? p.num_splits : splits_of<D>(tile_hi - tile_lo, p.num_splits);
   if (split >= splits) return;
   const int per_split = splits == 1 ? tile_hi - tile_lo : ceil_quotient(tile_hi - tile_lo, splits);
   const int my_lo = tile_lo + split * per_split, my_hi = min(tile_hi, my_lo + per_split);

@@ -855,6 +855,28 @@ def test_splits_that_are_asked_for_are_taken(head_dim, splits, monkeypatch):
     assert written == ([] if splits == 1 else [splits is not None])      # None: the short ones have one block, and no partial result
 
 
+# Launches that know the longest context only, one sequence at every edge of what the kernel gives its own keys: the last that one block
+# takes and the next, a tile a block, sixteen blocks, the last with sixteen and the first with more, beside others; from 32 blocks down to 2.
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("kv_heads,ctx_lens", [(2, [1, 64, 256, 257, 320, 321, 1024, 1025, 3072, 3073, 6145]), (8, [256, 257, 320, 321, 448, 449, 700, 6145]),
+                                               (8, [60 + 61 * i for i in range(24)])])
+@pytest.mark.parametrize("window,softcap,sink", [(0, 0.0, False), (300, 0.0, True), (0, 20.0, False)])
+def test_decode_takes_the_splits_its_keys_pay_for(head_dim, kv_heads, ctx_lens, window, softcap, sink):
+    from liteinfer_b200 import ops
+
+    heads, q_lens = 16, [1] * len(ctx_lens)
+    case = _paged_case(torch.bfloat16, heads, kv_heads, head_dim, 16, q_lens, ctx_lens, poison=False)
+    args = (case["qkv"], case["qkv"].shape[1])
+    rest = (case["k_pool"], case["v_pool"], case["table"], case["qsl"], case["ctx"], case["B"], 1, heads, kv_heads, head_dim,
+            head_dim ** -0.5, window)
+    extra = dict(softcap=softcap, sink=_randn(heads, dtype=torch.float32, seed=9) if sink else None)
+    out = lambda: torch.full((case["T"], heads * head_dim), float("nan"), dtype=torch.bfloat16, device="cuda")
+    want = ref.paged_attention(*args, out(), *rest, **extra)
+    got = ops.paged_attention(*args, out(), *rest, plan=_plan_for(q_lens, ctx_lens), **extra)
+    torch.testing.assert_close(got.float(), want.float(), rtol=2 ** -6, atol=2 ** -6)
+    assert ops.gemm_error_flag("cuda:0") == 0
+
+
 @pytest.mark.parametrize("heads,kv_heads,head_dim,page_size", [(32, 8, 64, 16), (8, 8, 64, 8), (16, 1, 128, 16),
                                                                (6, 2, 128, 5), (5, 1, 64, 32)])
 @pytest.mark.parametrize("window", [0, 100])
