@@ -51,11 +51,10 @@ struct SimtProduct {
 // tiles of 128 x 64 with one-wide multiply-adds); 400 rows of 768 x 768 33 (37), 256 of 16000 x 768 160 (169).
 //
 // bfloat16 is widened on its way to shared memory, by loads that a thread waits for: what counts is how many threads do that, and a
-// launch's tiles are 128 x 64 (or 32 x 64) by eight warps, with one-wide multiply-adds in fewer registers, two blocks an SM.  100 rows
+// launch's tiles are 128 x 64 (or 64 or 32 x 64) by eight warps, with one-wide multiply-adds in fewer registers, two blocks an SM.  100 rows
 // of 4096 x 4096 238 us, 390 by blocks of four warps as above; 12 rows of 2048 x 2048 94 and 99.
 constexpr int BN = 64, BK = 32, kTileStages = 4;
 template <typename T> constexpr int kTileThreads = sizeof(T) == 4 ? 128 : 256;
-template <typename T> constexpr int kLargeTile = sizeof(T) == 4 ? 64 : 128;        // rows
 constexpr int kTileRow = BK + 4;
 template <int BM> constexpr size_t kTileSmem = (size_t)kTileStages * (BM + BN) * kTileRow * sizeof(float);
 
@@ -393,20 +392,31 @@ int launch_tiles(const SimtProduct& p, bool vec, int batch, cudaStream_t stream)
   return 0;
 }
 
-// Which kernel, by what each was measured to take (B200, microseconds, float32).  The narrow one: 4 and 2.1 for every million
-// weights of a group of 16 rows (16384 x 2048: 70 for 12 rows; 1280 x 768: 11.3 for 64).  Tiles of 32 rows: 24 per 768 k
-// while each SM has one or none, 35 up to some 250, then 12 and 0.104 a tile (1280 x 768: 24.7 for 192 rows, 87 for 1,250); tiles of
-// 64 rows: 35.5 per 768 k up to one an SM, 58 up to two, then 12 and 0.155 a tile (1280 x 768: 35.6 for 256 rows, 79 for 1,250; 4096 x
-// 768: 213 for 1,250).  bfloat16: tiles of 32 rows 26, then 0.15 a tile; of 128 rows 54, up to two an SM 98, then 0.37 a tile.
+// Which kernel, by what each was measured to take (B200, microseconds).  float32, the narrow one: 3.6 and 0.12 a row up to 16, and for
+// every million weights 0.72 for one row, 0.85 for four, 1.4 for eight, 1.65 for twelve, 2.1 for every group of 16; a fifth more where k
+// is more than 2,048.  Tiles take their waves of 148, a whole step each: per 768 k 2 and 12.4 a wave for tiles of 32 rows (a lone wave 17.8),
+// 6.5 and 21 a wave for tiles of 64 (768 k, 140 tiles of 32 18.4, 156 27.7, 288 28.7, 300 39.5, 448 52.7, 640 64; of 64 rows 140 29.3, 156
+// 48.9, 320 70, 448 91).  By a line through these 257 rows of 4096 x 768 went to 320 tiles of 64 rows, 96 us (59 in 576 of 32).
+// Up to 16 rows of one product the narrow kernel is the faster wherever k is not short (16 of 16000 x 768: 29 and 40).
+// bfloat16, whose blocks are two an SM: waves in pairs, of 32 rows 46 a pair and 34 for one over (a lone wave 35), of 64 rows 63 and 58 (46.5), of
+// 128 rows 106 and 76 (68).  (Without tiles of 64 rows 300 of 2048 x 2048 took 202 us, 170 with them.)
 constexpr int kMostRows = 256;
 inline float rows_cost(const SimtProduct& p, int batch) {
-  return 4.f + 2.1e-6f * (float)p.N * p.K * ((p.M + 15) / 16) * batch;
+  if (p.M <= 16 && p.K >= 256 && batch == 1) return 0.f;
+  const float each = p.M == 1 ? 0.72f : p.M <= 4 ? 0.85f : p.M <= 8 ? 1.4f : p.M <= 12 ? 1.65f : 2.1f * ((p.M + 15) / 16);
+  return 3.6f + 0.12f * (p.M < 16 ? p.M : 16) + 1e-6f * each * (p.K > 2048 ? 1.2f : 1.f) * (float)p.N * p.K * batch;
 }
 inline float tiles_cost(int dtype, const SimtProduct& p, int batch, int rows) {
   const float tiles = (float)((p.N + BN - 1) / BN) * ((p.M + rows - 1) / rows) * batch, depth = p.K / 768.f;
-  if (dtype != kFloat32) return depth * (rows == 32 ? fmaxf(26.f, 0.15f * tiles) : tiles <= 148.f ? 54.f : fmaxf(98.f, 0.37f * tiles));
-  if (rows == 32) return depth * (tiles <= 148.f ? 24.f : fmaxf(35.f, 12.f + 0.104f * tiles));
-  return depth * (tiles <= 148.f ? 35.5f : fmaxf(58.f, 12.f + 0.155f * tiles));
+  const float waves = ceilf(tiles / 148.f);
+  if (dtype != kFloat32) {
+    const float two = floorf(waves / 2.f), over = waves - 2.f * two;
+    const float cost = rows == 32 ? (waves <= 1.f ? 35.f : 46.f * two + 34.f * over) :
+                       rows == 64 ? (waves <= 1.f ? 46.5f : 63.f * two + 58.f * over) : waves <= 1.f ? 68.f : 106.f * two + 76.f * over;
+    return 1.5f + depth * cost;
+  }
+  if (rows == 32) return 1.5f + (waves <= 1.f ? 17.8f * depth : 2.f * depth + waves * (0.5f + 11.9f * depth));
+  return 2.f + 6.5f * depth + waves * (0.45f + 20.6f * depth);
 }
 
 int launch_product(int dtype, const SimtProduct& p, int batch, cudaStream_t stream) {
@@ -414,7 +424,8 @@ int launch_product(int dtype, const SimtProduct& p, int batch, cudaStream_t stre
   // Loads of four k at once: every row of x and w starts on their size.
   const bool vec = p.K % 4 == 0 && p.ldx % 4 == 0 && p.x_batch % 4 == 0 && p.w_batch % 4 == 0 &&
                    reinterpret_cast<uintptr_t>(p.x) % four == 0 && reinterpret_cast<uintptr_t>(p.w) % four == 0;
-  const float small = tiles_cost(dtype, p, batch, 32), large = tiles_cost(dtype, p, batch, dtype == kFloat32 ? kLargeTile<float> : kLargeTile<bf16>);
+  const float small = tiles_cost(dtype, p, batch, 32), medium = tiles_cost(dtype, p, batch, 64);
+  const float large = dtype == kFloat32 ? medium : tiles_cost(dtype, p, batch, 128);
   if (dtype == kFloat32 && vec && p.K > 0 && p.M <= kMostRows && p.K <= kMostEach * kMostCluster * kChunk &&
       batch <= 65535 && rows_cost(p, batch) < fminf(small, large)) {
     if (p.M == 1) return launch_rows<1, 1>(p, batch, stream);
@@ -423,10 +434,10 @@ int launch_product(int dtype, const SimtProduct& p, int batch, cudaStream_t stre
     if (p.M <= 12) return launch_rows<6, 2>(p, batch, stream);
     return launch_rows<8, 2>(p, batch, stream);
   }
-  const bool narrow = small < large && (p.M + 31) / 32 <= 65535;
-  if (dtype == kFloat32)
-    return narrow ? launch_tiles<float, 32>(p, vec, batch, stream) : launch_tiles<float, kLargeTile<float>>(p, vec, batch, stream);
-  return narrow ? launch_tiles<bf16, 32>(p, vec, batch, stream) : launch_tiles<bf16, kLargeTile<bf16>>(p, vec, batch, stream);
+  const bool narrow = small < fminf(medium, large) && (p.M + 31) / 32 <= 65535;
+  if (dtype == kFloat32) return narrow ? launch_tiles<float, 32>(p, vec, batch, stream) : launch_tiles<float, 64>(p, vec, batch, stream);
+  if (narrow) return launch_tiles<bf16, 32>(p, vec, batch, stream);
+  return medium < large ? launch_tiles<bf16, 64>(p, vec, batch, stream) : launch_tiles<bf16, 128>(p, vec, batch, stream);
 }
 
 }  // namespace li
