@@ -80,10 +80,11 @@ class _Views:
 class _Batch:
     """Where each array of a step lies in the one int32 staging buffer."""
 
-    def __init__(self, B: int, T: int, R: int, widths: list[int], n_decode: int, n_prefill: int) -> None:
+    def __init__(self, B: int, T: int, R: int, widths: list[int], n_decode: int, n_prefill: int, ordered: bool = True) -> None:
         self.B, self.T, self.R, self.widths = B, T, R, widths
         self.n_decode, self.n_prefill = n_decode, n_prefill
-        sizes = [T, T, T, B + 1, B, B, R, n_decode, n_decode, n_decode, n_prefill, B, B] + [B * w for w in widths]
+        self.ordered = ordered      # the single tokens are listed by falling context too (`dlong`)
+        sizes = [T, T, T, B + 1, B, B, R, n_decode, n_decode, n_decode if ordered else 0, n_prefill, B, B] + [B * w for w in widths]
         # Every array starts on a 16-byte boundary.
         self.sizes = sizes
         self.offsets = []
@@ -106,6 +107,15 @@ class _Batch:
 def _longest_first(seqs: np.ndarray, context_lens: np.ndarray) -> np.ndarray:
     """Sequences by falling context, those of one length in their order."""
     return seqs[np.argsort(-context_lens[seqs], kind="stable")]
+
+
+def _order_pays(cache: CacheManager, n_decode: int, decode_splits: int | None) -> bool:
+    """Whether an attention launch over this many single tokens may have more blocks than the device has places: it then takes the longest
+    contexts first.  The sort is 8 us of the host in every step, more than a narrow step has to spare: twelve steps of seven sequences through four
+    layers 1,024 wide took 2,380 us with it and 2,363 without.  (Splits that nobody asked for never exceed the places.)"""
+    blocks = n_decode * (decode_splits or 1)
+    return any(blocks * need.kv_heads * max(1, need.value_dim // need.head_dim) > kernels.decode_capacity(need.head_dim, True)
+               for need in (group.need for group in cache.groups) if need.head_dim in (64, 128))
 
 
 def _fill(batch: _Batch, flat: np.ndarray, entries: list[StepEntry], cache: CacheManager,
@@ -137,7 +147,8 @@ def _fill(batch: _Batch, flat: np.ndarray, entries: list[StepEntry], cache: Cach
         qsl[i + 1] = cursor
         ctxl[i] = starts[i] + n
         slots[i] = cache.state_slot(entry.request_id)
-    dlong[:nd] = _longest_first(dseq[:nd], ctxl)
+    if batch.ordered:
+        dlong[:nd] = _longest_first(dseq[:nd], ctxl)
     for g, width in enumerate(batch.widths):
         if not width:
             continue
@@ -155,8 +166,8 @@ def _context(batch: _Batch, dev: torch.Tensor, device, counts, totals, decode_sp
               for t, w in zip(tables, batch.widths)]
     prefill_lens = [c for c in counts if c > 1]
     plan = AttentionPlan(
-        num_decode=batch.n_decode, decode_seqs=dseq, decode_tokens=dtok, decode_longest_first=dlong, num_prefill=batch.n_prefill,
-        prefill_seqs=pseq, max_prefill_query_len=max(prefill_lens, default=0), max_decode_context_len=decode_bound,
+        num_decode=batch.n_decode, decode_seqs=dseq, decode_tokens=dtok, decode_longest_first=dlong if batch.ordered else None,
+        num_prefill=batch.n_prefill, prefill_seqs=pseq, max_prefill_query_len=max(prefill_lens, default=0), max_decode_context_len=decode_bound,
         max_prefill_context_len=max((t for t, c in zip(totals, counts) if c > 1), default=0))
     return StepContext(
         num_tokens=batch.T, num_seqs=B, token_ids=tok, positions=pos, seq_of_token=seq, query_start_loc=qsl,
@@ -171,7 +182,8 @@ class _DecodeGraph:
     def __init__(self, runner: ModelRunner, width: int, max_model_len: int) -> None:
         cache = runner.cache
         pages = -(-max_model_len // cache.page_size)
-        self.batch = _Batch(width, width, width, [pages] * len(cache.groups), width, 0)
+        self.batch = _Batch(width, width, width, [pages] * len(cache.groups), width, 0,
+                            _order_pays(cache, width, runner.decode_splits))
         self.device_buffer = torch.zeros(self.batch.total, dtype=torch.int32, device=runner.device)
         counts, totals = [1] * width, [max_model_len] * width
         self.ctx = _context(self.batch, self.device_buffer, runner.device, counts, totals, runner.decode_splits,
@@ -198,7 +210,8 @@ class _DecodeGraph:
         rows[:] = seq
         dseq[:] = seq
         dtok[:] = seq
-        dlong[:] = seq
+        if self.batch.ordered:
+            dlong[:] = seq
         for table in tables:
             table.fill(-1)
         self.row_keys = [None] * width
@@ -220,7 +233,8 @@ class _DecodeGraph:
         late_src[:] = [entry.late or 0 for entry in entries]
         pos[:] = starts
         np.add(pos, 1, out=ctxl)
-        dlong[:] = _longest_first(dseq, ctxl)
+        if self.batch.ordered:
+            dlong[:] = _longest_first(dseq, ctxl)
         for i, entry in enumerate(entries):
             key = (entry.request_id, cache.table_version(entry.request_id))
             if self.row_keys[i] == key:
@@ -284,13 +298,14 @@ class _PaddedGraph:
         cache = runner.cache
         pages = -(-max_model_len // cache.page_size)
         n_decode = seqs if decode else 0
-        self.batch = batch = _Batch(seqs, tokens, rows, [pages] * len(cache.groups), n_decode, prefill)
+        self.batch = batch = _Batch(seqs, tokens, rows, [pages] * len(cache.groups), n_decode, prefill,
+                                    _order_pays(cache, n_decode, runner.decode_splits))
         self.device_buffer = torch.zeros(batch.total, dtype=torch.int32, device=runner.device)
         tok, pos, seq, qsl, ctxl, slots, wanted, dseq, dtok, dlong, pseq, _, _, *tables = batch.views(self.device_buffer)
         tables = [t.view(seqs, w) for t, w in zip(tables, batch.widths)]
         # The kernels' launch bounds are those of the padded shape; what a step really holds is in the buffers.
-        plan = AttentionPlan(num_decode=n_decode, decode_seqs=dseq, decode_tokens=dtok, decode_longest_first=dlong, num_prefill=prefill,
-                             prefill_seqs=pseq, max_prefill_query_len=portion if prefill else 0,
+        plan = AttentionPlan(num_decode=n_decode, decode_seqs=dseq, decode_tokens=dtok,
+                             decode_longest_first=dlong if batch.ordered else None, num_prefill=prefill, prefill_seqs=pseq, max_prefill_query_len=portion if prefill else 0,
                              max_decode_context_len=max_model_len, max_prefill_context_len=prefill_context)
         self.ctx = StepContext(
             num_tokens=tokens, num_seqs=seqs, token_ids=tok, positions=pos, seq_of_token=seq, query_start_loc=qsl,
@@ -406,7 +421,7 @@ class ModelRunner:
         widths = [max(len(cache.block_table(g, e.request_id)) for e in entries) for g in range(len(cache.groups))]
         n_decode = sum(1 for c in counts if c == 1)
         batch = _Batch(len(entries), sum(counts), sum(len(e.want) for e in entries), widths, n_decode,
-                       len(entries) - n_decode)
+                       len(entries) - n_decode, _order_pays(cache, n_decode, self.decode_splits))
         host = torch.empty(batch.total, dtype=torch.int32, pin_memory=self._pinned)
         _fill(batch, host.numpy(), entries, cache, starts)
         dev = host.to(self.device, non_blocking=True)

@@ -189,6 +189,27 @@ def test_steps_name_their_single_tokens_longest_first():
     assert views.dlong.tolist() == views.dseq.tolist() == [-1] * 3
 
 
+def test_steps_sort_their_single_tokens_where_a_launch_reads_the_order():
+    """Sorting is host work in every step: only for as many sequences as have more blocks than the device has places."""
+    from types import SimpleNamespace
+    from liteinfer_b200.engine.runner import _Batch, _context, _order_pays
+    from liteinfer_b200.ops import kernels
+    from liteinfer_b200.parts.context import KVNeed
+
+    held = lambda *needs: SimpleNamespace(groups=[SimpleNamespace(need=need) for need in needs])
+    for need in (KVNeed(8, 64), KVNeed(8, 128), KVNeed(2, 128, v_head_dim=256)):
+        each = need.kv_heads * need.value_dim // need.head_dim
+        most = kernels.decode_capacity(need.head_dim, True) // each
+        for cache in (held(need), held(KVNeed(1, 64), need)):
+            assert [_order_pays(cache, n, None) for n in (0, 1, most, most + 1)] == [False, False, False, True]
+            assert _order_pays(cache, most // 4 + 1, 4) and not _order_pays(cache, most // 4, 4)
+    assert not _order_pays(held(KVNeed(8, 96)), 1000, None) and not _order_pays(held(), 1000, None)      # (no streaming kernel)
+    for ordered in (False, True):
+        batch = _Batch(3, 3, 3, [2], 3, 0, ordered)
+        plan = _context(batch, torch.zeros(batch.total, dtype=torch.int32), "cpu", [1] * 3, [5] * 3, None, 5).plan
+        assert (plan.decode_longest_first is not None) == ordered and plan.decode_tokens.numel() == 3
+
+
 def test_sampler_streams_do_not_depend_on_the_batch(cpu_kernels):
     """A seeded request draws the same tokens alone and beside others; greedy rows are the arg-max."""
     from liteinfer_b200 import SamplingParams
